@@ -5,18 +5,15 @@
 // inside each 2^16-element chunk (src/sample.rs:38-50, src/state.rs:143-156),
 // chunk partials combined serially in chunk order, so norm_sqr, prob_one and
 // every sampled index are bit-identical to the CPU oracle for the same state
-// bits. A dependent f64 add costs ~64 cycles on GB300 and the FP64 pipe
-// issues one warp instruction per ~19 cycles per SM, so the chains are
-// warp-specialised: seven producer warps load amplitudes and compute
-// |a|^2 = r*r + i*i into a shared-memory ring (all lanes busy, loads
-// batched), and one consumer warp runs 32 chains, one per lane, at one
-// dependent add per element. The sampler's rescan records each chain's value
-// at every 32-element stage boundary; draws then resolve in parallel by a
-// binary search over those values and a replay of one stage, which repeats
-// the chain's own additions bit for bit.
-#include <atomic>
+// bits. The chains are evaluated in parallel with the same roundings
+// (zc_chain.h). The sampler's rescan records each chain's value at every
+// 32-element stage boundary; draws then resolve in parallel by a binary
+// search over those values and a replay of one stage, which repeats the
+// chain's own additions bit for bit.
+#include <algorithm>
 
 #include "zc_arith.cuh"
+#include "zc_chain.h"
 #include "zc_internal.h"
 
 namespace zc {
@@ -28,152 +25,194 @@ __device__ __forceinline__ double p2(double r, double i) { return radd(rmul(r, r
 // Non-negative doubles order like their IEEE bit patterns.
 __device__ __forceinline__ unsigned long long dkey(double x) { return (unsigned long long)__double_as_longlong(x); }
 
-// Named-barrier wait / arrive (non-.aligned forms: safe after divergence).
-__device__ __forceinline__ void nb_sync(int id, int count) {
-    asm volatile("barrier.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
+constexpr int kChainThreads = 256;
+constexpr int kStageElems = 32;  // elements per row: one warp-wide load, one recorded chain value
+constexpr int kRowsPerWarp = 8;
+constexpr int kTileRows = kRowsPerWarp * kChainThreads / 32;  // 64 rows, two per lane in the scan
+
+__device__ __forceinline__ ChainFn shfl_down_fn(const ChainFn &f, int o) {
+    return ChainFn{__shfl_down_sync(0xffffffffu, f.a, o), __shfl_down_sync(0xffffffffu, f.b, o)};
 }
-__device__ __forceinline__ void nb_arrive(int id, int count) {
-    asm volatile("barrier.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
+
+// One row (32 values, one per lane) as one function of the running mantissa
+// in the binade e; capped at kChainCross so that 64 rows add up in 64 bits.
+// Lane 0's result counts.
+__device__ __forceinline__ ChainFn row_fn(uint64_t vbits, uint32_t e) {
+    bool tie;
+    const uint64_t k = chain_inc(vbits, e, tie);
+    ChainFn f;
+    if (__any_sync(0xffffffffu, tie)) {  // ties look at parity: compose in order
+        f = chain_fn(k, tie);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) f = chain_then(f, shfl_down_fn(f, o));
+    } else {  // plain sum: two 32-bit warp reductions (27 low bits, <= 27 high bits)
+        const uint32_t lo = __reduce_add_sync(0xffffffffu, (uint32_t)k & 0x7ffffffu);
+        const uint32_t hi = __reduce_add_sync(0xffffffffu, (uint32_t)(k >> 27));
+        f.a = f.b = ((uint64_t)hi << 27) + lo;
+    }
+    f.a = f.a < kChainCross ? f.a : kChainCross;
+    f.b = f.b < kChainCross ? f.b : kChainCross;
+    return f;
 }
 
-constexpr int kChainProducers = 7;  // producer warps; producer p owns ring slot p
-constexpr int kChainThreads = 32 * (kChainProducers + 1);
-constexpr int kStageElems = 32;     // elements per chain per stage
-constexpr int kRowPad = kStageElems + 1;
-constexpr size_t kChainSmem = (size_t)kChainProducers * 32 * kRowPad * sizeof(double);
-
-// Named barriers: FULL(p) = 1 + p (producer p arrives, consumer waits),
-// EMPTY(p) = 1 + kChainProducers + p (consumer arrives, producer p waits).
-__device__ __forceinline__ int bar_full(int p) { return 1 + p; }
-__device__ __forceinline__ int bar_empty(int p) { return 1 + kChainProducers + p; }
-
-// Up to 32 serial chains per CTA (row r = consumer lane r).
-// SCAN = false: rows are chunks blockIdx.x*32 + r of the index space (mode 0:
-//   index h; mode 1, prob_one of qubit q: insert_zero(h, q) + 2^q); the final
-//   chain value goes to part[row].
-// SCAN = true: rows are the touched chunks cs[...]; a chain starts at the
-//   chunk's cum_before and stops (for all rows together) once every row
-//   exceeded its largest draw or ran out; rec[row][stage] holds the chain
-//   value at each stage start, rec_nst[row] the stages run and rec_last[row]
-//   1 + the last element with nonzero mass (0: none).
+// One serial f64 chain per CTA (row blockIdx.x), in tiles of 64 rows of 32
+// elements. A tile is reduced to one function per row, the rows are scanned
+// (every warp repeats the scan: no broadcast barrier), and the first row
+// that leaves the accumulator's binade is added serially, after which the
+// rows behind it are reduced again in the new binade.
+//
+// What bounds it: the three FP64 operations per element (|a|^2 must be
+// rounded as f64), 60 us per 2^16-element chunk on one SM, with about
+// twelve serial rows of 1 us per chunk beside them. One lane per chain, fed
+// by producer warps, took 2.9 ms per chunk at any state size (2^16 dependent
+// adds of 64 cycles).
+//
+// SCAN = false: chunk blockIdx.x of the index space (mode 0: index h; mode 1,
+//   prob_one of qubit q: insert_zero(h, q) + 2^q; mode 2: re holds the
+//   values themselves); the final chain value goes to part[row].
+// SCAN = true: touched chunk cs[row]; the chain starts at the chunk's
+//   cum_before and stops once it exceeded the chunk's largest draw;
+//   rec[row][stage] holds the chain value at each stage start, rec_nst[row]
+//   the stages run and rec_last[row] 1 + the last element with nonzero mass
+//   (0: none).
 template <typename T, bool SCAN>
-__global__ void __launch_bounds__(kChainThreads) k_chain(const T *__restrict__ re, const T *__restrict__ im,
-                                                         uint64_t total, uint64_t chunk, uint64_t nrows, int mode,
-                                                         uint32_t q, const SampleChunk *__restrict__ cs,
-                                                         const double *__restrict__ us, double *__restrict__ part,
-                                                         double *__restrict__ rec, uint32_t *__restrict__ rec_nst,
-                                                         unsigned long long *__restrict__ rec_last,
-                                                         uint32_t rec_stride) {
-    extern __shared__ double ring[];  // [kChainProducers][32][kRowPad]
-    __shared__ uint64_t s_first[32], s_len[32];
-    __shared__ volatile int s_done;
+__global__ void __launch_bounds__(kChainThreads, 2)
+    k_chain(const T *__restrict__ re, const T *__restrict__ im, uint64_t total, uint64_t chunk, int mode, uint32_t q,
+            const SampleChunk *__restrict__ cs, const double *__restrict__ us, double *__restrict__ part,
+            double *__restrict__ rec, uint32_t *__restrict__ rec_nst, unsigned long long *__restrict__ rec_last,
+            uint32_t rec_stride) {
+    __shared__ ChainFn s_row[2][kTileRows];  // double-buffered: one barrier per scan
+    __shared__ uint64_t s_acc;
+    __shared__ unsigned long long s_last;
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    const uint64_t row0 = (uint64_t)blockIdx.x * 32;
-    const int R = nrows - row0 < 32 ? (int)(nrows - row0) : 32;
-    if (warp == 0) {
-        uint64_t first = 0, len = 0;
-        if (lane < R) {
-            const uint64_t c = SCAN ? cs[row0 + lane].chunk : row0 + lane;
-            first = c * chunk;
-            len = total - first < chunk ? total - first : chunk;
-        }
-        s_first[lane] = first;
-        s_len[lane] = len;
-        if (lane == 0) s_done = 0;
-    }
-    __syncthreads();
-    uint64_t maxlen = 0;
-    for (int r = 0; r < R; r++) maxlen = s_len[r] > maxlen ? s_len[r] : maxlen;
-    const uint32_t nst = (uint32_t)((maxlen + kStageElems - 1) / kStageElems);
-    const uint64_t sbit = 1ull << q;
-    if (warp > 0) {
-        const int p = warp - 1;
-        double *buf = ring + (size_t)p * 32 * kRowPad;
-        for (uint32_t s = p; s < nst; s += kChainProducers) {
-            if (s >= (uint32_t)kChainProducers) nb_sync(bar_empty(p), 64);
-            if (!s_done) {
-                const uint64_t e = (uint64_t)s * kStageElems + lane;
-                for (int r0 = 0; r0 < R; r0 += 8) {
-                    T vr[8], vi[8];
-#pragma unroll
-                    for (int u = 0; u < 8; u++) {
-                        const int r = r0 + u;
-                        vr[u] = vi[u] = (T)0;
-                        if (r < R && e < s_len[r]) {
-                            const uint64_t h = s_first[r] + e;
-                            const uint64_t idx = mode == 0 ? h : insert_zero(h, q) + sbit;
-                            vr[u] = re[idx];
-                            vi[u] = im[idx];
-                        }
-                    }
-#pragma unroll
-                    for (int u = 0; u < 8; u++)
-                        if (r0 + u < R) buf[(r0 + u) * kRowPad + lane] = p2(widen(vr[u]), widen(vi[u]));
-                }
-            }
-            nb_arrive(bar_full(p), 64);
-        }
-        return;
-    }
-    // consumer warp: lane r runs row r's chain
-    double acc = 0.0;
-    unsigned long long stop = ~0ull, last = 0;
-    if (SCAN && lane < R) {
-        const SampleChunk sc = cs[row0 + lane];
-        acc = sc.cum;
+    const uint64_t row = blockIdx.x;
+    uint64_t c = row, acc = 0;
+    unsigned long long stop = ~0ull, my_last = 0;
+    if (SCAN) {
+        const SampleChunk sc = cs[row];
+        c = sc.chunk;
+        acc = dkey(sc.cum);
         stop = dkey(us[sc.s1 - 1]);
+        if (threadIdx.x == 0) s_last = 0;
     }
-    const uint64_t my_len = lane < R ? s_len[lane] : 0;
-    bool all_done = false;
+    const uint64_t first = c * chunk, len = total - first < chunk ? total - first : chunk;
+    const uint64_t sbit = 1ull << q;
+    const uint32_t nst = (uint32_t)((len + kStageElems - 1) / kStageElems);
     uint32_t ran = nst;
-    for (uint32_t s = 0; s < nst; s++) {
-        const int p = (int)(s % kChainProducers);
-        nb_sync(bar_full(p), 64);
-        if (!all_done) {
-            if (lane < R) {
-                if (SCAN) rec[(row0 + lane) * rec_stride + s] = acc;
-                const double *row = ring + ((size_t)p * 32 + lane) * kRowPad;
-#pragma unroll 8
-                for (int e = 0; e < kStageElems; e++) {
-                    const double v = row[e];
-                    acc = radd(acc, v);
-                    if (SCAN && dkey(v) != 0ull) last = (unsigned long long)s * kStageElems + e + 1;
+    T nr[kRowsPerWarp], ni[kRowsPerWarp];  // the next tile's amplitudes, in flight while this one is summed
+    auto fetch = [&](uint64_t t0) {
+#pragma unroll
+        for (int j = 0; j < kRowsPerWarp; j++) {
+            const uint64_t e = t0 + (uint64_t)((warp * kRowsPerWarp + j) * kStageElems + lane);
+            nr[j] = ni[j] = (T)0;
+            if (e < len) {
+                const uint64_t h = first + e;
+                const uint64_t idx = mode == 1 ? insert_zero(h, q) + sbit : h;
+                nr[j] = re[idx];
+                if (mode != 2) ni[j] = im[idx];
+            }
+        }
+    };
+    int buf = 0;
+    fetch(0);
+    for (uint64_t t0 = 0; t0 < len; t0 += kTileRows * kStageElems) {
+        uint64_t v[kRowsPerWarp];
+#pragma unroll
+        for (int j = 0; j < kRowsPerWarp; j++) {
+            v[j] = dkey(mode == 2 ? widen(nr[j]) : p2(widen(nr[j]), widen(ni[j])));
+            if (SCAN && v[j]) my_last = t0 + (uint64_t)((warp * kRowsPerWarp + j) * kStageElems + lane) + 1;
+        }
+        if (t0 + kTileRows * kStageElems < len) fetch(t0 + kTileRows * kStageElems);
+        for (int from = 0; from < kTileRows;) {
+            uint32_t e;
+            uint64_t m;
+            chain_split(acc, e, m);
+            buf ^= 1;
+#pragma unroll
+            for (int j = 0; j < kRowsPerWarp; j++) {
+                const int r = warp * kRowsPerWarp + j;
+                ChainFn f{0, 0};
+                if (r >= from) f = row_fn(v[j], e);
+                if (lane == 0) s_row[buf][r] = f;
+            }
+            __syncthreads();
+            const ChainFn f0 = s_row[buf][2 * lane], f1 = s_row[buf][2 * lane + 1];
+            ChainFn g = chain_then(f0, f1);
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const ChainFn h{__shfl_up_sync(0xffffffffu, g.a, o), __shfl_up_sync(0xffffffffu, g.b, o)};
+                if (lane >= o) g = chain_then(h, g);
+            }
+            ChainFn ex{__shfl_up_sync(0xffffffffu, g.a, 1), __shfl_up_sync(0xffffffffu, g.b, 1)};
+            if (lane == 0) ex = ChainFn{0, 0};
+            const uint64_t m0 = chain_apply(ex, m), m1 = chain_apply(f0, m0), m2 = chain_apply(f1, m1);
+            const uint32_t c1 = __ballot_sync(0xffffffffu, m1 >= kChainCross);
+            const uint32_t c2 = __ballot_sync(0xffffffffu, m2 >= kChainCross);
+            int x = kTileRows;  // the first row that leaves the binade
+            if (c1 | c2) {
+                const int l = __ffs(c1 | c2) - 1;
+                x = 2 * l + (int)(((c1 >> l) & 1u) ^ 1u);
+            }
+            if (SCAN && warp == 0) {
+                const uint32_t st0 = (uint32_t)(t0 / kStageElems);
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int r = 2 * lane + h;
+                    if (r >= from && r <= x && st0 + r < nst)
+                        rec[row * rec_stride + st0 + r] = __longlong_as_double((long long)chain_pack(e, h ? m1 : m0));
                 }
             }
-            const bool mine = lane >= R || (uint64_t)(s + 1) * kStageElems >= my_len || (SCAN && dkey(acc) > stop);
-            if (__all_sync(0xffffffffu, mine)) {
-                all_done = true;
-                ran = s + 1;
-                if (lane == 0) s_done = 1;
+            if (x == kTileRows) {
+                acc = chain_pack(e, __shfl_sync(0xffffffffu, m2, 31));
+                break;
             }
+            const uint64_t ax = __shfl_sync(0xffffffffu, (x & 1) ? m1 : m0, x >> 1);
+            if (warp == x / kRowsPerWarp) {
+                uint64_t vx = 0;
+#pragma unroll
+                for (int j = 0; j < kRowsPerWarp; j++)
+                    vx |= x % kRowsPerWarp == j ? v[j] : 0;
+                double a = __longlong_as_double((long long)chain_pack(e, ax));
+#pragma unroll 8
+                for (int i = 0; i < 32; i++)
+                    a = radd(a, __longlong_as_double((long long)__shfl_sync(0xffffffffu, vx, i)));
+                if (lane == 0) s_acc = dkey(a);
+            }
+            __syncthreads();
+            acc = s_acc;
+            from = x + 1;
         }
-        if (s + kChainProducers < nst) nb_arrive(bar_empty(p), 64);
+        if (SCAN && acc > stop) {
+            const uint64_t done = (t0 / kStageElems) + kTileRows;
+            ran = done < nst ? (uint32_t)done : nst;
+            break;
+        }
     }
-    if (lane < R) {
-        if (SCAN) {
-            const uint32_t full = (uint32_t)((my_len + kStageElems - 1) / kStageElems);
-            rec_nst[row0 + lane] = ran < full ? ran : full;
-            rec_last[row0 + lane] = last;
-        } else {
-            part[row0 + lane] = acc;
+    if (SCAN) {
+        if (my_last) atomicMax(&s_last, my_last);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            rec_nst[row] = ran;
+            rec_last[row] = s_last;
         }
+    } else if (threadIdx.x == 0) {
+        part[row] = __longlong_as_double((long long)acc);
     }
 }
 
-__global__ void k_serial_sum(const double *__restrict__ part, uint64_t n, double *out) {
-    double acc = 0.0;
-    for (uint64_t i = 0; i < n; i++) acc = radd(acc, part[i]);
-    *out = acc;
-}
-
-// Sampler pass 2 resolution (src/sample.rs:64-108), one CTA per touched
+// Sampler pass 2 resolution (src/sample.rs:64-108), blockIdx.x a touched
 // chunk, one thread per draw: the draw lands in the last stage t whose start
 // value is <= u; replaying stage t's additions from that value gives the
 // first index i with u < acc_i, the index the serial rescan emits. A draw
 // never exceeded by the chain goes to the chunk's last index with nonzero
 // mass (its last index if none).
+// A replay costs up to 128 FP64 operations, so the draws of a chunk are
+// spread over blockIdx.y when there are few chunks: 1000 draws of one chunk
+// keep one SM's FP64 pipe busy for 40 us, 32 SMs' for 1.
+constexpr int kResolveThreads = 32;
+
 template <typename T>
-__global__ void __launch_bounds__(128) k_resolve(const T *__restrict__ re, const T *__restrict__ im,
+__global__ void __launch_bounds__(kResolveThreads) k_resolve(const T *__restrict__ re, const T *__restrict__ im,
                                                  const SampleChunk *__restrict__ cs, const double *__restrict__ us,
                                                  uint64_t *__restrict__ out, uint64_t chunk_len, uint64_t total,
                                                  const double *__restrict__ rec, const uint32_t *__restrict__ rec_nst,
@@ -185,7 +224,7 @@ __global__ void __launch_bounds__(128) k_resolve(const T *__restrict__ re, const
     const uint64_t len = total - first < chunk_len ? total - first : chunk_len;
     const uint32_t n = rec_nst[b];
     const double *A = rec + b * rec_stride;
-    for (uint64_t d = sc.s0 + threadIdx.x; d < sc.s1; d += blockDim.x) {
+    for (uint64_t d = sc.s0 + blockIdx.y * blockDim.x + threadIdx.x; d < sc.s1; d += gridDim.y * blockDim.x) {
         const unsigned long long uk = dkey(us[d]);
         uint32_t lo = 0, hi = n - 1;  // A[0] = cum_before <= u by the host's routing
         while (lo < hi) {
@@ -392,24 +431,19 @@ __global__ void __launch_bounds__(kDfThreads) k_sample_scan_df(const T *__restri
     }
 }
 
-// Launch k_chain (the exact chunk chains); rec != nullptr selects SCAN.
+// Launch k_chain, one CTA per chain; rec != nullptr selects SCAN.
 template <typename T, bool SCAN>
-int run_chain(zc_state *st, unsigned blocks, uint64_t total, uint64_t chunk, uint64_t nrows, int mode, uint32_t q,
+int run_chain(zc_state *st, uint64_t total, uint64_t chunk, uint64_t nrows, int mode, uint32_t q,
               const SampleChunk *cs, const double *us, double *part, double *rec, uint32_t stride) {
-    static std::atomic<bool> attr{false};  // set once per process; racing first calls repeat it
-    if (!attr) {
-        ZC_CUDA(cudaFuncSetAttribute(k_chain<T, SCAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChainSmem));
-        attr = true;
-    }
     unsigned long long *rec_last = nullptr;
     uint32_t *rec_nst = nullptr;
     if (SCAN) {
         rec_last = (unsigned long long *)(rec + nrows * stride);
         rec_nst = (uint32_t *)(rec_last + nrows);
     }
-    k_chain<T, SCAN><<<blocks, kChainThreads, kChainSmem, st->stream>>>(
-        (const T *)st->re, (const T *)st->im, total, chunk, nrows, mode, q, cs, us, part, rec, rec_nst, rec_last,
-        stride);
+    k_chain<T, SCAN><<<(unsigned)nrows, kChainThreads, 0, st->stream>>>((const T *)st->re, (const T *)st->im, total,
+                                                                       chunk, mode, q, cs, us, part, rec, rec_nst,
+                                                                       rec_last, stride);
     ZC_CUDA(cudaGetLastError());
     return ZC_OK;
 }
@@ -440,17 +474,18 @@ int launch_chunk_sums(zc_state *st, int mode, uint32_t q, size_t *nchunks_out, b
         ZC_CUDA(cudaGetLastError());
         return ZC_OK;
     }
-    const unsigned blocks = (unsigned)((nch + 31) / 32);
     if (st->prec == 64)
-        return run_chain<double, false>(st, blocks, total, chunk, nch, mode, q, nullptr, nullptr, part, nullptr, 0);
-    return run_chain<float, false>(st, blocks, total, chunk, nch, mode, q, nullptr, nullptr, part, nullptr, 0);
+        return run_chain<double, false>(st, total, chunk, nch, mode, q, nullptr, nullptr, part, nullptr, 0);
+    return run_chain<float, false>(st, total, chunk, nch, mode, q, nullptr, nullptr, part, nullptr, 0);
 }
 
 int launch_serial_sum(zc_state *st, size_t nchunks, bool exact) {
     ProfScope ps(st, K_SERIAL_SUM, 8.0 * nchunks);
     st->ctr.launches++;
     if (exact)
-        k_serial_sum<<<1, 1, 0, st->stream>>>(st->d_part, nchunks, st->d_scalar);
+        k_chain<double, false><<<1, kChainThreads, 0, st->stream>>>(st->d_part, nullptr, nchunks, nchunks, 2, 0,
+                                                                    nullptr, nullptr, st->d_scalar, nullptr, nullptr,
+                                                                    nullptr, 0);
     else
         k_sum_df<<<1, kDfThreads, 0, st->stream>>>(st->d_part, nchunks, st->d_scalar);
     ZC_CUDA(cudaGetLastError());
@@ -476,20 +511,22 @@ int launch_sample_scan(zc_state *st, const SampleChunk *d_chunks, size_t nchunks
     double *rec = (double *)d_scratch;
     unsigned long long *rec_last = (unsigned long long *)(rec + nchunks * stride);
     uint32_t *rec_nst = (uint32_t *)(rec_last + nchunks);
-    const unsigned blocks = (unsigned)((nchunks + 31) / 32);
-    int rc = st->prec == 64 ? run_chain<double, true>(st, blocks, st->len, chunk_len, nchunks, 0, 0, d_chunks, d_us,
-                                                      nullptr, rec, stride)
-                            : run_chain<float, true>(st, blocks, st->len, chunk_len, nchunks, 0, 0, d_chunks, d_us,
-                                                     nullptr, rec, stride);
+    int rc = st->prec == 64 ? run_chain<double, true>(st, st->len, chunk_len, nchunks, 0, 0, d_chunks, d_us, nullptr,
+                                                      rec, stride)
+                            : run_chain<float, true>(st, st->len, chunk_len, nchunks, 0, 0, d_chunks, d_us, nullptr,
+                                                     rec, stride);
     if (rc) return rc;
+    // about eight CTAs per SM in all; those past a chunk's draws exit at once
+    const uint64_t split = std::max<uint64_t>(1, (uint64_t)st->num_sms * 8 / nchunks);
+    const dim3 grid((unsigned)nchunks, (unsigned)std::min<uint64_t>(split, 256));
     if (st->prec == 64)
-        k_resolve<double><<<(unsigned)nchunks, 128, 0, st->stream>>>((const double *)st->re, (const double *)st->im,
-                                                                     d_chunks, d_us, d_out, chunk_len, st->len, rec,
-                                                                     rec_nst, rec_last, stride);
-    else
-        k_resolve<float><<<(unsigned)nchunks, 128, 0, st->stream>>>((const float *)st->re, (const float *)st->im,
+        k_resolve<double><<<grid, kResolveThreads, 0, st->stream>>>((const double *)st->re, (const double *)st->im,
                                                                     d_chunks, d_us, d_out, chunk_len, st->len, rec,
                                                                     rec_nst, rec_last, stride);
+    else
+        k_resolve<float><<<grid, kResolveThreads, 0, st->stream>>>((const float *)st->re, (const float *)st->im,
+                                                                   d_chunks, d_us, d_out, chunk_len, st->len, rec,
+                                                                   rec_nst, rec_last, stride);
     ZC_CUDA(cudaGetLastError());
     return ZC_OK;
 }
