@@ -680,8 +680,8 @@ bool batchable(const zc_program *p) {
 // Noisy or dynamic program, all shots as trajectories in one launch.
 int run_batched(const zc_program *p, const zc_run_options *opt, const zc_noise &nz,
                 std::vector<std::pair<uint64_t, uint64_t>> *hist, zc_run_result *res) {
-    std::vector<TrajOp> tops;
-    std::vector<double> mats = {1, 0, 0, 0, 0, 0, 1, 0};  // 2x2 identity for measure / reset
+    std::vector<TrajRec> recs;
+    std::vector<float> mats = {1, 0, 0, 0, 0, 0, 1, 0};  // 2x2 identity for measure / reset
     for (const Op &o : p->ops) {
         TrajOp t{};
         if (o.kind == ZC_OP_MEASURE || o.kind == ZC_OP_RESET) {
@@ -690,6 +690,8 @@ int run_batched(const zc_program *p, const zc_run_options *opt, const zc_noise &
             t.kind = o.kind == ZC_OP_MEASURE ? TOP_MEASURE : TOP_RESET;
             t.clbit = o.b;
             t.mat_off = 0;
+            t.mono = 1;
+            t.cols = 1u << 3;  // row r in column r
         } else {
             std::vector<uint32_t> sup;
             Mat m = dense_of(o, &sup);
@@ -698,8 +700,21 @@ int run_batched(const zc_program *p, const zc_run_options *opt, const zc_noise &
             t.kind = TOP_GATE;
             t.mat_off = (uint32_t)mats.size();
             for (const Cx &c : m) {
-                mats.push_back(c.re);
-                mats.push_back(c.im);
+                mats.push_back((float)c.re);
+                mats.push_back((float)c.im);
+            }
+            // one nonzero entry per row (as f32): the kernel takes the column directly
+            const uint32_t dim = 1u << t.k;
+            t.mono = 1;
+            for (uint32_t r = 0; r < dim; r++) {
+                uint32_t nz_cols = 0;
+                for (uint32_t c = 0; c < dim; c++) {
+                    const float *e = &mats[t.mat_off + 2 * (r * dim + c)];
+                    if (e[0] == 0.f && e[1] == 0.f) continue;
+                    nz_cols++;
+                    t.cols |= c << (3 * r);
+                }
+                t.mono &= nz_cols == 1;
             }
         }
         if (o.has_if) {
@@ -708,7 +723,10 @@ int run_batched(const zc_program *p, const zc_run_options *opt, const zc_noise &
             t.cond_len = o.creg_len;
             t.cond_value = o.value;
         }
-        tops.push_back(t);
+        TrajRec rec{};
+        rec.op = t;
+        if (t.k <= 2) std::copy_n(mats.begin() + t.mat_off, (size_t)2 << (2 * t.k), rec.m);
+        recs.push_back(rec);
     }
     std::vector<uint32_t> fq, fc;
     for (const auto &f : p->finals) {
@@ -716,18 +734,20 @@ int run_batched(const zc_program *p, const zc_run_options *opt, const zc_noise &
         fc.push_back(f.second);
     }
     TrajNoise tn{{nz.depolarizing_1q, nz.depolarizing_2q, nz.bit_flip, nz.phase_flip, nz.amplitude_damping,
-                  nz.readout_flip_0to1, nz.readout_flip_1to0}};
+                  nz.readout_flip_0to1, nz.readout_flip_1to0},
+                 0};
+    for (int i = 0; i < 7; i++) tn.mask |= (uint32_t)(tn.p[i] > 0.0) << i;
     zc_state *ctx = nullptr;
     int rc = zc_create_ex(1, 32, opt->flags, &ctx);
     if (rc) return rc;
     const uint64_t ntraj = opt->shots;
-    const size_t per_cta = ((size_t)2 << p->n_qubits) * sizeof(float);
+    TrajPlan plan = plan_trajectories(p->n_qubits, ntraj, ctx->num_sms);
+    const size_t per_cta = plan.global_bytes;
     uint64_t budget = 0;
     zc_device_budget(opt->mem_fraction > 0 ? opt->mem_fraction : 0.75, &budget);
-    uint64_t ctas = std::min<uint64_t>(ntraj, (uint64_t)ctx->num_sms * 4);  // four trajectories per SM
-    ctas = std::min<uint64_t>(ctas, std::max<uint64_t>(1, budget / std::max<size_t>(per_cta, 1)));
+    if (per_cta) plan.ctas = (int)std::min<uint64_t>(plan.ctas, std::max<uint64_t>(1, budget / per_cta));
     void *d_work = nullptr, *d_buf = nullptr;
-    const size_t ops_b = tops.size() * sizeof(TrajOp), mats_b = mats.size() * sizeof(double);
+    const size_t ops_b = recs.size() * sizeof(TrajRec), mats_b = mats.size() * sizeof(float);
     const size_t f_b = (fq.size() + 1) * sizeof(uint32_t), out_b = ntraj * sizeof(uint64_t);
     const size_t off_mats = (ops_b + 255) & ~(size_t)255, off_fq = off_mats + ((mats_b + 255) & ~(size_t)255);
     const size_t off_fc = off_fq + ((f_b + 255) & ~(size_t)255), off_out = off_fc + ((f_b + 255) & ~(size_t)255);
@@ -741,20 +761,20 @@ int run_batched(const zc_program *p, const zc_run_options *opt, const zc_noise &
         zc_destroy(ctx);
         return code;
     };
-    cudaError_t e = cudaMalloc(&d_work, per_cta * ctas);
+    cudaError_t e = per_cta ? cudaMalloc(&d_work, per_cta * plan.ctas) : cudaSuccess;
     if (e == cudaSuccess) e = cudaMalloc(&d_buf, off_out + out_b);
     if (e != cudaSuccess) return cleanup(cuda_fail(e, "cudaMalloc (trajectory buffers)"));
     char *b = (char *)d_buf;
     cudaStream_t s = ctx->stream;
-    if (!tops.empty()) cudaMemcpyAsync(b, tops.data(), ops_b, cudaMemcpyHostToDevice, s);
+    if (!recs.empty()) cudaMemcpyAsync(b, recs.data(), ops_b, cudaMemcpyHostToDevice, s);
     if (!mats.empty()) cudaMemcpyAsync(b + off_mats, mats.data(), mats_b, cudaMemcpyHostToDevice, s);
     if (!fq.empty()) {
         cudaMemcpyAsync(b + off_fq, fq.data(), fq.size() * 4, cudaMemcpyHostToDevice, s);
         cudaMemcpyAsync(b + off_fc, fc.data(), fc.size() * 4, cudaMemcpyHostToDevice, s);
     }
-    rc = launch_trajectories(ctx, p->n_qubits, (const TrajOp *)b, (int)tops.size(), (const double *)(b + off_mats),
+    rc = launch_trajectories(ctx, plan, p->n_qubits, (const TrajRec *)b, (int)recs.size(), (const float *)(b + off_mats),
                              (const uint32_t *)(b + off_fq), (const uint32_t *)(b + off_fc), (int)fq.size(), tn, ntraj,
-                             opt->seed, (uint64_t *)(b + off_out), d_work, (int)ctas);
+                             opt->seed, (uint64_t *)(b + off_out), d_work);
     if (rc) return cleanup(rc);
     e = cudaMemcpyAsync(words.data(), b + off_out, out_b, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);

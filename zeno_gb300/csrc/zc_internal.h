@@ -184,11 +184,13 @@ int arena_put(zc_state *st, const void *src, size_t bytes, const void **dev);
 int launch_df_to_f64(zc_state *st);
 int launch_sweep(zc_state *st, const SweepGeom &g, const MicroOp *dev_ops, int nops, const char *dev_tables,
                  bool exact);
-struct TrajOp;
+struct TrajRec;
 struct TrajNoise;
-int launch_trajectories(zc_state *st, uint32_t n, const TrajOp *d_ops, int nops, const double *d_mats,
-                        const uint32_t *d_fq, const uint32_t *d_fc, int nfinal, const TrajNoise &nz, uint64_t ntraj,
-                        uint64_t seed, uint64_t *d_out, void *d_work, int ctas);
+struct TrajPlan;
+TrajPlan plan_trajectories(uint32_t n, uint64_t ntraj, int num_sms);
+int launch_trajectories(zc_state *st, const TrajPlan &plan, uint32_t n, const TrajRec *d_recs, int nops,
+                        const float *d_mats, const uint32_t *d_fq, const uint32_t *d_fc, int nfinal,
+                        const TrajNoise &nz, uint64_t ntraj, uint64_t seed, uint64_t *d_out, void *d_work);
 // d_scratch: sample_scan_scratch(nchunks, chunk_len, exact) bytes of device memory.
 int launch_sample_scan(zc_state *st, const SampleChunk *d_chunks, size_t nchunks, const double *d_us,
                        uint64_t *d_out, uint64_t chunk_len, bool exact, void *d_scratch);

@@ -6,18 +6,36 @@
 // phase flip and amplitude damping (whose jump probability gamma * P(1)
 // needs a reduction over the state), then readout flips at measurement.
 //
-// Here a persistent CTA owns one trajectory at a time; its state (2^n
-// amplitudes) stays in a per-CTA buffer that fits in L2. Per op the CTA
-// makes one pass over the state that (a) applies the previous op's pending
-// noise operators that are diagonal as a per-element factor, (b) applies the
-// gate (times the depolarizing Pauli string drawn for this op), and
-// (c) accumulates the joint probability table of the op's qubits. Thread 0
-// then resolves flips and damping for the touched qubits in the reference's
-// order on that table (each decision updates the table) and leaves the
-// resulting 2x2 operators pending for the next pass. All draws of an op are
-// independent of the state, so they are taken up front in the reference's
-// order from a per-trajectory Philox4x32-10 stream (zc_philox.h).
-// Probabilities are summed in double-float per thread and reduced in FP64.
+// Here a persistent CTA owns one trajectory at a time. Per op the CTA makes
+// one pass over the state that (a) applies the previous op's pending noise
+// operators that are diagonal as a per-element factor, (b) applies the gate
+// (times the depolarizing Pauli string drawn for this op), and (c) accumulates
+// the joint probability table of the op's qubits. Warp 0 then resolves flips
+// and damping for the touched qubits in the reference's order on that table
+// (each decision updates the table), leaves the resulting 2x2 operators
+// pending for the next pass and prepares the next op; two CTA barriers per op.
+// All draws of an op are independent of the state and come in the
+// reference's order from a per-trajectory Philox4x32-10 stream
+// (zc_philox.h). Probabilities are summed in double-float.
+//
+// Where the state lives. The pass is bound by moving the state (2S per op),
+// so it stays as close as it fits: up to 14 qubits (128 KiB) in shared
+// memory; above, the first part in shared memory and the rest in a per-CTA
+// buffer, one CTA per SM so that all SMs' buffers stay in the L2 (16 qubits:
+// 152 x 320 KiB = 47 MiB).
+//
+// The pass moves 16-byte vectors and works on four independent groups per
+// thread (the vector's lanes) as packed f32x2 arithmetic; ops on qubits 0 and
+// 1 permute lanes in registers (see lanes). While a gate's pass runs, warp 1
+// prepares the next op (look_ahead), so that only what the table decides
+// stands between two passes. Measured for 2048 trajectories of the 16-qubit
+// depth-20 circuit under damping: 402 ms with one scalar pass per op over
+// global memory (114 instructions per amplitude, four CTAs per SM, half the
+// traffic from DRAM), 106 ms now (15 us per op and SM; bound by the latency of
+// the L2 half of the state and the decisions between passes); 1500 shots of a
+// 13-qubit dynamic circuit: 10.2 -> 2.3 ms. Measured and dropped: two units
+// per thread for one-qubit ops (+17%, registers), 256-bit accesses to an
+// interleaved global part (2x, spills), passes out of line (+20%).
 #include <algorithm>
 
 #include "zc_arith.cuh"
@@ -27,8 +45,6 @@
 
 namespace zc {
 namespace {
-
-constexpr int kTrajThreads = 256;  // four CTAs (trajectories) per SM at 64 registers
 
 // ---------------------------------------------------------------- complex helpers
 
@@ -64,438 +80,1121 @@ struct Pending {
     C2 m[4];
 };
 
+// Ring of Philox blocks held ahead: at least 32 when a pass begins, of which
+// its op takes at most nine (three per qubit) and the next one two.
+constexpr uint32_t kDraws = 64;
+
+template <int NT>
 struct Shared {
-    float mr[64], mi[64];        // current op matrix (gate x Pauli string), f32
-    double J[8];                  // joint probability table of the op's qubits
-    Pending pend[3];              // operators left by the previous op's noise
-    int npend;
-    uint32_t dq[3];               // qubits of diagonal pending factors
-    float dr[8], di[8];           // per-element factor table over dq bits
+    float4 w[2][64];              // op matrix (gate x Pauli string): (re, re, im, im) per entry
+    float2 nw[2][64];             // (-im, -im)
+    float4 ft[8];                 // diagonal pending factor per vector lane, by the high factor bits
+    TrajRec recs[4];              // op i's record at i % 4: the pass's, the next, the one being copied in
+    int o;                        // behind finish_op: the op of the next pass (nops at the end),
+    int cur;                      //   whose matrix is w[cur]
+    uint32_t xm[2];               // row flips of the op's Pauli string
+    int look[2];                  // by o % 2: how far look_ahead got with op o + 1 (LOOK_*)
+    int look_draws;               // draws that took
+    Pending pend[3];              // operators left by the previous op's noise that are not diagonal
+    int npend;                    //   (three-qubit ops: all of them, until their tables are built)
+    uint32_t fqv[3];              // high qubits of the factor table, in vector units
+    int nfv;                      // -1: no factor differs from one
+    uint32_t dq[3];               // all qubits of the diagonal factors, and the factors by their bits
+    float dr[8], di[8];
     int nd;
-    int nondiag;                  // some pending operator is not diagonal
-    double red[kTrajThreads / 32][8];
-    double seg[kTrajThreads];
-    uint64_t draw;                // next draw number of this trajectory
-    uint64_t pick;                // sampled basis index
+    float2 red[NT / 32][8];       // per-warp tables (double-float)
+    double J[8];                  // joint probability table of a three-qubit op
+    double seg[32], blk[32];      // final sampling: region and block masses
+    double el[1024];              //   and the element masses of one block
+    double us[kDraws];            // draw i at i % kDraws: as f64, and the integer half of the block
+    uint64_t zw[kDraws];
+    uint64_t draw, drawn;         // stream positions of the next draw and behind the last one held
+    double keep, keep2;           // sqrt(1 - gamma), 1 - gamma
     uint64_t cl;                  // classical bits of this trajectory
-    int skip;                     // the current op's condition is false
-    int fail;
+    double u;                     // final sampling: what is left of the draw
+    int region, block;
+    __device__ __forceinline__ const TrajOp &op(int i) const { return recs[i & 3].op; }
+};
+
+// The next op is still to be found (LOOK_NO); its matrix is ready (LOOK_READY);
+// ready, and this op leaves nothing to decide either (LOOK_GO).
+enum : int { LOOK_NO = 0, LOOK_READY = 1, LOOK_GO = 2 };
+
+// An op's probability table is read: measurements, and gates under damping.
+__device__ __forceinline__ bool wants_table(const TrajOp &op, const TrajNoise &nz) {
+    return op.kind != TOP_GATE || nz.on(4);
+}
+
+// The CTA's tables. Functions reach them here rather than by reference, so
+// that those kept out of line still address shared memory directly.
+template <int NT>
+__device__ __forceinline__ Shared<NT> &shared_of() {
+    __shared__ Shared<NT> s;
+    return s;
+}
+
+// Two f32 lanes in one 64-bit register pair, the form loads, stores and the
+// packed arithmetic share.
+typedef unsigned long long P2;
+__device__ __forceinline__ P2 p2_make(float x, float y) { return pk_bits(make_float2(x, y)); }
+__device__ __forceinline__ P2 p2_mul(P2 a, P2 b) {
+    P2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ P2 p2_fma(P2 a, P2 b, P2 c) {
+    P2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ P2 p2_add(P2 a, P2 b) {
+    P2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ P2 p2_sub(P2 a, P2 b) {
+    P2 d;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
+// Where the trajectory's state is: amplitudes below ns in shared memory, the
+// others in the CTA's global buffer. SMEM: all of it in shared memory.
+template <bool SMEM>
+struct StateMem {
+    float *sre, *sim, *gre, *gim;
+    uint64_t ns;
+    // work: the CTA's global buffer (2^(n + 1) floats), unused if SMEM
+    __device__ __forceinline__ StateMem(float *work, uint32_t n) {
+        extern __shared__ __align__(16) float smem[];
+        ns = 1ull << n;
+        if (!SMEM && ns > kTrajSplitElems) ns = kTrajSplitElems;
+        sre = smem;
+        sim = smem + ns;
+        gre = work;
+        gim = work + (1ull << n);
+    }
+    __device__ __forceinline__ float &re(uint64_t i) const { return SMEM || i < ns ? sre[i] : gre[i]; }
+    __device__ __forceinline__ float &im(uint64_t i) const { return SMEM || i < ns ? sim[i] : gim[i]; }
+    // vector v (amplitudes 4v .. 4v + 3) as two pairs
+    __device__ __forceinline__ ulonglong2 *re4(uint32_t v) const {
+        return reinterpret_cast<ulonglong2 *>(SMEM || v < (uint32_t)(ns >> 2) ? sre : gre) + v;
+    }
+    __device__ __forceinline__ ulonglong2 *im4(uint32_t v) const {
+        return reinterpret_cast<ulonglong2 *>(SMEM || v < (uint32_t)(ns >> 2) ? sim : gim) + v;
+    }
 };
 
 // Apply every non-diagonal pending operator as a 1-qubit pass.
-template <typename T>
-__device__ void apply_nondiag_pending(T *re, T *im, uint32_t n, Shared &s) {
+template <int NT, bool SMEM>
+__device__ __noinline__ void apply_nondiag_pending(float *work, uint32_t n) {
+    Shared<NT> &s = shared_of<NT>();
+    const StateMem<SMEM> sm(work, n);
     const uint64_t half = 1ull << (n - 1);
     for (int p = 0; p < s.npend; p++) {
         const Pending &P = s.pend[p];
-        if (P.m[1].re == 0 && P.m[1].im == 0 && P.m[2].re == 0 && P.m[2].im == 0) continue;
         const float m00r = P.m[0].re, m00i = P.m[0].im, m01r = P.m[1].re, m01i = P.m[1].im;
         const float m10r = P.m[2].re, m10i = P.m[2].im, m11r = P.m[3].re, m11i = P.m[3].im;
-        for (uint64_t h = threadIdx.x; h < half; h += blockDim.x) {
+        for (uint64_t h = threadIdx.x; h < half; h += NT) {
             const uint64_t a = insert_zero(h, P.q), b = a | (1ull << P.q);
-            const float ar = re[a], ai = im[a], br = re[b], bi = im[b];
-            re[a] = m00r * ar - m00i * ai + m01r * br - m01i * bi;
-            im[a] = m00r * ai + m00i * ar + m01r * bi + m01i * br;
-            re[b] = m10r * ar - m10i * ai + m11r * br - m11i * bi;
-            im[b] = m10r * ai + m10i * ar + m11r * bi + m11i * br;
+            const float ar = sm.re(a), ai = sm.im(a), br = sm.re(b), bi = sm.im(b);
+            sm.re(a) = m00r * ar - m00i * ai + m01r * br - m01i * bi;
+            sm.im(a) = m00r * ai + m00i * ar + m01r * bi + m01i * br;
+            sm.re(b) = m10r * ar - m10i * ai + m11r * br - m11i * bi;
+            sm.im(b) = m10r * ai + m10i * ar + m11r * bi + m11i * br;
         }
         __syncthreads();
     }
 }
 
 // Per-element factor of the diagonal pending operators.
-__device__ __forceinline__ void diag_factor(const Shared &s, uint64_t idx, float &fr, float &fi) {
+template <int NT>
+__device__ __forceinline__ void diag_factor(const Shared<NT> &s, uint64_t idx, float &fr, float &fi) {
     uint32_t j = 0;
     for (int b = 0; b < s.nd; b++) j |= (uint32_t)((idx >> s.dq[b]) & 1) << b;
     fr = s.dr[j];
     fi = s.di[j];
 }
 
-// Build the diagonal-factor table from the pending list.
-__device__ void prepare_pending(Shared &s) {
-    s.nd = 0;
-    s.nondiag = 0;
-    for (int p = 0; p < s.npend; p++) {
-        const Pending &P = s.pend[p];
-        const bool diag = P.m[1].re == 0 && P.m[1].im == 0 && P.m[2].re == 0 && P.m[2].im == 0;
-        if (!diag) {
-            s.nondiag = 1;
-            continue;
+// Warp 0, every lane with the same arguments: the tables of the real diagonal
+// factors (f0[b], f1[b]) on qubits q[b], b < nd, per element and per vector.
+template <int NT>
+__device__ __forceinline__ void factor_tables(Shared<NT> &s, int nd, const uint32_t *q, const float *f0,
+                                              const float *f1) {
+    const int lane = threadIdx.x % 32;
+    bool one = true;
+    int nfv = 0;
+    float f = 1.f, fv = 1.f;  // this lane's entry per element (bits: lane), per vector (lane & 3, lane >> 2)
+#pragma unroll
+    for (int b = 0; b < 3; b++)
+        if (b < nd) {
+            one &= f0[b] == 1.f && f1[b] == 1.f;
+            f = __fmul_rn(f, (lane >> b) & 1 ? f1[b] : f0[b]);
+            const int bit = q[b] < 2 ? (lane >> q[b]) & 1 : (lane >> (2 + nfv)) & 1;
+            fv = __fmul_rn(fv, bit ? f1[b] : f0[b]);
+            if (q[b] >= 2) {
+                if (lane == 0) s.fqv[nfv] = q[b] - 2;
+                nfv++;
+            }
+            if (lane == 0) s.dq[b] = q[b];
         }
-        s.dq[s.nd++] = p;  // temporarily the pending index
+    if (lane < 8) {
+        s.dr[lane] = f;
+        s.di[lane] = 0.f;
     }
-    const int nd = s.nd;
-    uint32_t pidx[3];
-    for (int b = 0; b < nd; b++) {
-        pidx[b] = s.dq[b];
-        s.dq[b] = s.pend[pidx[b]].q;
-    }
-    for (uint32_t j = 0; j < (1u << nd); j++) {
-        C2 f{1, 0};
-        for (int b = 0; b < nd; b++) f = cmul(f, s.pend[pidx[b]].m[((j >> b) & 1) ? 3 : 0]);
-        s.dr[j] = (float)f.re;
-        s.di[j] = (float)f.im;
+    reinterpret_cast<float *>(s.ft)[lane] = fv;
+    if (lane == 0) {
+        s.nd = nd;
+        s.nfv = one ? -1 : nfv;
     }
 }
 
-// df accumulate |v|^2 (exact square via FMA, TwoSum into (hi, lo)).
-__device__ __forceinline__ void acc_p2(float r, float i, float &hi, float &lo) {
-    const float p0 = __fmul_rn(r, r), e0 = __fmaf_rn(r, r, -p0);
-    const float p1 = __fmul_rn(i, i), e1 = __fmaf_rn(i, i, -p1);
-    float err0, err1;
-    float s = two_sum(hi, p0, err0);
-    s = two_sum(s, p1, err1);
-    hi = s;
-    lo = __fadd_rn(lo, __fadd_rn(__fadd_rn(err0, err1), __fadd_rn(e0, e1)));
+// The same from the pending list of a three-qubit op, which also keeps only
+// its operators that are not diagonal. (All operators are real.)
+template <int NT>
+__device__ void split_pending(Shared<NT> &s) {
+    uint32_t q[3] = {0, 0, 0};
+    float f0[3] = {1.f, 1.f, 1.f}, f1[3] = {1.f, 1.f, 1.f};
+    int nd = 0, np = 0;
+    for (int p = 0; p < s.npend; p++) {
+        const Pending P = s.pend[p];
+        if (P.m[1].re == 0 && P.m[2].re == 0) {
+            q[nd] = P.q;
+            f0[nd] = P.m[0].re;
+            f1[nd++] = P.m[3].re;
+        } else {
+            __syncwarp();
+            if (threadIdx.x == 0) s.pend[np] = P;
+            np++;
+        }
+    }
+    factor_tables(s, nd, q, f0, f1);
+    __syncwarp();
+    if (threadIdx.x == 0) s.npend = np;
 }
 
-// CTA reduction of per-thread tables (hi + lo in FP64) into s.J[0..cnt).
-__device__ void reduce_table(Shared &s, const float *hi, const float *lo, int cnt) {
-    const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
-    for (int j = 0; j < cnt; j++) {
-        double v = (double)hi[j] + (double)lo[j];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if (lane == 0) s.red[warp][j] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < cnt) {
-        double v = 0.0;
-        for (int w = 0; w < (int)(blockDim.x / 32); w++) v += s.red[w][threadIdx.x];
-        s.J[threadIdx.x] = v;
-    }
-    __syncthreads();
+// a + b in double-float (TwoSum on the high parts, low parts summed).
+__device__ __forceinline__ float2 tdf_add(float2 a, float2 b) {
+    float e;
+    const float s = two_sum(a.x, b.x, e);
+    return df_norm(s, __fadd_rn(e, __fadd_rn(a.y, b.y)));
+}
+__device__ __forceinline__ float2 shfl_xor_f2(float2 v, int m) {
+    return make_float2(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m));
 }
 
-// One op's pass for a K-qubit op (K = 1, 2, so the group's amplitudes and
-// its probability table stay in registers): the pending diagonal factors,
-// then the gate, accumulating |amplitude|^2 per group row into (hi, lo).
-template <int K, typename T>
-__device__ __forceinline__ void traj_pass(T *re, T *im, uint64_t len, const TrajOp &op, const Shared &s, float *hi,
-                                          float *lo) {
-    constexpr uint32_t D = 1u << K;
-    uint32_t qs[K];
+// Sum D per-thread double-float values over the warp into red[0..D): lanes
+// halve the values they carry as they exchange them (D - 1 + 5 - log2 D
+// additions instead of 5 D).
+template <int D>
+__device__ __forceinline__ void warp_table(float2 *v, float2 *red) {
+    const int lane = threadIdx.x % 32;
+    int off = 16, base = 0;
 #pragma unroll
-    for (int b = 0; b < K; b++) qs[b] = op.qs[b];
-    // the op matrix is read from shared memory at each use: hoisted into
-    // registers it would spill at the 64-register cap of four CTAs per SM
-    const volatile float *mr = s.mr, *mi = s.mi;
-    float h[D], l[D];
+    for (int w = D; w > 1; w >>= 1, off >>= 1) {
+        const bool upper = lane & off;
 #pragma unroll
-    for (uint32_t r = 0; r < D; r++) h[r] = l[r] = 0.f;
-    const uint64_t groups = len >> K;
-    for (uint64_t g = threadIdx.x; g < groups; g += blockDim.x) {
-        const uint64_t base = insert_zeros(g, qs, K);
-        float xr[D], xi[D];
+        for (int j = 0; j < w / 2; j++) {
+            const float2 give = upper ? v[j] : v[j + w / 2], keep = upper ? v[j + w / 2] : v[j];
+            v[j] = tdf_add(keep, shfl_xor_f2(give, off));
+        }
+        if (upper) base += w / 2;
+    }
 #pragma unroll
-        for (uint32_t j = 0; j < D; j++) {
+    for (int o = off; o > 0; o >>= 1) v[0] = tdf_add(v[0], shfl_xor_f2(v[0], o));
+    if ((lane & (2 * off - 1)) == 0) red[base] = v[0];
+}
+
+// |y|^2 of both halves into (h, l), h >= |y|^2: the sum's high part in one
+// FMA, t - h exact (h <= t <= 2h), and the square minus that difference is
+// what the rounding dropped. The accumulators start at kBias, above any
+// |amplitude|^2 of a normalised state, and give it back at the end; the sum
+// keeps 2^-46 of the state's norm.
+constexpr float kBias = 1.0f;
+__device__ __forceinline__ void acc_sq2(float2 y, float2 &h, float2 &l) {
+    const float2 t = fma2(y, y, h);
+    l = add2(l, fma2(y, y, sub2(h, t)));
+    h = t;
+}
+__device__ __forceinline__ float2 acc_end(float2 h, float2 l) {
+    return tdf_add(df_norm(__fsub_rn(h.x, kBias), l.x), df_norm(__fsub_rn(h.y, kBias), l.y));
+}
+
+__device__ __forceinline__ void acc_pair(P2 y, P2 &h, P2 &l) {
+    const P2 t = p2_fma(y, y, h);
+    l = p2_add(l, p2_fma(y, y, p2_sub(h, t)));
+    h = t;
+}
+
+// Matrix entries read where they are used: hoisted out of the pass loop, the
+// sixteen entries of a dense two-qubit op (96 registers) spill.
+template <bool IN_PLACE>
+__device__ __forceinline__ void entry(const float4 *w, const float2 *nw, P2 &wr, P2 &wi, P2 &nwi) {
+    const uint32_t aw = (uint32_t)__cvta_generic_to_shared(w), an = (uint32_t)__cvta_generic_to_shared(nw);
+    if (IN_PLACE) {
+        asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(wr), "=l"(wi) : "r"(aw));
+        asm volatile("ld.shared.b64 %0, [%1];" : "=l"(nwi) : "r"(an));
+    } else {
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(w);
+        wr = a.x;
+        wi = a.y;
+        nwi = *reinterpret_cast<const P2 *>(nw);
+    }
+}
+
+// Qubits of the op among the lanes of a vector (0, 1) or above.
+enum : int { LOW_NONE = 0, LOW_Q0 = 1, LOW_Q1 = 2, LOW_BOTH = 3 };
+
+// A thread's 2^K vectors, two pairs each, as x[j][p]: j the op's qubits, p
+// numbering pairs of independent groups. Above the lanes a vector is a
+// coordinate and its halves the pairs, as loaded; an op qubit among the lanes
+// takes its coordinate from the lane (qubit 1: the vector's halves, qubit 0:
+// the lanes of a half), and a vector bit numbers pairs instead.
+__device__ __forceinline__ void lanes_2x2(P2 &a, P2 &b) {  // (a0 a1) (b0 b1) -> (a0 b0) (a1 b1)
+    const float2 x = pk_float2(a), y = pk_float2(b);
+    a = p2_make(x.x, y.x);
+    b = p2_make(x.y, y.y);
+}
+__device__ __forceinline__ void p2_swap(P2 &a, P2 &b) {
+    const P2 t = a;
+    a = b;
+    b = t;
+}
+template <int K, bool IN>
+__device__ __forceinline__ void lanes(P2 (&x)[1 << K][2], int low) {
+    constexpr int D = 1 << K;
+    if (low == LOW_NONE) return;
+    if (K == 2 && low == LOW_BOTH) {  // lane j of vectors 2p, 2p + 1 <-> x[j][p]
+#pragma unroll
+        for (int i = 0; i < 2; i++)  // order of the two steps is reversed on the way out
+            if ((i == 0) == IN) {
+#pragma unroll
+                for (int p = 0; p < D / 2; p++)
+#pragma unroll
+                    for (int e = 0; e < 2; e++) lanes_2x2(x[2 * p][e], x[(2 * p + 1) % D][e]);
+            } else {
+                // (2p + l, e) holds lane 2e + l of pair p: move to (2e + l, p)
+                p2_swap(x[0][1], x[2 % D][0]);
+                p2_swap(x[1][1], x[3 % D][0]);
+            }
+        return;
+    }
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+        if ((i == 0) == IN) {
+            if (low == LOW_Q0) {
+#pragma unroll
+                for (int v = 0; v < D; v++) lanes_2x2(x[v][0], x[v][1]);
+            }
+        } else {
+            // half e of vector (p, h) <-> x[e | h][p]
+#pragma unroll
+            for (int h = 0; h < D; h += 2) p2_swap(x[h][1], x[h + 1][0]);
+        }
+}
+
+// One op's pass for a K-qubit op (K = 1, 2): a thread loads 2^K vectors (four
+// groups), scales them by the pending factors, applies the gate and
+// accumulates |amplitude|^2 per group coordinate into the warp's table.
+// MONO: every matrix row has one entry (CX, SWAP, phases, Pauli strings) and
+// no qubit is among the lanes: row r loads its column's vector. The skipped
+// terms are exact zeros, so the values are those of the dense sum.
+template <int K, bool MONO, int NT, bool SMEM>
+__device__ __forceinline__ void traj_pass_body(float *work, uint32_t n, int o, int cur, bool acc) {
+    Shared<NT> &s = shared_of<NT>();
+    const StateMem<SMEM> sm(work, n);
+    constexpr int D = 1 << K;
+    const uint32_t q0 = s.op(o).qs[0], q1 = s.op(o).qs[1];
+    const int low = MONO || q0 >= 2 ? LOW_NONE : K == 2 && q1 == 1 ? LOW_BOTH : q0 == 0 ? LOW_Q0 : LOW_Q1;
+    // the vector bits the thread's vectors span: the op's qubits above the
+    // lanes, else the highest free ones (so a warp's loads stay contiguous)
+    uint32_t pos[2] = {q0 - 2, q1 - 2};
+    if (K == 1) {
+        if (low) pos[0] = n - 3;
+    } else if (low == LOW_BOTH) {
+        pos[0] = n - 4;
+        pos[1] = n - 3;
+    } else if (low) {  // bit 0 of v numbers groups, bit 1 is qs[1]
+        pos[0] = pos[1] == n - 3 ? n - 4 : n - 3;
+    }
+    const uint32_t plo = K == 1 ? pos[0] : min(pos[0], pos[1]), phi = K == 1 ? 0 : max(pos[0], pos[1]);
+    const float4 *W = s.w[cur];
+    const float2 *NW = s.nw[cur];
+    int col[D];
+    if (MONO) {
+#pragma unroll
+        for (int r = 0; r < D; r++) col[r] = (int)((s.op(o).cols >> (3 * (r ^ s.xm[cur]))) & 7u);
+    }
+    const int nfv = s.nfv;
+    // factor index bits; qubits that are not there read bit 31 of the vector
+    // number, which is zero
+    const uint32_t fq0 = nfv > 0 ? s.fqv[0] : 31, fq1 = nfv > 1 ? s.fqv[1] : 31, fq2 = nfv > 2 ? s.fqv[2] : 31;
+    P2 h[D], l[D];
+#pragma unroll
+    for (int r = 0; r < D; r++) {
+        h[r] = p2_make(kBias, kBias);
+        l[r] = p2_make(0.f, 0.f);
+    }
+    // the thread's vectors: unit u spread around the spanned bits, then those
+    auto vector = [&](uint32_t u, int v) {
+        uint32_t vb = ((u >> plo) << (plo + 1)) | (u & ((1u << plo) - 1));
+        if (K == 2) vb = ((vb >> phi) << (phi + 1)) | (vb & ((1u << phi) - 1));
+        uint32_t vi = vb | ((uint32_t)(v & 1) << pos[0]);
+        if (K == 2) vi |= (uint32_t)(v >> 1) << pos[1];
+        return vi;
+    };
+    auto source = [&](int v) { return MONO ? col[v] : v; };
+    const uint32_t units = 1u << (n - 2 - K);
+    constexpr int U = 1;
+#pragma unroll 1
+    for (uint32_t u0 = threadIdx.x; u0 < units; u0 += U * NT) {
+        P2 xr[U][D][2], xi[U][D][2];
+#pragma unroll
+        for (int i = 0; i < U; i++)
+            if (i == 0 || u0 + i * NT < units) {
+#pragma unroll
+                for (int v = 0; v < D; v++) {
+                    const uint32_t vi = vector(u0 + i * NT, source(v));
+                    const ulonglong2 a = *sm.re4(vi), c = *sm.im4(vi);
+                    xr[i][v][0] = a.x;
+                    xr[i][v][1] = a.y;
+                    xi[i][v][0] = c.x;
+                    xi[i][v][1] = c.y;
+                }
+            }
+#pragma unroll
+        for (int i = 0; i < U; i++)
+            if (i == 0 || u0 + i * NT < units) {
+                const uint32_t u = u0 + i * NT;
+                if (nfv >= 0) {  // factors are real: flips and damping have real operators
+#pragma unroll
+                    for (int v = 0; v < D; v++) {
+                        const uint32_t vi = vector(u, source(v));
+                        uint32_t j = ((vi >> fq0) & 1u) | (((vi >> fq1) & 1u) << 1);
+                        if (nfv > 2) j |= ((vi >> fq2) & 1u) << 2;
+                        const ulonglong2 f = *reinterpret_cast<const ulonglong2 *>(&s.ft[j]);
+                        xr[i][v][0] = p2_mul(f.x, xr[i][v][0]);
+                        xr[i][v][1] = p2_mul(f.y, xr[i][v][1]);
+                        xi[i][v][0] = p2_mul(f.x, xi[i][v][0]);
+                        xi[i][v][1] = p2_mul(f.y, xi[i][v][1]);
+                    }
+                }
+                if (!MONO) {
+                    lanes<K, true>(xr[i], low);
+                    lanes<K, true>(xi[i], low);
+                }
+                // one pair of groups at a time, results over the inputs they came from
+#pragma unroll
+                for (int p = 0; p < 2; p++) {
+                    P2 br[D], bi[D];
+#pragma unroll
+                    for (int r = 0; r < D; r++) {
+                        P2 wr, wi, nwi;
+                        if (MONO) {
+                            entry<(K > 1)>(&W[r * D + col[r]], &NW[r * D + col[r]], wr, wi, nwi);
+                            br[r] = p2_fma(wr, xr[i][r][p], p2_mul(nwi, xi[i][r][p]));
+                            bi[r] = p2_fma(wr, xi[i][r][p], p2_mul(wi, xr[i][r][p]));
+                        } else {
+#pragma unroll
+                            for (int c = 0; c < D; c++) {
+                                entry<(K > 1)>(&W[r * D + c], &NW[r * D + c], wr, wi, nwi);
+                                const P2 ar = xr[i][c][p], ai = xi[i][c][p];
+                                br[r] = p2_fma(wr, ar, c ? p2_fma(nwi, ai, br[r]) : p2_mul(nwi, ai));
+                                bi[r] = p2_fma(wr, ai, c ? p2_fma(wi, ar, bi[r]) : p2_mul(wi, ar));
+                            }
+                        }
+                        if (acc) {
+                            acc_pair(br[r], h[r], l[r]);
+                            acc_pair(bi[r], h[r], l[r]);
+                        }
+                    }
+#pragma unroll
+                    for (int r = 0; r < D; r++) {
+                        xr[i][r][p] = br[r];
+                        xi[i][r][p] = bi[r];
+                    }
+                }
+                if (!MONO) {
+                    lanes<K, false>(xr[i], low);
+                    lanes<K, false>(xi[i], low);
+                }
+#pragma unroll
+                for (int v = 0; v < D; v++) {
+                    const uint32_t vi = vector(u, v);
+                    *sm.re4(vi) = make_ulonglong2(xr[i][v][0], xr[i][v][1]);
+                    *sm.im4(vi) = make_ulonglong2(xi[i][v][0], xi[i][v][1]);
+                }
+            }
+    }
+    float2 tab[D];
+#pragma unroll
+    for (int r = 0; r < D; r++) tab[r] = acc_end(pk_float2(h[r]), pk_float2(l[r]));
+    if (acc) warp_table<D>(tab, s.red[threadIdx.x / 32]);
+}
+
+// A dense two-qubit op's pass, out of line: its registers would crowd the
+// common passes (one-qubit ops, CX) out of theirs.
+template <int NT, bool SMEM>
+__device__ __noinline__ void traj_pass_dense2(float *work, uint32_t n, int o, int cur, bool acc) {
+    traj_pass_body<2, false, NT, SMEM>(work, n, o, cur, acc);
+}
+
+// The general pass, element by element: three-qubit ops and states of fewer
+// than five or more than 31 qubits.
+template <int NT, bool SMEM>
+__device__ __noinline__ void traj_pass_general(float *work, uint32_t n, int o, int cur, bool table) {
+    Shared<NT> &s = shared_of<NT>();
+    const StateMem<SMEM> sm(work, n);
+    const uint64_t len = 1ull << n;
+    const uint32_t k = s.op(o).k, dim = 1u << k;
+    float2 acc[8];
+#pragma unroll
+    for (int r = 0; r < 8; r++) acc[r] = make_float2(kBias, 0.f);
+    const uint64_t groups = len >> k;
+    for (uint64_t g = threadIdx.x; g < groups; g += NT) {
+        const uint64_t base = insert_zeros(g, s.op(o).qs, (int)k);
+        float xr[8], xi[8];
+#pragma unroll
+        for (uint32_t j = 0; j < 8; j++) {
+            if (j >= dim) break;
             uint64_t idx = base;
-#pragma unroll
-            for (int b = 0; b < K; b++) idx |= (uint64_t)((j >> b) & 1) << qs[b];
+            for (uint32_t b = 0; b < k; b++) idx |= (uint64_t)((j >> b) & 1) << s.op(o).qs[b];
             float fr, fi;
             diag_factor(s, idx, fr, fi);
-            const float a = (float)re[idx], c = (float)im[idx];
+            const float a = sm.re(idx), c = sm.im(idx);
             xr[j] = fr * a - fi * c;
             xi[j] = fr * c + fi * a;
         }
 #pragma unroll
-        for (uint32_t r = 0; r < D; r++) {
+        for (uint32_t r = 0; r < 8; r++) {
+            if (r >= dim) break;
             float yr = 0.f, yi = 0.f;
 #pragma unroll
-            for (uint32_t c = 0; c < D; c++) {
-                const float wr = mr[r * D + c], wi = mi[r * D + c];
+            for (uint32_t c = 0; c < 8; c++) {
+                if (c >= dim) break;
+                const float wr = s.w[cur][r * dim + c].x, wi = s.w[cur][r * dim + c].z;
                 yr = fmaf(wr, xr[c], fmaf(-wi, xi[c], yr));
                 yi = fmaf(wr, xi[c], fmaf(wi, xr[c], yi));
             }
             uint64_t idx = base;
-#pragma unroll
-            for (int b = 0; b < K; b++) idx |= (uint64_t)((r >> b) & 1) << qs[b];
-            re[idx] = (T)yr;
-            im[idx] = (T)yi;
-            acc_p2(yr, yi, h[r], l[r]);
+            for (uint32_t b = 0; b < k; b++) idx |= (uint64_t)((r >> b) & 1) << s.op(o).qs[b];
+            sm.re(idx) = yr;
+            sm.im(idx) = yi;
+            float2 h = make_float2(acc[r].x, kBias), l = make_float2(acc[r].y, 0.f);
+            acc_sq2(make_float2(yr, 0.f), h, l);
+            acc_sq2(make_float2(yi, 0.f), h, l);
+            acc[r] = make_float2(h.x, l.x);
         }
     }
 #pragma unroll
-    for (uint32_t r = 0; r < D; r++) {
-        hi[r] = h[r];
-        lo[r] = l[r];
+    for (int r = 0; r < 8; r++) acc[r] = df_norm(__fsub_rn(acc[r].x, kBias), acc[r].y);
+    if (!table) return;
+    if (k == 1) warp_table<2>(acc, s.red[threadIdx.x / 32]);
+    else if (k == 2) warp_table<4>(acc, s.red[threadIdx.x / 32]);
+    else warp_table<8>(acc, s.red[threadIdx.x / 32]);
+}
+
+// One warp: the next 32 Philox blocks of trajectory t, one per lane, when
+// fewer than 32 are held.
+template <int NT>
+__device__ __forceinline__ void refill(Shared<NT> &s, uint64_t seed, uint64_t t) {
+    __syncwarp();
+    if (s.drawn - s.draw < 32) {
+        const uint64_t i = s.drawn + threadIdx.x % 32;
+        s.us[i % kDraws] = philox_f64(seed, t, i);
+        const PhiloxU4 b = philox_block(seed, t, i);
+        s.zw[i % kDraws] = ((uint64_t)b.z << 32) | b.w;
+        __syncwarp();
+        if (threadIdx.x % 32 == 0) s.drawn += 32;
+    }
+    __syncwarp();
+}
+template <int NT>
+__device__ __forceinline__ double next_f64(Shared<NT> &s) {
+    return s.us[s.draw++ % kDraws];
+}
+
+// One warp: op `op`'s matrix (gate x the depolarizing string drawn for it,
+// draws from stream position `draw` on) into buffer `buf`. Returns the draws
+// taken.
+template <int NT>
+__device__ int prepare_matrix(Shared<NT> &s, const TrajRec &rec, int buf, uint64_t draw, const float *mats,
+                              const TrajNoise &nz) {
+    const int lane = threadIdx.x % 32;
+    const TrajOp &op = rec.op;
+    const uint32_t k = op.k, dim = 1u << k;
+    uint32_t idx = 0;
+    int taken = 0;
+    if (op.kind == TOP_GATE && nz.on(k == 1 ? 0 : 1)) {
+        taken = 1;
+        if (s.us[draw % kDraws] < nz.p[k == 1 ? 0 : 1]) {
+            taken = 2;
+            idx = 1 + (uint32_t)(((unsigned __int128)s.zw[(draw + 1) % kDraws] * ((1ull << (2 * k)) - 1)) >> 64);
+        }
+    }
+    // P_string . M: the Pauli string is a signed permutation, row r
+    // holding its one entry in column r ^ xm (X and Y flip the bit),
+    // of value prod_b v_b(r_b) (Y: -i on 0, i on 1; Z: -1 on 1)
+    uint32_t xm = 0;
+    for (uint32_t b = 0; idx && b < k; b++) {
+        const uint32_t code = (idx >> (2 * b)) & 3u;
+        if (code == 1 || code == 2) xm |= 1u << b;
+    }
+    const float *M = k <= 2 ? rec.m : mats + op.mat_off;
+    for (uint32_t i = lane; i < dim * dim; i += 32) {
+        const uint32_t r = i >> k, c = i & (dim - 1), j = r ^ xm;
+        int re_sign = 1, swap = 0;  // phase = re_sign * (swap ? i : 1)
+        for (uint32_t b = 0; idx && b < k; b++) {
+            const uint32_t code = (idx >> (2 * b)) & 3u, rb = (r >> b) & 1u;
+            if (code == 2) {  // multiply by -i (rb = 0) or i (rb = 1)
+                if (swap) re_sign = rb ? -re_sign : re_sign;  // i * i = -1, i * -i = 1
+                else re_sign = rb ? re_sign : -re_sign;
+                swap ^= 1;
+            } else if (code == 3 && rb) {
+                re_sign = -re_sign;
+            }
+        }
+        const float mr = M[2 * (j * dim + c)], mi = M[2 * (j * dim + c) + 1];
+        // (re_sign * (swap ? i : 1)) * (mr + i mi)
+        const float wr = swap ? -re_sign * mi : re_sign * mr, wi = swap ? re_sign * mr : re_sign * mi;
+        s.w[buf][i] = make_float4(wr, wr, wi, wi);
+        s.nw[buf][i] = make_float2(-wi, -wi);
+    }
+    if (lane == 0) s.xm[buf] = xm;
+    return taken;
+}
+
+__device__ __forceinline__ bool op_runs(const TrajOp &op, uint64_t cl) {
+    if (!op.cond) return true;
+    const uint64_t mask = op.cond_len >= 64 ? ~0ull : ((1ull << op.cond_len) - 1);
+    return ((cl >> op.cond_off) & mask) == op.cond_value;
+}
+
+// Warp 1, during the pass of gate o: copy record o + 2 in, draw ahead, and
+// prepare op o + 1, all of which the pass's result has no part in. (What a
+// measurement decides, and ops behind one whose condition fails, is left to
+// next_op.)
+template <int NT>
+__device__ __noinline__ void look_ahead(int o, int cur, const TrajRec *recs, int nops, const float *mats,
+                                        const TrajNoise &nz, uint64_t seed, uint64_t t) {
+    Shared<NT> &s = shared_of<NT>();
+    const int lane = threadIdx.x % 32;
+    if (o + 2 < nops && lane < (int)(sizeof(TrajRec) / 16))
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                         (uint32_t)__cvta_generic_to_shared(reinterpret_cast<char *>(&s.recs[(o + 2) & 3]) + 16 * lane)),
+                     "l"(reinterpret_cast<const char *>(recs + o + 2) + 16 * lane)
+                     : "memory");
+    refill(s, seed, t);
+    const TrajRec &next = s.recs[(o + 1) & 3];
+    const bool gate = s.op(o).kind == TOP_GATE;
+    int look = LOOK_NO, taken = 0;
+    if (gate && o + 1 < nops && op_runs(next.op, s.cl)) {
+        // gates take a known number of draws behind their pass
+        const int before = s.op(o).k * (nz.on(2) + nz.on(3) + nz.on(4));
+        taken = prepare_matrix(s, next, cur ^ 1, s.draw + before, mats, nz);
+        look = before ? LOOK_READY : LOOK_GO;
+    }
+    __syncwarp();
+    if (lane == 0) {
+        s.look[o & 1] = look;
+        s.look_draws = taken;
+        if (look == LOOK_GO) s.draw += taken;
     }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kTrajThreads, 4)
-    k_trajectories(T *__restrict__ work, uint32_t n, const TrajOp *__restrict__ ops, int nops,
-                   const double *__restrict__ mats, const uint32_t *__restrict__ fq, const uint32_t *__restrict__ fc,
-                   int nfinal, TrajNoise nz, uint64_t ntraj, uint64_t seed, uint64_t *__restrict__ out,
-                   int *__restrict__ err) {
-    __shared__ Shared s;
-    const uint64_t len = 1ull << n;
-    T *re = work + (size_t)blockIdx.x * 2 * len;
-    T *im = re + len;
-    const int tid = threadIdx.x;
-    for (uint64_t t = blockIdx.x; t < ntraj; t += gridDim.x) {
-        for (uint64_t i = tid; i < len; i += blockDim.x) {
-            re[i] = T(i == 0);
-            im[i] = T(0);
+// Warp 0: the next op that runs, from o on, and its matrix (what look_ahead
+// could not do). Records o and o + 1 are held already if `held`.
+template <int NT>
+__device__ __noinline__ void next_op(int o, int buf, bool held, const TrajRec *recs, int nops, const float *mats,
+                                     const TrajNoise &nz) {
+    Shared<NT> &s = shared_of<NT>();
+    const int lane = threadIdx.x;
+    constexpr int kWords = (int)(sizeof(TrajRec) / 4);
+    for (;; o++, held = false) {
+        __syncwarp();
+        for (int r = o; !held && r < o + 2 && r < nops; r++)
+            for (int i = lane; i < kWords; i += 32)
+                reinterpret_cast<uint32_t *>(&s.recs[r & 3])[i] = reinterpret_cast<const uint32_t *>(recs + r)[i];
+        __syncwarp();
+        if (o >= nops || op_runs(s.recs[o & 3].op, s.cl)) break;
+    }
+    int taken = 0;
+    if (o < nops) taken = prepare_matrix(s, s.recs[o & 3], buf, s.draw, mats, nz);
+    __syncwarp();
+    if (lane == 0) {
+        s.o = o;
+        s.cur = buf;
+        s.draw += taken;
+    }
+    __syncwarp();
+}
+
+// Warp 0 after a pass: the flips and damping of a K-qubit gate, resolved on
+// the joint table J in the reference's order; the operators are left pending
+// (diagonal ones as factors). Every lane computes the same in registers: the
+// whole CTA waits for this chain, and a dependent FP64 operation takes 64
+// cycles.
+template <int K, int NT>
+__device__ __forceinline__ void resolve_gate(Shared<NT> &s, int o, const double *Jin, const TrajNoise &nz) {
+    constexpr int D = 1 << K;
+    double J[D];
+#pragma unroll
+    for (int j = 0; j < D; j++) J[j] = Jin[j];
+    uint64_t draw = s.draw;
+    uint32_t q[3] = {0, 0, 0};
+    float f0[3] = {1.f, 1.f, 1.f}, f1[3] = {1.f, 1.f, 1.f};
+    int nd = 0, np = 0;
+    uint32_t qs[K];
+#pragma unroll
+    for (int b = 0; b < K; b++) qs[b] = s.op(o).qs[b];
+#pragma unroll
+    for (int b = 0; b < K; b++) {
+        float m0 = 1.f, m1 = 0.f, m2 = 0.f, m3 = 1.f;  // row-major, real
+        if (nz.on(2) && s.us[draw++ % kDraws] < nz.p[2]) {  // X
+            m0 = m3 = 0.f;
+            m1 = m2 = 1.f;
+#pragma unroll
+            for (int j = 0; j < D; j++)
+                if (!((j >> b) & 1)) {
+                    const double x = J[j];
+                    J[j] = J[j | (1 << b)];
+                    J[j | (1 << b)] = x;
+                }
         }
-        if (tid == 0) {
-            s.npend = 0;
-            s.draw = 0;
-            s.cl = 0;
+        if (nz.on(3) && s.us[draw++ % kDraws] < nz.p[3]) {  // Z
+            m2 = -m2;
+            m3 = -m3;
         }
-        __syncthreads();
-        for (int o = 0; o < nops; o++) {
-            const TrajOp op = ops[o];
-            const uint32_t k = op.k, dim = 1u << k;
-            const bool gate = op.kind == TOP_GATE;
-            // ---- thread 0: condition, depolarizing draws, gate x Pauli string, pending factors
-            if (tid == 0) {
-                s.skip = 0;
-                if (op.cond) {
-                    const uint64_t mask = op.cond_len >= 64 ? ~0ull : ((1ull << op.cond_len) - 1);
-                    s.skip = ((s.cl >> op.cond_off) & mask) != op.cond_value;
+        if (nz.on(4)) {
+            const double u = s.us[draw++ % kDraws];
+            // mass0, mass1: of the qubit's two values; P(1) = mass1 / tot
+            double mass0 = J[0], mass1 = J[1 << b];
+#pragma unroll
+            for (int j = 1; j < D; j++)
+                if (j != (1 << b)) {
+                    if ((j >> b) & 1) mass1 += J[j];
+                    else mass0 += J[j];
+                }
+            const double tot = mass0 + mass1, jump = nz.p[4] * mass1;
+            if (u * tot < jump) {
+                // jump: collapse to 1 (scale 1/sqrt(P1)) then X
+                const float sc = (float)(1.0 / sqrt(mass1 / tot));
+                m0 = sc * m2;
+                m1 = sc * m3;
+                m2 = m3 = 0.f;
+#pragma unroll
+                for (int j = 0; j < D; j++)
+                    if (!((j >> b) & 1)) {
+                        J[j] = J[j | (1 << b)] * tot / mass1;
+                        J[j | (1 << b)] = 0.0;
+                    }
+            } else {
+                // 1 / sqrt(1 - gamma P(1)) in one rsqrt
+                const double sc = tot > 0.0 ? tot * rsqrt((tot - jump) * tot) : 1.0;
+                const float k0 = (float)sc, k1 = (float)(sc * s.keep);
+                m0 *= k0;
+                m1 *= k0;
+                m2 *= k1;
+                m3 *= k1;
+                if (b + 1 < K) {  // the next qubit's masses; the common sc^2 cancels
+#pragma unroll
+                    for (int j = 0; j < D; j++)
+                        if ((j >> b) & 1) J[j] *= s.keep2;
                 }
             }
-            __syncthreads();
-            if (s.skip) {  // pending operators wait for the next op that runs
-                __syncthreads();  // every thread has read s.skip before thread 0 sets it again
-                continue;
-            }
-            if (tid == 0) {
-                prepare_pending(s);
-                const double pdep = gate ? (k == 1 ? nz.p[0] : nz.p[1]) : 0.0;
-                uint64_t idx = 0;
-                if (pdep > 0.0 && philox_f64(seed, t, s.draw++) < pdep)
-                    idx = 1 + philox_range(seed, t, s.draw++, (1ull << (2 * k)) - 1);
-                const double *M = mats + op.mat_off;
-                // P_string . M: the Pauli string is a signed permutation, row r
-                // holding its one entry in column r ^ xm (X and Y flip the bit),
-                // of value prod_b v_b(r_b) (Y: -i on 0, i on 1; Z: -1 on 1)
-                uint32_t xm = 0;
-                for (uint32_t b = 0; b < k; b++) {
-                    const uint32_t code = (uint32_t)(idx >> (2 * b)) & 3u;
-                    if (code == 1 || code == 2) xm |= 1u << b;
-                }
-                for (uint32_t r = 0; r < dim; r++) {
-                    int re_sign = 1, swap = 0;  // phase = re_sign * (swap ? i : 1)
-                    for (uint32_t b = 0; b < k; b++) {
-                        const uint32_t code = (uint32_t)(idx >> (2 * b)) & 3u, rb = (r >> b) & 1u;
-                        if (code == 2) {  // multiply by -i (rb = 0) or i (rb = 1)
-                            if (swap) re_sign = rb ? -re_sign : re_sign;  // i * i = -1, i * -i = 1
-                            else re_sign = rb ? re_sign : -re_sign;
-                            swap ^= 1;
-                        } else if (code == 3 && rb) {
-                            re_sign = -re_sign;
-                        }
-                    }
-                    const uint32_t j = r ^ xm;
-                    for (uint32_t c = 0; c < dim; c++) {
-                        const float mr = (float)M[2 * (j * dim + c)], mi = (float)M[2 * (j * dim + c) + 1];
-                        // (re_sign * (swap ? i : 1)) * (mr + i mi)
-                        s.mr[r * dim + c] = swap ? -re_sign * mi : re_sign * mr;
-                        s.mi[r * dim + c] = swap ? re_sign * mr : re_sign * mi;
-                    }
-                }
-            }
-            __syncthreads();
-            if (s.nondiag) apply_nondiag_pending(re, im, n, s);
-            // ---- one pass: pending diagonal factors, gate, joint table
-            float hi[8] = {0}, lo[8] = {0};
-            if (k == 1) {
-                traj_pass<1>(re, im, len, op, s, hi, lo);
-            } else if (k == 2) {
-                traj_pass<2>(re, im, len, op, s, hi, lo);
-            } else {  // three-qubit ops (rare): generic loop
-                const uint64_t groups = len >> k;
-                for (uint64_t g = tid; g < groups; g += blockDim.x) {
-                    const uint64_t base = insert_zeros(g, op.qs, (int)k);
-                    float xr[8], xi[8];
-                    for (uint32_t j = 0; j < dim; j++) {
-                        uint64_t idx = base;
-                        for (uint32_t b = 0; b < k; b++) idx |= (uint64_t)((j >> b) & 1) << op.qs[b];
-                        float fr, fi;
-                        diag_factor(s, idx, fr, fi);
-                        const float a = (float)re[idx], c = (float)im[idx];
-                        xr[j] = fr * a - fi * c;
-                        xi[j] = fr * c + fi * a;
-                    }
-                    for (uint32_t r = 0; r < dim; r++) {
-                        float yr = 0.f, yi = 0.f;
-                        for (uint32_t c = 0; c < dim; c++) {
-                            const float wr = s.mr[r * dim + c], wi = s.mi[r * dim + c];
-                            yr = fmaf(wr, xr[c], fmaf(-wi, xi[c], yr));
-                            yi = fmaf(wr, xi[c], fmaf(wi, xr[c], yi));
-                        }
-                        uint64_t idx = base;
-                        for (uint32_t b = 0; b < k; b++) idx |= (uint64_t)((r >> b) & 1) << op.qs[b];
-                        re[idx] = (T)yr;
-                        im[idx] = (T)yi;
-                        acc_p2(yr, yi, hi[r], lo[r]);
-                    }
-                }
-            }
-            __syncthreads();
-            if (tid == 0) s.npend = 0;
-            reduce_table(s, hi, lo, (int)dim);
-            // ---- thread 0, measure / reset: outcome from the table, collapse (and X) left pending
-            if (tid == 0 && !gate) {
-                const double tot = s.J[0] + s.J[1];
-                const double p1 = tot > 0.0 ? s.J[1] / tot : 0.0;
-                const bool one = philox_f64(seed, t, s.draw++) < p1;  // src/exec.rs:201-207
-                const double sc = 1.0 / sqrt(one ? p1 : 1.0 - p1);
-                Pending &P = s.pend[s.npend++];
-                P.q = op.qs[0];
-                for (int i = 0; i < 4; i++) P.m[i] = C2{0, 0};
-                if (!one) P.m[0] = C2{(float)sc, 0};
-                else if (op.kind == TOP_RESET) P.m[1] = C2{(float)sc, 0};  // X . diag(0, sc)
-                else P.m[3] = C2{(float)sc, 0};
-                if (op.kind == TOP_MEASURE) {
-                    bool bit = one;
-                    const double pr = bit ? nz.p[6] : nz.p[5];  // readout_flip (src/noise.rs:181-192)
-                    if (pr > 0.0 && philox_f64(seed, t, s.draw++) < pr) bit = !bit;
-                    s.cl = (s.cl & ~(1ull << op.clbit)) | ((uint64_t)bit << op.clbit);
-                }
-            }
-            // ---- thread 0: flips and damping on the table, in the reference's order
-            if (tid == 0 && gate) {
-                double J[8];
-                for (uint32_t j = 0; j < dim; j++) J[j] = s.J[j];
-                for (uint32_t b = 0; b < k; b++) {
-                    C2 M[4];
-                    pauli(0, M);
-                    if (nz.p[2] > 0.0 && philox_f64(seed, t, s.draw++) < nz.p[2]) {
-                        C2 X[4];
-                        pauli(1, X);
-                        mul22(X, M, M);
-                        for (uint32_t j = 0; j < dim; j++)
-                            if (!((j >> b) & 1)) {
-                                const double x = J[j];
-                                J[j] = J[j | (1u << b)];
-                                J[j | (1u << b)] = x;
-                            }
-                    }
-                    if (nz.p[3] > 0.0 && philox_f64(seed, t, s.draw++) < nz.p[3]) {
-                        C2 Z[4];
-                        pauli(3, Z);
-                        mul22(Z, M, M);
-                    }
-                    if (nz.p[4] > 0.0) {
-                        const double u = philox_f64(seed, t, s.draw++);
-                        double tot = 0.0, p1 = 0.0;
-                        for (uint32_t j = 0; j < dim; j++) {
-                            tot += J[j];
-                            if ((j >> b) & 1) p1 += J[j];
-                        }
-                        p1 = tot > 0.0 ? p1 / tot : 0.0;
-                        const double pj = nz.p[4] * p1;
-                        C2 D[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
-                        if (u < pj) {
-                            // jump: collapse to 1 (scale 1/sqrt(P1)) then X
-                            D[1] = C2{(float)(1.0 / sqrt(p1)), 0};
-                            for (uint32_t j = 0; j < dim; j++)
-                                if (!((j >> b) & 1)) {
-                                    J[j] = J[j | (1u << b)] / p1;
-                                    J[j | (1u << b)] = 0.0;
-                                }
-                        } else {
-                            const double sc = 1.0 / sqrt(1.0 - pj);
-                            const double d3 = sc * sqrt(1.0 - nz.p[4]);
-                            D[0] = C2{(float)sc, 0};
-                            D[3] = C2{(float)d3, 0};
-                            for (uint32_t j = 0; j < dim; j++) J[j] *= ((j >> b) & 1) ? d3 * d3 : sc * sc;
-                        }
-                        mul22(D, M, M);
-                    }
-                    Pending &P = s.pend[s.npend++];
-                    P.q = op.qs[b];
-                    for (int i = 0; i < 4; i++) P.m[i] = M[i];
-                }
-            }
-            __syncthreads();
         }
-        // ---- final: pending operators, then one basis index from |psi|^2
-        if (tid == 0) prepare_pending(s);
-        __syncthreads();
-        if (s.nondiag) apply_nondiag_pending(re, im, n, s);
-        const uint64_t per = (len + blockDim.x - 1) / blockDim.x;
-        const uint64_t i0 = tid * per, i1 = min(len, i0 + per);
-        {
-            float hi = 0.f, lo = 0.f;
-            for (uint64_t i = i0; i < i1; i++) {
-                float fr, fi;
-                diag_factor(s, i, fr, fi);
-                const float a = (float)re[i], c = (float)im[i];
-                acc_p2(fr * a - fi * c, fr * c + fi * a, hi, lo);
-            }
-            s.seg[tid] = (double)hi + (double)lo;
+        if (m1 == 0.f && m2 == 0.f) {
+            q[nd] = qs[b];
+            f0[nd] = m0;
+            f1[nd++] = m3;
+        } else {
+            if (threadIdx.x == 0) s.pend[np] = Pending{qs[b], {{m0, 0}, {m1, 0}, {m2, 0}, {m3, 0}}};
+            np++;
         }
-        __syncthreads();
-        if (tid == 0) {
-            double tot = 0.0;
-            for (int i = 0; i < (int)blockDim.x; i++) tot += s.seg[i];
-            double u = philox_f64(seed, t, s.draw++) * tot;
-            uint64_t pick = len;
-            bool found = false;
-            for (int w = 0; w < (int)blockDim.x && !found; w++) {
-                if (u < s.seg[w]) {
-                    const uint64_t a0 = (uint64_t)w * per, a1 = min(len, a0 + per);
-                    for (uint64_t i = a0; i < a1; i++) {
-                        float fr, fi;
-                        diag_factor(s, i, fr, fi);
-                        const float a = (float)re[i], c = (float)im[i];
-                        const float xr = fr * a - fi * c, xi = fr * c + fi * a;
-                        const double p = (double)xr * xr + (double)xi * xi;
-                        if (p > 0.0) pick = i;  // last nonzero so far
-                        if (u < p) {
-                            pick = i;
-                            found = true;
-                            break;
-                        }
-                        u -= p;
+    }
+    factor_tables(s, nd, q, f0, f1);
+    if (threadIdx.x == 0) {
+        s.npend = np;
+        s.draw = draw;
+    }
+}
+
+// The same for a three-qubit gate (rare): thread 0, on s.J.
+template <int NT>
+__device__ __noinline__ void resolve_gate3(int o, const TrajNoise &nz) {
+    Shared<NT> &s = shared_of<NT>();
+    if (threadIdx.x == 0) {
+        const TrajOp &op = s.op(o);
+        s.npend = 0;
+        for (uint32_t b = 0; b < 3; b++) {
+            C2 M[4];
+            pauli(0, M);
+            if (nz.on(2) && next_f64(s) < nz.p[2]) {
+                C2 X[4];
+                pauli(1, X);
+                mul22(X, M, M);
+                for (uint32_t j = 0; j < 8; j++)
+                    if (!((j >> b) & 1)) {
+                        const double x = s.J[j];
+                        s.J[j] = s.J[j | (1u << b)];
+                        s.J[j | (1u << b)] = x;
                     }
-                    found = true;
+            }
+            if (nz.on(3) && next_f64(s) < nz.p[3]) {
+                C2 Z[4];
+                pauli(3, Z);
+                mul22(Z, M, M);
+            }
+            if (nz.on(4)) {
+                const double u = next_f64(s);
+                double mass0 = 0.0, mass1 = 0.0;
+                for (uint32_t j = 0; j < 8; j++)
+                    if ((j >> b) & 1) mass1 += s.J[j];
+                    else mass0 += s.J[j];
+                const double tot = mass0 + mass1, jump = nz.p[4] * mass1;
+                C2 D[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
+                if (u * tot < jump) {
+                    D[1] = C2{(float)(1.0 / sqrt(mass1 / tot)), 0};
+                    for (uint32_t j = 0; j < 8; j++)
+                        if (!((j >> b) & 1)) {
+                            s.J[j] = s.J[j | (1u << b)] * tot / mass1;
+                            s.J[j | (1u << b)] = 0.0;
+                        }
                 } else {
-                    u -= s.seg[w];
+                    const double sc = tot > 0.0 ? tot * rsqrt((tot - jump) * tot) : 1.0;
+                    D[0] = C2{(float)sc, 0};
+                    D[3] = C2{(float)(sc * s.keep), 0};
+                    for (uint32_t j = 0; j < 8; j++)
+                        if ((j >> b) & 1) s.J[j] *= s.keep2;
                 }
+                mul22(D, M, M);
             }
-            if (pick == len) {
-                // rounding left the draw past the last segment: last index with nonzero probability
-                pick = 0;
-                for (uint64_t i = len; i-- > 0;) {
-                    float fr, fi;
-                    diag_factor(s, i, fr, fi);
-                    const float a = (float)re[i], c = (float)im[i];
-                    if ((fr * a - fi * c) != 0.f || (fr * c + fi * a) != 0.f) {
-                        pick = i;
+            Pending &P = s.pend[s.npend++];
+            P.q = op.qs[b];
+            for (int i = 0; i < 4; i++) P.m[i] = M[i];
+        }
+    }
+    __syncwarp();
+    split_pending(s);
+}
+
+// Warp 0 after a measure or reset's pass: the outcome from the table, the
+// collapse (and X) left pending.
+template <int NT>
+__device__ __forceinline__ void resolve_measure(Shared<NT> &s, int o, double J0, double J1, const TrajNoise &nz) {
+    const TrajOp &op = s.op(o);
+    uint64_t draw = s.draw;
+    const double tot = J0 + J1;
+    const bool one = s.us[draw++ % kDraws] * tot < J1;  // u < P(1), src/exec.rs:201-207
+    const float sc = (float)(tot * rsqrt((one ? J1 : J0) * tot));  // 1 / sqrt(P(outcome))
+    const uint32_t q[3] = {op.qs[0], 0, 0};
+    const bool flip = one && op.kind == TOP_RESET;  // X . diag(0, sc)
+    const float f0[3] = {one ? 0.f : sc, 1.f, 1.f}, f1[3] = {one ? sc : 0.f, 1.f, 1.f};
+    factor_tables(s, flip ? 0 : 1, q, f0, f1);
+    uint64_t cl = s.cl;
+    if (op.kind == TOP_MEASURE) {
+        bool bit = one;
+        const double pr = bit ? nz.p[6] : nz.p[5];  // readout_flip (src/noise.rs:181-192)
+        if (nz.on(bit ? 6 : 5) && s.us[draw++ % kDraws] < pr) bit = !bit;
+        cl = (cl & ~(1ull << op.clbit)) | ((uint64_t)bit << op.clbit);
+    }
+    __syncwarp();
+    if (threadIdx.x == 0) {
+        if (flip) s.pend[0] = Pending{op.qs[0], {{0, 0}, {sc, 0}, {0, 0}, {0, 0}}};
+        s.npend = flip;
+        s.cl = cl;
+        s.draw = draw;
+    }
+}
+
+// Warp 0 behind a pass of a K-qubit op: the CTA's table from the warps'
+// (lanes in groups of NW, each summing one entry or every 32 / NW-th), the
+// op's noise or outcome, and the step to the next op.
+template <int K, int NT>
+__device__ __noinline__ void finish_op(int o, int cur, bool acc, const TrajRec *recs, int nops, const float *mats,
+                                       const TrajNoise &nz) {
+    constexpr int NW = NT / 32, G = 32 / NW, D = 1 << K;
+    Shared<NT> &s = shared_of<NT>();
+    const int lane = threadIdx.x;
+    double J[D];
+#pragma unroll
+    for (int j = 0; j < D; j++) J[j] = 0.0;
+    if (acc) {
+        float2 v[D];
+#pragma unroll
+        for (int j = 0; j < D; j += G) v[j] = s.red[lane % NW][(j + lane / NW) & (D - 1)];
+#pragma unroll
+        for (int o = NW / 2; o > 0; o >>= 1)
+#pragma unroll
+            for (int j = 0; j < D; j += G) v[j] = tdf_add(v[j], shfl_xor_f2(v[j], o));
+#pragma unroll
+        for (int j = 0; j < D; j++) {
+            const int src = (j % G) * NW;
+            const float hi = __shfl_sync(0xffffffffu, v[j - j % G].x, src), lo = __shfl_sync(0xffffffffu, v[j - j % G].y, src);
+            J[j] = (double)hi + (double)lo;
+        }
+    }
+    const bool gate = s.op(o).kind == TOP_GATE;
+    if constexpr (K == 3) {
+#pragma unroll
+        for (int j = 0; j < D; j++) s.J[j] = J[j];  // every lane the same
+        __syncwarp();
+        resolve_gate3<NT>(o, nz);
+    } else {
+        if (gate) resolve_gate<K>(s, o, J, nz);
+        else resolve_measure(s, o, J[0], J[1], nz);
+    }
+    __syncwarp();
+    const int look = s.look[o & 1];
+    if (look != LOOK_NO) {
+        if (lane == 0) {
+            if (look == LOOK_READY) s.draw += s.look_draws;
+            s.o = o + 1;
+            s.cur = cur ^ 1;
+        }
+    } else {
+        next_op<NT>(o + 1, cur ^ 1, true, recs, nops, mats, nz);
+    }
+}
+
+// |a|^2 of element i with the pending factors, as f64.
+template <int NT, bool SMEM>
+__device__ __forceinline__ double mass_at(const StateMem<SMEM> &sm, const Shared<NT> &s, uint64_t i) {
+    float fr, fi;
+    diag_factor(s, i, fr, fi);
+    const float a = sm.re(i), c = sm.im(i);
+    const float xr = fr * a - fi * c, xi = fr * c + fi * a;
+    return (double)xr * xr + (double)xi * xi;
+}
+
+// Warp: the mass of elements [i0, i1) in double-float.
+template <int NT, bool SMEM>
+__device__ double range_mass(const StateMem<SMEM> &sm, const Shared<NT> &s, uint64_t i0, uint64_t i1) {
+    float2 h = make_float2(kBias, kBias), l = make_float2(0.f, 0.f);
+    for (uint64_t i = i0 + threadIdx.x % 32; i < i1; i += 32) {
+        float fr, fi;
+        diag_factor(s, i, fr, fi);
+        const float a = sm.re(i), c = sm.im(i);
+        acc_sq2(make_float2(fr * a - fi * c, fr * c + fi * a), h, l);
+    }
+    float2 v = acc_end(h, l);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = tdf_add(v, shfl_xor_f2(v, o));
+    return (double)v.x + (double)v.y;
+}
+
+// One basis index from |psi|^2 by the draw u in [0, 1): region (one per
+// warp), block (32 per region) and element whose cumulative mass first
+// exceeds it. Left in s.u's stead as an index in every thread.
+template <int NT, bool SMEM>
+__device__ __noinline__ uint64_t sample_index(float *work, uint32_t n) {
+    Shared<NT> &s = shared_of<NT>();
+    const StateMem<SMEM> sm(work, n);
+    const uint64_t len = 1ull << n;
+    constexpr int NW = NT / 32;
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const uint64_t W = (len + NW - 1) / NW, B = (W + 31) / 32;  // elements per region, per block
+    const uint64_t w0 = min(len, warp * W), w1 = min(len, w0 + W);
+    const double seg = range_mass(sm, s, w0, w1);
+    if (lane == 0) s.seg[warp] = seg;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double tot = 0.0;
+        for (int i = 0; i < NW; i++) tot += s.seg[i];
+        double u = next_f64(s) * tot;
+        int r = 0;
+        while (r < NW && !(u < s.seg[r])) u -= s.seg[r++];
+        s.region = r;
+        s.u = u;
+    }
+    __syncthreads();
+    const int region = s.region;
+    uint64_t pick = len;
+    if (region < NW) {
+        const uint64_t r0 = min(len, region * W), r1 = min(len, r0 + W);
+        for (int b = warp; b < 32; b += NW) {
+            const uint64_t b0 = min(r1, r0 + b * B), b1 = min(r1, b0 + B);
+            const double m = range_mass(sm, s, b0, b1);
+            if (lane == 0) s.blk[b] = m;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double u = s.u;
+            int b = 0, last = 0;
+            for (; b < 32 && !(u < s.blk[b]); b++) {
+                if (s.blk[b] > 0.0) last = b;
+                u -= s.blk[b];
+            }
+            s.block = b < 32 ? b : last;  // rounding past the region's end: its last block with mass
+            s.u = b < 32 ? u : __longlong_as_double(0x7ff0000000000000ll);
+        }
+        __syncthreads();
+        // the block's elements, in order, 1024 at a time
+        const uint64_t b0 = min(r1, r0 + s.block * B), b1 = min(r1, b0 + B);
+        double u = s.u;
+        bool found = false;
+        for (uint64_t c0 = b0; c0 < b1 && !found; c0 += 1024) {
+            const uint64_t c1 = min(b1, c0 + 1024);
+            __syncthreads();
+            for (uint64_t i = c0 + threadIdx.x; i < c1; i += NT) s.el[i - c0] = mass_at(sm, s, i);
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                for (uint64_t i = c0; i < c1; i++) {
+                    const double p = s.el[i - c0];
+                    if (p > 0.0) pick = i;  // last nonzero so far
+                    if (u < p) {
+                        found = true;
                         break;
                     }
+                    u -= p;
                 }
             }
+            found = __syncthreads_or(found);
+        }
+    }
+    if (threadIdx.x == 0 && pick == len) {
+        // rounding left the draw past the last region: last index with nonzero probability
+        pick = 0;
+        for (uint64_t i = len; i-- > 0;)
+            if (mass_at(sm, s, i) > 0.0) {
+                pick = i;
+                break;
+            }
+    }
+    return pick;  // thread 0's counts
+}
+
+// NT threads per CTA. SMEM: the whole state in shared memory (ns unused).
+template <int NT, int CTAS, bool SMEM>
+__global__ void __launch_bounds__(NT, CTAS)
+    k_trajectories(float *__restrict__ work, uint32_t n, const TrajRec *__restrict__ recs, int nops,
+                   const float *__restrict__ mats, const uint32_t *__restrict__ fq, const uint32_t *__restrict__ fc,
+                   int nfinal, TrajNoise nz, uint64_t ntraj, uint64_t seed, uint64_t *__restrict__ out) {
+    Shared<NT> &s = shared_of<NT>();
+    constexpr int NW = NT / 32;
+    const uint64_t len = 1ull << n;
+    if (!SMEM) work += (size_t)blockIdx.x * 2 * len;
+    const StateMem<SMEM> sm(work, n);
+    const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+    const bool vec = n >= 5 && n <= 31;
+    if (tid == 0) {
+        s.keep = sqrt(1.0 - nz.p[4]);
+        s.keep2 = s.keep * s.keep;
+    }
+    for (uint64_t t = blockIdx.x; t < ntraj; t += gridDim.x) {
+        for (uint64_t i = tid; i < len; i += NT) {
+            sm.re(i) = i == 0 ? 1.f : 0.f;
+            sm.im(i) = 0.f;
+        }
+        if (warp == 0) {
+            const uint32_t q[3] = {0, 0, 0};
+            const float f[3] = {1.f, 1.f, 1.f};
+            factor_tables(s, 0, q, f, f);
+            if (tid == 0) {
+                s.npend = 0;
+                s.draw = s.drawn = 0;
+                s.cl = 0;
+            }
+            refill(s, seed, t);
+            next_op<NT>(0, 0, false, recs, nops, mats, nz);
+        }
+        __syncthreads();
+        int o = s.o, cur = s.cur;
+        while (o < nops) {
+            const bool factors = s.npend || s.nfv >= 0;
+            if (s.npend) apply_nondiag_pending<NT, SMEM>(work, n);
+            const uint32_t k = s.op(o).k;
+            const bool acc = wants_table(s.op(o), nz);
+            if (warp == 1) look_ahead<NT>(o, cur, recs, nops, mats, nz, seed, t);
+            const bool mono = s.op(o).mono && s.op(o).qs[0] >= 2;
+            if (!vec || k > 2) traj_pass_general<NT, SMEM>(work, n, o, cur, acc);
+            else if (k == 1 && !mono) traj_pass_body<1, false, NT, SMEM>(work, n, o, cur, acc);
+            else if (k == 1) traj_pass_body<1, true, NT, SMEM>(work, n, o, cur, acc);
+            else if (mono) traj_pass_body<2, true, NT, SMEM>(work, n, o, cur, acc);
+            else traj_pass_dense2<NT, SMEM>(work, n, o, cur, acc);
+            if (warp == 1) asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();
+            // nothing to decide and nothing pending before or after: on to the
+            // next pass with this one barrier
+            if (s.look[o & 1] == LOOK_GO && !factors) {
+                o++;
+                cur ^= 1;
+                continue;
+            }
+            if (warp == 0) {
+                if (k == 1) finish_op<1, NT>(o, cur, acc, recs, nops, mats, nz);
+                else if (k == 2) finish_op<2, NT>(o, cur, acc, recs, nops, mats, nz);
+                else finish_op<3, NT>(o, cur, acc, recs, nops, mats, nz);
+            }
+            __syncthreads();
+            o = s.o;
+            cur = s.cur;
+        }
+        // ---- final: pending operators, then one basis index from |psi|^2
+        if (s.npend) apply_nondiag_pending<NT, SMEM>(work, n);
+        if (warp == 0) refill(s, seed, t);
+        const uint64_t pick = sample_index<NT, SMEM>(work, n);
+        if (warp == 0) {
             uint64_t cl = s.cl;
             for (int f = 0; f < nfinal; f++) {
-                bool bit = (pick >> fq[f]) & 1;
-                const double pr = bit ? nz.p[6] : nz.p[5];
-                if (pr > 0.0 && philox_f64(seed, t, s.draw++) < pr) bit = !bit;
-                cl = (cl & ~(1ull << fc[f])) | ((uint64_t)bit << fc[f]);
+                refill(s, seed, t);
+                if (tid == 0) {
+                    bool bit = (pick >> fq[f]) & 1;
+                    const double pr = bit ? nz.p[6] : nz.p[5];
+                    if (nz.on(bit ? 6 : 5) && next_f64(s) < pr) bit = !bit;
+                    cl = (cl & ~(1ull << fc[f])) | ((uint64_t)bit << fc[f]);
+                }
             }
-            out[t] = cl;
+            if (tid == 0) out[t] = cl;
         }
         __syncthreads();
     }
-    (void)err;
+}
+
+template <int NT, int CTAS, bool SMEM>
+int run_trajectories(zc_state *st, const TrajPlan &plan, uint32_t n, const TrajRec *d_recs, int nops,
+                     const float *d_mats, const uint32_t *d_fq, const uint32_t *d_fc, int nfinal, const TrajNoise &nz,
+                     uint64_t ntraj, uint64_t seed, uint64_t *d_out, float *d_work) {
+    ZC_CUDA(cudaFuncSetAttribute(k_trajectories<NT, CTAS, SMEM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)kTrajSmemMax));
+    k_trajectories<NT, CTAS, SMEM><<<plan.ctas, NT, plan.smem, st->stream>>>(
+        d_work, n, d_recs, nops, d_mats, d_fq, d_fc, nfinal, nz, ntraj, seed, d_out);
+    ZC_CUDA(cudaGetLastError());
+    return ZC_OK;
 }
 
 }  // namespace
 
-int launch_trajectories(zc_state *st, uint32_t n, const TrajOp *d_ops, int nops, const double *d_mats,
-                        const uint32_t *d_fq, const uint32_t *d_fc, int nfinal, const TrajNoise &nz, uint64_t ntraj,
-                        uint64_t seed, uint64_t *d_out, void *d_work, int ctas) {
+// CTA size and placement by state size (f32, 8 bytes per amplitude), 128
+// registers per thread everywhere:
+//   <= 10 qubits (8 KiB)    64 threads, eight per SM: a pass is a few vectors
+//                           per thread, latency is hidden across trajectories
+//   <= 12 qubits (32 KiB)   128 threads, four per SM
+//   13 qubits (64 KiB)      256 threads, two per SM; all these in shared memory
+//   14 qubits (128 KiB)     512 threads, one per SM, all in shared memory
+//   above                   512 threads, one per SM, the first 24576
+//                           amplitudes in shared memory, the rest in global
+TrajPlan plan_trajectories(uint32_t n, uint64_t ntraj, int num_sms) {
+    TrajPlan p{};
+    const uint64_t len = 1ull << n;
+    p.threads = n <= 10 ? 64 : n <= 12 ? 128 : n == 13 ? 256 : 512;
+    p.smem = std::min<uint64_t>(len, kTrajSplitElems) * 8;
+    p.global_bytes = n <= 14 ? 0 : len * 8;
+    p.ctas = (int)std::min<uint64_t>(ntraj, (uint64_t)num_sms * (512 / p.threads));
+    return p;
+}
+
+int launch_trajectories(zc_state *st, const TrajPlan &plan, uint32_t n, const TrajRec *d_recs, int nops,
+                        const float *d_mats, const uint32_t *d_fq, const uint32_t *d_fc, int nfinal,
+                        const TrajNoise &nz, uint64_t ntraj, uint64_t seed, uint64_t *d_out, void *d_work) {
     ProfScope ps(st, K_TRAJ, 0.0);
     st->ctr.launches++;
     if (st->prec != 32) return fail(ZC_ERR_UNSUPPORTED, "the batched trajectory engine runs f32 states");
-    k_trajectories<float><<<ctas, kTrajThreads, 0, st->stream>>>((float *)d_work, n, d_ops, nops, d_mats, d_fq, d_fc,
-                                                                 nfinal, nz, ntraj, seed, d_out, st->d_err);
-    ZC_CUDA(cudaGetLastError());
-    return ZC_OK;
+    auto run = plan.threads == 64    ? run_trajectories<64, 8, true>
+               : plan.threads == 128 ? run_trajectories<128, 4, true>
+               : plan.threads == 256 ? run_trajectories<256, 2, true>
+                                     : run_trajectories<512, 1, false>;
+    return run(st, plan, n, d_recs, nops, d_mats, d_fq, d_fc, nfinal, nz, ntraj, seed, d_out, (float *)d_work);
 }
 
 }  // namespace zc
