@@ -204,12 +204,27 @@ __device__ __forceinline__ float2 df_dot4(float2 x0, float2 y0, float2 x1, float
     return df_norm(s, lo);
 }
 
+// The residual of a sum with a rounded product p = fl(x y) in it: TwoSum's last
+// difference p - pp (pp: p as the sum sees it) plus the product's own rounding
+// error x y - p is x y - pp, one FMA, rounded once where the two were added.
+// A sum of two products so takes 8 operations for hi and residual (against 13
+// for two split products and a TwoSum), x + t y takes 7 (against 9).
+
+// x0*y0 + x1*y1 in double-float, unnormalised.
+__device__ __forceinline__ float2 df_dot2_u(float2 x0, float2 y0, float2 x1, float2 y1) {
+    const float p0 = __fmul_rn(x0.x, y0.x), p1 = __fmul_rn(x1.x, y1.x);
+    const float s = __fadd_rn(p0, p1);
+    const float b = __fsub_rn(s, p0), a = __fsub_rn(s, b);
+    float l0 = __fmaf_rn(x0.x, y0.x, -a), l1 = __fmaf_rn(x1.x, y1.x, -b);
+    l0 = __fmaf_rn(x0.x, y0.y, l0);
+    l1 = __fmaf_rn(x1.x, y1.y, l1);
+    l0 = __fmaf_rn(x0.y, y0.x, l0);
+    l1 = __fmaf_rn(x1.y, y1.x, l1);
+    return make_float2(s, __fadd_rn(l0, l1));
+}
 __device__ __forceinline__ float2 df_dot2(float2 x0, float2 y0, float2 x1, float2 y1) {
-    float p0, e0, p1, e1, r1;
-    df_prod(x0, y0, p0, e0);
-    df_prod(x1, y1, p1, e1);
-    const float s = two_sum(p0, p1, r1);
-    return df_norm(s, __fadd_rn(r1, __fadd_rn(e0, e1)));
+    const float2 r = df_dot2_u(x0, y0, x1, y1);
+    return df_norm(r.x, r.y);
 }
 
 // Gate matrix in double-float: m00r m00i m01r m01i m10r m10i m11r m11i.
@@ -250,32 +265,28 @@ __device__ __forceinline__ void pair_update_rdf(const float2 *r, float2 &ar, flo
     bi = nbi;
 }
 
-// x + t*y in double-float (one product, one TwoSum).
-__device__ __forceinline__ float2 df_axpy(float2 x, float2 t, float2 y) {
-    float p, e, r;
-    df_prod(t, y, p, e);
-    const float s = two_sum(x.x, p, r);
-    return df_norm(s, __fadd_rn(x.y, __fadd_rn(e, r)));
-}
+// Unnormalised variants (also df_dot2_u above) for chains of operations
+// inside one register pass: the (s, lo) pair is left as the sum and its error
+// terms give it (|lo| a few ulps of s at most); products and sums of the next
+// operation stay exact in their hi parts whatever the pair's normalisation, so
+// the chain keeps the double-float error bound relative to its inputs. df_norm
+// once at the end.
 
-// Unnormalised variants for chains of operations inside one register pass:
-// the (s, lo) pair is left as TwoSum and the error terms give it (|lo| a few
-// ulps of s at most); products and TwoSums of the next operation stay exact in
-// their hi parts whatever the pair's normalisation, so the chain keeps the
-// double-float error bound relative to its inputs. df_norm once at the end.
+// x + t*y in double-float.
 __device__ __forceinline__ float2 df_axpy_u(float2 x, float2 t, float2 y) {
-    float p, e, r;
-    df_prod(t, y, p, e);
-    const float s = two_sum(x.x, p, r);
-    return make_float2(s, __fadd_rn(x.y, __fadd_rn(e, r)));
+    const float p = __fmul_rn(t.x, y.x);
+    const float s = __fadd_rn(x.x, p);
+    const float b = __fsub_rn(s, x.x);
+    const float da = __fsub_rn(x.x, __fsub_rn(s, b));
+    // the small terms first: x.y may have grown over a chain
+    float lo = __fadd_rn(da, __fmaf_rn(t.x, y.x, -b));
+    lo = __fmaf_rn(t.x, y.y, lo);
+    lo = __fmaf_rn(t.y, y.x, lo);
+    return make_float2(s, __fadd_rn(x.y, lo));
 }
-
-__device__ __forceinline__ float2 df_dot2_u(float2 x0, float2 y0, float2 x1, float2 y1) {
-    float p0, e0, p1, e1, r1;
-    df_prod(x0, y0, p0, e0);
-    df_prod(x1, y1, p1, e1);
-    const float s = two_sum(p0, p1, r1);
-    return make_float2(s, __fadd_rn(r1, __fadd_rn(e0, e1)));
+__device__ __forceinline__ float2 df_axpy(float2 x, float2 t, float2 y) {
+    const float2 r = df_axpy_u(x, t, y);
+    return df_norm(r.x, r.y);
 }
 
 __device__ __forceinline__ float2 df_renorm(float2 v) { return df_norm(v.x, v.y); }
@@ -345,9 +356,9 @@ __device__ __forceinline__ void cscale_df(float2 wr, float2 wi, float2 &ar, floa
 //   H = (re hi, im hi),  L = (re lo, im lo)
 // and run the real and imaginary halves of a rotation through one
 // instruction stream. Each half sees the operations of the scalar
-// routines above in the same order; where a routine subtracts a product p,
-// the packed one adds q = -p (negation is exact and rounding to nearest is
-// symmetric), so both give the same values (a zero may carry the other
+// routines above in the same order; where a routine subtracts a value, the
+// packed one may add its negative (negation is exact and rounding to nearest
+// is symmetric), so both give the same values (a zero may carry the other
 // sign).
 
 __device__ __forceinline__ unsigned long long pk_bits(float2 v) {
@@ -381,37 +392,34 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
     return pk_float2(d);
 }
 
-// A real double-float coefficient t as pairs: (t hi, t hi), (t lo, t lo),
-// (-t hi, -t hi).
+// A real double-float coefficient t as pairs: (t hi, t hi), (t lo, t lo) and
+// their negatives.
 struct PkReal {
-    float2 h, l, nh;
+    float2 h, l, nh, nl;
 };
 
-// [[1, -t], [t, 1]] on (a, b), unnormalised: per half, a - t b equals
-// df_axpy_u(a, -t, b) and b + t a equals df_axpy_u(b, t, a). Both use the
-// product of +t; q = -(t hi * y hi) serves the error term and the sums.
+// x + t*y per half: df_axpy_u on (H, L) pairs (h, l the pairs of t).
+__device__ __forceinline__ void pk_axpy_u(float2 h, float2 l, float2 Hx, float2 Lx, float2 Hy, float2 Ly, float2 &Hr,
+                                          float2 &Lr) {
+    // the product as an FMA: a packed mul whose only use is an add gets
+    // contracted with it (measured: results lose the low parts)
+    const float2 s = add2(Hx, fma2(h, Hy, make_float2(0.f, 0.f)));
+    const float2 nb = sub2(Hx, s);
+    const float2 da = sub2(Hx, add2(s, nb));
+    float2 lo = add2(da, fma2(h, Hy, nb));
+    lo = fma2(h, Ly, lo);
+    lo = fma2(l, Hy, lo);
+    Hr = s;
+    Lr = add2(Lx, lo);
+}
+
+// [[1, -t], [t, 1]] on (a, b), unnormalised.
 __device__ __forceinline__ void pk_rot_u(const PkReal &t, float2 &Ha, float2 &La, float2 &Hb, float2 &Lb) {
-    // a - t b
-    float2 q = mul2(t.nh, Hb);
-    float2 e = fma2(t.h, Hb, q);
-    e = fma2(t.h, Lb, e);
-    e = fma2(t.l, Hb, e);  // t b = -q + e
-    float2 s = add2(Ha, q);
-    float2 bb = sub2(s, Ha);
-    float2 r = add2(sub2(Ha, sub2(s, bb)), sub2(q, bb));
-    const float2 nHa = s, nLa = add2(La, sub2(r, e));
-    // b + t a
-    q = mul2(t.nh, Ha);
-    e = fma2(t.h, Ha, q);
-    e = fma2(t.h, La, e);
-    e = fma2(t.l, Ha, e);  // t a = -q + e
-    s = sub2(Hb, q);
-    bb = sub2(s, Hb);
-    r = sub2(sub2(Hb, sub2(s, bb)), add2(q, bb));
-    Lb = add2(Lb, add2(e, r));
-    Hb = s;
-    Ha = nHa;
-    La = nLa;
+    float2 Hn, Ln;
+    pk_axpy_u(t.nh, t.nl, Ha, La, Hb, Lb, Hn, Ln);
+    pk_axpy_u(t.h, t.l, Hb, Lb, Ha, La, Hb, Lb);
+    Ha = Hn;
+    La = Ln;
 }
 
 // (H, L) <-> the scalar routines' (re, im) double-float pairs.

@@ -134,7 +134,7 @@ __device__ void apply_perm(T *sr, T *si, const OpHead &op, uint64_t base, uint32
 // Per-op coefficients converted once per CTA into the compute representation.
 // U1: the 2x2 matrix; D1: entries 0..3 = d0r d0i d1r d1i. Double-float
 // pairs for A == AR_DF, else values of T. Double-float RT: v[0] = t, and
-// v[2..5) its packed pairs (PkReal: t hi, t lo, -t hi, each twice).
+// v[2..6) its packed pairs (PkReal: t hi, t lo, -t hi, -t lo, each twice).
 template <typename T, int A>
 struct alignas(16) OpCoef {
     typename std::conditional<A == AR_DF, float2, T>::type v[8];
@@ -142,16 +142,17 @@ struct alignas(16) OpCoef {
 
 // The packed pairs of a double-float rotation's t, read where the rotation
 // runs: hoisted above a group's amplitude loads, the pairs of three
-// rotations (18 registers) spill at the 80-register cap.
+// rotations (24 registers) spill at the 80-register cap.
 template <typename T, int A>
 __device__ __forceinline__ PkReal rot_pairs(const OpCoef<T, A> &c) {
-    float4 a;
-    float2 b;
+    float4 a, b;
     asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
                  : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w)
                  : "r"(smem_addr(&c.v[2])));
-    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(b.x), "=f"(b.y) : "r"(smem_addr(&c.v[4])));
-    return PkReal{make_float2(a.x, a.y), make_float2(a.z, a.w), b};
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "r"(smem_addr(&c.v[4])));
+    return PkReal{make_float2(a.x, a.y), make_float2(a.z, a.w), make_float2(b.x, b.y), make_float2(b.z, b.w)};
 }
 
 // Double-float sweeps hold each amplitude as packed pairs: slot v of the
@@ -792,6 +793,7 @@ __device__ void load_job(SweepSmem<T, A> &c, const MicroOp *gops, int nops, uint
                     c.coef[tid].v[2] = make_float2(t.x, t.x);
                     c.coef[tid].v[3] = make_float2(t.y, t.y);
                     c.coef[tid].v[4] = make_float2(-t.x, -t.x);
+                    c.coef[tid].v[5] = make_float2(-t.y, -t.y);
                 }
             }
         }
