@@ -542,11 +542,8 @@ int check_device_error(zc_state *st) {
         if (h[0] == 3)
             return fail(ZC_ERR_CUDA, "tensor-core block kernel gave up waiting for a copy or an MMA (device wait limit)");
         char buf[320];
-        snprintf(buf, sizeof(buf),
-                 "sweep kernel %s (cta %d tile %d phase %d barrier %08x%08x L %d H %d ops %d tiles done %d index %08x)",
-                 h[0] == 1 ? "gave up waiting for a bulk copy (device wait limit reached)"
-                           : "found a tile index out of range",
-                 h[1], h[2], h[3], (unsigned)h[5], (unsigned)h[4], h[6], h[7], h[8], h[9], (unsigned)h[10]);
+        snprintf(buf, sizeof(buf), "sweep kernel found a tile index out of range (cta %d L %d H %d ops %d index %08x)",
+                 h[1], h[6], h[7], h[8], (unsigned)h[10]);
         return fail(ZC_ERR_CUDA, buf);
     }
     return ZC_OK;

@@ -1,5 +1,5 @@
 // Shared-memory asynchronous-copy helpers (TMA bulk copies, mbarriers)
-// used by the sweep and tensor-core kernels. Every wait is bounded.
+// used by the tensor-core kernel. Every wait is bounded.
 #pragma once
 
 #include <stdint.h>
@@ -54,15 +54,6 @@ __device__ __forceinline__ void bulk_load(void *dst_smem, const void *src_gmem, 
         : "memory");
 }
 
-__device__ __forceinline__ void bulk_store(void *dst_gmem, const void *src_smem, uint32_t bytes) {
-    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst_gmem),
-                 "r"(smem_addr(src_smem)), "r"(bytes)
-                 : "memory");
-}
-
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 }  // namespace

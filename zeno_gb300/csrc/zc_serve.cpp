@@ -479,7 +479,7 @@ int zc_server_step(zc_server *s, zc_server_status *status) {
     s->steps++;
     int h = 0;
     ZC_CUDA(cudaMemcpy(&h, s->ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost));
-    if (h) return fail(ZC_ERR_CUDA, "packed sweep gave up waiting for a bulk copy");
+    if (h) return fail(ZC_ERR_CUDA, "packed sweep found a tile index out of range");
     if (status) {
         status->pending = s->pending.size();
         status->active = s->active.size();

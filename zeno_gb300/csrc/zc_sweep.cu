@@ -3,11 +3,10 @@
 // The state is cut into tiles of 2^T amplitudes: the L lowest qubits (a
 // contiguous row of 2^L elements, 256 bytes) plus H chosen higher qubits
 // ("local" qubits); the other n - T qubits pick the tile. A persistent CTA
-// streams tiles through one shared-memory buffer: every row of a tile is
-// fetched with one TMA bulk copy (cp.async.bulk, completion on an
-// mbarrier), the sweep's micro-ops are applied in shared memory, and the
-// rows go back with TMA bulk stores; three CTAs per SM overlap one tile's
-// copies with the others' arithmetic. In exact mode every micro-op uses the
+// streams tiles through one shared-memory buffer: a tile is fetched with
+// asynchronous 16-byte copies, the sweep's micro-ops are applied in shared
+// memory, and it goes back with 16-byte stores; three CTAs per SM overlap one
+// tile's copies with the others' arithmetic. In exact mode every micro-op uses the
 // same arithmetic as the per-op kernels, so a sweep is bit-identical to
 // launching its ops one by one; fast f64 sweeps run the lowered ops
 // (zc_lower.cpp) in register passes of packed double-float arithmetic.
@@ -732,19 +731,17 @@ __device__ void apply_ops(R *sr, R *si, const OpHead *ops, const OpCoef<T, A> *c
 }
 
 // Per-CTA state of a sweep: the current job's micro-ops, coefficients and
-// row offsets, plus the tile buffer's mbarrier.
+// row offsets.
 template <typename T, int A>
 struct SweepSmem {
-    uint64_t bar;
     OpHead ops[kMaxMicroOps];
     OpCoef<T, A> coef[kMaxMicroOps];
-    uint32_t hpos[16];     // tile bit L + j holds qubit hpos[j] (any order)
-    uint32_t hsorted[16];  // the same qubits ascending (tile base)
+    uint32_t rows[1u << kMaxSweepHigh];  // row r of a tile starts at element rows[r] << L of it
+    uint32_t hsorted[8];                 // the high qubits ascending (tile base)
     int nops;
     uint32_t L, H;
     int has_arith;
-    int fail;
-    uint32_t fail_tile, done_tiles, bad;
+    uint32_t bad;
     uint16_t jlut[kJlutLen];  // diagonal index tables of the current DK op
     // register passes (double-float sweeps), or the job's diagonal index tables
     typename std::conditional<A == AR_DF, GroupInfo[kMaxMicroOps], uint16_t[kJobLuts * kJlutLen]>::type gi;
@@ -763,7 +760,11 @@ __device__ void load_job(SweepSmem<T, A> &c, const MicroOp *gops, int nops, uint
     for (int i = tid; i < nops * kHeadWords; i += blockDim.x)
         reinterpret_cast<uint32_t *>(c.ops)[i] =
             reinterpret_cast<const uint32_t *>(gops)[(i / kHeadWords) * kOpWords + i % kHeadWords];
-    if (tid < 16) c.hpos[tid] = tid < (int)H ? hpos[tid] : 0u;
+    for (uint32_t r = tid; r < (1u << H); r += blockDim.x) {  // tile bit L + j holds qubit hpos[j] (any order)
+        uint32_t o = 0;
+        for (uint32_t j = 0; j < H; j++) o |= ((r >> j) & 1u) << (hpos[j] - L);
+        c.rows[r] = o;
+    }
     if (tid == 0) {
         for (uint32_t j = 0; j < H; j++) {  // insertion sort, H <= 7
             uint32_t x = hpos[j], i = j;
@@ -823,40 +824,65 @@ __device__ void load_job(SweepSmem<T, A> &c, const MicroOp *gops, int nops, uint
     }
 }
 
-// Global offset of row r of a tile: bit j of r at qubit hpos[j].
+// All threads: one array of a tile between global and shared memory, 16
+// bytes per access (a row is 256 bytes, or less for states under 2^L).
+// Loads are asynchronous copies (wait_all, then a barrier); stores go
+// through registers, four in flight.
 template <typename T, int A>
-__device__ __forceinline__ uint64_t row_offset(const SweepSmem<T, A> &c, uint32_t r) {
-    uint64_t o = 0;
-    for (uint32_t j = 0; j < c.H; j++) o |= (uint64_t)((r >> j) & 1u) << c.hpos[j];
-    return o;
+__device__ __forceinline__ void tile_load(const SweepSmem<T, A> &c, T *dst, const T *src, uint32_t vecs) {
+    constexpr uint32_t VW = 16 / sizeof(T), VB = VW == 4 ? 2 : 1;
+    const uint32_t lv = c.L - VB, cm = (1u << lv) - 1;  // vectors per row (log2), column mask
+    const uint32_t d = smem_addr(dst);
+    if (c.L < VB) {  // a state shorter than one vector
+        if (threadIdx.x < (1u << c.L)) dst[threadIdx.x] = src[threadIdx.x];
+        return;
+    }
+    for (uint32_t i = threadIdx.x; i < vecs; i += kSweepThreads) {
+        const T *g = src + ((size_t)c.rows[i >> lv] << c.L) + (size_t)(i & cm) * VW;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16 * i), "l"(g) : "memory");
+    }
+}
+template <typename T, int A>
+__device__ __forceinline__ void tile_store(const SweepSmem<T, A> &c, T *dst, const T *src, uint32_t vecs) {
+    constexpr uint32_t VW = 16 / sizeof(T), VB = VW == 4 ? 2 : 1;
+    const uint32_t lv = c.L - VB, cm = (1u << lv) - 1;
+    if (c.L < VB) {
+        if (threadIdx.x < (1u << c.L)) dst[threadIdx.x] = src[threadIdx.x];
+        return;
+    }
+    const uint4 *sv = reinterpret_cast<const uint4 *>(src);
+    auto at = [&](uint32_t i) {
+        return reinterpret_cast<uint4 *>(dst + ((size_t)c.rows[i >> lv] << c.L) + (size_t)(i & cm) * VW);
+    };
+    uint32_t i = threadIdx.x;
+    for (; i + 3 * kSweepThreads < vecs; i += 4 * kSweepThreads) {
+        uint4 x[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) x[k] = sv[i + k * kSweepThreads];
+#pragma unroll
+        for (int k = 0; k < 4; k++) *at(i + k * kSweepThreads) = x[k];
+    }
+    for (; i < vecs; i += kSweepThreads) *at(i) = sv[i];
 }
 
-// All threads: one tile of the current job — TMA row loads, micro-ops in
-// shared memory, TMA row stores. Returns false if a wait ran out.
+// All threads: one tile of the current job — load, micro-ops in shared
+// memory, store.
+// The tile moves by plain 16-byte accesses of all threads (32 per thread and
+// tile). One TMA bulk copy per 256-byte row, issued by one warp, kept the
+// copy unit busy ~75 cycles per row: 20k cycles for a tile's loads and 22k
+// for its stores beside 38k of arithmetic, at three CTAs per SM
+// (clock64 at 26 qubits). The same circuits with
+// this: 27q depth-10 fast f64 84.3 -> 72.3 ms, 26q f32 gate mix 22.3 -> 18.8.
 template <typename T, int A>
-__device__ bool process_tile(SweepSmem<T, A> &c, T *re, T *im, uint64_t t, const char *tables, T *sre, T *sim,
-                             uint32_t &phase, uint32_t form) {
-    const uint32_t size = 1u << (c.L + c.H);
-    const uint32_t rows = 1u << c.H, row_elems = 1u << c.L, row_bytes = row_elems * (uint32_t)sizeof(T);
-    const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+__device__ void process_tile(SweepSmem<T, A> &c, T *re, T *im, uint64_t t, const char *tables, T *sre, T *sim,
+                             uint32_t form) {
+    const uint32_t size = 1u << (c.L + c.H), vecs = size / (16 / (uint32_t)sizeof(T));
+    const int tid = threadIdx.x;
     const uint64_t base = tile_base(t, c.L, c.hsorted, c.H);
-    if (warp == 0) {
-        if (lane == 0) mbar_expect_tx(&c.bar, 2u * rows * row_bytes);
-        __syncwarp();
-        for (uint32_t r = lane; r < rows; r += 32) {
-            const uint64_t gi = base | row_offset(c, r);
-            bulk_load(sre + (size_t)r * row_elems, re + gi, row_bytes, &c.bar);
-            bulk_load(sim + (size_t)r * row_elems, im + gi, row_bytes, &c.bar);
-        }
-    }
-    // Every thread waits; a timeout anywhere makes all threads leave together.
-    if (!mbar_wait(&c.bar, phase)) {
-        c.fail = 1;
-        c.fail_tile = (uint32_t)t;
-    }
+    tile_load(c, sre, re + base, vecs);
+    tile_load(c, sim, im + base, vecs);
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    if (c.fail) return false;
-    phase ^= 1;
     if constexpr (A == AR_DF) {
         // The slots hold f64, or (form & kFormInDf) the normalised packed
         // pairs the previous sweep left (re slot H, im slot L); on exit f64,
@@ -906,62 +932,29 @@ __device__ bool process_tile(SweepSmem<T, A> &c, T *re, T *im, uint64_t t, const
     } else {
         apply_ops<T, A, T>(sre, sim, c.ops, c.coef, c.nops, base, size, tables, &c.bad, c.jlut, c.gi, nullptr);
     }
-    fence_async_smem();
     __syncthreads();
-    if (warp == 0) {
-        for (uint32_t r = lane; r < rows; r += 32) {
-            const uint64_t gi = base | row_offset(c, r);
-            bulk_store(re + gi, sre + (size_t)r * row_elems, row_bytes);
-            bulk_store(im + gi, sim + (size_t)r * row_elems, row_bytes);
-        }
-        bulk_commit();
-        bulk_wait_read_all();  // the buffer is free once the stores have read it
-    }
-    if (tid == 0) c.done_tiles++;
-    __syncthreads();
-    return true;
+    tile_store(c, re + base, sre, vecs);
+    tile_store(c, im + base, sim, vecs);
+    __syncthreads();  // the buffer is free
 }
 
+// Error record (the first CTA that found a bad index fills it): err[0] = 2;
+// then CTA, L, H, ops and the offending index at 1, 6, 7, 8, 10.
 template <typename T, int A>
-__device__ void sweep_init(SweepSmem<T, A> &c) {
-    if (threadIdx.x == 0) {
-        c.fail = 0;
-        c.fail_tile = c.done_tiles = c.bad = 0;
-        mbar_init(&c.bar, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
+__device__ void sweep_exit(SweepSmem<T, A> &c, int *err) {
     __syncthreads();
-}
-
-// Error record (the first failing CTA fills it): err[0] = 1 wait ran out /
-// 2 index check; then CTA, tile, phase, raw barrier word, L, H, ops, tiles
-// done, offending index.
-template <typename T, int A>
-__device__ void sweep_exit(SweepSmem<T, A> &c, uint32_t phase, int *err) {
-    if (threadIdx.x == 0 && (c.fail || c.bad)) {
-        // Give the loads still in flight a bounded chance to land before exit.
-        if (c.fail) mbar_wait(&c.bar, phase);
-        uint64_t raw;
-        asm volatile("ld.shared.b64 %0, [%1];" : "=l"(raw) : "r"(smem_addr(&c.bar)) : "memory");
-        if (atomicCAS(err, 0, c.fail ? 1 : 2) == 0) {
-            err[1] = (int)blockIdx.x;
-            err[2] = (int)c.fail_tile;
-            err[3] = (int)phase;
-            err[4] = (int)(uint32_t)raw;
-            err[5] = (int)(uint32_t)(raw >> 32);
-            err[6] = (int)c.L;
-            err[7] = (int)c.H;
-            err[8] = c.nops;
-            err[9] = (int)c.done_tiles;
-            err[10] = (int)c.bad;
-            __threadfence();
-        }
+    if (threadIdx.x == 0 && c.bad && atomicCAS(err, 0, 2) == 0) {
+        err[1] = (int)blockIdx.x;
+        err[6] = (int)c.L;
+        err[7] = (int)c.H;
+        err[8] = c.nops;
+        err[10] = (int)c.bad;
+        __threadfence();
     }
-    if (threadIdx.x / 32 == 0) bulk_wait_all();
 }
 
 // One state. One CTA streams tiles through a single shared-memory buffer;
-// three CTAs per SM overlap one tile's TMA traffic with the others' arithmetic.
+// three CTAs per SM overlap one tile's traffic with the others' arithmetic.
 // FORM (g.form as a compile-time constant): each hand-over of double-float
 // pairs between sweeps is its own instantiation, so the tile loop carries no
 // run-time branches for it (they cost registers at the 80-register cap).
@@ -973,12 +966,10 @@ __global__ void __launch_bounds__(kSweepThreads, kSweepCtasPerSm)
     __shared__ SweepSmem<T, A> c;
     T *sre = reinterpret_cast<T *>(smem);
     T *sim = sre + (1u << (g.L + g.H));
-    sweep_init(c);
+    if (threadIdx.x == 0) c.bad = 0;
     load_job(c, gops, nops, g.L, g.H, g.hpos, true);
-    uint32_t phase = 0;
-    for (uint64_t t = blockIdx.x; t < g.ntiles; t += gridDim.x)
-        if (!process_tile(c, re, im, t, tables, sre, sim, phase, FORM)) break;
-    sweep_exit(c, phase, err);
+    for (uint64_t t = blockIdx.x; t < g.ntiles; t += gridDim.x) process_tile(c, re, im, t, tables, sre, sim, FORM);
+    sweep_exit(c, err);
 }
 
 // Many states in one launch (the serving engine's packed step): the tiles
@@ -993,8 +984,7 @@ __global__ void __launch_bounds__(kSweepThreads, kSweepCtasPerSm)
     const SweepJob *jobs = reinterpret_cast<const SweepJob *>(blob + sizeof(SweepBatch));
     const uint32_t njobs = hdr->njobs;
     const uint64_t total = hdr->total_tiles;
-    sweep_init(c);
-    uint32_t phase = 0;
+    if (threadIdx.x == 0) c.bad = 0;
     int cur = -1;
     // Tiles go to CTAs round-robin (concurrent tiles stay adjacent in memory
     // and big and small jobs mix evenly); the job is looked up only when a
@@ -1019,11 +1009,10 @@ __global__ void __launch_bounds__(kSweepThreads, kSweepCtasPerSm)
         const SweepJob &J = jobs[cur];
         T *sre = reinterpret_cast<T *>(smem);
         T *sim = sre + (1u << (J.L + J.H));
-        if (!process_tile(c, reinterpret_cast<T *>(J.re), reinterpret_cast<T *>(J.im), t - J.tile_start,
-                          blob + J.tables_off, sre, sim, phase, 0u))
-            break;
+        process_tile(c, reinterpret_cast<T *>(J.re), reinterpret_cast<T *>(J.im), t - J.tile_start,
+                     blob + J.tables_off, sre, sim, 0u);
     }
-    sweep_exit(c, phase, err);
+    sweep_exit(c, err);
 }
 
 template <typename T, int A, uint32_t FORM>
