@@ -81,6 +81,7 @@ struct GroupInfo {
     uint16_t pm[3];                // load pattern of coordinate g (column g of M, as slots)
     uint16_t trw[4];               // translation patterns
     uint16_t fmask;                // store pattern of the flipped coordinates
+    uint16_t so_step, lo_step, jb_step;  // the kernel's, for a thread's second group (set there)
     uint32_t tab_off;
 };
 

@@ -37,6 +37,21 @@ constexpr uint32_t kJlutLen = 256 + kJlutHigh;
 // CTA's copy of the micro-ops) names its job table, or kNoJobLut.
 constexpr int kJobLuts = 5;
 constexpr uint32_t kNoJobLut = 0xffffffffu;
+// The tile's re array, then, this far behind it whatever the tile's size, im.
+constexpr uint32_t kTileArrayBytes = (uint32_t)(kSweepSmemBytes / 2);
+
+// Where element v of a tile array of ES-byte elements sits: 16-byte vectors
+// stay whole and in their 128-byte row, and the vector's place in the row is
+// XORed with higher index bits. A pass that pairs low index bits otherwise
+// reads with power-of-two strides and hits the same banks: conflicts were
+// 30-45% of the shared-memory wavefronts of a sweep, and those wavefronts are
+// what bounds it (65-84% of peak). The map is linear over XOR and its own
+// inverse: swz(a ^ b) = swz(a) ^ swz(b), swz(swz(v)) = v.
+template <int ES>
+__device__ __forceinline__ uint32_t swz(uint32_t v) {
+    constexpr uint32_t VB = ES == 4 ? 2 : ES == 8 ? 1 : 0;  // elements per vector, log2 (16: vectors themselves)
+    return v ^ ((((v >> (VB + 3)) ^ (v >> (VB + 6))) & 7u) << VB);
+}
 
 // Global index of the first element of tile t: the tile number fills the
 // non-local positions above the L low bits.
@@ -78,54 +93,55 @@ __device__ void apply_perm(T *sr, T *si, const OpHead &op, uint64_t base, uint32
     const int tid = threadIdx.x, nt = blockDim.x;
     constexpr uint32_t VW = 16 / sizeof(T), VB = VW == 4 ? 2 : 1;  // elements per vector, log2
     const uint32_t nv = size / VW;                                   // vectors in the tile
+    constexpr int ES = (int)sizeof(T);
     if (op.kind == MOP_CX && !(op.a & kOuterFlag) && min(op.a, op.b) >= VB) {
         const uint32_t c = op.a - VB, t = op.b - VB, lo = min(c, t), hi = max(c, t);
+        const uint32_t ct = swz<16>(1u << c), tt = swz<16>(1u << t);
         for (uint32_t p = tid; p < nv / 4; p += nt) {
-            const uint32_t v0 = insert_zero32(insert_zero32(p, lo), hi) | (1u << c);
-            swap_vec(sr, si, v0, v0 | (1u << t));
+            const uint32_t v0 = swz<16>(insert_zero32(insert_zero32(p, lo), hi)) ^ ct;
+            swap_vec(sr, si, v0, v0 ^ tt);
         }
         return;
     }
     if (op.kind == MOP_CX && (op.a & kOuterFlag) && op.b >= VB) {
         if (!((base >> (op.a & ~kOuterFlag)) & 1)) return;
-        const uint32_t t = op.b - VB;
+        const uint32_t t = op.b - VB, tt = swz<16>(1u << t);
         for (uint32_t p = tid; p < nv / 2; p += nt) {
-            const uint32_t v0 = insert_zero32(p, t);
-            swap_vec(sr, si, v0, v0 | (1u << t));
+            const uint32_t v0 = swz<16>(insert_zero32(p, t));
+            swap_vec(sr, si, v0, v0 ^ tt);
         }
         return;
     }
     if (op.kind == MOP_SWAP && min(op.a, op.b) >= VB) {
         const uint32_t lo = min(op.a, op.b) - VB, hi = max(op.a, op.b) - VB;
+        const uint32_t tl = swz<16>(1u << lo), th = swz<16>(1u << hi);
         for (uint32_t p = tid; p < nv / 4; p += nt) {
-            const uint32_t v = insert_zero32(insert_zero32(p, lo), hi);
-            swap_vec(sr, si, v | (1u << lo), v | (1u << hi));
+            const uint32_t v = swz<16>(insert_zero32(insert_zero32(p, lo), hi));
+            swap_vec(sr, si, v ^ tl, v ^ th);
         }
         return;
     }
     if (op.kind == MOP_CX) {
-        const uint32_t t = op.b;
+        const uint32_t t = op.b, tt = swz<ES>(1u << t);
         if (op.a & kOuterFlag) {
             if (!((base >> (op.a & ~kOuterFlag)) & 1)) return;
             for (uint32_t p = tid; p < size / 2; p += nt) {
-                const uint32_t v0 = ((p >> t) << (t + 1)) | (p & ((1u << t) - 1));
-                swap_slots(sr, si, v0, v0 | (1u << t));
+                const uint32_t v0 = swz<ES>(insert_zero32(p, t));
+                swap_slots(sr, si, v0, v0 ^ tt);
             }
         } else {
-            const uint32_t c = op.a, lo = min(c, t), hi = max(c, t);
+            const uint32_t c = op.a, lo = min(c, t), hi = max(c, t), ct = swz<ES>(1u << c);
             for (uint32_t p = tid; p < size / 4; p += nt) {
-                uint32_t v = ((p >> lo) << (lo + 1)) | (p & ((1u << lo) - 1));
-                v = ((v >> hi) << (hi + 1)) | (v & ((1u << hi) - 1));
-                const uint32_t v0 = v | (1u << c);
-                swap_slots(sr, si, v0, v0 | (1u << t));
+                const uint32_t v0 = swz<ES>(insert_zero32(insert_zero32(p, lo), hi)) ^ ct;
+                swap_slots(sr, si, v0, v0 ^ tt);
             }
         }
     } else {
         const uint32_t lo = min(op.a, op.b), hi = max(op.a, op.b);
+        const uint32_t tl = swz<ES>(1u << lo), th = swz<ES>(1u << hi);
         for (uint32_t p = tid; p < size / 4; p += nt) {
-            uint32_t v = ((p >> lo) << (lo + 1)) | (p & ((1u << lo) - 1));
-            v = ((v >> hi) << (hi + 1)) | (v & ((1u << hi) - 1));
-            swap_slots(sr, si, v | (1u << lo), v | (1u << hi));
+            const uint32_t v = swz<ES>(insert_zero32(insert_zero32(p, lo), hi));
+            swap_slots(sr, si, v ^ tl, v ^ th);
         }
     }
 }
@@ -313,10 +329,14 @@ __device__ void apply_u1_group(R *sr, R *si, const OpHead *ops, const OpCoef<T, 
     constexpr int E = 1 << G;
     uint32_t bits[G], sorted[G], fmask;
     if (!group_bits<G>(ops, o, size, 0u, bits, sorted, fmask, bad)) return;
+#pragma unroll
+    for (int g = 0; g < G; g++) bits[g] = swz<(int)sizeof(R)>(1u << bits[g]);
+    fmask = swz<(int)sizeof(R)>(fmask);
     for (uint32_t p = threadIdx.x; p < size / E; p += blockDim.x) {
         uint32_t v = p;
 #pragma unroll
         for (int g = 0; g < G; g++) v = ((v >> sorted[g]) << (sorted[g] + 1)) | (v & ((1u << sorted[g]) - 1));
+        v = swz<(int)sizeof(R)>(v);
         // element e of the group sits at v ^ (bits selected by e)
         // (recomputed at the store so the indices need no registers across
         // the arithmetic); flipped elements: slot(e ^ flips) = slot(e) ^ fmask
@@ -324,7 +344,7 @@ __device__ void apply_u1_group(R *sr, R *si, const OpHead *ops, const OpCoef<T, 
             uint32_t w = base_v;
 #pragma unroll
             for (int g = 0; g < G; g++)
-                if ((e >> g) & 1u) w ^= 1u << bits[g];
+                if ((e >> g) & 1u) w ^= bits[g];
             return w;
         };
         R xr[E], xi[E];
@@ -355,16 +375,20 @@ __device__ void apply_u1_group_v2(float *sr, float *si, const OpHead *ops, const
     constexpr int E = 1 << G;
     uint32_t bits[G], sorted[G], fmask;
     if (!group_bits<G>(ops, o, size, 1u, bits, sorted, fmask, bad)) return;
+#pragma unroll
+    for (int g = 0; g < G; g++) bits[g] = swz<8>(1u << bits[g]);  // 8-byte units of a 4-byte array: the same places
+    fmask = swz<8>(fmask);
     float2 *vr = reinterpret_cast<float2 *>(sr), *vi = reinterpret_cast<float2 *>(si);
     for (uint32_t p = threadIdx.x; p < size / 2 / E; p += blockDim.x) {
         uint32_t v = p;
 #pragma unroll
         for (int g = 0; g < G; g++) v = ((v >> sorted[g]) << (sorted[g] + 1)) | (v & ((1u << sorted[g]) - 1));
+        v = swz<8>(v);
         auto slot = [&](uint32_t base_v, uint32_t e) {
             uint32_t w = base_v;
 #pragma unroll
             for (int g = 0; g < G; g++)
-                if ((e >> g) & 1u) w ^= 1u << bits[g];
+                if ((e >> g) & 1u) w ^= bits[g];
             return w;
         };
         float xr[2 * E], xi[2 * E];  // lane 0 (even element) at e, lane 1 at E + e
@@ -388,66 +412,77 @@ __device__ void apply_u1_group_v2(float *sr, float *si, const OpHead *ops, const
     }
 }
 
-// One pass (see GroupInfo) of a double-float sweep. The descriptor's fields
-// are read from shared memory where they are used, which keeps the 80-register
-// budget for the group's amplitudes. xr / xi hold the packed pairs H / L;
-// the rotations run as f32x2 arithmetic.
+// One pass (see GroupInfo) of a double-float sweep. xr / xi hold the packed
+// pairs H / L; the rotations run as f32x2 arithmetic.
+// Every index a thread needs (its slot, its load slot under the folded CX
+// block, its table entry) is linear over XOR in the group number p, so it is
+// worked out once per pass, as byte offsets, and a group of three bits (two
+// groups per thread) steps to its second group by XORing the descriptor's
+// step patterns; the im array sits a fixed distance behind re. Index work was
+// half of a pass's instructions when it was redone per group and element.
 // in_f64 / out_f64: the slots hold f64 on entry / must hold f64 on exit (the
 // sweep's first / last pass does the tile's conversion in registers).
 template <typename T, int A, int G, bool ROT_ONLY, bool HAS_DK, bool HAS_CX>
-__device__ void run_pass(const GroupInfo &gi, float2 *sr, float2 *si, const OpHead *ops, const OpCoef<T, A> *coef,
-                         uint32_t size, const char *tables, uint64_t base, bool in_f64, bool out_f64) {
+__device__ void run_pass(const GroupInfo &gi, char *tile, const OpHead *ops, const OpCoef<T, A> *coef, uint32_t size,
+                         const char *tables, uint64_t base, bool in_f64, bool out_f64) {
     constexpr int E = 1 << G;
     const int o = gi.first;
     uint32_t jo = 0, u0 = 0;
     if constexpr (HAS_DK) {
-        for (int i = 0; i < gi.nout; i++) jo |= (uint32_t)((base >> gi.outq[i]) & 1u) << gi.outb[i];
+        for (int i = 0; i < gi.nout; i++) jo |= (uint32_t)((base >> gi.outq[i]) & 1u) << (gi.outb[i] + 4);
     }
     if constexpr (HAS_CX) {
         for (int t = 0; t < gi.ntr; t++)
             if ((gi.trc[t] & 0x80u) && ((base >> (gi.trc[t] & 0x7fu)) & 1u)) u0 ^= gi.trw[t];
     }
-    for (uint32_t p = threadIdx.x; p < size / E; p += blockDim.x) {
-        uint32_t v = p;
+    uint32_t so = 0, lo = 0, jb = 0;  // slot, load slot, table entry of element 0, in bytes
+    for (uint32_t p = threadIdx.x; p < size / E; p += kSweepThreads) {
+        if (G == 3 && p >= kSweepThreads) {  // at most one step: tiles have 2^12 elements
+            so ^= gi.so_step;
+            lo ^= gi.lo_step;
+            jb ^= gi.jb_step;
+        } else {
+            uint32_t v = p;
 #pragma unroll
-        for (int g = 0; g < G; g++) {
-            const uint32_t s = gi.sorted[g];
-            v = ((v >> s) << (s + 1)) | (v & ((1u << s) - 1));
+            for (int g = 0; g < G; g++) v = insert_zero32(v, gi.sorted[g]);
+            so = lo = swz<8>(v) << 3;
+            if constexpr (HAS_CX) {  // the descriptor's slot patterns are byte offsets of swizzled slots
+                lo ^= u0;
+                for (int t = 0; t < gi.ntr; t++)
+                    if (!(gi.trc[t] & 0x80u) && ((v >> gi.trc[t]) & 1u)) lo ^= gi.trw[t];
+            }
+            if constexpr (HAS_DK) {
+                jb = jo;
+                for (int i = 0; i < gi.nloc; i++) jb |= ((v >> gi.loc[i]) & 1u) << (gi.locb[i] + 4);
+            }
         }
         float2 xr[E], xi[E];
-        {
-            uint32_t lv = v;
-            if constexpr (HAS_CX) {
-                lv ^= u0;
-                for (int t = 0; t < gi.ntr; t++)
-                    if (!(gi.trc[t] & 0x80u) && ((v >> gi.trc[t]) & 1u)) lv ^= gi.trw[t];
-            }
 #pragma unroll
-            for (int e = 0; e < E; e++) {
-                uint32_t w = lv;
+        for (int e = 0; e < E; e++) {
+            uint32_t w = lo;
 #pragma unroll
-                for (int g = 0; g < G; g++)
-                    if ((e >> g) & 1) w ^= HAS_CX ? gi.pm[g] : gi.gm[g];
-                if (in_f64) {
-                    pk_from_f64(reinterpret_cast<const double *>(sr)[w], reinterpret_cast<const double *>(si)[w],
-                                xr[e], xi[e]);
-                } else {
-                    xr[e] = sr[w];
-                    xi[e] = si[w];
-                }
+            for (int g = 0; g < G; g++)
+                if ((e >> g) & 1) w ^= HAS_CX ? gi.pm[g] : gi.gm[g];
+            if (in_f64) {
+                pk_from_f64(*reinterpret_cast<const double *>(tile + w),
+                            *reinterpret_cast<const double *>(tile + kTileArrayBytes + w), xr[e], xi[e]);
+            } else {
+                xr[e] = *reinterpret_cast<const float2 *>(tile + w);
+                xi[e] = *reinterpret_cast<const float2 *>(tile + kTileArrayBytes + w);
             }
         }
         if constexpr (HAS_DK) {
-            const float4 *dtab = reinterpret_cast<const float4 *>(tables + gi.tab_off);
-            uint32_t jb = jo;
-            for (int i = 0; i < gi.nloc; i++) jb |= ((v >> gi.loc[i]) & 1u) << gi.locb[i];
+            const char *dtab = tables + gi.tab_off;
+            uint32_t tm[G];
+#pragma unroll
+            for (int g = 0; g < G; g++) tm[g] = gi.tb[g] != 0xff ? 16u << gi.tb[g] : 0u;
 #pragma unroll
             for (int e = 0; e < E; e++) {
                 uint32_t j = jb;
 #pragma unroll
                 for (int g = 0; g < G; g++)
-                    if (((e >> g) & 1) && gi.tb[g] != 0xff) j ^= 1u << gi.tb[g];
-                const float4 w = __ldg(dtab + j);
+                    if ((e >> g) & 1) j ^= tm[g];
+                const float4 w = __ldg(reinterpret_cast<const float4 *>(dtab + j));
                 float2 ar, ai;  // scalar: the packed form needs eight registers per entry
                 pk_split(xr[e], xi[e], ar, ai);
                 cscale_df_u(make_float2(w.x, w.y), make_float2(w.z, w.w), ar, ai);
@@ -481,35 +516,36 @@ __device__ void run_pass(const GroupInfo &gi, float2 *sr, float2 *si, const OpHe
                     if (!((e >> g) & 1)) hl_udf(m, xr[e], xi[e], xr[e | (1 << g)], xi[e | (1 << g)]);
             }
         }
-        const uint32_t vs = v ^ gi.fmask;
+        const uint32_t fo = so ^ gi.fmask;
 #pragma unroll
         for (int e = 0; e < E; e++) {
-            uint32_t w = vs;
+            uint32_t w = fo;
 #pragma unroll
             for (int g = 0; g < G; g++)
                 if ((e >> g) & 1) w ^= gi.gm[g];
             if (out_f64) {
-                pk_to_f64(xr[e], xi[e], reinterpret_cast<double *>(sr)[w], reinterpret_cast<double *>(si)[w]);
+                pk_to_f64(xr[e], xi[e], *reinterpret_cast<double *>(tile + w),
+                          *reinterpret_cast<double *>(tile + kTileArrayBytes + w));
             } else {  // the next pass accepts unnormalised pairs
-                sr[w] = xr[e];
-                si[w] = xi[e];
+                *reinterpret_cast<float2 *>(tile + w) = xr[e];
+                *reinterpret_cast<float2 *>(tile + kTileArrayBytes + w) = xi[e];
             }
         }
     }
 }
 
 template <typename T, int A, int G, bool ROT_ONLY>
-__device__ void run_pass_any(const GroupInfo &gi, float2 *sr, float2 *si, const OpHead *ops,
+__device__ void run_pass_any(const GroupInfo &gi, char *tile, const OpHead *ops,
                              const OpCoef<T, A> *coef, uint32_t size, const char *tables, uint64_t base, bool in_f64,
                              bool out_f64) {
     const bool cx = gi.ntr || gi.pm[0] != gi.gm[0] || (G > 1 && gi.pm[G - 1] != gi.gm[G - 1]) ||
                     (G > 2 && gi.pm[1] != gi.gm[1]);
     if (gi.has_dk) {
-        if (cx) run_pass<T, A, G, ROT_ONLY, true, true>(gi, sr, si, ops, coef, size, tables, base, in_f64, out_f64);
-        else run_pass<T, A, G, ROT_ONLY, true, false>(gi, sr, si, ops, coef, size, tables, base, in_f64, out_f64);
+        if (cx) run_pass<T, A, G, ROT_ONLY, true, true>(gi, tile, ops, coef, size, tables, base, in_f64, out_f64);
+        else run_pass<T, A, G, ROT_ONLY, true, false>(gi, tile, ops, coef, size, tables, base, in_f64, out_f64);
     } else {
-        if (cx) run_pass<T, A, G, ROT_ONLY, false, true>(gi, sr, si, ops, coef, size, tables, base, in_f64, out_f64);
-        else run_pass<T, A, G, ROT_ONLY, false, false>(gi, sr, si, ops, coef, size, tables, base, in_f64, out_f64);
+        if (cx) run_pass<T, A, G, ROT_ONLY, false, true>(gi, tile, ops, coef, size, tables, base, in_f64, out_f64);
+        else run_pass<T, A, G, ROT_ONLY, false, false>(gi, tile, ops, coef, size, tables, base, in_f64, out_f64);
     }
 }
 
@@ -528,11 +564,11 @@ __device__ void apply_ops(R *sr, R *si, const OpHead *ops, const OpCoef<T, A> *c
             if (gi.G) {
                 const bool in_f64 = o == 0 && fuse_in, out_f64 = o + gi.skip == nops && fuse_out;
                 if (gi.rot3)
-                    run_pass_any<T, A, 3, true>(gi, sr, si, ops, coef, size, tables, base, in_f64, out_f64);
+                    run_pass_any<T, A, 3, true>(gi, reinterpret_cast<char *>(sr), ops, coef, size, tables, base, in_f64, out_f64);
                 else if (gi.G == 2)
-                    run_pass_any<T, A, 2, false>(gi, sr, si, ops, coef, size, tables, base, in_f64, out_f64);
+                    run_pass_any<T, A, 2, false>(gi, reinterpret_cast<char *>(sr), ops, coef, size, tables, base, in_f64, out_f64);
                 else
-                    run_pass_any<T, A, 1, false>(gi, sr, si, ops, coef, size, tables, base, in_f64, out_f64);
+                    run_pass_any<T, A, 1, false>(gi, reinterpret_cast<char *>(sr), ops, coef, size, tables, base, in_f64, out_f64);
                 o += gi.skip - 1;
                 __syncthreads();
                 continue;
@@ -574,12 +610,12 @@ __device__ void apply_ops(R *sr, R *si, const OpHead *ops, const OpCoef<T, A> *c
                 __syncthreads();
                 continue;
             }
-            const uint32_t b = op.a;
+            const uint32_t b = op.a, bs = swz<(int)sizeof(R)>(1u << b);
             if (op.kind == MOP_RT) {
                 const R t = coef[o].v[0];
-                const uint32_t flip = op.b ? 1u << b : 0u;
+                const uint32_t flip = op.b ? bs : 0u;
                 for (uint32_t p = tid; p < size / 2; p += nt) {
-                    const uint32_t v0 = ((p >> b) << (b + 1)) | (p & ((1u << b) - 1)), v1 = v0 | (1u << b);
+                    const uint32_t v0 = swz<(int)sizeof(R)>(insert_zero32(p, b)), v1 = v0 ^ bs;
                     R ar = sr[v0], ai = si[v0], br = sr[v1], bi = si[v1];
                     if constexpr (A == AR_DF) hl_rot_df(t, ar, ai, br, bi);
                     else pair_update_rot<T>(t, ar, ai, br, bi);
@@ -596,7 +632,7 @@ __device__ void apply_ops(R *sr, R *si, const OpHead *ops, const OpCoef<T, A> *c
 #pragma unroll
                 for (int i = 0; i < 4; i++) r[i] = coef[o].v[i];
                 for (uint32_t p = tid; p < size / 2; p += nt) {
-                    const uint32_t v0 = ((p >> b) << (b + 1)) | (p & ((1u << b) - 1)), v1 = v0 | (1u << b);
+                    const uint32_t v0 = swz<(int)sizeof(R)>(insert_zero32(p, b)), v1 = v0 ^ bs;
                     if constexpr (A == AR_DF) hl_rdf(r, sr[v0], si[v0], sr[v1], si[v1]);
                     else pair_update_real<T>(r, sr[v0], si[v0], sr[v1], si[v1]);
                 }
@@ -611,7 +647,7 @@ __device__ void apply_ops(R *sr, R *si, const OpHead *ops, const OpCoef<T, A> *c
                 else pair_update<T, A == AR_EXACT>(m, ar, ai, br, bi);
             };
             for (uint32_t p = tid; p < size / 2; p += nt) {
-                const uint32_t v0 = ((p >> b) << (b + 1)) | (p & ((1u << b) - 1)), v1 = v0 | (1u << b);
+                const uint32_t v0 = swz<(int)sizeof(R)>(insert_zero32(p, b)), v1 = v0 ^ bs;
                 upd(sr[v0], si[v0], sr[v1], si[v1]);
             }
         } else if (op.kind == MOP_D1) {
@@ -626,9 +662,10 @@ __device__ void apply_ops(R *sr, R *si, const OpHead *ops, const OpCoef<T, A> *c
                 float4 *vr = reinterpret_cast<float4 *>(sr), *vi = reinterpret_cast<float4 *>(si);
                 for (uint32_t q = tid; q < size / 4; q += nt) {
                     const float4 a = vr[q], b = vi[q];
+                    const uint32_t v0 = 4 * swz<16>(q);  // the elements this vector holds
                     R xr[4] = {a.x, a.y, a.z, a.w}, xi[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
-                    for (int k = 0; k < 4; k++) scl(4 * q + k, xr[k], xi[k]);
+                    for (int k = 0; k < 4; k++) scl(v0 + k, xr[k], xi[k]);
                     vr[q] = make_float4(xr[0], xr[1], xr[2], xr[3]);
                     vi[q] = make_float4(xi[0], xi[1], xi[2], xi[3]);
                 }
@@ -643,12 +680,12 @@ __device__ void apply_ops(R *sr, R *si, const OpHead *ops, const OpCoef<T, A> *c
                     }
 #pragma unroll
                     for (int k = 0; k < 4; k++) {
-                        scl(v + k * nt, xr[k], xi[k]);
+                        scl(swz<(int)sizeof(R)>(v + k * nt), xr[k], xi[k]);
                         sr[v + k * nt] = xr[k];
                         si[v + k * nt] = xi[k];
                     }
                 }
-                for (; v < size; v += nt) scl(v, sr[v], si[v]);
+                for (; v < size; v += nt) scl(swz<(int)sizeof(R)>(v), sr[v], si[v]);
             }
         } else if (op.kind == MOP_DK) {
             const uint32_t jo = jouter(op, base);
@@ -685,7 +722,7 @@ __device__ void apply_ops(R *sr, R *si, const OpHead *ops, const OpCoef<T, A> *c
             if constexpr (sizeof(R) == 4) {  // four consecutive elements per 16-byte vector
                 float4 *vr = reinterpret_cast<float4 *>(sr), *vi = reinterpret_cast<float4 *>(si);
                 for (uint32_t q = tid; q < size / 4; q += nt) {
-                    const uint32_t v0 = 4 * q, jh = jo | lut[256 + (v0 >> 8)];  // same high bits for all four
+                    const uint32_t v0 = 4 * swz<16>(q), jh = jo | lut[256 + (v0 >> 8)];  // same high bits for all four
                     W wr[4], wi[4];
 #pragma unroll
                     for (int k = 0; k < 4; k++) load_w(jh | lut[(v0 & 255u) + k], wr[k], wi[k]);
@@ -703,11 +740,11 @@ __device__ void apply_ops(R *sr, R *si, const OpHead *ops, const OpCoef<T, A> *c
                     W wr[4], wi[4];
 #pragma unroll
                     for (int k = 0; k < 4; k++) {
-                        const uint32_t vk = v + k * nt;
+                        const uint32_t vk = swz<(int)sizeof(R)>(v + k * nt);
                         const uint32_t j = jo | lut[vk & 255u] | lut[256 + (vk >> 8)];
                         load_w(j, wr[k], wi[k]);
-                        xr[k] = sr[vk];
-                        xi[k] = si[vk];
+                        xr[k] = sr[v + k * nt];
+                        xi[k] = si[v + k * nt];
                     }
 #pragma unroll
                     for (int k = 0; k < 4; k++) {
@@ -717,7 +754,8 @@ __device__ void apply_ops(R *sr, R *si, const OpHead *ops, const OpCoef<T, A> *c
                     }
                 }
                 for (; v < size; v += nt) {
-                    const uint32_t j = jo | lut[v & 255u] | lut[256 + (v >> 8)];
+                    const uint32_t vk = swz<(int)sizeof(R)>(v);
+                    const uint32_t j = jo | lut[vk & 255u] | lut[256 + (vk >> 8)];
                     W wr, wi;
                     load_w(j, wr, wi);
                     scl(wr, wi, sr[v], si[v]);
@@ -812,6 +850,28 @@ __device__ void load_job(SweepSmem<T, A> &c, const MicroOp *gops, int nops, uint
             plan_passes(c.ops, nops, L + H, fold, max_group_of<T, A>(), c.gi, &c.bad, &c.fuse_in, &c.fuse_out);
     }
     __syncthreads();
+    if constexpr (A == AR_DF) {  // slot patterns as byte offsets into the swizzled tile, step patterns
+        if (tid < nops) {
+            GroupInfo &q = c.gi[tid];
+            if (q.G) {
+                for (int g = 0; g < q.G; g++) {
+                    q.gm[g] = (uint16_t)(swz<8>(q.gm[g]) << 3);
+                    q.pm[g] = (uint16_t)(swz<8>(q.pm[g]) << 3);
+                }
+                for (int i = 0; i < q.ntr; i++) q.trw[i] = (uint16_t)(swz<8>(q.trw[i]) << 3);
+                q.fmask = (uint16_t)(swz<8>(q.fmask) << 3);
+                uint32_t v = kSweepThreads, lo = 0, jb = 0;  // group number p + kSweepThreads against p
+                for (int g = 0; g < q.G; g++) v = insert_zero32(v, q.sorted[g]);
+                for (int i = 0; i < q.ntr; i++)
+                    if (!(q.trc[i] & 0x80u) && ((v >> q.trc[i]) & 1u)) lo ^= q.trw[i];
+                for (int i = 0; i < q.nloc; i++) jb |= ((v >> q.loc[i]) & 1u) << (q.locb[i] + 4);
+                q.so_step = (uint16_t)(swz<8>(v) << 3);
+                q.lo_step = (uint16_t)(q.so_step ^ lo);
+                q.jb_step = (uint16_t)jb;
+            }
+        }
+        __syncthreads();
+    }
     if constexpr (A != AR_DF) {  // the job's diagonal index tables, once per job
         for (int o = 0; o < nops; o++) {
             const OpHead &op = c.ops[o];
@@ -839,7 +899,7 @@ __device__ __forceinline__ void tile_load(const SweepSmem<T, A> &c, T *dst, cons
     }
     for (uint32_t i = threadIdx.x; i < vecs; i += kSweepThreads) {
         const T *g = src + ((size_t)c.rows[i >> lv] << c.L) + (size_t)(i & cm) * VW;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16 * i), "l"(g) : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16 * swz<16>(i)), "l"(g) : "memory");
     }
 }
 template <typename T, int A>
@@ -858,11 +918,11 @@ __device__ __forceinline__ void tile_store(const SweepSmem<T, A> &c, T *dst, con
     for (; i + 3 * kSweepThreads < vecs; i += 4 * kSweepThreads) {
         uint4 x[4];
 #pragma unroll
-        for (int k = 0; k < 4; k++) x[k] = sv[i + k * kSweepThreads];
+        for (int k = 0; k < 4; k++) x[k] = sv[swz<16>(i + k * kSweepThreads)];
 #pragma unroll
         for (int k = 0; k < 4; k++) *at(i + k * kSweepThreads) = x[k];
     }
-    for (; i < vecs; i += kSweepThreads) *at(i) = sv[i];
+    for (; i < vecs; i += kSweepThreads) *at(i) = sv[swz<16>(i)];
 }
 
 // All threads: one tile of the current job — load, micro-ops in shared
@@ -962,10 +1022,10 @@ template <typename T, int A, uint32_t FORM>
 __global__ void __launch_bounds__(kSweepThreads, kSweepCtasPerSm)
     k_sweep(T *__restrict__ re, T *__restrict__ im, const SweepGeom g, const MicroOp *__restrict__ gops, int nops,
             const char *__restrict__ tables, int *__restrict__ err) {
-    extern __shared__ __align__(1024) unsigned char smem[];
+    extern __shared__ __align__(128) unsigned char smem[];
     __shared__ SweepSmem<T, A> c;
     T *sre = reinterpret_cast<T *>(smem);
-    T *sim = sre + (1u << (g.L + g.H));
+    T *sim = sre + kTileArrayBytes / sizeof(T);
     if (threadIdx.x == 0) c.bad = 0;
     load_job(c, gops, nops, g.L, g.H, g.hpos, true);
     for (uint64_t t = blockIdx.x; t < g.ntiles; t += gridDim.x) process_tile(c, re, im, t, tables, sre, sim, FORM);
@@ -978,7 +1038,7 @@ __global__ void __launch_bounds__(kSweepThreads, kSweepCtasPerSm)
 template <typename T, int A>
 __global__ void __launch_bounds__(kSweepThreads, kSweepCtasPerSm)
     k_sweep_multi(const char *__restrict__ blob, int *__restrict__ err) {
-    extern __shared__ __align__(1024) unsigned char smem[];
+    extern __shared__ __align__(128) unsigned char smem[];
     __shared__ SweepSmem<T, A> c;
     const SweepBatch *hdr = reinterpret_cast<const SweepBatch *>(blob);
     const SweepJob *jobs = reinterpret_cast<const SweepJob *>(blob + sizeof(SweepBatch));
@@ -1008,7 +1068,7 @@ __global__ void __launch_bounds__(kSweepThreads, kSweepCtasPerSm)
         }
         const SweepJob &J = jobs[cur];
         T *sre = reinterpret_cast<T *>(smem);
-        T *sim = sre + (1u << (J.L + J.H));
+        T *sim = sre + kTileArrayBytes / sizeof(T);
         process_tile(c, reinterpret_cast<T *>(J.re), reinterpret_cast<T *>(J.im), t - J.tile_start,
                      blob + J.tables_off, sre, sim, 0u);
     }
@@ -1027,7 +1087,7 @@ int run_sweep_form(zc_state *st, const SweepGeom &g, const MicroOp *dev_ops, int
     if (smem > kSweepSmemBytes || g.H > kMaxSweepHigh || nops > kMaxMicroOps)
         return fail(ZC_ERR_INVALID, "sweep shape exceeds the kernel's limits");
     const uint64_t blocks = std::min<uint64_t>(g.ntiles, (uint64_t)st->num_sms * kSweepCtasPerSm);
-    k_sweep<T, A, FORM><<<(int)blocks, kSweepThreads, smem, st->stream>>>((T *)st->re, (T *)st->im, g, dev_ops,
+    k_sweep<T, A, FORM><<<(int)blocks, kSweepThreads, kSweepSmemBytes, st->stream>>>((T *)st->re, (T *)st->im, g, dev_ops,
                                                                              nops, dev_tables, st->d_err);
     ZC_CUDA(cudaGetLastError());
     return ZC_OK;
