@@ -480,13 +480,14 @@ static int run_one_sweep(zc_state *st) {
         q.erase(q.begin());
         return rc;
     }
-    const size_t ops_bytes = plan.mops.size() * sizeof(MicroOp);
-    const size_t tab_off = (ops_bytes + 255) & ~(size_t)255;
-    std::vector<char> blob(tab_off + plan.tables.size());
-    memcpy(blob.data(), plan.mops.data(), ops_bytes);
+    std::vector<char> blob;
+    int rc = encode_job(st->prec, exact(st), plan, &blob);
+    if (rc) return rc;
+    const size_t tab_off = (blob.size() + 255) & ~(size_t)255;
+    blob.resize(tab_off + plan.tables.size());
     if (!plan.tables.empty()) memcpy(blob.data() + tab_off, plan.tables.data(), plan.tables.size());
     const void *dev = nullptr;
-    int rc = arena_put(st, blob.data(), blob.size(), &dev);
+    rc = arena_put(st, blob.data(), blob.size(), &dev);
     if (rc) return rc;
     consume_plan(q, plan);
     // Fast f64: consecutive sweeps of one flush hand the state over as
@@ -495,8 +496,7 @@ static int run_one_sweep(zc_state *st) {
     const bool df = st->prec == 64 && !exact(st);
     const bool out_df = df && !q.empty() && sweepable(q.front());
     plan.g.form = (st->df_resident ? kFormInDf : 0u) | (out_df ? kFormOutDf : 0u);
-    rc = launch_sweep(st, plan.g, (const MicroOp *)dev, (int)plan.mops.size(), (const char *)dev + tab_off,
-                      exact(st));
+    rc = launch_sweep(st, plan.g, (const char *)dev, (const char *)dev + tab_off, exact(st));
     st->df_resident = out_df;
     for (const MicroOp &m : plan.mops) st->ctr.micro_ops[m.kind & 7]++;
     return rc;

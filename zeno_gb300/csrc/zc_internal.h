@@ -182,8 +182,9 @@ int launch_sweep_multi(cudaStream_t stream, int num_sms, int prec, bool exact, c
 int arena_put(zc_state *st, const void *src, size_t bytes, const void **dev);
 // Round an f64 state left as double-float pairs (g.form kFormOutDf) back to f64.
 int launch_df_to_f64(zc_state *st);
-int launch_sweep(zc_state *st, const SweepGeom &g, const MicroOp *dev_ops, int nops, const char *dev_tables,
-                 bool exact);
+// The plan's job block for the sweep kernels (JobHead).
+int encode_job(int prec, bool exact, const SweepPlan &plan, std::vector<char> *out);
+int launch_sweep(zc_state *st, const SweepGeom &g, const char *dev_job, const char *dev_tables, bool exact);
 struct TrajRec;
 struct TrajNoise;
 struct TrajPlan;

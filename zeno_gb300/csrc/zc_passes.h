@@ -1,7 +1,7 @@
 // Register passes of double-float sweeps: the micro-op head the tile loop
 // reads, the pass descriptor and the planning of the passes of a job. Shared
-// by the sweep kernel (zc_sweep.cu, one thread per CTA per job) and the host
-// check of the pass logic (tests/passes_harness.cpp).
+// by the sweep kernel (zc_sweep.cu) and the host check of the pass logic
+// (tests/passes_harness.cpp).
 #pragma once
 #include <stddef.h>
 #include <stdint.h>
@@ -10,10 +10,8 @@
 
 #ifdef __CUDACC__
 #define ZC_HD __host__ __device__ __forceinline__
-#define ZC_HD_NOINLINE __host__ __device__ __noinline__
 #else
 #define ZC_HD inline
-#define ZC_HD_NOINLINE inline
 #endif
 
 namespace zc {
@@ -21,7 +19,7 @@ namespace zc {
 constexpr int kMaxFoldCx = 4;  // CX ops one register group takes into its loads
 
 // The part of a MicroOp the tile loop reads (its first 72 bytes); the matrix
-// entries are read once per job, from global memory, into the coefficients.
+// entries go into the job's coefficients.
 struct OpHead {
     uint32_t kind, a, b, k;
     uint32_t loc[12];
@@ -67,8 +65,8 @@ ZC_HD int group_at(const OpHead *ops, int o, int nops, int max_group, bool *rot3
 // pi_1(pi_2(...pi_n(y))), pi_i flipping the target where the control is
 // set. Over GF(2) that is y -> M y + sum_i ctl_i(v) w_i: controls among the
 // group bits make M, controls outside them (local bits of v, or outer qubits
-// fixed per tile) add the translations w_i. One thread derives all of it in
-// load_job; per tile a pass reads a few shared words.
+// fixed per tile) add the translations w_i. The host derives all of it per
+// job (encode_job); per tile a pass reads a few shared words.
 struct GroupInfo {
     uint8_t G, rot3, skip, first;  // G = 0: no pass starts at this op
     uint8_t nloc, nout, ntr, has_dk;
@@ -81,17 +79,16 @@ struct GroupInfo {
     uint16_t pm[3];                // load pattern of coordinate g (column g of M, as slots)
     uint16_t trw[4];               // translation patterns
     uint16_t fmask;                // store pattern of the flipped coordinates
-    uint16_t so_step, lo_step, jb_step;  // the kernel's, for a thread's second group (set there)
+    uint16_t so_step, lo_step, jb_step;  // for a thread's second group (set by encode_job)
     uint32_t tab_off;
 };
 
-// One thread: walk the ops the way apply_ops will and describe each pass
+// Walk the ops the way apply_ops will and describe each pass
 // (max_group: the kernel's register group size). *fuse_in / *fuse_out: the
 // job starts / ends with a pass, which then also converts the tile between
 // f64 and double-float in registers.
-// (Out of line on the device: one thread runs it once per job.)
-ZC_HD_NOINLINE void plan_passes(const OpHead *ops, int nops, uint32_t tile_log2, bool fold, int max_group,
-                                       GroupInfo *gi, uint32_t *bad, int *fuse_in, int *fuse_out) {
+inline void plan_passes(const OpHead *ops, int nops, uint32_t tile_log2, bool fold, int max_group, GroupInfo *gi,
+                        uint32_t *bad, int *fuse_in, int *fuse_out) {
     for (int i = 0; i < nops; i++) gi[i].G = 0;
     *fuse_out = 0;
     int o = 0;

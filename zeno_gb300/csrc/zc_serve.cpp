@@ -156,7 +156,7 @@ int packed_step(zc_server *s, int gi, int round, int *issued) {
     const int prec = gi ? 64 : 32;
     const bool ex = (s->flags & ZC_FLAG_FAST) == 0;
     std::vector<SweepJob> jobs;
-    std::vector<char> body;  // micro-ops + tables, offsets relative to the body
+    std::vector<char> body, blk;  // job blocks + tables, offsets relative to the body
     std::vector<std::pair<Request *, SweepPlan>> planned;
     uint64_t tiles = 0;
     for (Request *r : s->active) {
@@ -179,17 +179,15 @@ int packed_step(zc_server *s, int gi, int round, int *issued) {
         SweepJob j{};
         j.re = r->view.re;
         j.im = r->view.im;
-        j.L = plan.g.L;
-        j.H = plan.g.H;
-        j.nops = (uint32_t)plan.mops.size();
-        for (uint32_t k = 0; k < plan.g.H && k < 8; k++) j.hpos[k] = plan.g.hpos[k];
         j.ntiles = plan.g.ntiles;
         j.tile_start = tiles;
         tiles += plan.g.ntiles;
         size_t off = (body.size() + 15) & ~(size_t)15;
-        body.resize(off + plan.mops.size() * sizeof(MicroOp));
-        memcpy(body.data() + off, plan.mops.data(), plan.mops.size() * sizeof(MicroOp));
-        j.ops_off = off;
+        int rc = encode_job(prec, ex, plan, &blk);
+        if (rc) return rc;
+        body.resize(off + blk.size());
+        memcpy(body.data() + off, blk.data(), blk.size());
+        j.job_off = off;
         off = (body.size() + 15) & ~(size_t)15;
         body.resize(off + plan.tables.size());
         if (!plan.tables.empty()) memcpy(body.data() + off, plan.tables.data(), plan.tables.size());
@@ -203,7 +201,7 @@ int packed_step(zc_server *s, int gi, int round, int *issued) {
     const size_t total = body_off + body.size();
     if (total > kBlobBytes) return fail(ZC_ERR_INVALID, "packed launch exceeds its parameter buffer");
     for (auto &j : jobs) {
-        j.ops_off += body_off;
+        j.job_off += body_off;
         j.tables_off += body_off;
     }
     SweepBatch hdr{(uint32_t)jobs.size(), 0, tiles};

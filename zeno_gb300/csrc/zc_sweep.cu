@@ -14,8 +14,10 @@
 // Which ops fit a sweep: unitaries whose qubits are all local; diagonals
 // on any qubits (bits of non-local qubits are constant per tile); CX with a
 // local target and any control; SWAP of two local qubits.
-#include <atomic>
+#include <string.h>
+
 #include <algorithm>
+#include <atomic>
 
 #include "zc_arith.cuh"
 #include "zc_async.cuh"
@@ -48,7 +50,7 @@ constexpr uint32_t kTileArrayBytes = (uint32_t)(kSweepSmemBytes / 2);
 // what bounds it (65-84% of peak). The map is linear over XOR and its own
 // inverse: swz(a ^ b) = swz(a) ^ swz(b), swz(swz(v)) = v.
 template <int ES>
-__device__ __forceinline__ uint32_t swz(uint32_t v) {
+__host__ __device__ __forceinline__ uint32_t swz(uint32_t v) {
     constexpr uint32_t VB = ES == 4 ? 2 : ES == 8 ? 1 : 0;  // elements per vector, log2 (16: vectors themselves)
     return v ^ ((((v >> (VB + 3)) ^ (v >> (VB + 6))) & 7u) << VB);
 }
@@ -80,7 +82,7 @@ __device__ __forceinline__ void swap_vec(void *sr, void *si, uint32_t v0, uint32
     i[v1] = c;
 }
 
-__device__ __forceinline__ uint32_t insert_zero32(uint32_t v, uint32_t b) {
+__host__ __device__ __forceinline__ uint32_t insert_zero32(uint32_t v, uint32_t b) {
     return ((v >> b) << (b + 1)) | (v & ((1u << b) - 1));
 }
 
@@ -775,112 +777,129 @@ struct SweepSmem {
     OpHead ops[kMaxMicroOps];
     OpCoef<T, A> coef[kMaxMicroOps];
     uint32_t rows[1u << kMaxSweepHigh];  // row r of a tile starts at element rows[r] << L of it
-    uint32_t hsorted[8];                 // the high qubits ascending (tile base)
-    int nops;
-    uint32_t L, H;
-    int has_arith;
+    JobHead job;
     uint32_t bad;
     uint16_t jlut[kJlutLen];  // diagonal index tables of the current DK op
     // register passes (double-float sweeps), or the job's diagonal index tables
-    typename std::conditional<A == AR_DF, GroupInfo[kMaxMicroOps], uint16_t[kJobLuts * kJlutLen]>::type gi;
-    int fuse_in, fuse_out;  // the first / last pass converts the tile
+    alignas(16) typename std::conditional<A == AR_DF, GroupInfo[kMaxMicroOps], uint16_t[kJobLuts * kJlutLen]>::type gi;
 };
 static_assert(sizeof(uint16_t[kJobLuts * kJlutLen]) <= sizeof(GroupInfo[kMaxMicroOps]),
               "job index tables fit where the pass descriptors go");
+static_assert(sizeof(OpHead[kMaxMicroOps]) % 16 == 0 && sizeof(GroupInfo[kMaxMicroOps]) % 16 == 0,
+              "job sections are copied in 16-byte pieces");
 
-// All threads: make (gops, nops, L, H, hpos) the CTA's current job.
+// A job's block for the kernel (see JobHead). Everything that depends on the
+// job alone is worked out here, once: a CTA of a small or mid-size state has
+// one tile, and the passes resolved there by one thread took longer than the
+// tile (a 4-qubit double-float sweep: 95 us; a 19-qubit one 52 us).
 template <typename T, int A>
-__device__ void load_job(SweepSmem<T, A> &c, const MicroOp *gops, int nops, uint32_t L, uint32_t H,
-                         const uint32_t *hpos, bool fold) {
+int encode_job_as(const SweepPlan &plan, std::vector<char> *out) {
+    const int nops = (int)plan.mops.size();
+    JobHead h{};
+    h.nops = (uint32_t)nops;
+    h.L = plan.g.L;
+    h.H = plan.g.H;
+    for (uint32_t j = 0; j < h.H && j < 8; j++) h.hpos[j] = plan.g.hpos[j];
+    std::vector<OpHead> ops((size_t)nops);
+    std::vector<OpCoef<T, A>> coef((size_t)nops);
+    uint32_t nlut = 0;
+    for (int o = 0; o < nops; o++) {
+        const MicroOp &m = plan.mops[(size_t)o];
+        memcpy(&ops[(size_t)o], &m, sizeof(OpHead));
+        h.has_arith |= m.kind != MOP_CX && m.kind != MOP_SWAP;
+        if (m.kind == MOP_DK) ops[(size_t)o].b = A != AR_DF && nlut < (uint32_t)kJobLuts ? nlut++ : kNoJobLut;
+        const int cnt = m.kind == MOP_U1 ? 8 : m.kind == MOP_RT ? 1 : m.kind == MOP_D1 || m.kind == MOP_R1 ? 4 : 0;
+        OpCoef<T, A> &c = coef[(size_t)o];
+        for (int i = 0; i < cnt; i++) {
+            if constexpr (A == AR_DF) {
+                const float hi = (float)m.m[i];
+                c.v[i] = make_float2(hi, (float)(m.m[i] - (double)hi));
+            } else {
+                c.v[i] = (T)m.m[i];
+            }
+        }
+        if constexpr (A == AR_DF) {
+            if (m.kind == MOP_RT) {  // the rotation's packed pairs
+                const float2 t = c.v[0];
+                c.v[2] = make_float2(t.x, t.x);
+                c.v[3] = make_float2(t.y, t.y);
+                c.v[4] = make_float2(-t.x, -t.x);
+                c.v[5] = make_float2(-t.y, -t.y);
+            }
+        }
+    }
+    std::vector<GroupInfo> gi;
+    if constexpr (A == AR_DF) {
+        gi.resize((size_t)nops);
+        uint32_t bad = 0;
+        int fuse_in = 0, fuse_out = 0;
+        plan_passes(ops.data(), nops, h.L + h.H, true, max_group_of<T, A>(), gi.data(), &bad, &fuse_in, &fuse_out);
+        if (bad) return fail(ZC_ERR_INVALID, "sweep plan: a group bit lies outside the tile");
+        h.fuse_in = (uint32_t)fuse_in;
+        h.fuse_out = (uint32_t)fuse_out;
+        for (GroupInfo &q : gi) {  // slot patterns as byte offsets into the swizzled tile, step patterns
+            if (!q.G) continue;
+            for (int g = 0; g < q.G; g++) {
+                q.gm[g] = (uint16_t)(swz<8>(q.gm[g]) << 3);
+                q.pm[g] = (uint16_t)(swz<8>(q.pm[g]) << 3);
+            }
+            for (int i = 0; i < q.ntr; i++) q.trw[i] = (uint16_t)(swz<8>(q.trw[i]) << 3);
+            q.fmask = (uint16_t)(swz<8>(q.fmask) << 3);
+            uint32_t v = kSweepThreads, lo = 0, jb = 0;  // group number p + kSweepThreads against p
+            for (int g = 0; g < q.G; g++) v = insert_zero32(v, q.sorted[g]);
+            for (int i = 0; i < q.ntr; i++)
+                if (!(q.trc[i] & 0x80u) && ((v >> q.trc[i]) & 1u)) lo ^= q.trw[i];
+            for (int i = 0; i < q.nloc; i++) jb |= ((v >> q.loc[i]) & 1u) << (q.locb[i] + 4);
+            q.so_step = (uint16_t)(swz<8>(v) << 3);
+            q.lo_step = (uint16_t)(q.so_step ^ lo);
+            q.jb_step = (uint16_t)jb;
+        }
+    }
+    auto up16 = [](size_t b) { return (b + 15) & ~(size_t)15; };
+    const size_t ops_b = up16(ops.size() * sizeof(OpHead)), coef_b = up16(coef.size() * sizeof(OpCoef<T, A>));
+    h.coef_off = (uint32_t)(sizeof(JobHead) + ops_b);
+    h.gi_off = (uint32_t)(h.coef_off + coef_b);
+    out->assign(h.gi_off + up16(gi.size() * sizeof(GroupInfo)), 0);
+    memcpy(out->data(), &h, sizeof h);
+    memcpy(out->data() + sizeof(JobHead), ops.data(), ops.size() * sizeof(OpHead));
+    memcpy(out->data() + h.coef_off, (const void *)coef.data(), coef.size() * sizeof(OpCoef<T, A>));
+    if (!gi.empty()) memcpy(out->data() + h.gi_off, gi.data(), gi.size() * sizeof(GroupInfo));
+    return ZC_OK;
+}
+
+__device__ __forceinline__ void copy16(void *dst, const char *src, uint32_t bytes) {
+    for (uint32_t i = threadIdx.x; i < (bytes + 15) / 16; i += blockDim.x)
+        reinterpret_cast<uint4 *>(dst)[i] = __ldg(reinterpret_cast<const uint4 *>(src) + i);
+}
+
+// All threads: make the job block at `blk` the CTA's current job.
+template <typename T, int A>
+__device__ void load_job(SweepSmem<T, A> &c, const char *blk) {
     const int tid = threadIdx.x;
+    const JobHead *h = reinterpret_cast<const JobHead *>(blk);
+    const uint32_t nops = h->nops, L = h->L, H = h->H;
     __syncthreads();  // the previous job's tiles are done with the tables
-    constexpr int kHeadWords = (int)(sizeof(OpHead) / 4), kOpWords = (int)(sizeof(MicroOp) / 4);
-    for (int i = tid; i < nops * kHeadWords; i += blockDim.x)
-        reinterpret_cast<uint32_t *>(c.ops)[i] =
-            reinterpret_cast<const uint32_t *>(gops)[(i / kHeadWords) * kOpWords + i % kHeadWords];
-    for (uint32_t r = tid; r < (1u << H); r += blockDim.x) {  // tile bit L + j holds qubit hpos[j] (any order)
+    copy16(&c.job, blk, sizeof(JobHead));
+    copy16(c.ops, blk + sizeof(JobHead), nops * (uint32_t)sizeof(OpHead));
+    copy16(c.coef, blk + h->coef_off, nops * (uint32_t)sizeof(OpCoef<T, A>));
+    if constexpr (A == AR_DF) copy16(c.gi, blk + h->gi_off, nops * (uint32_t)sizeof(GroupInfo));
+    for (uint32_t r = tid; r < (1u << H); r += blockDim.x) {  // tile bit L + j holds qubit hpos[j]
         uint32_t o = 0;
-        for (uint32_t j = 0; j < H; j++) o |= ((r >> j) & 1u) << (hpos[j] - L);
+        for (uint32_t j = 0; j < H; j++) o |= ((r >> j) & 1u) << (h->hpos[j] - L);
         c.rows[r] = o;
     }
-    if (tid == 0) {
-        for (uint32_t j = 0; j < H; j++) {  // insertion sort, H <= 7
-            uint32_t x = hpos[j], i = j;
-            for (; i > 0 && c.hsorted[i - 1] > x; i--) c.hsorted[i] = c.hsorted[i - 1];
-            c.hsorted[i] = x;
-        }
-    }
-    if (tid == 0) {
-        c.nops = nops;
-        c.L = L;
-        c.H = H;
-    }
     __syncthreads();
-    if (tid < nops) {
-        const MicroOp &op = gops[tid];  // matrix entries from global memory
-        if (op.kind == MOP_U1 || op.kind == MOP_D1 || op.kind == MOP_R1 || op.kind == MOP_RT) {
-            const int cnt = op.kind == MOP_U1 ? 8 : op.kind == MOP_RT ? 1 : 4;
-            for (int i = 0; i < cnt; i++) {
-                if constexpr (A == AR_DF)
-                    c.coef[tid].v[i] = df_from_f64(op.m[i]);
-                else
-                    c.coef[tid].v[i] = (T)op.m[i];
-            }
-            if constexpr (A == AR_DF) {
-                if (op.kind == MOP_RT) {  // the rotation's packed pairs
-                    const float2 t = c.coef[tid].v[0];
-                    c.coef[tid].v[2] = make_float2(t.x, t.x);
-                    c.coef[tid].v[3] = make_float2(t.y, t.y);
-                    c.coef[tid].v[4] = make_float2(-t.x, -t.x);
-                    c.coef[tid].v[5] = make_float2(-t.y, -t.y);
-                }
-            }
-        }
-    }
-    if (tid == 0) {
-        int ar = 0, nlut = 0;
-        for (int o = 0; o < nops; o++) {
-            ar |= c.ops[o].kind != MOP_CX && c.ops[o].kind != MOP_SWAP;
-            if (c.ops[o].kind == MOP_DK)
-                c.ops[o].b = A != AR_DF && nlut < kJobLuts ? (uint32_t)nlut++ : kNoJobLut;
-        }
-        c.has_arith = ar;
-        c.fuse_in = c.fuse_out = 0;
-        if constexpr (A == AR_DF)
-            plan_passes(c.ops, nops, L + H, fold, max_group_of<T, A>(), c.gi, &c.bad, &c.fuse_in, &c.fuse_out);
-    }
-    __syncthreads();
-    if constexpr (A == AR_DF) {  // slot patterns as byte offsets into the swizzled tile, step patterns
-        if (tid < nops) {
-            GroupInfo &q = c.gi[tid];
-            if (q.G) {
-                for (int g = 0; g < q.G; g++) {
-                    q.gm[g] = (uint16_t)(swz<8>(q.gm[g]) << 3);
-                    q.pm[g] = (uint16_t)(swz<8>(q.pm[g]) << 3);
-                }
-                for (int i = 0; i < q.ntr; i++) q.trw[i] = (uint16_t)(swz<8>(q.trw[i]) << 3);
-                q.fmask = (uint16_t)(swz<8>(q.fmask) << 3);
-                uint32_t v = kSweepThreads, lo = 0, jb = 0;  // group number p + kSweepThreads against p
-                for (int g = 0; g < q.G; g++) v = insert_zero32(v, q.sorted[g]);
-                for (int i = 0; i < q.ntr; i++)
-                    if (!(q.trc[i] & 0x80u) && ((v >> q.trc[i]) & 1u)) lo ^= q.trw[i];
-                for (int i = 0; i < q.nloc; i++) jb |= ((v >> q.loc[i]) & 1u) << (q.locb[i] + 4);
-                q.so_step = (uint16_t)(swz<8>(v) << 3);
-                q.lo_step = (uint16_t)(q.so_step ^ lo);
-                q.jb_step = (uint16_t)jb;
-            }
-        }
-        __syncthreads();
-    }
     if constexpr (A != AR_DF) {  // the job's diagonal index tables, once per job
-        for (int o = 0; o < nops; o++) {
+        bool any = false;
+        for (uint32_t o = 0; o < nops; o++) {
             const OpHead &op = c.ops[o];
             if (op.kind != MOP_DK || op.b == kNoJobLut) continue;
+            any = true;
             uint16_t *lut = c.gi + (size_t)op.b * kJlutLen;
             for (uint32_t x = tid; x < kJlutLen; x += blockDim.x)
                 lut[x] = (uint16_t)jgather<T>(op, 0u, x < 256 ? x : (x - 256) << 8);
         }
-        __syncthreads();
+        if (any) __syncthreads();
     }
 }
 
@@ -891,28 +910,28 @@ __device__ void load_job(SweepSmem<T, A> &c, const MicroOp *gops, int nops, uint
 template <typename T, int A>
 __device__ __forceinline__ void tile_load(const SweepSmem<T, A> &c, T *dst, const T *src, uint32_t vecs) {
     constexpr uint32_t VW = 16 / sizeof(T), VB = VW == 4 ? 2 : 1;
-    const uint32_t lv = c.L - VB, cm = (1u << lv) - 1;  // vectors per row (log2), column mask
+    const uint32_t lv = c.job.L - VB, cm = (1u << lv) - 1;  // vectors per row (log2), column mask
     const uint32_t d = smem_addr(dst);
-    if (c.L < VB) {  // a state shorter than one vector
-        if (threadIdx.x < (1u << c.L)) dst[threadIdx.x] = src[threadIdx.x];
+    if (c.job.L < VB) {  // a state shorter than one vector
+        if (threadIdx.x < (1u << c.job.L)) dst[threadIdx.x] = src[threadIdx.x];
         return;
     }
     for (uint32_t i = threadIdx.x; i < vecs; i += kSweepThreads) {
-        const T *g = src + ((size_t)c.rows[i >> lv] << c.L) + (size_t)(i & cm) * VW;
+        const T *g = src + ((size_t)c.rows[i >> lv] << c.job.L) + (size_t)(i & cm) * VW;
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16 * swz<16>(i)), "l"(g) : "memory");
     }
 }
 template <typename T, int A>
 __device__ __forceinline__ void tile_store(const SweepSmem<T, A> &c, T *dst, const T *src, uint32_t vecs) {
     constexpr uint32_t VW = 16 / sizeof(T), VB = VW == 4 ? 2 : 1;
-    const uint32_t lv = c.L - VB, cm = (1u << lv) - 1;
-    if (c.L < VB) {
-        if (threadIdx.x < (1u << c.L)) dst[threadIdx.x] = src[threadIdx.x];
+    const uint32_t lv = c.job.L - VB, cm = (1u << lv) - 1;
+    if (c.job.L < VB) {
+        if (threadIdx.x < (1u << c.job.L)) dst[threadIdx.x] = src[threadIdx.x];
         return;
     }
     const uint4 *sv = reinterpret_cast<const uint4 *>(src);
     auto at = [&](uint32_t i) {
-        return reinterpret_cast<uint4 *>(dst + ((size_t)c.rows[i >> lv] << c.L) + (size_t)(i & cm) * VW);
+        return reinterpret_cast<uint4 *>(dst + ((size_t)c.rows[i >> lv] << c.job.L) + (size_t)(i & cm) * VW);
     };
     uint32_t i = threadIdx.x;
     for (; i + 3 * kSweepThreads < vecs; i += 4 * kSweepThreads) {
@@ -936,9 +955,9 @@ __device__ __forceinline__ void tile_store(const SweepSmem<T, A> &c, T *dst, con
 template <typename T, int A>
 __device__ void process_tile(SweepSmem<T, A> &c, T *re, T *im, uint64_t t, const char *tables, T *sre, T *sim,
                              uint32_t form) {
-    const uint32_t size = 1u << (c.L + c.H), vecs = size / (16 / (uint32_t)sizeof(T));
+    const uint32_t size = 1u << (c.job.L + c.job.H), vecs = size / (16 / (uint32_t)sizeof(T));
     const int tid = threadIdx.x;
-    const uint64_t base = tile_base(t, c.L, c.hsorted, c.H);
+    const uint64_t base = tile_base(t, c.job.L, c.job.hpos, c.job.H);
     tile_load(c, sre, re + base, vecs);
     tile_load(c, sim, im + base, vecs);
     asm volatile("cp.async.wait_all;" ::: "memory");
@@ -952,7 +971,7 @@ __device__ void process_tile(SweepSmem<T, A> &c, T *re, T *im, uint64_t t, const
         double *dr = reinterpret_cast<double *>(sre), *di = reinterpret_cast<double *>(sim);
         float2 *fr = reinterpret_cast<float2 *>(sre), *fi = reinterpret_cast<float2 *>(sim);
         const bool in_df = form & kFormInDf, out_df = form & kFormOutDf;
-        const bool fuse_in = c.fuse_in && !in_df, fuse_out = c.fuse_out && !out_df;
+        const bool fuse_in = c.job.fuse_in && !in_df, fuse_out = c.job.fuse_out && !out_df;
         auto to_pairs = [&](uint32_t v) {
             float2 H, L;
             pk_from_f64(dr[v], di[v], H, L);
@@ -965,14 +984,14 @@ __device__ void process_tile(SweepSmem<T, A> &c, T *re, T *im, uint64_t t, const
             dr[v] = a;
             di[v] = b;
         };
-        if (c.has_arith && !in_df && !c.fuse_in) {
+        if (c.job.has_arith && !in_df && !c.job.fuse_in) {
             for (uint32_t v = tid; v < size; v += blockDim.x) to_pairs(v);
             __syncthreads();
         }
-        apply_ops<T, A, float2>(fr, fi, c.ops, c.coef, c.nops, base, size, tables, &c.bad, c.jlut, nullptr, c.gi,
+        apply_ops<T, A, float2>(fr, fi, c.ops, c.coef, (int)c.job.nops, base, size, tables, &c.bad, c.jlut, nullptr, c.gi,
                                 fuse_in,
                                 fuse_out);
-        if (c.has_arith && !fuse_out) {  // register passes leave pairs unnormalised
+        if (c.job.has_arith && !fuse_out) {  // register passes leave pairs unnormalised
             for (uint32_t v = tid; v < size; v += blockDim.x) {
                 if (out_df) {
                     float2 H = fr[v], L = fi[v];
@@ -983,14 +1002,14 @@ __device__ void process_tile(SweepSmem<T, A> &c, T *re, T *im, uint64_t t, const
                     to_f64(v);
                 }
             }
-        } else if (!c.has_arith && in_df != out_df) {  // permutations only: change the form alone
+        } else if (!c.job.has_arith && in_df != out_df) {  // permutations only: change the form alone
             for (uint32_t v = tid; v < size; v += blockDim.x) {
                 if (in_df) to_f64(v);
                 else to_pairs(v);
             }
         }
     } else {
-        apply_ops<T, A, T>(sre, sim, c.ops, c.coef, c.nops, base, size, tables, &c.bad, c.jlut, c.gi, nullptr);
+        apply_ops<T, A, T>(sre, sim, c.ops, c.coef, (int)c.job.nops, base, size, tables, &c.bad, c.jlut, c.gi, nullptr);
     }
     __syncthreads();
     tile_store(c, re + base, sre, vecs);
@@ -1005,9 +1024,9 @@ __device__ void sweep_exit(SweepSmem<T, A> &c, int *err) {
     __syncthreads();
     if (threadIdx.x == 0 && c.bad && atomicCAS(err, 0, 2) == 0) {
         err[1] = (int)blockIdx.x;
-        err[6] = (int)c.L;
-        err[7] = (int)c.H;
-        err[8] = c.nops;
+        err[6] = (int)c.job.L;
+        err[7] = (int)c.job.H;
+        err[8] = (int)c.job.nops;
         err[10] = (int)c.bad;
         __threadfence();
     }
@@ -1020,15 +1039,15 @@ __device__ void sweep_exit(SweepSmem<T, A> &c, int *err) {
 // run-time branches for it (they cost registers at the 80-register cap).
 template <typename T, int A, uint32_t FORM>
 __global__ void __launch_bounds__(kSweepThreads, kSweepCtasPerSm)
-    k_sweep(T *__restrict__ re, T *__restrict__ im, const SweepGeom g, const MicroOp *__restrict__ gops, int nops,
+    k_sweep(T *__restrict__ re, T *__restrict__ im, uint64_t ntiles, const char *__restrict__ job,
             const char *__restrict__ tables, int *__restrict__ err) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ SweepSmem<T, A> c;
     T *sre = reinterpret_cast<T *>(smem);
     T *sim = sre + kTileArrayBytes / sizeof(T);
     if (threadIdx.x == 0) c.bad = 0;
-    load_job(c, gops, nops, g.L, g.H, g.hpos, true);
-    for (uint64_t t = blockIdx.x; t < g.ntiles; t += gridDim.x) process_tile(c, re, im, t, tables, sre, sim, FORM);
+    load_job(c, job);
+    for (uint64_t t = blockIdx.x; t < ntiles; t += gridDim.x) process_tile(c, re, im, t, tables, sre, sim, FORM);
     sweep_exit(c, err);
 }
 
@@ -1059,9 +1078,7 @@ __global__ void __launch_bounds__(kSweepThreads, kSweepCtasPerSm)
                 else hi = mid;
             }
             const SweepJob &Jn = jobs[lo];
-            // CX folding stays off here: the packed kernel's extra live state spills
-            load_job(c, reinterpret_cast<const MicroOp *>(blob + Jn.ops_off), (int)Jn.nops, Jn.L, Jn.H, Jn.hpos,
-                     false);
+            load_job(c, blob + Jn.job_off);
             cur = (int)lo;
             job_lo = Jn.tile_start;
             job_hi = Jn.tile_start + Jn.ntiles;
@@ -1076,35 +1093,34 @@ __global__ void __launch_bounds__(kSweepThreads, kSweepCtasPerSm)
 }
 
 template <typename T, int A, uint32_t FORM>
-int run_sweep_form(zc_state *st, const SweepGeom &g, const MicroOp *dev_ops, int nops, const char *dev_tables) {
-    const size_t smem = (size_t)2 * (1u << (g.L + g.H)) * sizeof(T);
+int run_sweep_form(zc_state *st, const SweepGeom &g, const char *dev_job, const char *dev_tables) {
     static std::atomic<bool> attr{false};  // set once per process; racing first calls repeat it
     if (!attr) {
         ZC_CUDA(cudaFuncSetAttribute(k_sweep<T, A, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)kSweepSmemBytes));
         attr = true;
     }
-    if (smem > kSweepSmemBytes || g.H > kMaxSweepHigh || nops > kMaxMicroOps)
+    if (((size_t)2 << (g.L + g.H)) * sizeof(T) > kSweepSmemBytes || g.H > kMaxSweepHigh)
         return fail(ZC_ERR_INVALID, "sweep shape exceeds the kernel's limits");
     const uint64_t blocks = std::min<uint64_t>(g.ntiles, (uint64_t)st->num_sms * kSweepCtasPerSm);
-    k_sweep<T, A, FORM><<<(int)blocks, kSweepThreads, kSweepSmemBytes, st->stream>>>((T *)st->re, (T *)st->im, g, dev_ops,
-                                                                             nops, dev_tables, st->d_err);
+    k_sweep<T, A, FORM><<<(int)blocks, kSweepThreads, kSweepSmemBytes, st->stream>>>(
+        (T *)st->re, (T *)st->im, g.ntiles, dev_job, dev_tables, st->d_err);
     ZC_CUDA(cudaGetLastError());
     return ZC_OK;
 }
 
 template <typename T, int A>
-int run_sweep(zc_state *st, const SweepGeom &g, const MicroOp *dev_ops, int nops, const char *dev_tables) {
+int run_sweep(zc_state *st, const SweepGeom &g, const char *dev_job, const char *dev_tables) {
     if constexpr (A == AR_DF) {
         switch (g.form) {
-            case 0: return run_sweep_form<T, A, 0>(st, g, dev_ops, nops, dev_tables);
-            case kFormInDf: return run_sweep_form<T, A, kFormInDf>(st, g, dev_ops, nops, dev_tables);
-            case kFormOutDf: return run_sweep_form<T, A, kFormOutDf>(st, g, dev_ops, nops, dev_tables);
-            default: return run_sweep_form<T, A, kFormInDf | kFormOutDf>(st, g, dev_ops, nops, dev_tables);
+            case 0: return run_sweep_form<T, A, 0>(st, g, dev_job, dev_tables);
+            case kFormInDf: return run_sweep_form<T, A, kFormInDf>(st, g, dev_job, dev_tables);
+            case kFormOutDf: return run_sweep_form<T, A, kFormOutDf>(st, g, dev_job, dev_tables);
+            default: return run_sweep_form<T, A, kFormInDf | kFormOutDf>(st, g, dev_job, dev_tables);
         }
     }
     if (g.form) return fail(ZC_ERR_INVALID, "double-float hand-over requested outside a double-float sweep");
-    return run_sweep_form<T, A, 0>(st, g, dev_ops, nops, dev_tables);
+    return run_sweep_form<T, A, 0>(st, g, dev_job, dev_tables);
 }
 
 template <typename T, int A>
@@ -1159,17 +1175,23 @@ int launch_sweep_multi(cudaStream_t stream, int num_sms, int prec, bool exact, c
                  : run_sweep_multi<float, AR_FMA>(stream, num_sms, dev_blob, d_err);
 }
 
-int launch_sweep(zc_state *st, const SweepGeom &g, const MicroOp *dev_ops, int nops, const char *dev_tables,
-                 bool exact) {
+int encode_job(int prec, bool exact, const SweepPlan &plan, std::vector<char> *out) {
+    if (plan.mops.size() > (size_t)kMaxMicroOps || plan.g.H > kMaxSweepHigh)
+        return fail(ZC_ERR_INVALID, "sweep shape exceeds the kernel's limits");
+    if (prec == 64) return exact ? encode_job_as<double, AR_EXACT>(plan, out) : encode_job_as<double, AR_DF>(plan, out);
+    return exact ? encode_job_as<float, AR_EXACT>(plan, out) : encode_job_as<float, AR_FMA>(plan, out);
+}
+
+int launch_sweep(zc_state *st, const SweepGeom &g, const char *dev_job, const char *dev_tables, bool exact) {
     ProfScope ps(st, K_SWEEP, 2.0 * st->len * (st->prec / 8) * 2);
     st->ctr.launches++;
     st->ctr.sweeps++;
     st->ctr.bytes_moved += 2 * st->len * (st->prec / 8) * 2;
     if (st->prec == 64)
-        return exact ? run_sweep<double, AR_EXACT>(st, g, dev_ops, nops, dev_tables)
-                     : run_sweep<double, AR_DF>(st, g, dev_ops, nops, dev_tables);
-    return exact ? run_sweep<float, AR_EXACT>(st, g, dev_ops, nops, dev_tables)
-                 : run_sweep<float, AR_FMA>(st, g, dev_ops, nops, dev_tables);
+        return exact ? run_sweep<double, AR_EXACT>(st, g, dev_job, dev_tables)
+                     : run_sweep<double, AR_DF>(st, g, dev_job, dev_tables);
+    return exact ? run_sweep<float, AR_EXACT>(st, g, dev_job, dev_tables)
+                 : run_sweep<float, AR_FMA>(st, g, dev_job, dev_tables);
 }
 
 }  // namespace zc

@@ -24,7 +24,7 @@ struct SweepGeom {
     uint64_t ntiles;
 };
 
-// One op inside a sweep, operands as local bit indices (0..L+H) or
+// One op as the planner leaves it, operands as local bit indices (0..L+H) or
 // kOuterFlag | global qubit. U1: a = bit, m = 2x2 row-major (re, im);
 // D1: a = bit, m[0..4) = d0, d1; DK: k, loc[], table = byte offset of 2^k
 // (re, im) pairs in the sweep's table block (for double-float sweeps of f64
@@ -39,8 +39,18 @@ struct MicroOp {
     double m[8];
 };
 
+// A job as the kernel takes it (encode_job, zc_sweep.cu): this head, then at
+// 16-byte boundaries the op heads, the coefficients in the arithmetic's form
+// (coef_off), and for double-float sweeps the register passes (gi_off),
+// copied as they are into the CTA's shared tables.
+struct JobHead {
+    uint32_t nops, L, H, has_arith;
+    uint32_t fuse_in, fuse_out, coef_off, gi_off;
+    uint32_t hpos[8];  // the tile's high qubits, ascending
+};
+
 // Packed launch over many states: header, then jobs, then each job's
-// micro-ops and tables at the given byte offsets of the same blob.
+// block and tables at the given byte offsets of the same blob.
 struct SweepBatch {
     uint32_t njobs, pad;
     uint64_t total_tiles;
@@ -48,11 +58,9 @@ struct SweepBatch {
 
 struct SweepJob {
     void *re, *im;  // the state's device arrays
-    uint32_t L, H, nops, pad;
-    uint32_t hpos[8];
     uint64_t ntiles;
     uint64_t tile_start;  // first tile of this job in the packed index space
-    uint64_t ops_off;     // byte offset of its MicroOps in the blob (16-byte aligned)
+    uint64_t job_off;     // byte offset of its JobHead in the blob (16-byte aligned)
     uint64_t tables_off;  // byte offset of its tables in the blob
 };
 
