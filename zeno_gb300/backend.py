@@ -446,18 +446,25 @@ def run(p, shots: int = 1024, seed: int = 0, precision: int = 0, fusion: Optiona
     nz = NoiseC(*[getattr(noise, f.name) for f in fields(noise)]) if noisy else None
     opts = RunOptions(precision, flags, shots, seed, C.pointer(nz) if nz is not None else None, 0.0, sweep_high, 0)
     cap = max(16, min(shots, 1 << 22) + 1)
-    keys = np.zeros(cap, dtype=np.uint64)
-    counts = np.zeros(cap, dtype=np.uint64)
-    sv = np.zeros(1 << p.n_qubits, dtype=np.complex128) if statevector else None
+    keys = np.empty(cap, dtype=np.uint64)
+    counts = np.empty(cap, dtype=np.uint64)
+    sv = np.empty(1 << p.n_qubits, dtype=np.complex128) if statevector else None
     res = RunResultC()
     _check(load().zc_run(program._h, C.byref(opts), C.byref(res), keys.ctypes.data_as(C.POINTER(C.c_uint64)),
                          counts.ctypes.data_as(C.POINTER(C.c_uint64)), cap,
                          sv.ctypes.data_as(C.POINTER(C.c_double)) if sv is not None else None))
-    raw = {int(keys[i]): int(counts[i]) for i in range(min(res.n_keys, cap))}
+    nk = min(res.n_keys, cap)
+    raw = dict(zip(keys[:nk].tolist(), counts[:nk].tolist()))
     fmt: Dict[str, int] = {}
-    for k, v in raw.items():
-        key = _circ.format_key(k, p.cregs)
-        fmt[key] = fmt.get(key, 0) + v
+    if len(p.cregs) == 1 and p.cregs[0][1] >= p.n_clbits and p.n_clbits:  # one register: the word itself, in binary
+        spec, mask = "0%db" % p.cregs[0][1], (1 << p.cregs[0][1]) - 1
+        for k, v in raw.items():
+            key = format(k & mask, spec)
+            fmt[key] = fmt.get(key, 0) + v
+    else:
+        for k, v in raw.items():
+            key = _circ.format_key(k, p.cregs)
+            fmt[key] = fmt.get(key, 0) + v
     prec = res.precision_bits
     return RunResult(fmt, raw, shots, p.n_qubits, prec, "cuda-f%d" % prec, seed, res.sim_seconds, sv,
                      program.stats, res.launches, res.sweeps, res.bytes_moved, bool(res.batched),

@@ -298,43 +298,50 @@ size_t plan_sweep(uint32_t n, int prec, bool ex, uint32_t L, uint32_t Hcap, cons
     if (!ex) {
         const size_t m = taken.size();
         std::vector<char> done(m, 0);
-        auto ready = [&](size_t i) {
-            for (size_t j = 0; j < i; j++)
-                if (!done[j] && (touch_mask(q[taken[j]]) & touch_mask(q[taken[i]]))) return false;
-            return true;
-        };
+        std::vector<uint64_t> touch(m);
+        for (size_t i = 0; i < m; i++) touch[i] = touch_mask(q[taken[i]]);
         auto is1q = [&](size_t i) { return q[taken[i]].kind == Q_UNITARY && q[taken[i]].k == 1; };
+        const uint64_t all = n >= 64 ? ~0ull : ((1ull << n) - 1);
         order.clear();
         uint64_t cx_targets = 0;  // targets of the CX ops since the last run
+        size_t first = 0;         // ops before it are emitted
         while (order.size() < m) {
+            while (done[first]) first++;
             // ready one-qubit ops on distinct qubits, program order; those on
             // targets of the CX ops just emitted first (the kernel folds a CX
-            // into the register group that holds its target)
+            // into the register group that holds its target). An op is ready
+            // when no op before it that is still to come touches its qubits.
             std::vector<size_t> run;
             uint64_t used = 0;
-            for (int pass = 0; pass < 2; pass++)
-                for (size_t i = 0; i < m && run.size() < run_cap; i++) {
-                    if (done[i] || !is1q(i) || !ready(i)) continue;
+            size_t other = m;  // the first ready op of another kind
+            for (int pass = 0; pass < 2 && run.size() < run_cap; pass++) {
+                uint64_t ahead = 0;
+                for (size_t i = first; i < m && run.size() < run_cap && ahead != all; i++) {
+                    if (done[i]) continue;
+                    const bool ready = !(touch[i] & ahead);
+                    ahead |= touch[i];
+                    if (!ready) continue;
+                    if (!is1q(i)) {
+                        other = std::min(other, i);
+                        continue;
+                    }
                     const uint32_t qb = q[taken[i]].qs[0];
                     if ((used >> qb) & 1) continue;
                     if (pass == 0 && !((cx_targets >> qb) & 1)) continue;
                     run.push_back(i);
                     used |= 1ull << qb;
                 }
+            }
             std::sort(run.begin(), run.end());
             // a full run goes out at once; otherwise a ready op of another
             // kind goes first (it can make more one-qubit ops ready), and a
             // short run only when nothing else is ready
-            bool emitted = false;
-            if (run.size() < run_cap)
-                for (size_t i = 0; i < m && !emitted; i++)
-                    if (!done[i] && !is1q(i) && ready(i)) {
-                        done[i] = 1;
-                        order.push_back(i);
-                        emitted = true;
-                        if (q[taken[i]].kind == Q_CX) cx_targets |= 1ull << q[taken[i]].b;
-                    }
-            if (emitted) continue;
+            if (run.size() < run_cap && other < m) {
+                done[other] = 1;
+                order.push_back(other);
+                if (q[taken[other]].kind == Q_CX) cx_targets |= 1ull << q[taken[other]].b;
+                continue;
+            }
             for (size_t i : run) {
                 done[i] = 1;
                 order.push_back(i);
@@ -373,9 +380,12 @@ size_t plan_sweep(uint32_t n, int prec, bool ex, uint32_t L, uint32_t Hcap, cons
     }
     if (low.size() <= (size_t)kMaxMicroOps) break;
     // lowering added table ops: take fewer queue ops (dropping the last
-    // taken op never breaks an ordering constraint)
-    taken.pop_back();
+    // taken ops never breaks an ordering constraint), first in proportion
+    // (lowering again costs more than an op in the next sweep), then singly
+    const size_t fit = taken.size() * (size_t)kMaxMicroOps / low.size();
+    taken.resize(std::min(fit, taken.size() - 1));
     if (taken.size() <= 1) {
+        taken.resize(1);
         plan->carry.clear();
         return taken.size();
     }

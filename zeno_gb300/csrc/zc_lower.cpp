@@ -46,42 +46,58 @@ struct Term {
     std::vector<cd> tab;      // index bit b <-> b-th set bit of mask (ascending)
 };
 
-uint64_t scatter(uint64_t y, uint64_t mask) {
-    uint64_t g = 0;
+// Bits of g at the positions of mask, packed ascending.
+uint32_t gather(uint64_t g, uint64_t mask) {
+    uint32_t y = 0;
     for (int b = 0; mask; b++) {
         const uint64_t low = mask & (~mask + 1);
-        if ((y >> b) & 1) g |= low;
-        mask ^= low;
-    }
-    return g;
-}
-
-uint64_t gather(uint64_t g, uint64_t mask) {
-    uint64_t y = 0;
-    for (int b = 0; mask; b++) {
-        const uint64_t low = mask & (~mask + 1);
-        if (g & low) y |= 1ull << b;
+        if (g & low) y |= 1u << b;
         mask ^= low;
     }
     return y;
 }
 
+// Plain complex product (std::complex's operator checks for NaN and calls out).
+inline cd cmul(cd a, cd b) {
+    return cd(a.real() * b.real() - a.imag() * b.imag(), a.real() * b.imag() + a.imag() * b.real());
+}
+
+// For every assignment y over `mask` (bit b on its b-th qubit) the index into
+// a table over tmask that f(assignment) has, f linear over XOR: built by
+// doubling, one XOR per entry.
+template <typename F>
+const std::vector<uint32_t> &index_map(uint64_t mask, uint64_t tmask, F f) {
+    static thread_local std::vector<uint32_t> idx;  // valid until the next call
+    idx.resize((size_t)1 << __builtin_popcountll(mask));
+    idx[0] = 0;
+    size_t n = 1;
+    for (uint64_t m = mask; m; m &= m - 1, n *= 2) {
+        const uint32_t c = gather(f(m & (~m + 1)), tmask);
+        for (size_t y = 0; y < n; y++) idx[n + y] = idx[y] ^ c;
+    }
+    return idx;
+}
+
 // Term over `mask` whose value at assignment g is t(f(g)).
 template <typename F>
 Term remap(const Term &t, uint64_t mask, F f) {
-    Term r{mask, std::vector<cd>((size_t)1 << __builtin_popcountll(mask))};
-    for (uint64_t y = 0; y < r.tab.size(); y++) r.tab[y] = t.tab[gather(f(scatter(y, mask)), t.mask)];
+    const std::vector<uint32_t> &idx = index_map(mask, t.mask, f);
+    Term r{mask, std::vector<cd>(idx.size())};
+    for (size_t y = 0; y < idx.size(); y++) r.tab[y] = t.tab[idx[y]];
     return r;
 }
 
-// Product of several terms over the union of their supports.
-Term merge(const std::vector<Term> &ts) {
-    uint64_t mask = 0;
-    for (const Term &t : ts) mask |= t.mask;
-    Term r{mask, std::vector<cd>((size_t)1 << __builtin_popcountll(mask), cd(1.0, 0.0))};
-    for (uint64_t y = 0; y < r.tab.size(); y++) {
-        const uint64_t g = scatter(y, mask);
-        for (const Term &t : ts) r.tab[y] *= t.tab[gather(g, t.mask)];
+// Product of several terms over `mask`, the union of their supports.
+Term merge(const std::vector<const Term *> &ts, uint64_t mask) {
+    if (ts.size() == 1) return *ts[0];
+    Term r{mask, std::vector<cd>((size_t)1 << __builtin_popcountll(mask))};
+    for (size_t k = 0; k < ts.size(); k++) {
+        const Term &t = *ts[k];
+        const std::vector<uint32_t> &idx = index_map(mask, t.mask, [](uint64_t g) { return g; });
+        if (k == 0)
+            for (size_t y = 0; y < idx.size(); y++) r.tab[y] = t.tab[idx[y]];
+        else
+            for (size_t y = 0; y < idx.size(); y++) r.tab[y] = cmul(r.tab[y], t.tab[idx[y]]);
     }
     return r;
 }
@@ -129,20 +145,22 @@ LoweredOp diag_op(const Term &t) {
 
 // Merge `ts` into as few diagonals of at most kFlushCap qubits as a greedy
 // packing gives, appending them to `out`.
-void emit_terms(std::vector<Term> ts, std::vector<LoweredOp> *out) {
+void emit_terms(const std::vector<Term> &all, std::vector<LoweredOp> *out) {
+    std::vector<const Term *> ts, pack, rest;
+    for (const Term &t : all) ts.push_back(&t);
     while (!ts.empty()) {
-        std::vector<Term> pack{ts.front()};
-        uint64_t mask = ts.front().mask;
-        std::vector<Term> rest;
+        pack.assign(1, ts.front());
+        rest.clear();
+        uint64_t mask = ts.front()->mask;
         for (size_t i = 1; i < ts.size(); i++) {
-            if (__builtin_popcountll(mask | ts[i].mask) <= kFlushCap) {
-                mask |= ts[i].mask;
+            if (__builtin_popcountll(mask | ts[i]->mask) <= kFlushCap) {
+                mask |= ts[i]->mask;
                 pack.push_back(ts[i]);
             } else {
                 rest.push_back(ts[i]);
             }
         }
-        out->push_back(diag_op(merge(pack)));
+        out->push_back(diag_op(merge(pack, mask)));
         ts.swap(rest);
     }
 }
@@ -324,7 +342,7 @@ void lower_df(const std::vector<const QOp *> &seq, int run_cap, std::vector<Lowe
                     o.kind = MOP_U1;
                     for (int k = 0; k < 8; k++) o.m[k] = items[g].op->data[k];
                 }
-                out->push_back(o);
+                out->push_back(std::move(o));
             }
             for (size_t g = i; g < j; g++)
                 if (items[g].real) {
@@ -350,7 +368,7 @@ void lower_df(const std::vector<const QOp *> &seq, int run_cap, std::vector<Lowe
                 }
                 pending.push_back(remap(d, mask, [&](uint64_t g) { return g ^ (((g >> c) & 1) << t); }));
             }
-            emit_terms(std::move(flush_now), out);
+            emit_terms(flush_now, out);
             LoweredOp o{};
             o.kind = MOP_CX;
             o.a = c;
@@ -388,7 +406,7 @@ void lower_df(const std::vector<const QOp *> &seq, int run_cap, std::vector<Lowe
             carry->push_back(std::move(q));
         }
     } else {
-        emit_terms(std::move(pending), out);
+        emit_terms(pending, out);
     }
 }
 
