@@ -142,7 +142,10 @@ static int grow(void **p, size_t *cap, size_t need) {
 
 static constexpr size_t kQueueWindow = 2048;  // ops examined per sweep plan
 static constexpr size_t kQueueFlushAt = 8192; // queue length that forces a flush
-static constexpr uint32_t kMinSweepQubits = 14;
+static constexpr uint32_t kMinSweepQubits = 3;
+// f32 states below this size keep program order in fast mode too (see
+// program_order).
+static constexpr uint32_t kF32OrderQubits = 14;
 
 int launch_single(zc_state *st, const QOp &op) {
     const bool ex = exact(st);
@@ -208,17 +211,40 @@ struct SweepShape {
     uint32_t L, Hcap;
 };
 
+// How many high qubits a tile takes. A sweep costs ~15 us of planning, copy and
+// launch, so a small state wants tiles that hold many of its qubits (fewer
+// sweeps), against enough tiles for the SMs. Measured per whole zc_run
+// (depth-12 u3 + matching CX; f32: gate mix), us:
+//   exact f64, bound by each SM's FP64 pipe: 2^8 amplitudes per tile up to 15
+//   qubits (12q: 773 with 2^8, 1641 with 2^11, 1615 one launch per op), 2^9
+//   for 16-17, 2^10 for 18-21 (20q: 8133, 2^11 8924), whole tiles beyond
+//   double-float: about half the qubits plus two, at least 2^8 (10q 355, one
+//   launch per op 842; 16q 544 with 2^10, 918 with 2^7; 20q 1080 with 2^12)
+//   f32: up to 13 qubits the state is one tile (10q 155, one launch per op
+//   408); larger states keep at least two tiles per SM
 static SweepShape shape_for(const zc_state *st) {
-    const uint32_t L = std::min<uint32_t>(st->n, st->prec == 64 ? 5 : 6);  // 256-byte rows
-    const uint32_t Tmax = st->prec == 64 ? 12 : 13;                       // 64 KiB per tile buffer
-    uint32_t Hcap = std::min<uint32_t>(Tmax - L, st->n - L);
+    const uint32_t n = st->n, L = std::min<uint32_t>(n, st->prec == 64 ? 5 : 6);  // 256-byte rows
+    const uint32_t Tmax = st->prec == 64 ? 12 : 13;                                // 64 KiB per tile buffer
+    uint32_t Hcap = std::min<uint32_t>(Tmax - L, n - L);
     if (st->sweep_high) return SweepShape{L, std::min<uint32_t>(Hcap, st->sweep_high)};  // tuned
-    // keep at least ~2 tiles per SM so every SM streams
-    uint32_t tiles_log2 = 0;
-    while ((1u << tiles_log2) < (uint32_t)(2 * st->num_sms)) tiles_log2++;
-    if (st->n - L > tiles_log2) Hcap = std::min<uint32_t>(Hcap, st->n - L - tiles_log2);
-    else Hcap = 0;
-    return SweepShape{L, Hcap};
+    uint32_t T = Tmax;
+    if (st->prec == 64 && exact(st)) {
+        T = n <= 15 ? 8 : n <= 17 ? 9 : n <= 21 ? 10 : Tmax;
+    } else if (st->prec == 64) {
+        T = std::max<uint32_t>(8, n / 2 + 2);
+    } else if (n >= kF32OrderQubits) {
+        uint32_t tiles_log2 = 0;
+        while ((1u << tiles_log2) < (uint32_t)(2 * st->num_sms)) tiles_log2++;
+        T = n - std::min(tiles_log2, n - L);
+    }
+    return SweepShape{L, std::min(Hcap, std::max(T, L) - L)};
+}
+
+// Whether ops keep program order. Exact mode does (reordering two gates
+// changes the rounding); so do f32 states under kF32OrderQubits, whose
+// results stay those of one launch per op.
+static bool program_order(const zc_state *st) {
+    return exact(st) || (st->prec == 32 && st->n < kF32OrderQubits);
 }
 
 static uint32_t loc_of(uint32_t q, uint32_t L, const std::vector<uint32_t> &highs) {
@@ -482,7 +508,7 @@ static int run_one_sweep(zc_state *st) {
     std::vector<QOp> &q = st->queue;
     const SweepShape sh = shape_for(st);
     SweepPlan plan;
-    if (plan_sweep(st->n, st->prec, exact(st), sh.L, sh.Hcap, q, &plan) <= 1) {
+    if (plan_sweep(st->n, st->prec, program_order(st), sh.L, sh.Hcap, q, &plan) <= 1) {
         // nothing to batch: the per-op kernel is the same work
         int rc = settle_form(st);
         if (rc) return rc;
@@ -513,13 +539,11 @@ static int run_one_sweep(zc_state *st) {
 }
 
 static bool sweeps_enabled(const zc_state *st) {
-    if (st->flags & ZC_FLAG_NO_SWEEPS) return false;
-    if (st->flags & ZC_FLAG_FORCE_SWEEPS) return st->n >= 3;
-    return st->n >= kMinSweepQubits;
+    return !(st->flags & ZC_FLAG_NO_SWEEPS) && st->n >= kMinSweepQubits;
 }
 
 // Launch everything queued (program order preserved where results depend on it).
-static int flush(zc_state *st) {
+int flush(zc_state *st) {
     int rc = ZC_OK;
     while (!st->queue.empty() && rc == ZC_OK) {
         if (!sweeps_enabled(st) || !sweepable(st->queue.front())) {

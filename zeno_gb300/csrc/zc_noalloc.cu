@@ -213,6 +213,12 @@ extern "C" int zc_sample_noalloc(zc_state *st, uint64_t shots, uint64_t seed, ui
     if (!st) return fail(ZC_ERR_INVALID, "null state");
     if (shots == 0) return ZC_OK;
     if (!out) return fail(ZC_ERR_INVALID, "sample_noalloc: null output");
+    // states below 14 qubits never needed a zc_finish before this call; their
+    // few queued ops are launched here (from the parameter ring: no allocation)
+    if (!st->queue.empty() && st->n < 14) {
+        const int rc = flush(st);
+        if (rc) return rc;
+    }
     if (!st->queue.empty())
         return fail(ZC_ERR_INVALID, "sample_noalloc: ops are still queued; call zc_finish first");
     if (shots > kMaxShots) return fail(ZC_ERR_INVALID, "sample_noalloc: at most 16384 shots per call");
