@@ -1018,22 +1018,22 @@ int zc_statevector(zc_state *st, double *out) {
     if (!st || !out) return fail(ZC_ERR_INVALID, "null argument");
     int rc = flush(st);
     if (rc) return rc;
-    const size_t es = st->prec / 8;
-    std::vector<char> re(st->len * es), im(st->len * es);
-    ZC_CUDA(cudaMemcpyAsync(re.data(), st->re, st->len * es, cudaMemcpyDeviceToHost, st->stream));
-    ZC_CUDA(cudaMemcpyAsync(im.data(), st->im, st->len * es, cudaMemcpyDeviceToHost, st->stream));
-    ZC_CUDA(cudaStreamSynchronize(st->stream));
-    if ((rc = check_device_error(st))) return rc;
-    for (size_t i = 0; i < st->len; i++) {
-        if (st->prec == 64) {
-            out[2 * i] = ((double *)re.data())[i];
-            out[2 * i + 1] = ((double *)im.data())[i];
-        } else {
-            out[2 * i] = (double)((float *)re.data())[i];
-            out[2 * i + 1] = (double)((float *)im.data())[i];
-        }
+    // The device interleaves and widens, a staging buffer at a time, and the
+    // copy engine writes the caller's array: 176 GB/s into touched pages. (The
+    // host loop over two copied arrays took 8.6 ms for 2^22 amplitudes, this 3.9
+    // into a fresh array, most of it the array's page faults.) The staging
+    // buffer is the device half of the parameter ring: everything that reads
+    // the ring precedes these launches on the stream, everything that refills
+    // it follows them.
+    const uint64_t chunk = st->arena.cap / (2 * sizeof(double));
+    for (uint64_t i = 0; i < st->len; i += chunk) {
+        const uint64_t count = std::min<uint64_t>(chunk, st->len - i);
+        if ((rc = launch_interleave(st, i, count, st->arena.dev))) return rc;
+        ZC_CUDA(cudaMemcpyAsync(out + 2 * i, st->arena.dev, count * 2 * sizeof(double), cudaMemcpyDeviceToHost,
+                                st->stream));
     }
-    return ZC_OK;
+    ZC_CUDA(cudaStreamSynchronize(st->stream));
+    return check_device_error(st);
 }
 
 int zc_load_state(zc_state *st, const double *in) {

@@ -194,6 +194,8 @@ TrajPlan plan_trajectories(uint32_t n, uint64_t ntraj, int num_sms);
 int launch_trajectories(zc_state *st, const TrajPlan &plan, uint32_t n, const TrajRec *d_recs, int nops,
                         const float *d_mats, const uint32_t *d_fq, const uint32_t *d_fc, int nfinal,
                         const TrajNoise &nz, uint64_t ntraj, uint64_t seed, uint64_t *d_out, void *d_work);
+// Amplitudes [first, first + count) as interleaved f64 pairs into device memory.
+int launch_interleave(zc_state *st, uint64_t first, uint64_t count, void *dst);
 // d_scratch: sample_scan_scratch(nchunks, chunk_len, exact) bytes of device memory.
 int launch_sample_scan(zc_state *st, const SampleChunk *d_chunks, size_t nchunks, const double *d_us,
                        uint64_t *d_out, uint64_t chunk_len, bool exact, void *d_scratch);

@@ -448,7 +448,42 @@ int run_chain(zc_state *st, uint64_t total, uint64_t chunk, uint64_t nrows, int 
     return ZC_OK;
 }
 
+// Split re / im arrays -> interleaved f64 (re, im) pairs, four amplitudes per
+// thread (16-byte loads, 64 bytes of stores).
+template <typename T>
+__global__ void __launch_bounds__(256) k_interleave(const T *__restrict__ re, const T *__restrict__ im,
+                                                    double2 *__restrict__ out, uint64_t len) {
+    const uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) * 4;
+    if (i + 4 <= len) {
+        T r[4], m[4];
+        using VT = typename Vec<T>::type;
+        constexpr int V = Vec<T>::N;
+#pragma unroll
+        for (int k = 0; k < 4; k += V) {
+            *reinterpret_cast<VT *>(r + k) = *reinterpret_cast<const VT *>(re + i + k);
+            *reinterpret_cast<VT *>(m + k) = *reinterpret_cast<const VT *>(im + i + k);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) out[i + k] = make_double2(widen(r[k]), widen(m[k]));
+    } else {
+        for (uint64_t k = i; k < len; k++) out[k] = make_double2(widen(re[k]), widen(im[k]));
+    }
+}
+
 }  // namespace
+
+int launch_interleave(zc_state *st, uint64_t first, uint64_t count, void *dst) {
+    const unsigned blocks = (unsigned)((count + 1023) / 1024);
+    st->ctr.launches++;
+    if (st->prec == 64)
+        k_interleave<double><<<blocks, 256, 0, st->stream>>>((const double *)st->re + first,
+                                                             (const double *)st->im + first, (double2 *)dst, count);
+    else
+        k_interleave<float><<<blocks, 256, 0, st->stream>>>((const float *)st->re + first,
+                                                            (const float *)st->im + first, (double2 *)dst, count);
+    ZC_CUDA(cudaGetLastError());
+    return ZC_OK;
+}
 
 int launch_chunk_sums(zc_state *st, int mode, uint32_t q, size_t *nchunks_out, bool exact, double *out) {
     const uint64_t total = mode == 0 ? st->len : st->len / 2;
