@@ -154,6 +154,7 @@ int launch_single(zc_state *st, const QOp &op) {
             if (op.k == 1) return launch_1q(st, op.qs[0], op.data.data(), ex);
             if (op.k >= 3 && st->prec == 32 && (st->flags & ZC_FLAG_TENSOR))
                 return launch_block_tc(st, op.qs, op.k, op.data.data());
+            if (op.k <= kMaxRegUnitary) return launch_kq_small(st, op.qs, op.k, op.data.data(), ex);
             const void *dev = nullptr;
             if (st->prec == 64 && !ex) {  // fast f64: double-float on the FP32 pipe
                 const size_t cnt = (size_t)1 << (2 * op.k);
@@ -492,7 +493,8 @@ void consume_plan(std::vector<QOp> &q, SweepPlan &plan) {
     }
 }
 
-static bool sweepable(const QOp &op);
+// Ops of a fast f64 state that read and leave packed double-float pairs.
+static bool takes_pairs(const QOp &op) { return sweepable(op) || (op.kind == Q_UNITARY && op.k <= kMaxRegUnitary); }
 static bool sweeps_enabled(const zc_state *st);
 
 // Before any kernel other than a sweep: a state that double-float sweeps
@@ -509,8 +511,10 @@ static int run_one_sweep(zc_state *st) {
     const SweepShape sh = shape_for(st);
     SweepPlan plan;
     if (plan_sweep(st->n, st->prec, program_order(st), sh.L, sh.Hcap, q, &plan) <= 1) {
-        // nothing to batch: the per-op kernel is the same work
-        int rc = settle_form(st);
+        // nothing to batch: the per-op kernel is the same work (a permutation
+        // moves slots whatever they hold)
+        const bool perm = q.front().kind == Q_CX || q.front().kind == Q_SWAP;
+        int rc = perm ? ZC_OK : settle_form(st);
         if (rc) return rc;
         rc = launch_single(st, q.front());
         q.erase(q.begin());
@@ -527,10 +531,10 @@ static int run_one_sweep(zc_state *st) {
     if (rc) return rc;
     consume_plan(q, plan);
     // Fast f64: consecutive sweeps of one flush hand the state over as
-    // (hi, lo) float pairs; the last one (nothing sweepable queued behind
-    // it) rounds it back to f64.
+    // (hi, lo) float pairs, also to and from small dense blocks; the last one
+    // (nothing that takes pairs queued behind it) rounds it back to f64.
     const bool df = st->prec == 64 && !exact(st);
-    const bool out_df = df && !q.empty() && sweepable(q.front());
+    const bool out_df = df && !q.empty() && takes_pairs(q.front());
     plan.g.form = (st->df_resident ? kFormInDf : 0u) | (out_df ? kFormOutDf : 0u);
     rc = launch_sweep(st, plan.g, (const char *)dev, (const char *)dev + tab_off, exact(st));
     st->df_resident = out_df;
@@ -547,8 +551,15 @@ int flush(zc_state *st) {
     int rc = ZC_OK;
     while (!st->queue.empty() && rc == ZC_OK) {
         if (!sweeps_enabled(st) || !sweepable(st->queue.front())) {
-            rc = settle_form(st);
-            if (rc == ZC_OK) rc = launch_single(st, st->queue.front());
+            const QOp &op = st->queue.front();
+            if (st->prec == 64 && !exact(st) && sweeps_enabled(st) && takes_pairs(op)) {  // a small dense block
+                const bool out_df = st->queue.size() > 1 && takes_pairs(st->queue[1]);
+                rc = launch_kq_small(st, op.qs, op.k, op.data.data(), false, st->df_resident, out_df);
+                st->df_resident = out_df;
+            } else {
+                rc = settle_form(st);
+                if (rc == ZC_OK) rc = launch_single(st, op);
+            }
             st->queue.erase(st->queue.begin());
             continue;
         }

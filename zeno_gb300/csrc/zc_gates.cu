@@ -121,8 +121,8 @@ struct KqParams {
 
 constexpr int kKqTile = 2048;  // amplitudes staged per CTA iteration
 
-// Fused k-qubit unitary (kern_kq_scalar, src/state.rs:355-392): a CTA
-// stages G = 2048 / 2^k groups in shared memory (gather), each thread
+// Fused k-qubit unitary of five to seven qubits (kern_kq_scalar,
+// src/state.rs:355-392): a CTA stages G = 2048 / 2^k groups in shared memory (gather), each thread
 // forms output rows with the column sum in ascending order, then scatters.
 template <typename T, bool EXACT>
 __global__ void __launch_bounds__(kThreads) k_kq(T *__restrict__ re, T *__restrict__ im, KqParams p,
@@ -204,8 +204,164 @@ int run_kq(zc_state *st, const uint32_t *qs, uint32_t k, const void *dev_mat) {
     return ZC_OK;
 }
 
-// Fused k-qubit unitary on an f64 state in fast mode: the same gather /
-// row sums / scatter as k_kq, in double-float arithmetic on the FP32 pipe
+// Blocks of up to four qubits, a group per thread: the 2^K amplitudes stay in
+// registers, each output row is summed and stored at once, and the matrix
+// comes as a kernel parameter (constant bank: uniform loads, no shared memory,
+// no barriers). Staging groups in shared memory (k_kq below five qubits
+// before) spent more on the staging than on the sums.
+// The sums are k_kq's, column by column, so results are the same bits.
+template <typename T, int K>
+struct KqMat {
+    T re[1 << (2 * K)], im[1 << (2 * K)];
+};
+struct KqQubits {
+    uint32_t q[4];
+};
+
+template <int K>
+__device__ __forceinline__ uint64_t kq_offset(const KqQubits &qs, int j) {
+    uint64_t o = 0;
+#pragma unroll
+    for (int b = 0; b < K; b++)
+        if ((j >> b) & 1) o |= 1ull << qs.q[b];
+    return o;
+}
+
+template <typename T, bool EXACT, int K>
+__global__ void __launch_bounds__(kThreads) k_kq_reg(T *__restrict__ re, T *__restrict__ im, uint64_t groups,
+                                                     const KqQubits qs, const __grid_constant__ KqMat<T, K> m) {
+    constexpr int D = 1 << K;
+    for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < groups;
+         g += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t base = insert_zeros(g, qs.q, K);
+        T xr[D], xi[D];
+#pragma unroll
+        for (int j = 0; j < D; j++) {
+            const uint64_t i = base | kq_offset<K>(qs, j);
+            xr[j] = re[i];
+            xi[j] = im[i];
+        }
+#pragma unroll 1
+        for (int r = 0; r < D; r++) {  // (unrolled, the compiler takes minutes over it)
+            T ar = T(0), ai = T(0);
+#pragma unroll
+            for (int c = 0; c < D; c++) cmac<T, EXACT>(m.re[r * D + c], m.im[r * D + c], xr[c], xi[c], ar, ai);
+            const uint64_t i = base | kq_offset<K>(qs, r);
+            re[i] = ar;
+            im[i] = ai;
+        }
+    }
+}
+
+template <typename T, bool EXACT, int K>
+int run_kq_reg(zc_state *st, const uint32_t *qs, const double *mat) {
+    KqMat<T, K> m;
+    for (int i = 0; i < 1 << (2 * K); i++) {
+        m.re[i] = (T)mat[2 * i];
+        m.im[i] = (T)mat[2 * i + 1];
+    }
+    KqQubits q{};
+    for (int b = 0; b < K; b++) q.q[b] = qs[b];
+    const uint64_t groups = st->len >> K;
+    Launch L = grid_for(st, groups);
+    k_kq_reg<T, EXACT, K><<<L.blocks, L.threads, 0, st->stream>>>((T *)st->re, (T *)st->im, groups, q, m);
+    ZC_CUDA(cudaGetLastError());
+    return ZC_OK;
+}
+
+template <typename T, bool EXACT>
+int run_kq_small(zc_state *st, const uint32_t *qs, uint32_t k, const double *mat) {
+    return k == 2   ? run_kq_reg<T, EXACT, 2>(st, qs, mat)
+           : k == 3 ? run_kq_reg<T, EXACT, 3>(st, qs, mat)
+                    : run_kq_reg<T, EXACT, 4>(st, qs, mat);
+}
+
+// The same on an f64 state in fast mode, in double-float on the FP32 pipe: an
+// amplitude is a packed pair H = (re hi, im hi), L = (re lo, im lo), and a row
+// keeps A = sum w_re * x and B = sum w_im * x, each one packed stream of
+// unnormalised axpys (10 instructions per entry for both halves), renormalised
+// every eight terms; the row is (A.re - B.im, A.im + B.re).
+// in_df / out_df: the slots hold packed pairs on entry / exit, as sweeps hand
+// them over, instead of f64 (a conversion costs as much as two entries).
+// Measured at 22 qubits, K = 3: 132 us per block staged through shared memory,
+// 54 here.
+template <int K>
+struct KqMatDf {
+    float2 rh[1 << (2 * K)], rl[1 << (2 * K)], ih[1 << (2 * K)], il[1 << (2 * K)];  // each value twice
+};
+
+template <int K, bool IN_DF, bool OUT_DF>
+__global__ void __launch_bounds__(kThreads, 2) k_kq_reg_df(double *__restrict__ re, double *__restrict__ im,
+                                                           uint64_t groups, const KqQubits qs,
+                                                           const __grid_constant__ KqMatDf<K> m) {
+    constexpr int D = 1 << K;
+    for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < groups;
+         g += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t base = insert_zeros(g, qs.q, K);
+        float2 H[D], L[D];
+#pragma unroll
+        for (int j = 0; j < D; j++) {
+            const uint64_t i = base | kq_offset<K>(qs, j);
+            if (IN_DF) {
+                H[j] = reinterpret_cast<const float2 *>(re)[i];
+                L[j] = reinterpret_cast<const float2 *>(im)[i];
+            } else {
+                pk_from_f64(re[i], im[i], H[j], L[j]);
+            }
+        }
+#pragma unroll 1
+        for (int r = 0; r < D; r++) {
+            float2 AH = make_float2(0.f, 0.f), AL = AH, BH = AH, BL = AH;
+#pragma unroll
+            for (int c = 0; c < D; c++) {
+                pk_axpy_u(m.rh[r * D + c], m.rl[r * D + c], AH, AL, H[c], L[c], AH, AL);
+                pk_axpy_u(m.ih[r * D + c], m.il[r * D + c], BH, BL, H[c], L[c], BH, BL);
+                if ((c & 7) == 7) {
+                    pk_renorm(AH, AL);
+                    pk_renorm(BH, BL);
+                }
+            }
+            float er, ei;
+            const float sr = two_sum(AH.x, -BH.y, er), si = two_sum(AH.y, BH.x, ei);
+            float2 YH = make_float2(sr, si);
+            float2 YL = make_float2(__fadd_rn(er, __fsub_rn(AL.x, BL.y)), __fadd_rn(ei, __fadd_rn(AL.y, BL.x)));
+            const uint64_t i = base | kq_offset<K>(qs, r);
+            if (OUT_DF) {
+                pk_renorm(YH, YL);
+                reinterpret_cast<float2 *>(re)[i] = YH;
+                reinterpret_cast<float2 *>(im)[i] = YL;
+            } else {
+                pk_to_f64(YH, YL, re[i], im[i]);
+            }
+        }
+    }
+}
+
+template <int K>
+int run_kq_reg_df(zc_state *st, const uint32_t *qs, const double *mat, bool in_df, bool out_df) {
+    KqMatDf<K> m;
+    auto split = [](double x, float2 *hi, float2 *lo) {
+        const float h = (float)x, l = (float)(x - (double)h);
+        *hi = make_float2(h, h);
+        *lo = make_float2(l, l);
+    };
+    for (int i = 0; i < 1 << (2 * K); i++) {
+        split(mat[2 * i], &m.rh[i], &m.rl[i]);
+        split(mat[2 * i + 1], &m.ih[i], &m.il[i]);
+    }
+    KqQubits q{};
+    for (int b = 0; b < K; b++) q.q[b] = qs[b];
+    const uint64_t groups = st->len >> K;
+    Launch L = grid_for(st, groups);
+    auto k = in_df ? (out_df ? k_kq_reg_df<K, true, true> : k_kq_reg_df<K, true, false>)
+                   : (out_df ? k_kq_reg_df<K, false, true> : k_kq_reg_df<K, false, false>);
+    k<<<L.blocks, L.threads, 0, st->stream>>>((double *)st->re, (double *)st->im, groups, q, m);
+    ZC_CUDA(cudaGetLastError());
+    return ZC_OK;
+}
+
+// Fused k-qubit unitary of five to seven qubits on an f64 state in fast mode: the
+// same gather / row sums / scatter as k_kq, in double-float arithmetic on the FP32 pipe
 // (GB300 issues FP64 ~68x slower than FP32). Amplitudes are split into
 // (hi, lo) pairs as they are staged; the matrix comes pre-split as float4
 // (re hi, re lo, im hi, im lo) per entry. Each output is a complex dot
@@ -511,13 +667,27 @@ int launch_1q(zc_state *st, uint32_t q, const double *m8, bool exact) {
     return exact ? run_1q<float, AR_EXACT>(st, q, m8) : run_1q<float, AR_FMA>(st, q, m8);
 }
 
+int launch_kq_small(zc_state *st, const uint32_t *qs, uint32_t k, const double *mat, bool exact, bool in_df,
+                    bool out_df) {
+    ProfScope ps(st, K_KQ, 2.0 * st->len * (st->prec / 8) * 2);
+    st->ctr.launches++;
+    st->ctr.sweeps++;
+    st->ctr.bytes_moved += 2 * st->len * (st->prec / 8) * 2;
+    if (st->prec == 64 && !exact)
+        return k == 2   ? run_kq_reg_df<2>(st, qs, mat, in_df, out_df)
+               : k == 3 ? run_kq_reg_df<3>(st, qs, mat, in_df, out_df)
+                        : run_kq_reg_df<4>(st, qs, mat, in_df, out_df);
+    if (in_df || out_df) return fail(ZC_ERR_INVALID, "double-float hand-over requested outside double-float blocks");
+    if (st->prec == 64) return run_kq_small<double, true>(st, qs, k, mat);
+    return exact ? run_kq_small<float, true>(st, qs, k, mat) : run_kq_small<float, false>(st, qs, k, mat);
+}
+
 int launch_kq(zc_state *st, const uint32_t *qs, uint32_t k, const void *dev_mat, bool exact) {
     ProfScope ps(st, K_KQ, 2.0 * st->len * (st->prec / 8) * 2);
     st->ctr.launches++;
     st->ctr.sweeps++;
     st->ctr.bytes_moved += 2 * st->len * (st->prec / 8) * 2;
-    if (st->prec == 64)
-        return exact ? run_kq<double, true>(st, qs, k, dev_mat) : run_kq<double, false>(st, qs, k, dev_mat);
+    if (st->prec == 64) return run_kq<double, true>(st, qs, k, dev_mat);  // fast: launch_kq_df
     return exact ? run_kq<float, true>(st, qs, k, dev_mat) : run_kq<float, false>(st, qs, k, dev_mat);
 }
 

@@ -117,8 +117,13 @@ int plan_state(uint32_t n, int prec, uint64_t budget);
 int create_state(uint32_t n, int prec, uint32_t flags, uint64_t budget, zc_state **out);
 
 int launch_1q(zc_state *st, uint32_t q, const double *m8, bool exact);
+// Dense blocks of 2 to kMaxRegUnitary qubits, a group per thread; mat: row-major
+// interleaved complex. in_df / out_df (fast f64): packed pairs in the slots.
+constexpr uint32_t kMaxRegUnitary = 4;
+int launch_kq_small(zc_state *st, const uint32_t *qs, uint32_t k, const double *mat, bool exact, bool in_df = false,
+                    bool out_df = false);
 int launch_kq(zc_state *st, const uint32_t *qs, uint32_t k, const void *dev_mat, bool exact);
-// Dense k-qubit block (k = 2..7) on an f64 state in fast mode, double-float
+// Dense k-qubit block (k = 5..7) on an f64 state in fast mode, double-float
 // on the FP32 pipe; dev_mat_df: row-major 2^k x 2^k float4 (re hi, re lo,
 // im hi, im lo) per entry.
 int launch_kq_df(zc_state *st, const uint32_t *qs, uint32_t k, const void *dev_mat_df);
