@@ -228,7 +228,7 @@ __device__ __forceinline__ uint64_t kq_offset(const KqQubits &qs, int j) {
 }
 
 template <typename T, bool EXACT, int K>
-__global__ void __launch_bounds__(kThreads) k_kq_reg(T *__restrict__ re, T *__restrict__ im, uint64_t groups,
+__global__ void __launch_bounds__(kThreads, 2) k_kq_reg(T *__restrict__ re, T *__restrict__ im, uint64_t groups,
                                                      const KqQubits qs, const __grid_constant__ KqMat<T, K> m) {
     constexpr int D = 1 << K;
     for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < groups;

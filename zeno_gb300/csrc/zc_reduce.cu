@@ -19,8 +19,15 @@
 namespace zc {
 namespace {
 
-// |a|^2 in f64 exactly as `r * r + im * im` after widening (no FMA).
-__device__ __forceinline__ double p2(double r, double i) { return radd(rmul(r, r), rmul(i, i)); }
+// |a|^2 in f64 exactly as `r * r + im * im` after widening (no FMA); the
+// squares on the integer pipe where they can be (zc_softmul.h).
+__device__ __forceinline__ double p2(double r, double i) {
+    if (soft_ok_right(f64_bits(r)) && soft_ok_right(f64_bits(i))) {
+        const uint64_t a = f64_bits(r), b = f64_bits(i);
+        return radd(soft_product(soft_left(a), soft_right(a)), soft_product(soft_left(b), soft_right(b)));
+    }
+    return radd(rmul(r, r), rmul(i, i));
+}
 
 // Non-negative doubles order like their IEEE bit patterns.
 __device__ __forceinline__ unsigned long long dkey(double x) { return (unsigned long long)__double_as_longlong(x); }

@@ -208,13 +208,14 @@ __device__ __forceinline__ void hl_cscale_df(float2 wr, float2 wi, float2 &H, fl
     pk_join(ar, ai, H, L);
 }
 
-// The kernel's register group size: f64 states outside FMA mode spill at the
+// The kernel's register group size: double-float sweeps spill at the
 // 80-register cap with more than two general ops (rotations: three); f32
 // states run groups of two as 8-byte vectors of element pairs (measured
-// faster than scalar groups of three, which spill as vectors).
+// faster than scalar groups of three, which spill as vectors); exact f64
+// gates are long enough one at a time (~400 integer instructions per pair).
 template <typename T, int A>
 __host__ __device__ constexpr int max_group_of() {
-    return sizeof(T) == 4 ? 2 : (A != AR_FMA ? 2 : 3);
+    return A == AR_EXACT && sizeof(T) == 8 ? 1 : 2;
 }
 
 template <typename R>
@@ -637,6 +638,22 @@ __device__ void apply_ops(R *sr, R *si, const OpHead *ops, const OpCoef<T, A> *c
                     const uint32_t v0 = swz<(int)sizeof(R)>(insert_zero32(p, b)), v1 = v0 ^ bs;
                     if constexpr (A == AR_DF) hl_rdf(r, sr[v0], si[v0], sr[v1], si[v1]);
                     else pair_update_real<T>(r, sr[v0], si[v0], sr[v1], si[v1]);
+                }
+                __syncthreads();
+                continue;
+            }
+            if constexpr (A == AR_EXACT && sizeof(T) == 8) {
+                const double *m = coef[o].v;
+                const ExactMask mask = exact_mask(m);
+#pragma unroll 1
+                for (uint32_t p = tid; p < size / 2; p += nt) {
+                    const uint32_t v0 = swz<(int)sizeof(R)>(insert_zero32(p, b)), v1 = v0 ^ bs;
+                    double ar = sr[v0], ai = si[v0], br = sr[v1], bi = si[v1];
+                    pair_update_f64(m, mask, ar, ai, br, bi);
+                    sr[v0] = ar;
+                    si[v0] = ai;
+                    sr[v1] = br;
+                    si[v1] = bi;
                 }
                 __syncthreads();
                 continue;
