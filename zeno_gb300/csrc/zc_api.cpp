@@ -120,11 +120,18 @@ static int check_support(const zc_state *st, const uint32_t *qs, uint32_t k, uin
 static inline bool exact(const zc_state *st) { return (st->flags & ZC_FLAG_FAST) == 0; }
 
 
-static int sync_read_scalar(zc_state *st, double *out) {
-    ZC_CUDA(cudaMemcpyAsync(st->h_scalar, st->d_scalar, sizeof(double), cudaMemcpyDeviceToHost, st->stream));
+int sync_status(zc_state *st) {
+    ZC_CUDA(cudaMemcpyAsync(st->h_scalar, st->d_scalar, kStatusErr + kErrWords * sizeof(int), cudaMemcpyDeviceToHost,
+                            st->stream));
     ZC_CUDA(cudaStreamSynchronize(st->stream));
+    const int *h = (const int *)((const char *)st->h_scalar + kStatusErr);
+    return h[0] ? check_device_error(st) : ZC_OK;  // a kernel that gave up leaves a wrong state behind
+}
+
+static int sync_read_scalar(zc_state *st, double *out) {
+    const int rc = sync_status(st);
     *out = *st->h_scalar;
-    return check_device_error(st);  // a kernel that gave up leaves a wrong state behind
+    return rc;
 }
 
 static int grow(void **p, size_t *cap, size_t need) {
@@ -796,7 +803,6 @@ void free_kit(Kit &k) {
     if (k.d_scalar) cudaFree(k.d_scalar);
     if (k.h_scalar) cudaFreeHost(k.h_scalar);
     if (k.d_samp) cudaFree(k.d_samp);
-    if (k.d_err) cudaFree(k.d_err);
     if (k.stream) cudaStreamDestroy(k.stream);
     k = Kit{};
 }
@@ -879,11 +885,11 @@ int zc::create_state(uint32_t n, int prec, uint32_t flags, uint64_t budget, zc_s
         TRY(cudaMallocHost(&st->arena.host, kArenaBytes));
         TRY(cudaMalloc(&st->arena.dev, kArenaBytes));
         st->arena.cap = kArenaBytes;
-        TRY(cudaMalloc(&st->d_scalar, sizeof(double)));
-        TRY(cudaMalloc(&st->d_err, kErrWords * sizeof(int)));
-        TRY(cudaMallocHost(&st->h_scalar, sizeof(double)));
+        TRY(cudaMalloc(&st->d_scalar, kStatusBytes));
+        st->d_err = (int *)((char *)st->d_scalar + kStatusErr);
+        TRY(cudaMallocHost(&st->h_scalar, kStatusBytes));
     }
-    TRY(cudaMemsetAsync(st->d_err, 0, kErrWords * sizeof(int), st->stream));
+    TRY(cudaMemsetAsync(st->d_scalar, 0, kStatusBytes, st->stream));
 #undef TRY
     rc = launch_reset(st);
     if (rc) {
@@ -960,10 +966,7 @@ int zc_prob_one(zc_state *st, uint32_t q, double *out) {
     if (q >= st->n) return fail(ZC_ERR_INVALID, "prob_one: qubit out of range");
     int rc = flush(st);
     if (rc) return rc;
-    size_t nch = 0;
-    rc = launch_chunk_sums(st, 1, q, &nch, exact(st));
-    if (rc) return rc;
-    rc = launch_serial_sum(st, nch, exact(st));
+    rc = launch_total(st, true, q, exact(st));
     if (rc) return rc;
     return sync_read_scalar(st, out);
 }
@@ -991,10 +994,7 @@ int zc_norm_sqr(zc_state *st, double *out) {
     if (!st || !out) return fail(ZC_ERR_INVALID, "null argument");
     int rc = flush(st);
     if (rc) return rc;
-    size_t nch = 0;
-    rc = launch_chunk_sums(st, 0, 0, &nch, exact(st));
-    if (rc) return rc;
-    rc = launch_serial_sum(st, nch, exact(st));
+    rc = launch_total(st, false, 0, exact(st));
     if (rc) return rc;
     return sync_read_scalar(st, out);
 }
@@ -1021,8 +1021,7 @@ int zc_sample(zc_state *st, uint64_t shots, uint64_t seed, uint64_t *out) {
     rc = sample_launch_pass2(st, route, (char *)st->d_samp, &d_out);
     if (rc) return rc;
     ZC_CUDA(cudaMemcpyAsync(out, d_out, shots * sizeof(uint64_t), cudaMemcpyDeviceToHost, st->stream));
-    ZC_CUDA(cudaStreamSynchronize(st->stream));
-    return check_device_error(st);
+    return sync_status(st);
 }
 
 int zc_statevector(zc_state *st, double *out) {
@@ -1043,8 +1042,7 @@ int zc_statevector(zc_state *st, double *out) {
         ZC_CUDA(cudaMemcpyAsync(out + 2 * i, st->arena.dev, count * 2 * sizeof(double), cudaMemcpyDeviceToHost,
                                 st->stream));
     }
-    ZC_CUDA(cudaStreamSynchronize(st->stream));
-    return check_device_error(st);
+    return sync_status(st);
 }
 
 int zc_load_state(zc_state *st, const double *in) {
@@ -1071,9 +1069,8 @@ int zc_finish(zc_state *st) {
     if (!st) return fail(ZC_ERR_INVALID, "null state");
     int rc = flush(st);
     if (rc) return rc;
-    ZC_CUDA(cudaStreamSynchronize(st->stream));
     ZC_CUDA(cudaGetLastError());
-    return check_device_error(st);
+    return sync_status(st);
 }
 
 int zc_get_stream(zc_state *st, void **stream) {

@@ -25,6 +25,9 @@ constexpr int kMaxUnitaryQubits = 7;
 constexpr int kMaxDiagQubits = 12;
 constexpr int kSampleChunkLog2 = 16;  // sample.rs CHUNK = 1 << 16
 constexpr int kErrWords = 16;         // device error record (d_err) in ints
+// A state's status block (d_scalar): the scalar result, the device error
+// record and a ticket for one-launch sums; one copy reads result and record.
+constexpr size_t kStatusErr = 64, kStatusTicket = 128, kStatusBytes = 256;
 
 // Device parameter arena: tables (matrices, diagonals) for queued ops are
 // staged in pinned host memory and copied into a device ring. Wrapping the
@@ -81,11 +84,11 @@ struct zc_state {
     // scratch for reductions and the sampler
     double *d_part = nullptr;  // chunk partial sums
     size_t part_cap = 0;
-    double *d_scalar = nullptr;  // single result
-    double *h_scalar = nullptr;  // pinned
+    double *d_scalar = nullptr;  // status block: the single result at its start
+    double *h_scalar = nullptr;  // pinned copy of it
     void *d_samp = nullptr;      // sampler work area
     size_t samp_cap = 0;
-    int *d_err = nullptr;        // device error record
+    int *d_err = nullptr;        // device error record, inside the status block
     bool df_resident = false;    // inside a flush: fast f64 sweeps left packed float pairs in re / im
     std::vector<zc::QOp> queue;  // ops waiting to be scheduled into sweeps
     bool prof = false;            // record CUDA events around every launch
@@ -111,6 +114,9 @@ struct ProfScope {
 // up on a bounded wait or found an index out of range): ZC_ERR_CUDA with
 // the record's text, and the record cleared; else ZC_OK.
 int check_device_error(zc_state *st);
+// The same where the stream is not yet synchronised: reads the status block
+// with one copy and one synchronisation (h_scalar[0] is the scalar result).
+int sync_status(zc_state *st);
 // mem::plan against `budget` bytes (ZC_ERR_MEMORY with zeno's text), and
 // zc_create_ex with that budget in place of 0.75 of the device memory.
 int plan_state(uint32_t n, int prec, uint64_t budget);
@@ -141,8 +147,9 @@ int launch_collapse(zc_state *st, uint32_t q, int outcome, double scale64);
 // mode 0: all amplitudes (norm / sampler pass 1); mode 1: the q=1 half of
 // qubit q (prob_one). Writes nchunks partials to `out` (default st->d_part).
 int launch_chunk_sums(zc_state *st, int mode, uint32_t q, size_t *nchunks, bool exact, double *out = nullptr);
-// Sum of st->d_part[0..nchunks) into st->d_scalar (exact: serial, in order).
-int launch_serial_sum(zc_state *st, size_t nchunks, bool exact);
+// Sum of |amp|^2 over all amplitudes, or the ones half of qubit q, into
+// st->d_scalar (exact: the chunk partials serially, in order).
+int launch_total(zc_state *st, bool ones, uint32_t q, bool exact);
 // Sampler pass 2 (sample.rs:64-108): a touched chunk and its draws.
 struct SampleChunk {
     uint64_t chunk;  // chunk index

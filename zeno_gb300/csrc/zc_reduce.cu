@@ -19,15 +19,8 @@
 namespace zc {
 namespace {
 
-// |a|^2 in f64 exactly as `r * r + im * im` after widening (no FMA); the
-// squares on the integer pipe where they can be (zc_softmul.h).
-__device__ __forceinline__ double p2(double r, double i) {
-    if (soft_ok_right(f64_bits(r)) && soft_ok_right(f64_bits(i))) {
-        const uint64_t a = f64_bits(r), b = f64_bits(i);
-        return radd(soft_product(soft_left(a), soft_right(a)), soft_product(soft_left(b), soft_right(b)));
-    }
-    return radd(rmul(r, r), rmul(i, i));
-}
+// |a|^2 in f64 exactly as `r * r + im * im` after widening (no FMA).
+__device__ __forceinline__ double p2(double r, double i) { return radd(rmul(r, r), rmul(i, i)); }
 
 // Non-negative doubles order like their IEEE bit patterns.
 __device__ __forceinline__ unsigned long long dkey(double x) { return (unsigned long long)__double_as_longlong(x); }
@@ -308,15 +301,14 @@ __device__ __forceinline__ float2 block_sum_df(float2 v, float2 *red) {
     return t;
 }
 
-// One CTA per chunk (mode and index map as k_chunk_sums); f64 partials.
+// One CTA per chunk; f64 partials (the sampler's chunk masses).
 template <typename T>
 __global__ void __launch_bounds__(kDfThreads) k_chunk_sums_df(const T *__restrict__ re, const T *__restrict__ im,
-                                                              uint64_t total, uint64_t chunk, int mode, uint32_t q,
+                                                              uint64_t total, uint64_t chunk,
                                                               double *__restrict__ part) {
     __shared__ float2 red[kDfThreads / 32];
     const uint64_t lo = (uint64_t)blockIdx.x * chunk;
     const uint64_t hi = lo + chunk < total ? lo + chunk : total;
-    const uint64_t s = 1ull << q;
     float2 acc[4] = {};
     for (uint64_t h0 = lo + threadIdx.x; h0 < hi; h0 += 4 * kDfThreads) {
         T vr[4], vi[4];
@@ -325,9 +317,8 @@ __global__ void __launch_bounds__(kDfThreads) k_chunk_sums_df(const T *__restric
             const uint64_t h = h0 + (uint64_t)u * kDfThreads;
             vr[u] = vi[u] = (T)0;
             if (h < hi) {
-                const uint64_t idx = mode == 0 ? h : insert_zero(h, q) + s;
-                vr[u] = re[idx];
-                vi[u] = im[idx];
+                vr[u] = re[h];
+                vi[u] = im[h];
             }
         }
 #pragma unroll
@@ -337,13 +328,71 @@ __global__ void __launch_bounds__(kDfThreads) k_chunk_sums_df(const T *__restric
     if (threadIdx.x == 0) part[blockIdx.x] = df_to_f64(t);
 }
 
-// Sum of n f64 partials into *out (one CTA).
-__global__ void __launch_bounds__(kDfThreads) k_sum_df(const double *__restrict__ part, uint64_t n, double *out) {
+// The whole sum (norm_sqr; ONES: the q = 1 half, prob_one) in one launch: CTAs
+// stride over 16-byte vectors, four in flight per thread and array, and the
+// last one to finish (a ticket) adds the CTAs' partials. A qubit whose halves
+// alternate inside a vector reads everything and keeps its elements; DRAM
+// moves whole sectors either way.
+// Bound by HBM. One CTA per 2^16 elements and a second launch took 124 us for
+// prob_one at 25 qubits (f64, 268 MB), this and one readback instead of two 79.
+template <typename T, bool ONES>
+__global__ void __launch_bounds__(kDfThreads) k_total_df(const T *__restrict__ re, const T *__restrict__ im,
+                                                         uint64_t units, uint32_t q, double *__restrict__ part,
+                                                         unsigned *__restrict__ ticket, double *__restrict__ out) {
     __shared__ float2 red[kDfThreads / 32];
-    float2 acc = make_float2(0.f, 0.f);
-    for (uint64_t i = threadIdx.x; i < n; i += kDfThreads) acc = df_add(acc, df_from_f64(part[i]));
-    const float2 t = block_sum_df(acc, red);
-    if (threadIdx.x == 0) *out = df_to_f64(t);
+    __shared__ bool s_last;
+    using VT = typename Vec<T>::type;
+    constexpr int V = Vec<T>::N, U = 4;
+    const bool inside = ONES && (1u << q) < (uint32_t)V;  // both halves in every vector
+    const uint64_t stride = (uint64_t)gridDim.x * kDfThreads;
+    float2 acc[U] = {};
+    auto element = [&](uint64_t u) {  // first element of vector u of the sum
+        return ONES && !inside ? insert_zero(u * V, q) + (1ull << q) : u * V;
+    };
+    for (uint64_t u0 = blockIdx.x * (uint64_t)kDfThreads + threadIdx.x; u0 < units; u0 += U * stride) {
+        VT vr[U], vi[U];
+#pragma unroll
+        for (int k = 0; k < U; k++)
+            if (u0 + k * stride < units) {
+                const uint64_t i = element(u0 + k * stride);
+                vr[k] = *reinterpret_cast<const VT *>(re + i);
+                vi[k] = *reinterpret_cast<const VT *>(im + i);
+            }
+#pragma unroll
+        for (int k = 0; k < U; k++)
+            if (u0 + k * stride < units) {
+                const T *r = reinterpret_cast<const T *>(&vr[k]), *m = reinterpret_cast<const T *>(&vi[k]);
+#pragma unroll
+                for (int e = 0; e < V; e++)
+                    if (!inside || ((e >> q) & 1)) acc[k] = df_add(acc[k], p2_df(r[e], m[e]));
+            }
+    }
+    const float2 t = block_sum_df(df_add(df_add(acc[0], acc[1]), df_add(acc[2], acc[3])), red);
+    if (threadIdx.x == 0) {
+        part[blockIdx.x] = df_to_f64(t);
+        __threadfence();
+        s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    float2 a = make_float2(0.f, 0.f);
+    for (uint32_t i = threadIdx.x; i < gridDim.x; i += kDfThreads) a = df_add(a, df_from_f64(__ldcg(part + i)));
+    const float2 sum = block_sum_df(a, red);
+    if (threadIdx.x == 0) {
+        *out = df_to_f64(sum);
+        *ticket = 0;  // for the next launch on this stream
+    }
+}
+
+template <typename T>
+__global__ void k_total_small(const T *re, const T *im, uint64_t total, int ones, uint32_t q, double *out) {
+    float2 a = make_float2(0.f, 0.f);  // states shorter than a vector
+    for (uint64_t h = 0; h < total; h++) {
+        const uint64_t i = ones ? insert_zero(h, q) + (1ull << q) : h;
+        a = df_add(a, p2_df(re[i], im[i]));
+    }
+    *out = df_to_f64(a);
 }
 
 // Sampler pass 2, one CTA per touched chunk: tiles of 2048 elements get a
@@ -506,13 +555,14 @@ int launch_chunk_sums(zc_state *st, int mode, uint32_t q, size_t *nchunks_out, b
     ProfScope ps(st, K_CHUNK_SUMS, (mode == 0 ? 1.0 : 0.5) * st->len * (st->prec / 8) * 2);
     st->ctr.launches++;
     *nchunks_out = nch;
-    if (!exact) {
+    if (!exact) {  // only whole-state masses: prob_one is launch_total's
+        if (mode != 0) return fail(ZC_ERR_INVALID, "fast chunk sums cover whole states");
         if (st->prec == 64)
             k_chunk_sums_df<double><<<(unsigned)nch, kDfThreads, 0, st->stream>>>(
-                (const double *)st->re, (const double *)st->im, total, chunk, mode, q, part);
+                (const double *)st->re, (const double *)st->im, total, chunk, part);
         else
             k_chunk_sums_df<float><<<(unsigned)nch, kDfThreads, 0, st->stream>>>(
-                (const float *)st->re, (const float *)st->im, total, chunk, mode, q, part);
+                (const float *)st->re, (const float *)st->im, total, chunk, part);
         ZC_CUDA(cudaGetLastError());
         return ZC_OK;
     }
@@ -521,17 +571,47 @@ int launch_chunk_sums(zc_state *st, int mode, uint32_t q, size_t *nchunks_out, b
     return run_chain<float, false>(st, total, chunk, nch, mode, q, nullptr, nullptr, part, nullptr, 0);
 }
 
-int launch_serial_sum(zc_state *st, size_t nchunks, bool exact) {
-    ProfScope ps(st, K_SERIAL_SUM, 8.0 * nchunks);
-    st->ctr.launches++;
-    if (exact)
-        k_chain<double, false><<<1, kChainThreads, 0, st->stream>>>(st->d_part, nullptr, nchunks, nchunks, 2, 0,
-                                                                    nullptr, nullptr, st->d_scalar, nullptr, nullptr,
-                                                                    nullptr, 0);
-    else
-        k_sum_df<<<1, kDfThreads, 0, st->stream>>>(st->d_part, nchunks, st->d_scalar);
+template <typename T>
+int run_total(zc_state *st, bool ones, uint32_t q) {
+    constexpr uint64_t V = Vec<T>::N;
+    const T *re = (const T *)st->re, *im = (const T *)st->im;
+    unsigned *ticket = (unsigned *)((char *)st->d_scalar + kStatusTicket);
+    if (st->len < 2 * V) {
+        k_total_small<T><<<1, 1, 0, st->stream>>>(re, im, ones ? st->len / 2 : st->len, ones, q, st->d_scalar);
+    } else {
+        const uint64_t units = (ones && (1ull << q) >= V ? st->len / 2 : st->len) / V;
+        const uint64_t want = (units + kDfThreads - 1) / kDfThreads, cap = (uint64_t)st->num_sms * 8;
+        const unsigned blocks = (unsigned)std::min(want, cap);
+        if (blocks > st->part_cap) {
+            if (st->d_part) cudaFree(st->d_part);
+            st->d_part = nullptr;
+            st->part_cap = 0;
+            ZC_CUDA(cudaMalloc(&st->d_part, cap * sizeof(double)));
+            st->part_cap = cap;
+        }
+        if (ones) k_total_df<T, true><<<blocks, kDfThreads, 0, st->stream>>>(re, im, units, q, st->d_part, ticket, st->d_scalar);
+        else k_total_df<T, false><<<blocks, kDfThreads, 0, st->stream>>>(re, im, units, q, st->d_part, ticket, st->d_scalar);
+    }
     ZC_CUDA(cudaGetLastError());
     return ZC_OK;
+}
+
+int launch_total(zc_state *st, bool ones, uint32_t q, bool exact) {
+    if (exact) {  // chunk chains, then the chunks in order
+        size_t nch = 0;
+        const int rc = launch_chunk_sums(st, ones ? 1 : 0, q, &nch, true);
+        if (rc) return rc;
+        ProfScope ps(st, K_SERIAL_SUM, 8.0 * nch);
+        st->ctr.launches++;
+        k_chain<double, false><<<1, kChainThreads, 0, st->stream>>>(st->d_part, nullptr, nch, nch, 2, 0, nullptr,
+                                                                    nullptr, st->d_scalar, nullptr, nullptr, nullptr,
+                                                                    0);
+        ZC_CUDA(cudaGetLastError());
+        return ZC_OK;
+    }
+    ProfScope ps(st, K_CHUNK_SUMS, (ones ? 0.5 : 1.0) * st->len * (st->prec / 8) * 2);
+    st->ctr.launches++;
+    return st->prec == 64 ? run_total<double>(st, ones, q) : run_total<float>(st, ones, q);
 }
 
 int launch_sample_scan(zc_state *st, const SampleChunk *d_chunks, size_t nchunks, const double *d_us,
