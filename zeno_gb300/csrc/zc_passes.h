@@ -53,9 +53,9 @@ ZC_HD int group_at(const OpHead *ops, int o, int nops, int max_group, bool *rot3
     return g;
 }
 
-// Register passes of double-float sweeps, resolved once per job.
+// Register passes of double-float and f32 sweeps, resolved once per job.
 //
-// A pass is a register group (one to three one-qubit ops on distinct tile
+// A pass is a register group (one to four one-qubit ops on distinct tile
 // bits, as group_at forms them) together with the table diagonal right
 // before it and, before that, a block of CX ops whose targets are all group
 // bits. The diagonal scales each element before the gates, exactly as its
@@ -70,13 +70,13 @@ ZC_HD int group_at(const OpHead *ops, int o, int nops, int max_group, bool *rot3
 struct GroupInfo {
     uint8_t G, rot3, skip, first;  // G = 0: no pass starts at this op
     uint8_t nloc, nout, ntr, has_dk;
-    uint8_t sorted[3];             // group bits ascending (zero insertion)
-    uint8_t tb[3];                 // table bit of each group coordinate (0xff: not in the support)
+    uint8_t sorted[4];             // group bits ascending (zero insertion)
+    uint8_t tb[4];                 // table bit of each group coordinate (0xff: not in the support)
     uint8_t loc[8], locb[8];       // support bits outside the group -> table bit
     uint8_t outq[8], outb[8];      // outer support qubits -> table bit
     uint8_t trc[4];                // translation controls: local bit, or 0x80 | outer qubit
-    uint16_t gm[3];                // slot pattern of group coordinate g (1 << bit)
-    uint16_t pm[3];                // load pattern of coordinate g (column g of M, as slots)
+    uint16_t gm[4];                // slot pattern of group coordinate g (1 << bit)
+    uint16_t pm[4];                // load pattern of coordinate g (column g of M, as slots)
     uint16_t trw[4];               // translation patterns
     uint16_t fmask;                // store pattern of the flipped coordinates
     uint16_t so_step, lo_step, jb_step;  // for a thread's second group (set by encode_job)
@@ -132,7 +132,7 @@ inline void plan_passes(const OpHead *ops, int nops, uint32_t tile_log2, bool fo
         bool rot3;
         const int G = group_at(ops, first, nops, max_group, &rot3);
         GroupInfo &q = gi[o];
-        uint32_t bits[3] = {0, 0, 0};
+        uint32_t bits[4] = {0, 0, 0, 0};
         bool in_tile = true;
         for (int g = 0; g < G; g++) {
             bits[g] = ops[first + g].a;
@@ -152,17 +152,17 @@ inline void plan_passes(const OpHead *ops, int nops, uint32_t tile_log2, bool fo
             q.gm[g] = q.pm[g] = (uint16_t)(1u << bits[g]);
             if (ops[first + g].kind == MOP_RT && ops[first + g].b) q.fmask |= (uint16_t)(1u << bits[g]);
         }
-        uint32_t srt[3] = {bits[0], bits[1], bits[2]};
+        uint32_t srt[4] = {bits[0], bits[1], bits[2], bits[3]};
         for (int a = 1; a < G; a++)
             for (int b = a; b > 0 && srt[b] < srt[b - 1]; b--) {
                 const uint32_t x = srt[b];
                 srt[b] = srt[b - 1];
                 srt[b - 1] = x;
             }
-        for (int g = 0; g < 3; g++) q.sorted[g] = (uint8_t)srt[g];
+        for (int g = 0; g < 4; g++) q.sorted[g] = (uint8_t)srt[g];
         q.has_dk = jdk >= 0;
         q.nloc = q.nout = 0;
-        for (int g = 0; g < 3; g++) q.tb[g] = 0xff;
+        for (int g = 0; g < 4; g++) q.tb[g] = 0xff;
         if (jdk >= 0) {
             const OpHead &d = ops[jdk];
             q.tab_off = (uint32_t)d.table;
@@ -188,7 +188,7 @@ inline void plan_passes(const OpHead *ops, int nops, uint32_t tile_log2, bool fo
         // from the last CX (applied to y first) to the first
         q.ntr = 0;
         if (ncx > 0) {
-            uint32_t col[3] = {1u, 2u, 4u}, trv[kMaxFoldCx];
+            uint32_t col[4] = {1u, 2u, 4u, 8u}, trv[kMaxFoldCx];
             uint8_t trc[kMaxFoldCx];
             int ntr = 0;
             for (int i = ncx - 1; i >= 0; i--) {

@@ -37,7 +37,8 @@ constexpr uint32_t kJlutLen = 256 + kJlutHigh;
 // memory the pass descriptors take in double-float sweeps; further table
 // diagonals build theirs per tile. A table diagonal's `b` field (in the
 // CTA's copy of the micro-ops) names its job table, or kNoJobLut.
-constexpr int kJobLuts = 5;
+// (Exact f64 sweeps; f32 sweeps have both and keep kF32Luts tables.)
+constexpr int kJobLuts = 5, kF32Luts = 2;
 constexpr uint32_t kNoJobLut = 0xffffffffu;
 // The tile's re array, then, this far behind it whatever the tile's size, im.
 constexpr uint32_t kTileArrayBytes = (uint32_t)(kSweepSmemBytes / 2);
@@ -217,6 +218,13 @@ template <typename T, int A>
 __host__ __device__ constexpr int max_group_of() {
     return A == AR_EXACT && sizeof(T) == 8 ? 1 : 2;
 }
+// Sweeps with register passes (GroupInfo): double-float ones and f32 ones, the
+// latter with groups of up to four ops.
+template <typename T, int A>
+__host__ __device__ constexpr bool has_passes() {
+    return A == AR_DF || sizeof(T) == 4;
+}
+constexpr int kF32Group = 4;
 
 template <typename R>
 __device__ __forceinline__ uint32_t jgather(const OpHead &op, uint32_t jo, uint32_t v) {
@@ -537,6 +545,105 @@ __device__ void run_pass(const GroupInfo &gi, char *tile, const OpHead *ops, con
     }
 }
 
+// A pass of an f32 sweep: the same indices (4-byte slots, 8-byte table
+// entries), each element's arithmetic in the order of the ops one by one. Up to
+// four gates, a diagonal and a block of CX in one round trip through shared
+// memory, whose wavefronts bound f32 sweeps.
+template <typename T, int A, int G, bool HAS_DK, bool HAS_CX>
+__device__ __noinline__ void run_pass_f32(const GroupInfo &gi, char *tile, const OpHead *ops, const OpCoef<T, A> *coef,
+                             uint32_t size, const char *tables, uint64_t base) {
+    constexpr int E = 1 << G;
+    const int o = gi.first;
+    uint32_t jo = 0, u0 = 0;
+    if constexpr (HAS_DK) {
+        for (int i = 0; i < gi.nout; i++) jo |= (uint32_t)((base >> gi.outq[i]) & 1u) << (gi.outb[i] + 3);
+    }
+    if constexpr (HAS_CX) {
+        for (int t = 0; t < gi.ntr; t++)
+            if ((gi.trc[t] & 0x80u) && ((base >> (gi.trc[t] & 0x7fu)) & 1u)) u0 ^= gi.trw[t];
+    }
+    uint32_t so = 0, lo = 0, jb = 0;
+    for (uint32_t p = threadIdx.x; p < size / E; p += kSweepThreads) {
+        if (G == 4 && p >= kSweepThreads) {  // at most one step: tiles have 2^13 elements
+            so ^= gi.so_step;
+            lo ^= gi.lo_step;
+            jb ^= gi.jb_step;
+        } else {
+            uint32_t v = p;
+#pragma unroll
+            for (int g = 0; g < G; g++) v = insert_zero32(v, gi.sorted[g]);
+            so = lo = swz<4>(v) << 2;
+            if constexpr (HAS_CX) {
+                lo ^= u0;
+                for (int t = 0; t < gi.ntr; t++)
+                    if (!(gi.trc[t] & 0x80u) && ((v >> gi.trc[t]) & 1u)) lo ^= gi.trw[t];
+            }
+            if constexpr (HAS_DK) {
+                jb = jo;
+                for (int i = 0; i < gi.nloc; i++) jb |= ((v >> gi.loc[i]) & 1u) << (gi.locb[i] + 3);
+            }
+        }
+        float xr[E], xi[E];
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            uint32_t w = lo;
+#pragma unroll
+            for (int g = 0; g < G; g++)
+                if ((e >> g) & 1) w ^= HAS_CX ? gi.pm[g] : gi.gm[g];
+            xr[e] = *reinterpret_cast<const float *>(tile + w);
+            xi[e] = *reinterpret_cast<const float *>(tile + kTileArrayBytes + w);
+        }
+        if constexpr (HAS_DK) {
+            const char *dtab = tables + gi.tab_off;
+            uint32_t tm[G];
+#pragma unroll
+            for (int g = 0; g < G; g++) tm[g] = gi.tb[g] != 0xff ? 8u << gi.tb[g] : 0u;
+#pragma unroll
+            for (int e = 0; e < E; e++) {
+                uint32_t j = jb;
+#pragma unroll
+                for (int g = 0; g < G; g++)
+                    if ((e >> g) & 1) j ^= tm[g];
+                const float2 w = __ldg(reinterpret_cast<const float2 *>(dtab + j));
+                cscale<float, A == AR_EXACT>(w.x, w.y, xr[e], xi[e]);
+            }
+        }
+#pragma unroll
+        for (int g = 0; g < G; g++) {
+            Mat2<float> m;
+#pragma unroll
+            for (int i = 0; i < 8; i++) m.v[i] = coef[o + g].v[i];
+#pragma unroll
+            for (int e = 0; e < E; e++)
+                if (!((e >> g) & 1))
+                    pair_update<float, A == AR_EXACT>(m, xr[e], xi[e], xr[e | (1 << g)], xi[e | (1 << g)]);
+        }
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            uint32_t w = so;
+#pragma unroll
+            for (int g = 0; g < G; g++)
+                if ((e >> g) & 1) w ^= gi.gm[g];
+            *reinterpret_cast<float *>(tile + w) = xr[e];
+            *reinterpret_cast<float *>(tile + kTileArrayBytes + w) = xi[e];
+        }
+    }
+}
+
+template <typename T, int A, int G>
+__device__ void run_pass_f32_any(const GroupInfo &gi, char *tile, const OpHead *ops, const OpCoef<T, A> *coef,
+                                 uint32_t size, const char *tables, uint64_t base) {
+    bool cx = gi.ntr;
+    for (int g = 0; g < G; g++) cx |= gi.pm[g] != gi.gm[g];
+    if (gi.has_dk) {
+        if (cx) run_pass_f32<T, A, G, true, true>(gi, tile, ops, coef, size, tables, base);
+        else run_pass_f32<T, A, G, true, false>(gi, tile, ops, coef, size, tables, base);
+    } else {
+        if (cx) run_pass_f32<T, A, G, false, true>(gi, tile, ops, coef, size, tables, base);
+        else run_pass_f32<T, A, G, false, false>(gi, tile, ops, coef, size, tables, base);
+    }
+}
+
 template <typename T, int A, int G, bool ROT_ONLY>
 __device__ void run_pass_any(const GroupInfo &gi, char *tile, const OpHead *ops,
                              const OpCoef<T, A> *coef, uint32_t size, const char *tables, uint64_t base, bool in_f64,
@@ -572,6 +679,19 @@ __device__ void apply_ops(R *sr, R *si, const OpHead *ops, const OpCoef<T, A> *c
                     run_pass_any<T, A, 2, false>(gi, reinterpret_cast<char *>(sr), ops, coef, size, tables, base, in_f64, out_f64);
                 else
                     run_pass_any<T, A, 1, false>(gi, reinterpret_cast<char *>(sr), ops, coef, size, tables, base, in_f64, out_f64);
+                o += gi.skip - 1;
+                __syncthreads();
+                continue;
+            }
+        }
+        if constexpr (sizeof(T) == 4) {
+            const GroupInfo &gi = gis[o];
+            if (gi.G) {
+                char *tile = reinterpret_cast<char *>(sr);
+                if (gi.G == 4) run_pass_f32_any<T, A, 4>(gi, tile, ops, coef, size, tables, base);
+                else if (gi.G == 3) run_pass_f32_any<T, A, 3>(gi, tile, ops, coef, size, tables, base);
+                else if (gi.G == 2) run_pass_f32_any<T, A, 2>(gi, tile, ops, coef, size, tables, base);
+                else run_pass_f32_any<T, A, 1>(gi, tile, ops, coef, size, tables, base);
                 o += gi.skip - 1;
                 __syncthreads();
                 continue;
@@ -797,11 +917,10 @@ struct SweepSmem {
     JobHead job;
     uint32_t bad;
     uint16_t jlut[kJlutLen];  // diagonal index tables of the current DK op
-    // register passes (double-float sweeps), or the job's diagonal index tables
-    alignas(16) typename std::conditional<A == AR_DF, GroupInfo[kMaxMicroOps], uint16_t[kJobLuts * kJlutLen]>::type gi;
+    alignas(16) GroupInfo gi[has_passes<T, A>() ? kMaxMicroOps : 1];  // register passes
+    static constexpr int kLuts = A == AR_DF ? 0 : sizeof(T) == 4 ? kF32Luts : kJobLuts;
+    uint16_t luts[kLuts * kJlutLen + 1];  // the job's diagonal index tables
 };
-static_assert(sizeof(uint16_t[kJobLuts * kJlutLen]) <= sizeof(GroupInfo[kMaxMicroOps]),
-              "job index tables fit where the pass descriptors go");
 static_assert(sizeof(OpHead[kMaxMicroOps]) % 16 == 0 && sizeof(GroupInfo[kMaxMicroOps]) % 16 == 0,
               "job sections are copied in 16-byte pieces");
 
@@ -824,7 +943,6 @@ int encode_job_as(const SweepPlan &plan, std::vector<char> *out) {
         const MicroOp &m = plan.mops[(size_t)o];
         memcpy(&ops[(size_t)o], &m, sizeof(OpHead));
         h.has_arith |= m.kind != MOP_CX && m.kind != MOP_SWAP;
-        if (m.kind == MOP_DK) ops[(size_t)o].b = A != AR_DF && nlut < (uint32_t)kJobLuts ? nlut++ : kNoJobLut;
         const int cnt = m.kind == MOP_U1 ? 8 : m.kind == MOP_RT ? 1 : m.kind == MOP_D1 || m.kind == MOP_R1 ? 4 : 0;
         OpCoef<T, A> &c = coef[(size_t)o];
         for (int i = 0; i < cnt; i++) {
@@ -846,31 +964,48 @@ int encode_job_as(const SweepPlan &plan, std::vector<char> *out) {
         }
     }
     std::vector<GroupInfo> gi;
-    if constexpr (A == AR_DF) {
+    if constexpr (has_passes<T, A>()) {
+        constexpr int SB = sizeof(T) == 4 ? 2 : 3, JB = sizeof(T) == 4 ? 3 : 4;  // slot and table entry bytes, log2
         gi.resize((size_t)nops);
         uint32_t bad = 0;
         int fuse_in = 0, fuse_out = 0;
-        plan_passes(ops.data(), nops, h.L + h.H, true, max_group_of<T, A>(), gi.data(), &bad, &fuse_in, &fuse_out);
+        plan_passes(ops.data(), nops, h.L + h.H, true, sizeof(T) == 4 ? kF32Group : max_group_of<T, A>(), gi.data(),
+                    &bad, &fuse_in, &fuse_out);
+        if constexpr (sizeof(T) == 4) {
+            // one or two bare gates move as vectors of element pairs instead
+            for (GroupInfo &q : gi)
+                if (q.G && q.G <= 2 && q.skip == q.G && !(q.gm[0] & 1) && !(q.G == 2 && (q.gm[1] & 1))) q.G = 0;
+        }
         if (bad) return fail(ZC_ERR_INVALID, "sweep plan: a group bit lies outside the tile");
         h.fuse_in = (uint32_t)fuse_in;
         h.fuse_out = (uint32_t)fuse_out;
         for (GroupInfo &q : gi) {  // slot patterns as byte offsets into the swizzled tile, step patterns
             if (!q.G) continue;
             for (int g = 0; g < q.G; g++) {
-                q.gm[g] = (uint16_t)(swz<8>(q.gm[g]) << 3);
-                q.pm[g] = (uint16_t)(swz<8>(q.pm[g]) << 3);
+                q.gm[g] = (uint16_t)(swz<(int)sizeof(T)>(q.gm[g]) << SB);
+                q.pm[g] = (uint16_t)(swz<(int)sizeof(T)>(q.pm[g]) << SB);
             }
-            for (int i = 0; i < q.ntr; i++) q.trw[i] = (uint16_t)(swz<8>(q.trw[i]) << 3);
-            q.fmask = (uint16_t)(swz<8>(q.fmask) << 3);
+            for (int i = 0; i < q.ntr; i++) q.trw[i] = (uint16_t)(swz<(int)sizeof(T)>(q.trw[i]) << SB);
+            q.fmask = (uint16_t)(swz<(int)sizeof(T)>(q.fmask) << SB);
             uint32_t v = kSweepThreads, lo = 0, jb = 0;  // group number p + kSweepThreads against p
             for (int g = 0; g < q.G; g++) v = insert_zero32(v, q.sorted[g]);
             for (int i = 0; i < q.ntr; i++)
                 if (!(q.trc[i] & 0x80u) && ((v >> q.trc[i]) & 1u)) lo ^= q.trw[i];
-            for (int i = 0; i < q.nloc; i++) jb |= ((v >> q.loc[i]) & 1u) << (q.locb[i] + 4);
-            q.so_step = (uint16_t)(swz<8>(v) << 3);
+            for (int i = 0; i < q.nloc; i++) jb |= ((v >> q.loc[i]) & 1u) << (q.locb[i] + JB);
+            q.so_step = (uint16_t)(swz<(int)sizeof(T)>(v) << SB);
             q.lo_step = (uint16_t)(q.so_step ^ lo);
             q.jb_step = (uint16_t)jb;
         }
+    }
+    // index tables for the table diagonals that no pass takes
+    for (int o = 0; o < nops;) {
+        if (!gi.empty() && gi[(size_t)o].G) {
+            o += gi[(size_t)o].skip;
+            continue;
+        }
+        if (ops[(size_t)o].kind == MOP_DK)
+            ops[(size_t)o].b = nlut < (uint32_t)SweepSmem<T, A>::kLuts ? nlut++ : kNoJobLut;
+        o++;
     }
     auto up16 = [](size_t b) { return (b + 15) & ~(size_t)15; };
     const size_t ops_b = up16(ops.size() * sizeof(OpHead)), coef_b = up16(coef.size() * sizeof(OpCoef<T, A>));
@@ -899,7 +1034,7 @@ __device__ void load_job(SweepSmem<T, A> &c, const char *blk) {
     copy16(&c.job, blk, sizeof(JobHead));
     copy16(c.ops, blk + sizeof(JobHead), nops * (uint32_t)sizeof(OpHead));
     copy16(c.coef, blk + h->coef_off, nops * (uint32_t)sizeof(OpCoef<T, A>));
-    if constexpr (A == AR_DF) copy16(c.gi, blk + h->gi_off, nops * (uint32_t)sizeof(GroupInfo));
+    if constexpr (has_passes<T, A>()) copy16(c.gi, blk + h->gi_off, nops * (uint32_t)sizeof(GroupInfo));
     for (uint32_t r = tid; r < (1u << H); r += blockDim.x) {  // tile bit L + j holds qubit hpos[j]
         uint32_t o = 0;
         for (uint32_t j = 0; j < H; j++) o |= ((r >> j) & 1u) << (h->hpos[j] - L);
@@ -910,9 +1045,13 @@ __device__ void load_job(SweepSmem<T, A> &c, const char *blk) {
         bool any = false;
         for (uint32_t o = 0; o < nops; o++) {
             const OpHead &op = c.ops[o];
+            if (has_passes<T, A>() && c.gi[o].G) {
+                o += c.gi[o].skip - 1;
+                continue;
+            }
             if (op.kind != MOP_DK || op.b == kNoJobLut) continue;
             any = true;
-            uint16_t *lut = c.gi + (size_t)op.b * kJlutLen;
+            uint16_t *lut = c.luts + (size_t)op.b * kJlutLen;
             for (uint32_t x = tid; x < kJlutLen; x += blockDim.x)
                 lut[x] = (uint16_t)jgather<T>(op, 0u, x < 256 ? x : (x - 256) << 8);
         }
@@ -1026,7 +1165,7 @@ __device__ void process_tile(SweepSmem<T, A> &c, T *re, T *im, uint64_t t, const
             }
         }
     } else {
-        apply_ops<T, A, T>(sre, sim, c.ops, c.coef, (int)c.job.nops, base, size, tables, &c.bad, c.jlut, c.gi, nullptr);
+        apply_ops<T, A, T>(sre, sim, c.ops, c.coef, (int)c.job.nops, base, size, tables, &c.bad, c.jlut, c.luts, c.gi);
     }
     __syncthreads();
     tile_store(c, re + base, sre, vecs);
