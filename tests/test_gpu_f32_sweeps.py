@@ -1,8 +1,7 @@
 """f32 sweeps against one launch per op, bit for bit.
 
-A register pass of an f32 sweep takes up to four one-qubit gates, the table
-diagonal and the CX before them, and rounds each element as the ops one by one
-do. Bit 0 and the highest tile bit, runs that end early, controls inside and
+A register pass of an f32 sweep takes a run of gates, diagonals and CX on four
+tile bits and rounds each element as the ops one by one do. Bit 0 and the highest tile bit, runs that end early, controls inside and
 outside a group and tiles from three qubits to several tiles are in the draw.
 The tolerance is none: the bits are the same.
 """

@@ -224,8 +224,8 @@ struct SweepShape {
 // sweeps), against enough tiles for the SMs. Measured per whole zc_run
 // (depth-12 u3 + matching CX; f32: gate mix), us:
 //   exact f64, bound by each SM's FP64 pipe: 2^8 amplitudes per tile up to 15
-//   qubits (12q: 773 with 2^8, 1641 with 2^11, 1615 one launch per op), 2^9
-//   for 16-17, 2^10 for 18-21 (20q: 8133, 2^11 8924), whole tiles beyond
+//   qubits (12q: 718 with 2^8, 1322 with 2^11), 2^9 for 16-17, 2^10 for 18-21
+//   (20q: 5529, 2^11 5699), whole tiles beyond (22q: 6600)
 //   double-float: about half the qubits plus two, at least 2^8 (10q 355, one
 //   launch per op 842; 16q 544 with 2^10, 918 with 2^7; 20q 1080 with 2^12)
 //   f32: up to 13 qubits the state is one tile (10q 155, one launch per op
@@ -320,9 +320,9 @@ size_t plan_sweep(uint32_t n, int prec, bool ex, uint32_t L, uint32_t Hcap, cons
     // Order of the micro-ops. Exact mode keeps program order (reordering two
     // gates changes the rounding). Fast mode lets ops on disjoint qubits
     // commute: one-qubit ops on distinct qubits are emitted back to back, in
-    // runs the size of the kernel's register groups (three for the rotations
-    // of lowered f64 sweeps, else two: f32 groups of two move element pairs
-    // as 8-byte vectors), so the kernel applies each run in one register pass.
+    // runs (three for the rotations of lowered f64 sweeps, their register group;
+    // else two: an f32 pass takes four tile bits in whatever order, and another
+    // run length would round f32 states differently).
     const size_t run_cap = prec == 32 ? 2 : (prec == 64 && !df_lowering ? 2 : 3);
     const bool df = df_lowering;
     std::vector<LoweredOp> low;

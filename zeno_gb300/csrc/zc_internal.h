@@ -192,7 +192,7 @@ void lower_df(const std::vector<const QOp *> &seq, int run_cap, std::vector<Lowe
 int launch_single(zc_state *st, const QOp &op);
 // Launch every queued op.
 int flush(zc_state *st);
-int launch_sweep_multi(cudaStream_t stream, int num_sms, int prec, bool exact, const char *dev_blob, int *d_err);
+int launch_sweep_multi(cudaStream_t stream, int num_sms, int prec, bool exact, const char *dev_blob);
 int arena_put(zc_state *st, const void *src, size_t bytes, const void **dev);
 // Round an f64 state left as double-float pairs (g.form kFormOutDf) back to f64.
 int launch_df_to_f64(zc_state *st);

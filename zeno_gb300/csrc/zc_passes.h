@@ -1,4 +1,4 @@
-// Register passes of double-float sweeps: the micro-op head the tile loop
+// Register passes of double-float and f32 sweeps: the micro-op head the tile loop
 // reads, the pass descriptor and the planning of the passes of a job. Shared
 // by the sweep kernel (zc_sweep.cu) and the host check of the pass logic
 // (tests/passes_harness.cpp).
@@ -29,6 +29,12 @@ static_assert(sizeof(OpHead) == 72 && offsetof(MicroOp, table) == offsetof(OpHea
                   offsetof(MicroOp, m) == sizeof(OpHead),
               "OpHead is the head of MicroOp");
 
+inline int popcount32(uint32_t v) {
+    int n = 0;
+    for (; v; v &= v - 1) n++;
+    return n;
+}
+
 ZC_HD bool is_1q(uint32_t kind) { return kind == MOP_U1 || kind == MOP_R1 || kind == MOP_RT; }
 
 // The register group starting at one-qubit op o: three rotations on distinct
@@ -53,9 +59,9 @@ ZC_HD int group_at(const OpHead *ops, int o, int nops, int max_group, bool *rot3
     return g;
 }
 
-// Register passes of double-float and f32 sweeps, resolved once per job.
+// Register passes of double-float sweeps, resolved once per job.
 //
-// A pass is a register group (one to four one-qubit ops on distinct tile
+// A pass is a register group (one to three one-qubit ops on distinct tile
 // bits, as group_at forms them) together with the table diagonal right
 // before it and, before that, a block of CX ops whose targets are all group
 // bits. The diagonal scales each element before the gates, exactly as its
@@ -70,13 +76,13 @@ ZC_HD int group_at(const OpHead *ops, int o, int nops, int max_group, bool *rot3
 struct GroupInfo {
     uint8_t G, rot3, skip, first;  // G = 0: no pass starts at this op
     uint8_t nloc, nout, ntr, has_dk;
-    uint8_t sorted[4];             // group bits ascending (zero insertion)
-    uint8_t tb[4];                 // table bit of each group coordinate (0xff: not in the support)
+    uint8_t sorted[3];             // group bits ascending (zero insertion)
+    uint8_t tb[3];                 // table bit of each group coordinate (0xff: not in the support)
     uint8_t loc[8], locb[8];       // support bits outside the group -> table bit
     uint8_t outq[8], outb[8];      // outer support qubits -> table bit
     uint8_t trc[4];                // translation controls: local bit, or 0x80 | outer qubit
-    uint16_t gm[4];                // slot pattern of group coordinate g (1 << bit)
-    uint16_t pm[4];                // load pattern of coordinate g (column g of M, as slots)
+    uint16_t gm[3];                // slot pattern of group coordinate g (1 << bit)
+    uint16_t pm[3];                // load pattern of coordinate g (column g of M, as slots)
     uint16_t trw[4];               // translation patterns
     uint16_t fmask;                // store pattern of the flipped coordinates
     uint16_t so_step, lo_step, jb_step;  // for a thread's second group (set by encode_job)
@@ -132,7 +138,7 @@ inline void plan_passes(const OpHead *ops, int nops, uint32_t tile_log2, bool fo
         bool rot3;
         const int G = group_at(ops, first, nops, max_group, &rot3);
         GroupInfo &q = gi[o];
-        uint32_t bits[4] = {0, 0, 0, 0};
+        uint32_t bits[3] = {0, 0, 0};
         bool in_tile = true;
         for (int g = 0; g < G; g++) {
             bits[g] = ops[first + g].a;
@@ -152,17 +158,17 @@ inline void plan_passes(const OpHead *ops, int nops, uint32_t tile_log2, bool fo
             q.gm[g] = q.pm[g] = (uint16_t)(1u << bits[g]);
             if (ops[first + g].kind == MOP_RT && ops[first + g].b) q.fmask |= (uint16_t)(1u << bits[g]);
         }
-        uint32_t srt[4] = {bits[0], bits[1], bits[2], bits[3]};
+        uint32_t srt[3] = {bits[0], bits[1], bits[2]};
         for (int a = 1; a < G; a++)
             for (int b = a; b > 0 && srt[b] < srt[b - 1]; b--) {
                 const uint32_t x = srt[b];
                 srt[b] = srt[b - 1];
                 srt[b - 1] = x;
             }
-        for (int g = 0; g < 4; g++) q.sorted[g] = (uint8_t)srt[g];
+        for (int g = 0; g < 3; g++) q.sorted[g] = (uint8_t)srt[g];
         q.has_dk = jdk >= 0;
         q.nloc = q.nout = 0;
-        for (int g = 0; g < 4; g++) q.tb[g] = 0xff;
+        for (int g = 0; g < 3; g++) q.tb[g] = 0xff;
         if (jdk >= 0) {
             const OpHead &d = ops[jdk];
             q.tab_off = (uint32_t)d.table;
@@ -188,7 +194,7 @@ inline void plan_passes(const OpHead *ops, int nops, uint32_t tile_log2, bool fo
         // from the last CX (applied to y first) to the first
         q.ntr = 0;
         if (ncx > 0) {
-            uint32_t col[4] = {1u, 2u, 4u, 8u}, trv[kMaxFoldCx];
+            uint32_t col[3] = {1u, 2u, 4u}, trv[kMaxFoldCx];
             uint8_t trc[kMaxFoldCx];
             int ntr = 0;
             for (int i = ncx - 1; i >= 0; i--) {
@@ -225,6 +231,77 @@ inline void plan_passes(const OpHead *ops, int nops, uint32_t tile_log2, bool fo
         *fuse_out = o == nops;
     }
     *fuse_in = nops > 0 && gi[0].G != 0;
+}
+
+// Register passes of f32 sweeps. A pass is a run of consecutive ops whose
+// gates and CX targets lie on at most kRegBits tile bits: a thread holds the
+// 2^kRegBits elements those bits span and applies the ops in order, each
+// element rounded as the ops one by one do. Diagonals join on any support, a
+// CX control may lie anywhere. A run with fewer bits is padded with high tile
+// bits (low ones would make the lanes of a warp collide in the banks). A lone
+// CX stays a permutation pass, which touches half the tile.
+constexpr int kRegBits = 4;
+
+struct RegOp {
+    uint8_t n;               // ops of the pass that starts here (0: none does)
+    uint8_t g;               // the gate's (CX target's) coordinate
+    uint8_t c;               // D1 / CX: the coordinate that selects (0xff: not a group bit)
+    uint8_t pad;
+    uint8_t sorted[4];       // the pass's bits, ascending; coordinate g is sorted[g]
+    uint16_t tm[4];          // DK: table index bit of each coordinate (0: not in the support)
+};
+static_assert(sizeof(RegOp) == 16, "RegOps are copied in 16-byte pieces");
+
+inline void plan_reg_passes(const OpHead *ops, int nops, uint32_t tile_log2, RegOp *out) {
+    for (int i = 0; i < nops; i++) out[i] = RegOp{};
+    if (tile_log2 < (uint32_t)kRegBits) return;
+    for (int o = 0; o < nops;) {
+        uint32_t set = 0;
+        int n = 0;
+        bool arith = false;
+        for (; o + n < nops; n++) {
+            const OpHead &op = ops[o + n];
+            uint32_t add = 0;
+            if (op.kind == MOP_U1 || op.kind == MOP_CX) {
+                const uint32_t bit = op.kind == MOP_U1 ? op.a : op.b;
+                if (bit >= tile_log2) break;  // not a planned op: the plain loop reports it
+                add = 1u << bit;
+            } else if (op.kind != MOP_D1 && op.kind != MOP_DK) {
+                break;
+            }
+            if (popcount32(set | add) > kRegBits) break;
+            set |= add;
+            arith |= op.kind != MOP_CX;
+        }
+        if (n == 0 || (n == 1 && !arith)) {
+            o++;
+            continue;
+        }
+        for (uint32_t b = tile_log2; b-- > 0 && popcount32(set) < kRegBits;) set |= 1u << b;
+        uint8_t bits[kRegBits];
+        int cnt = 0;
+        for (uint32_t b = 0; b < tile_log2; b++)
+            if ((set >> b) & 1u) bits[cnt++] = (uint8_t)b;
+        auto coord = [&](uint32_t loc) {  // outer locations match no bit
+            for (int g = 0; g < kRegBits; g++)
+                if (bits[g] == loc) return (uint8_t)g;
+            return (uint8_t)0xff;
+        };
+        out[o].n = (uint8_t)n;
+        for (int k = 0; k < n; k++) {
+            const OpHead &op = ops[o + k];
+            RegOp &r = out[o + k];
+            for (int g = 0; g < kRegBits; g++) r.sorted[g] = bits[g];
+            r.g = coord(op.kind == MOP_CX ? op.b : op.a);
+            r.c = coord(op.a);
+            if (op.kind == MOP_DK)
+                for (uint32_t b = 0; b < op.k; b++) {
+                    const uint8_t g = coord(op.loc[b]);
+                    if (g != 0xff) r.tm[g] = (uint16_t)(1u << b);
+                }
+        }
+        o += n;
+    }
 }
 
 }  // namespace zc

@@ -129,8 +129,7 @@ int capture_group(zc_server *s, int gi) {
     cudaStream_t st = s->ctx->stream;
     ZC_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     cudaMemcpyAsync(g.d_blob, g.h_blob[0], sizeof(SweepBatch), cudaMemcpyHostToDevice, st);
-    int rc = launch_sweep_multi(st, s->ctx->num_sms, gi ? 64 : 32, (s->flags & ZC_FLAG_FAST) == 0, g.d_blob,
-                                s->ctx->d_err);
+    int rc = launch_sweep_multi(st, s->ctx->num_sms, gi ? 64 : 32, (s->flags & ZC_FLAG_FAST) == 0, g.d_blob);
     cudaError_t e = cudaStreamEndCapture(st, &g.graph);
     if (rc) return rc;
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
@@ -219,7 +218,7 @@ int packed_step(zc_server *s, int gi, int round, int *issued) {
     } else {
         // first packed launch of the server runs uncaptured (kernel attributes get set here)
         ZC_CUDA(cudaMemcpyAsync(g.d_blob, hb, total, cudaMemcpyHostToDevice, s->ctx->stream));
-        int rc = launch_sweep_multi(s->ctx->stream, s->ctx->num_sms, prec, ex, g.d_blob, s->ctx->d_err);
+        int rc = launch_sweep_multi(s->ctx->stream, s->ctx->num_sms, prec, ex, g.d_blob);
         if (rc) return rc;
     }
     s->launches++;

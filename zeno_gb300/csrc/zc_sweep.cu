@@ -37,8 +37,8 @@ constexpr uint32_t kJlutLen = 256 + kJlutHigh;
 // memory the pass descriptors take in double-float sweeps; further table
 // diagonals build theirs per tile. A table diagonal's `b` field (in the
 // CTA's copy of the micro-ops) names its job table, or kNoJobLut.
-// (Exact f64 sweeps; f32 sweeps have both and keep kF32Luts tables.)
-constexpr int kJobLuts = 5, kF32Luts = 2;
+// (Exact f64 sweeps: the others' diagonals ride in register passes.)
+constexpr int kJobLuts = 5;
 constexpr uint32_t kNoJobLut = 0xffffffffu;
 // The tile's re array, then, this far behind it whatever the tile's size, im.
 constexpr uint32_t kTileArrayBytes = (uint32_t)(kSweepSmemBytes / 2);
@@ -209,22 +209,15 @@ __device__ __forceinline__ void hl_cscale_df(float2 wr, float2 wi, float2 &H, fl
     pk_join(ar, ai, H, L);
 }
 
-// The kernel's register group size: double-float sweeps spill at the
-// 80-register cap with more than two general ops (rotations: three); f32
-// states run groups of two as 8-byte vectors of element pairs (measured
-// faster than scalar groups of three, which spill as vectors); exact f64
-// gates are long enough one at a time (~400 integer instructions per pair).
+// The register group size of double-float sweeps: they spill at the
+// 80-register cap with more than two general ops (rotations: three).
+constexpr int kDfGroup = 2;
+// The pass descriptors of a job, one slot per op (exact f64 sweeps have none).
 template <typename T, int A>
-__host__ __device__ constexpr int max_group_of() {
-    return A == AR_EXACT && sizeof(T) == 8 ? 1 : 2;
-}
-// Sweeps with register passes (GroupInfo): double-float ones and f32 ones, the
-// latter with groups of up to four ops.
-template <typename T, int A>
-__host__ __device__ constexpr bool has_passes() {
-    return A == AR_DF || sizeof(T) == 4;
-}
-constexpr int kF32Group = 4;
+struct PassOf {
+    using type = typename std::conditional<A == AR_DF, GroupInfo, RegOp>::type;
+    static constexpr bool any = A == AR_DF || sizeof(T) == 4;
+};
 
 template <typename R>
 __device__ __forceinline__ uint32_t jgather(const OpHead &op, uint32_t jo, uint32_t v) {
@@ -239,188 +232,6 @@ __device__ __forceinline__ uint32_t jouter(const OpHead &op, uint64_t base) {
     for (uint32_t b = 0; b < op.k; b++)
         if (op.loc[b] & kOuterFlag) jo |= (uint32_t)((base >> (op.loc[b] & ~kOuterFlag)) & 1) << b;
     return jo;
-}
-
-// The arithmetic of G consecutive one-qubit micro-ops (U1, R1 or RT; only RT
-// when ROT_ONLY; ops[o..o+G), distinct tile bits) on a register-held group
-// of 2^G elements: element e sits at the slot of the group bits selected by
-// e. Each gate updates the same pairs with the same arithmetic, in the same
-// order, as one op at a time.
-// NE: elements held (a multiple of 2^G: several independent groups side by
-// side, element e of group h at index h * 2^G + e; each gate's coefficients
-// are read once for all of them).
-template <typename T, int A, typename R, int G, bool ROT_ONLY, int NE = (1 << G)>
-__device__ __forceinline__ void group_math(const OpHead *ops, const OpCoef<T, A> *coef, int o, R *xr, R *xi) {
-    constexpr int E = NE;
-#pragma unroll
-    for (int g = 0; g < G; g++) {
-        if (ROT_ONLY || ops[o + g].kind == MOP_RT) {
-            const R t = coef[o + g].v[0];
-#pragma unroll
-            for (int e = 0; e < E; e++)
-                if (!((e >> g) & 1)) {
-                    if constexpr (A == AR_DF)
-                        hl_rot_df(t, xr[e], xi[e], xr[e | (1 << g)], xi[e | (1 << g)]);
-                    else
-                        pair_update_rot<T>(t, xr[e], xi[e], xr[e | (1 << g)], xi[e | (1 << g)]);
-                }
-        } else if (ops[o + g].kind == MOP_R1) {
-            R r[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) r[i] = coef[o + g].v[i];
-#pragma unroll
-            for (int e = 0; e < E; e++)
-                if (!((e >> g) & 1)) {
-                    if constexpr (A == AR_DF)
-                        hl_rdf(r, xr[e], xi[e], xr[e | (1 << g)], xi[e | (1 << g)]);
-                    else
-                        pair_update_real<T>(r, xr[e], xi[e], xr[e | (1 << g)], xi[e | (1 << g)]);
-                }
-        } else if constexpr (A == AR_DF) {
-            MatDF m;
-#pragma unroll
-            for (int i = 0; i < 8; i++) m.v[i] = coef[o + g].v[i];
-#pragma unroll
-            for (int e = 0; e < E; e++)
-                if (!((e >> g) & 1)) hl_udf(m, xr[e], xi[e], xr[e | (1 << g)], xi[e | (1 << g)]);
-        } else {
-            Mat2<T> m;
-#pragma unroll
-            for (int i = 0; i < 8; i++) m.v[i] = coef[o + g].v[i];
-#pragma unroll
-            for (int e = 0; e < E; e++)
-                if (!((e >> g) & 1))
-                    pair_update<T, A == AR_EXACT>(m, xr[e], xi[e], xr[e | (1 << g)], xi[e | (1 << g)]);
-        }
-    }
-}
-
-// The group's tile bits (bits: op order; sorted: ascending), the pattern of
-// flipped RT ops and a range check. Returns false (and records the bad bit)
-// when a bit lies outside the tile; `shift` counts the low bits a vector of
-// consecutive elements covers (the bits are then in vector units).
-template <int G>
-__device__ __forceinline__ bool group_bits(const OpHead *ops, int o, uint32_t size, uint32_t shift, uint32_t *bits,
-                                           uint32_t *sorted, uint32_t &fmask, uint32_t *bad) {
-#pragma unroll
-    for (int g = 0; g < G; g++) bits[g] = sorted[g] = ops[o + g].a - shift;
-#pragma unroll
-    for (int i = 1; i < G; i++)
-#pragma unroll
-        for (int j = i; j > 0; j--)
-            if (sorted[j] < sorted[j - 1]) {
-                const uint32_t x = sorted[j];
-                sorted[j] = sorted[j - 1];
-                sorted[j - 1] = x;
-            }
-    uint32_t bad_bit = 0;
-    fmask = 0;
-#pragma unroll
-    for (int g = 0; g < G; g++) {
-        if (ops[o + g].kind == MOP_RT && ops[o + g].b) fmask |= 1u << bits[g];
-        if ((1u << ops[o + g].a) >= size) bad_bit = ops[o + g].a;
-    }
-    // every slot is inside the tile when the bits are (v < size / 2^G with
-    // G zero bits inserted below log2(size)); a bad bit is recorded and the
-    // group skipped
-    if (bad_bit) {
-        if (threadIdx.x == 0) *bad = bad_bit | 0x80000000u;
-        return false;
-    }
-    return true;
-}
-
-// Apply G consecutive one-qubit micro-ops to register-held groups of 2^G
-// elements (group_math). The pair swaps of flipped RT ops commute with the
-// group's other gates (other bits), so they all happen at the store: element
-// e goes to the slot of e ^ flips.
-template <typename T, int A, typename R, int G, bool ROT_ONLY = false>
-__device__ void apply_u1_group(R *sr, R *si, const OpHead *ops, const OpCoef<T, A> *coef, int o, uint32_t size,
-                               uint32_t *bad) {
-    constexpr int E = 1 << G;
-    uint32_t bits[G], sorted[G], fmask;
-    if (!group_bits<G>(ops, o, size, 0u, bits, sorted, fmask, bad)) return;
-#pragma unroll
-    for (int g = 0; g < G; g++) bits[g] = swz<(int)sizeof(R)>(1u << bits[g]);
-    fmask = swz<(int)sizeof(R)>(fmask);
-    for (uint32_t p = threadIdx.x; p < size / E; p += blockDim.x) {
-        uint32_t v = p;
-#pragma unroll
-        for (int g = 0; g < G; g++) v = ((v >> sorted[g]) << (sorted[g] + 1)) | (v & ((1u << sorted[g]) - 1));
-        v = swz<(int)sizeof(R)>(v);
-        // element e of the group sits at v ^ (bits selected by e)
-        // (recomputed at the store so the indices need no registers across
-        // the arithmetic); flipped elements: slot(e ^ flips) = slot(e) ^ fmask
-        auto slot = [&](uint32_t base_v, uint32_t e) {
-            uint32_t w = base_v;
-#pragma unroll
-            for (int g = 0; g < G; g++)
-                if ((e >> g) & 1u) w ^= bits[g];
-            return w;
-        };
-        R xr[E], xi[E];
-#pragma unroll
-        for (int e = 0; e < E; e++) {
-            const uint32_t w = slot(v, (uint32_t)e);
-            xr[e] = sr[w];
-            xi[e] = si[w];
-        }
-        group_math<T, A, R, G, ROT_ONLY>(ops, coef, o, xr, xi);
-        const uint32_t vs = v ^ fmask;
-#pragma unroll
-        for (int e = 0; e < E; e++) {
-            const uint32_t w = slot(vs, (uint32_t)e);
-            sr[w] = xr[e];
-            si[w] = xi[e];
-        }
-    }
-}
-
-// The same for 4-byte elements when no group bit is bit 0: each thread
-// moves element pairs (2m, 2m + 1) as one 8-byte vector, so a group of 2^G
-// vectors carries two independent element groups (the vector's two lanes)
-// with half the loads, stores and index arithmetic per element.
-template <typename T, int A, int G, bool ROT_ONLY = false>
-__device__ void apply_u1_group_v2(float *sr, float *si, const OpHead *ops, const OpCoef<T, A> *coef, int o,
-                                  uint32_t size, uint32_t *bad) {
-    constexpr int E = 1 << G;
-    uint32_t bits[G], sorted[G], fmask;
-    if (!group_bits<G>(ops, o, size, 1u, bits, sorted, fmask, bad)) return;
-#pragma unroll
-    for (int g = 0; g < G; g++) bits[g] = swz<8>(1u << bits[g]);  // 8-byte units of a 4-byte array: the same places
-    fmask = swz<8>(fmask);
-    float2 *vr = reinterpret_cast<float2 *>(sr), *vi = reinterpret_cast<float2 *>(si);
-    for (uint32_t p = threadIdx.x; p < size / 2 / E; p += blockDim.x) {
-        uint32_t v = p;
-#pragma unroll
-        for (int g = 0; g < G; g++) v = ((v >> sorted[g]) << (sorted[g] + 1)) | (v & ((1u << sorted[g]) - 1));
-        v = swz<8>(v);
-        auto slot = [&](uint32_t base_v, uint32_t e) {
-            uint32_t w = base_v;
-#pragma unroll
-            for (int g = 0; g < G; g++)
-                if ((e >> g) & 1u) w ^= bits[g];
-            return w;
-        };
-        float xr[2 * E], xi[2 * E];  // lane 0 (even element) at e, lane 1 at E + e
-#pragma unroll
-        for (int e = 0; e < E; e++) {
-            const uint32_t w = slot(v, (uint32_t)e);
-            const float2 a = vr[w], b = vi[w];
-            xr[e] = a.x;
-            xr[E + e] = a.y;
-            xi[e] = b.x;
-            xi[E + e] = b.y;
-        }
-        group_math<T, A, float, G, ROT_ONLY, 2 * E>(ops, coef, o, xr, xi);
-        const uint32_t vs = v ^ fmask;
-#pragma unroll
-        for (int e = 0; e < E; e++) {
-            const uint32_t w = slot(vs, (uint32_t)e);
-            vr[w] = make_float2(xr[e], xr[E + e]);
-            vi[w] = make_float2(xi[e], xi[E + e]);
-        }
-    }
 }
 
 // One pass (see GroupInfo) of a double-float sweep. xr / xi hold the packed
@@ -545,102 +356,122 @@ __device__ void run_pass(const GroupInfo &gi, char *tile, const OpHead *ops, con
     }
 }
 
-// A pass of an f32 sweep: the same indices (4-byte slots, 8-byte table
-// entries), each element's arithmetic in the order of the ops one by one. Up to
-// four gates, a diagonal and a block of CX in one round trip through shared
-// memory, whose wavefronts bound f32 sweeps.
-template <typename T, int A, int G, bool HAS_DK, bool HAS_CX>
-__device__ __noinline__ void run_pass_f32(const GroupInfo &gi, char *tile, const OpHead *ops, const OpCoef<T, A> *coef,
-                             uint32_t size, const char *tables, uint64_t base) {
-    constexpr int E = 1 << G;
-    const int o = gi.first;
-    uint32_t jo = 0, u0 = 0;
-    if constexpr (HAS_DK) {
-        for (int i = 0; i < gi.nout; i++) jo |= (uint32_t)((base >> gi.outq[i]) & 1u) << (gi.outb[i] + 3);
-    }
-    if constexpr (HAS_CX) {
-        for (int t = 0; t < gi.ntr; t++)
-            if ((gi.trc[t] & 0x80u) && ((base >> (gi.trc[t] & 0x7fu)) & 1u)) u0 ^= gi.trw[t];
-    }
-    uint32_t so = 0, lo = 0, jb = 0;
-    for (uint32_t p = threadIdx.x; p < size / E; p += kSweepThreads) {
-        if (G == 4 && p >= kSweepThreads) {  // at most one step: tiles have 2^13 elements
-            so ^= gi.so_step;
-            lo ^= gi.lo_step;
-            jb ^= gi.jb_step;
-        } else {
-            uint32_t v = p;
+// One gate of an f32 pass on the group coordinate G.
+template <int G, bool EXACT>
+__device__ __forceinline__ void reg_gate(const Mat2<float> &m, float *xr, float *xi) {
 #pragma unroll
-            for (int g = 0; g < G; g++) v = insert_zero32(v, gi.sorted[g]);
-            so = lo = swz<4>(v) << 2;
-            if constexpr (HAS_CX) {
-                lo ^= u0;
-                for (int t = 0; t < gi.ntr; t++)
-                    if (!(gi.trc[t] & 0x80u) && ((v >> gi.trc[t]) & 1u)) lo ^= gi.trw[t];
-            }
-            if constexpr (HAS_DK) {
-                jb = jo;
-                for (int i = 0; i < gi.nloc; i++) jb |= ((v >> gi.loc[i]) & 1u) << (gi.locb[i] + 3);
-            }
-        }
-        float xr[E], xi[E];
+    for (int e = 0; e < 1 << kRegBits; e++)
+        if (!((e >> G) & 1)) pair_update<float, EXACT>(m, xr[e], xi[e], xr[e | (1 << G)], xi[e | (1 << G)]);
+}
+
+// The CX with target coordinate G: pairs whose bit of `on` is set change places.
+template <int G>
+__device__ __forceinline__ void reg_cx(uint32_t on, float *xr, float *xi) {
 #pragma unroll
-        for (int e = 0; e < E; e++) {
-            uint32_t w = lo;
-#pragma unroll
-            for (int g = 0; g < G; g++)
-                if ((e >> g) & 1) w ^= HAS_CX ? gi.pm[g] : gi.gm[g];
-            xr[e] = *reinterpret_cast<const float *>(tile + w);
-            xi[e] = *reinterpret_cast<const float *>(tile + kTileArrayBytes + w);
-        }
-        if constexpr (HAS_DK) {
-            const char *dtab = tables + gi.tab_off;
-            uint32_t tm[G];
-#pragma unroll
-            for (int g = 0; g < G; g++) tm[g] = gi.tb[g] != 0xff ? 8u << gi.tb[g] : 0u;
-#pragma unroll
-            for (int e = 0; e < E; e++) {
-                uint32_t j = jb;
-#pragma unroll
-                for (int g = 0; g < G; g++)
-                    if ((e >> g) & 1) j ^= tm[g];
-                const float2 w = __ldg(reinterpret_cast<const float2 *>(dtab + j));
-                cscale<float, A == AR_EXACT>(w.x, w.y, xr[e], xi[e]);
-            }
-        }
-#pragma unroll
-        for (int g = 0; g < G; g++) {
-            Mat2<float> m;
-#pragma unroll
-            for (int i = 0; i < 8; i++) m.v[i] = coef[o + g].v[i];
-#pragma unroll
-            for (int e = 0; e < E; e++)
-                if (!((e >> g) & 1))
-                    pair_update<float, A == AR_EXACT>(m, xr[e], xi[e], xr[e | (1 << g)], xi[e | (1 << g)]);
-        }
-#pragma unroll
-        for (int e = 0; e < E; e++) {
-            uint32_t w = so;
-#pragma unroll
-            for (int g = 0; g < G; g++)
-                if ((e >> g) & 1) w ^= gi.gm[g];
-            *reinterpret_cast<float *>(tile + w) = xr[e];
-            *reinterpret_cast<float *>(tile + kTileArrayBytes + w) = xi[e];
-        }
+    for (int e = 0; e < 1 << kRegBits; e++) {
+        constexpr int F = 1 << G;
+        if ((e >> G) & 1) continue;
+        const bool sw = (on >> e) & 1u;
+        const float ar = xr[e], ai = xi[e], br = xr[e | F], bi = xi[e | F];
+        xr[e] = sw ? br : ar;
+        xi[e] = sw ? bi : ai;
+        xr[e | F] = sw ? ar : br;
+        xi[e | F] = sw ? ai : bi;
     }
 }
 
-template <typename T, int A, int G>
-__device__ void run_pass_f32_any(const GroupInfo &gi, char *tile, const OpHead *ops, const OpCoef<T, A> *coef,
-                                 uint32_t size, const char *tables, uint64_t base) {
-    bool cx = gi.ntr;
-    for (int g = 0; g < G; g++) cx |= gi.pm[g] != gi.gm[g];
-    if (gi.has_dk) {
-        if (cx) run_pass_f32<T, A, G, true, true>(gi, tile, ops, coef, size, tables, base);
-        else run_pass_f32<T, A, G, true, false>(gi, tile, ops, coef, size, tables, base);
-    } else {
-        if (cx) run_pass_f32<T, A, G, false, true>(gi, tile, ops, coef, size, tables, base);
-        else run_pass_f32<T, A, G, false, false>(gi, tile, ops, coef, size, tables, base);
+// A pass of an f32 sweep (RegOp): its ops in order on sixteen elements in
+// registers, one round trip through shared memory for all of them. The
+// wavefronts of a trip per op (per pair of gates) bound f32 sweeps; four bits
+// take four to five ops of a random circuit. Out of line: inlined into the tile
+// loop it spilled at the 80-register cap. Bound by instruction issue now (69%
+// of the slots at three CTAs per SM; f32x2 gates took 18% of the instructions
+// away and no time). 26 qubits, random gates: 17.2 -> 16.0 ms, 24 packed states
+// of 8 to 22 qubits 7.8 -> 7.4 (10.9 with a trip per pair of gates).
+template <typename T, int A>
+__device__ __noinline__ void run_pass_f32(const RegOp *pass, const OpHead *ops, const OpCoef<T, A> *coef, char *tile,
+                                          uint32_t size, const char *tables, uint64_t base) {
+    constexpr int E = 1 << kRegBits;
+    constexpr bool EX = A == AR_EXACT;
+    const int n = pass[0].n;
+    for (uint32_t p = threadIdx.x; p < size / E; p += kSweepThreads) {
+        uint32_t v = p, gm[kRegBits];
+#pragma unroll
+        for (int g = 0; g < kRegBits; g++) {
+            v = insert_zero32(v, pass[0].sorted[g]);
+            gm[g] = swz<4>(1u << pass[0].sorted[g]) << 2;
+        }
+        const uint32_t so = swz<4>(v) << 2;
+        auto slot = [&](int e) {
+            uint32_t w = so;
+#pragma unroll
+            for (int g = 0; g < kRegBits; g++)
+                if ((e >> g) & 1) w ^= gm[g];
+            return w;
+        };
+        float xr[E], xi[E];
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            const uint32_t w = slot(e);
+            xr[e] = *reinterpret_cast<const float *>(tile + w);
+            xi[e] = *reinterpret_cast<const float *>(tile + kTileArrayBytes + w);
+        }
+        // bit of location l (a tile bit outside the group, or an outer qubit)
+        auto bit_of = [&](uint32_t l) {
+            return (l & kOuterFlag) ? (uint32_t)(base >> (l & ~kOuterFlag)) & 1u : (v >> l) & 1u;
+        };
+        // elements whose selecting bit is set
+        auto chosen = [&](uint32_t c, uint32_t l) {
+            return c != 0xffu ? (uint32_t)(0xff00f0f0ccccaaaaull >> (16 * c)) & 0xffffu : 0u - bit_of(l);
+        };
+#pragma unroll 1
+        for (int k = 0; k < n; k++) {
+            const RegOp &r = pass[k];
+            const OpHead &op = ops[k];
+            if (op.kind == MOP_U1) {
+                Mat2<float> m;
+#pragma unroll
+                for (int i = 0; i < 8; i++) m.v[i] = coef[k].v[i];
+                if (r.g == 0) reg_gate<0, EX>(m, xr, xi);
+                else if (r.g == 1) reg_gate<1, EX>(m, xr, xi);
+                else if (r.g == 2) reg_gate<2, EX>(m, xr, xi);
+                else reg_gate<3, EX>(m, xr, xi);
+            } else if (op.kind == MOP_CX) {
+                const uint32_t on = chosen(r.c, op.a);
+                if (r.g == 0) reg_cx<0>(on, xr, xi);
+                else if (r.g == 1) reg_cx<1>(on, xr, xi);
+                else if (r.g == 2) reg_cx<2>(on, xr, xi);
+                else reg_cx<3>(on, xr, xi);
+            } else if (op.kind == MOP_D1) {
+                const uint32_t on = chosen(r.c, op.a);
+                const float d0r = coef[k].v[0], d0i = coef[k].v[1], d1r = coef[k].v[2], d1i = coef[k].v[3];
+#pragma unroll
+                for (int e = 0; e < E; e++) {
+                    const bool one = (on >> e) & 1u;
+                    cscale<float, EX>(one ? d1r : d0r, one ? d1i : d0i, xr[e], xi[e]);
+                }
+            } else {
+                uint32_t j = 0;
+                for (uint32_t b = 0; b < op.k; b++)
+                    if (!((r.tm[0] | r.tm[1] | r.tm[2] | r.tm[3]) >> b & 1u)) j |= bit_of(op.loc[b]) << b;
+                const float2 *tab = reinterpret_cast<const float2 *>(tables + op.table);
+#pragma unroll
+                for (int e = 0; e < E; e++) {
+                    uint32_t i = j;
+#pragma unroll
+                    for (int g = 0; g < kRegBits; g++)
+                        if ((e >> g) & 1) i |= r.tm[g];
+                    const float2 w = __ldg(tab + i);
+                    cscale<float, EX>(w.x, w.y, xr[e], xi[e]);
+                }
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            const uint32_t w = slot(e);
+            *reinterpret_cast<float *>(tile + w) = xr[e];
+            *reinterpret_cast<float *>(tile + kTileArrayBytes + w) = xi[e];
+        }
     }
 }
 
@@ -659,12 +490,12 @@ __device__ void run_pass_any(const GroupInfo &gi, char *tile, const OpHead *ops,
     }
 }
 
-// gis: the job's register passes (double-float sweeps; see GroupInfo);
+// gis: the job's register passes (double-float and f32 sweeps);
 // fuse_in / fuse_out: its first / last pass converts the tile.
 template <typename T, int A, typename R>
 __device__ void apply_ops(R *sr, R *si, const OpHead *ops, const OpCoef<T, A> *coef, int nops, uint64_t base,
-                          uint32_t size, const char *tables, uint32_t *bad, uint16_t *jlut, const uint16_t *job_luts,
-                          const GroupInfo *gis,
+                          uint32_t size, const char *tables, uint16_t *jlut, const uint16_t *job_luts,
+                          const typename PassOf<T, A>::type *gis,
                           int fuse_in = 0, int fuse_out = 0) {
     const int tid = threadIdx.x, nt = blockDim.x;
     for (int o = 0; o < nops; o++) {
@@ -685,111 +516,47 @@ __device__ void apply_ops(R *sr, R *si, const OpHead *ops, const OpCoef<T, A> *c
             }
         }
         if constexpr (sizeof(T) == 4) {
-            const GroupInfo &gi = gis[o];
-            if (gi.G) {
-                char *tile = reinterpret_cast<char *>(sr);
-                if (gi.G == 4) run_pass_f32_any<T, A, 4>(gi, tile, ops, coef, size, tables, base);
-                else if (gi.G == 3) run_pass_f32_any<T, A, 3>(gi, tile, ops, coef, size, tables, base);
-                else if (gi.G == 2) run_pass_f32_any<T, A, 2>(gi, tile, ops, coef, size, tables, base);
-                else run_pass_f32_any<T, A, 1>(gi, tile, ops, coef, size, tables, base);
-                o += gi.skip - 1;
+            const int n = gis[o].n;
+            if (n) {
+                run_pass_f32<T, A>(gis + o, ops + o, coef + o, reinterpret_cast<char *>(sr), size, tables, base);
+                o += n - 1;
                 __syncthreads();
                 continue;
             }
         }
-        if (is_1q(op.kind)) {
-            // runs of up to three one-qubit ops on distinct bits share one
-            // register pass (two for f64 states outside FMA mode, which would
-            // spill at the 80-register cap with three, except for rotations)
-            constexpr int kMaxGroup = max_group_of<T, A>();
-            bool rot3;
-            const int g = group_at(ops, o, nops, kMaxGroup, &rot3);
-            if constexpr (sizeof(R) == 4) {  // 4-byte elements: pairs of them as 8-byte vectors
-                bool vec = g <= 2;
-                for (int h = 0; h < g; h++) vec &= ops[o + h].a >= 1u;
-                if (vec) {
-                    if (g == 2) apply_u1_group_v2<T, A, 2>(sr, si, ops, coef, o, size, bad);
-                    else apply_u1_group_v2<T, A, 1>(sr, si, ops, coef, o, size, bad);
-                    o += g - 1;
+        // one gate: exact f64 (~400 integer instructions per pair hide the
+        // trip), and f32 states smaller than a pass's bits
+        if constexpr (A != AR_DF) {
+            if (op.kind == MOP_U1) {
+                const uint32_t b = op.a, bs = swz<(int)sizeof(R)>(1u << b);
+                if constexpr (A == AR_EXACT && sizeof(T) == 8) {
+                    const double *m = coef[o].v;
+                    const ExactMask mask = exact_mask(m);
+#pragma unroll 1
+                    for (uint32_t p = tid; p < size / 2; p += nt) {
+                        const uint32_t v0 = swz<(int)sizeof(R)>(insert_zero32(p, b)), v1 = v0 ^ bs;
+                        double ar = sr[v0], ai = si[v0], br = sr[v1], bi = si[v1];
+                        pair_update_f64(m, mask, ar, ai, br, bi);
+                        sr[v0] = ar;
+                        si[v0] = ai;
+                        sr[v1] = br;
+                        si[v1] = bi;
+                    }
                     __syncthreads();
                     continue;
                 }
-            }
-            if (rot3) {
-                apply_u1_group<T, A, R, 3, true>(sr, si, ops, coef, o, size, bad);
-                o += 2;
-                __syncthreads();
-                continue;
-            }
-            if (kMaxGroup == 3 && g == 3) {
-                apply_u1_group<T, A, R, kMaxGroup>(sr, si, ops, coef, o, size, bad);
-                o += 2;
-                __syncthreads();
-                continue;
-            }
-            if (g == 2) {
-                apply_u1_group<T, A, R, 2>(sr, si, ops, coef, o, size, bad);
-                o += 1;
-                __syncthreads();
-                continue;
-            }
-            const uint32_t b = op.a, bs = swz<(int)sizeof(R)>(1u << b);
-            if (op.kind == MOP_RT) {
-                const R t = coef[o].v[0];
-                const uint32_t flip = op.b ? bs : 0u;
-                for (uint32_t p = tid; p < size / 2; p += nt) {
-                    const uint32_t v0 = swz<(int)sizeof(R)>(insert_zero32(p, b)), v1 = v0 ^ bs;
-                    R ar = sr[v0], ai = si[v0], br = sr[v1], bi = si[v1];
-                    if constexpr (A == AR_DF) hl_rot_df(t, ar, ai, br, bi);
-                    else pair_update_rot<T>(t, ar, ai, br, bi);
-                    sr[v0 ^ flip] = ar;
-                    si[v0 ^ flip] = ai;
-                    sr[v1 ^ flip] = br;
-                    si[v1 ^ flip] = bi;
-                }
-                __syncthreads();
-                continue;
-            }
-            if (op.kind == MOP_R1) {
-                R r[4];
+                Mat2<T> m;
 #pragma unroll
-                for (int i = 0; i < 4; i++) r[i] = coef[o].v[i];
+                for (int i = 0; i < 8; i++) m.v[i] = coef[o].v[i];
                 for (uint32_t p = tid; p < size / 2; p += nt) {
                     const uint32_t v0 = swz<(int)sizeof(R)>(insert_zero32(p, b)), v1 = v0 ^ bs;
-                    if constexpr (A == AR_DF) hl_rdf(r, sr[v0], si[v0], sr[v1], si[v1]);
-                    else pair_update_real<T>(r, sr[v0], si[v0], sr[v1], si[v1]);
+                    pair_update<T, A == AR_EXACT>(m, sr[v0], si[v0], sr[v1], si[v1]);
                 }
                 __syncthreads();
                 continue;
             }
-            if constexpr (A == AR_EXACT && sizeof(T) == 8) {
-                const double *m = coef[o].v;
-                const ExactMask mask = exact_mask(m);
-#pragma unroll 1
-                for (uint32_t p = tid; p < size / 2; p += nt) {
-                    const uint32_t v0 = swz<(int)sizeof(R)>(insert_zero32(p, b)), v1 = v0 ^ bs;
-                    double ar = sr[v0], ai = si[v0], br = sr[v1], bi = si[v1];
-                    pair_update_f64(m, mask, ar, ai, br, bi);
-                    sr[v0] = ar;
-                    si[v0] = ai;
-                    sr[v1] = br;
-                    si[v1] = bi;
-                }
-                __syncthreads();
-                continue;
-            }
-            typename std::conditional<A == AR_DF, MatDF, Mat2<T>>::type m;
-#pragma unroll
-            for (int i = 0; i < 8; i++) m.v[i] = coef[o].v[i];
-            auto upd = [&](R &ar, R &ai, R &br, R &bi) {
-                if constexpr (A == AR_DF) hl_udf(m, ar, ai, br, bi);
-                else pair_update<T, A == AR_EXACT>(m, ar, ai, br, bi);
-            };
-            for (uint32_t p = tid; p < size / 2; p += nt) {
-                const uint32_t v0 = swz<(int)sizeof(R)>(insert_zero32(p, b)), v1 = v0 ^ bs;
-                upd(sr[v0], si[v0], sr[v1], si[v1]);
-            }
-        } else if (op.kind == MOP_D1) {
+        }
+        if (op.kind == MOP_D1) {
             const bool outer = op.a & kOuterFlag;
             const bool tile_one = outer && ((base >> (op.a & ~kOuterFlag)) & 1);
             auto scl = [&](uint32_t v, R &xr, R &xi) {
@@ -915,10 +682,9 @@ struct SweepSmem {
     OpCoef<T, A> coef[kMaxMicroOps];
     uint32_t rows[1u << kMaxSweepHigh];  // row r of a tile starts at element rows[r] << L of it
     JobHead job;
-    uint32_t bad;
     uint16_t jlut[kJlutLen];  // diagonal index tables of the current DK op
-    alignas(16) GroupInfo gi[has_passes<T, A>() ? kMaxMicroOps : 1];  // register passes
-    static constexpr int kLuts = A == AR_DF ? 0 : sizeof(T) == 4 ? kF32Luts : kJobLuts;
+    alignas(16) typename PassOf<T, A>::type gi[PassOf<T, A>::any ? kMaxMicroOps : 1];  // register passes
+    static constexpr int kLuts = PassOf<T, A>::any ? 0 : kJobLuts;
     uint16_t luts[kLuts * kJlutLen + 1];  // the job's diagonal index tables
 };
 static_assert(sizeof(OpHead[kMaxMicroOps]) % 16 == 0 && sizeof(GroupInfo[kMaxMicroOps]) % 16 == 0,
@@ -944,6 +710,8 @@ int encode_job_as(const SweepPlan &plan, std::vector<char> *out) {
         memcpy(&ops[(size_t)o], &m, sizeof(OpHead));
         h.has_arith |= m.kind != MOP_CX && m.kind != MOP_SWAP;
         const int cnt = m.kind == MOP_U1 ? 8 : m.kind == MOP_RT ? 1 : m.kind == MOP_D1 || m.kind == MOP_R1 ? 4 : 0;
+        if ((is_1q(m.kind) && m.a >= h.L + h.H) || (m.kind == MOP_CX && m.b >= h.L + h.H))
+            return fail(ZC_ERR_INVALID, "sweep plan: a gate bit lies outside the tile");
         OpCoef<T, A> &c = coef[(size_t)o];
         for (int i = 0; i < cnt; i++) {
             if constexpr (A == AR_DF) {
@@ -963,59 +731,48 @@ int encode_job_as(const SweepPlan &plan, std::vector<char> *out) {
             }
         }
     }
-    std::vector<GroupInfo> gi;
-    if constexpr (has_passes<T, A>()) {
-        constexpr int SB = sizeof(T) == 4 ? 2 : 3, JB = sizeof(T) == 4 ? 3 : 4;  // slot and table entry bytes, log2
+    std::vector<typename PassOf<T, A>::type> gi;
+    if constexpr (sizeof(T) == 4) {
+        gi.resize((size_t)nops);
+        plan_reg_passes(ops.data(), nops, h.L + h.H, gi.data());
+    }
+    if constexpr (A == AR_DF) {
         gi.resize((size_t)nops);
         uint32_t bad = 0;
         int fuse_in = 0, fuse_out = 0;
-        plan_passes(ops.data(), nops, h.L + h.H, true, sizeof(T) == 4 ? kF32Group : max_group_of<T, A>(), gi.data(),
-                    &bad, &fuse_in, &fuse_out);
-        if constexpr (sizeof(T) == 4) {
-            // one or two bare gates move as vectors of element pairs instead
-            for (GroupInfo &q : gi)
-                if (q.G && q.G <= 2 && q.skip == q.G && !(q.gm[0] & 1) && !(q.G == 2 && (q.gm[1] & 1))) q.G = 0;
-        }
+        plan_passes(ops.data(), nops, h.L + h.H, true, kDfGroup, gi.data(), &bad, &fuse_in, &fuse_out);
         if (bad) return fail(ZC_ERR_INVALID, "sweep plan: a group bit lies outside the tile");
         h.fuse_in = (uint32_t)fuse_in;
         h.fuse_out = (uint32_t)fuse_out;
         for (GroupInfo &q : gi) {  // slot patterns as byte offsets into the swizzled tile, step patterns
             if (!q.G) continue;
             for (int g = 0; g < q.G; g++) {
-                q.gm[g] = (uint16_t)(swz<(int)sizeof(T)>(q.gm[g]) << SB);
-                q.pm[g] = (uint16_t)(swz<(int)sizeof(T)>(q.pm[g]) << SB);
+                q.gm[g] = (uint16_t)(swz<8>(q.gm[g]) << 3);
+                q.pm[g] = (uint16_t)(swz<8>(q.pm[g]) << 3);
             }
-            for (int i = 0; i < q.ntr; i++) q.trw[i] = (uint16_t)(swz<(int)sizeof(T)>(q.trw[i]) << SB);
-            q.fmask = (uint16_t)(swz<(int)sizeof(T)>(q.fmask) << SB);
+            for (int i = 0; i < q.ntr; i++) q.trw[i] = (uint16_t)(swz<8>(q.trw[i]) << 3);
+            q.fmask = (uint16_t)(swz<8>(q.fmask) << 3);
             uint32_t v = kSweepThreads, lo = 0, jb = 0;  // group number p + kSweepThreads against p
             for (int g = 0; g < q.G; g++) v = insert_zero32(v, q.sorted[g]);
             for (int i = 0; i < q.ntr; i++)
                 if (!(q.trc[i] & 0x80u) && ((v >> q.trc[i]) & 1u)) lo ^= q.trw[i];
-            for (int i = 0; i < q.nloc; i++) jb |= ((v >> q.loc[i]) & 1u) << (q.locb[i] + JB);
-            q.so_step = (uint16_t)(swz<(int)sizeof(T)>(v) << SB);
+            for (int i = 0; i < q.nloc; i++) jb |= ((v >> q.loc[i]) & 1u) << (q.locb[i] + 4);
+            q.so_step = (uint16_t)(swz<8>(v) << 3);
             q.lo_step = (uint16_t)(q.so_step ^ lo);
             q.jb_step = (uint16_t)jb;
         }
     }
-    // index tables for the table diagonals that no pass takes
-    for (int o = 0; o < nops;) {
-        if (!gi.empty() && gi[(size_t)o].G) {
-            o += gi[(size_t)o].skip;
-            continue;
-        }
-        if (ops[(size_t)o].kind == MOP_DK)
-            ops[(size_t)o].b = nlut < (uint32_t)SweepSmem<T, A>::kLuts ? nlut++ : kNoJobLut;
-        o++;
-    }
+    for (OpHead &op : ops)
+        if (op.kind == MOP_DK) op.b = nlut < (uint32_t)SweepSmem<T, A>::kLuts ? nlut++ : kNoJobLut;
     auto up16 = [](size_t b) { return (b + 15) & ~(size_t)15; };
     const size_t ops_b = up16(ops.size() * sizeof(OpHead)), coef_b = up16(coef.size() * sizeof(OpCoef<T, A>));
     h.coef_off = (uint32_t)(sizeof(JobHead) + ops_b);
     h.gi_off = (uint32_t)(h.coef_off + coef_b);
-    out->assign(h.gi_off + up16(gi.size() * sizeof(GroupInfo)), 0);
+    out->assign(h.gi_off + up16(gi.size() * sizeof(gi[0])), 0);
     memcpy(out->data(), &h, sizeof h);
     memcpy(out->data() + sizeof(JobHead), ops.data(), ops.size() * sizeof(OpHead));
     memcpy(out->data() + h.coef_off, (const void *)coef.data(), coef.size() * sizeof(OpCoef<T, A>));
-    if (!gi.empty()) memcpy(out->data() + h.gi_off, gi.data(), gi.size() * sizeof(GroupInfo));
+    if (!gi.empty()) memcpy(out->data() + h.gi_off, gi.data(), gi.size() * sizeof(gi[0]));
     return ZC_OK;
 }
 
@@ -1034,21 +791,17 @@ __device__ void load_job(SweepSmem<T, A> &c, const char *blk) {
     copy16(&c.job, blk, sizeof(JobHead));
     copy16(c.ops, blk + sizeof(JobHead), nops * (uint32_t)sizeof(OpHead));
     copy16(c.coef, blk + h->coef_off, nops * (uint32_t)sizeof(OpCoef<T, A>));
-    if constexpr (has_passes<T, A>()) copy16(c.gi, blk + h->gi_off, nops * (uint32_t)sizeof(GroupInfo));
+    if constexpr (PassOf<T, A>::any) copy16(c.gi, blk + h->gi_off, nops * (uint32_t)sizeof(c.gi[0]));
     for (uint32_t r = tid; r < (1u << H); r += blockDim.x) {  // tile bit L + j holds qubit hpos[j]
         uint32_t o = 0;
         for (uint32_t j = 0; j < H; j++) o |= ((r >> j) & 1u) << (h->hpos[j] - L);
         c.rows[r] = o;
     }
     __syncthreads();
-    if constexpr (A != AR_DF) {  // the job's diagonal index tables, once per job
+    if constexpr (SweepSmem<T, A>::kLuts > 0) {  // the job's diagonal index tables, once per job
         bool any = false;
         for (uint32_t o = 0; o < nops; o++) {
             const OpHead &op = c.ops[o];
-            if (has_passes<T, A>() && c.gi[o].G) {
-                o += c.gi[o].skip - 1;
-                continue;
-            }
             if (op.kind != MOP_DK || op.b == kNoJobLut) continue;
             any = true;
             uint16_t *lut = c.luts + (size_t)op.b * kJlutLen;
@@ -1144,7 +897,7 @@ __device__ void process_tile(SweepSmem<T, A> &c, T *re, T *im, uint64_t t, const
             for (uint32_t v = tid; v < size; v += blockDim.x) to_pairs(v);
             __syncthreads();
         }
-        apply_ops<T, A, float2>(fr, fi, c.ops, c.coef, (int)c.job.nops, base, size, tables, &c.bad, c.jlut, nullptr, c.gi,
+        apply_ops<T, A, float2>(fr, fi, c.ops, c.coef, (int)c.job.nops, base, size, tables, c.jlut, nullptr, c.gi,
                                 fuse_in,
                                 fuse_out);
         if (c.job.has_arith && !fuse_out) {  // register passes leave pairs unnormalised
@@ -1165,27 +918,12 @@ __device__ void process_tile(SweepSmem<T, A> &c, T *re, T *im, uint64_t t, const
             }
         }
     } else {
-        apply_ops<T, A, T>(sre, sim, c.ops, c.coef, (int)c.job.nops, base, size, tables, &c.bad, c.jlut, c.luts, c.gi);
+        apply_ops<T, A, T>(sre, sim, c.ops, c.coef, (int)c.job.nops, base, size, tables, c.jlut, c.luts, c.gi);
     }
     __syncthreads();
     tile_store(c, re + base, sre, vecs);
     tile_store(c, im + base, sim, vecs);
     __syncthreads();  // the buffer is free
-}
-
-// Error record (the first CTA that found a bad index fills it): err[0] = 2;
-// then CTA, L, H, ops and the offending index at 1, 6, 7, 8, 10.
-template <typename T, int A>
-__device__ void sweep_exit(SweepSmem<T, A> &c, int *err) {
-    __syncthreads();
-    if (threadIdx.x == 0 && c.bad && atomicCAS(err, 0, 2) == 0) {
-        err[1] = (int)blockIdx.x;
-        err[6] = (int)c.job.L;
-        err[7] = (int)c.job.H;
-        err[8] = (int)c.job.nops;
-        err[10] = (int)c.bad;
-        __threadfence();
-    }
 }
 
 // One state. One CTA streams tiles through a single shared-memory buffer;
@@ -1196,15 +934,13 @@ __device__ void sweep_exit(SweepSmem<T, A> &c, int *err) {
 template <typename T, int A, uint32_t FORM>
 __global__ void __launch_bounds__(kSweepThreads, kSweepCtasPerSm)
     k_sweep(T *__restrict__ re, T *__restrict__ im, uint64_t ntiles, const char *__restrict__ job,
-            const char *__restrict__ tables, int *__restrict__ err) {
+            const char *__restrict__ tables) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ SweepSmem<T, A> c;
     T *sre = reinterpret_cast<T *>(smem);
     T *sim = sre + kTileArrayBytes / sizeof(T);
-    if (threadIdx.x == 0) c.bad = 0;
     load_job(c, job);
     for (uint64_t t = blockIdx.x; t < ntiles; t += gridDim.x) process_tile(c, re, im, t, tables, sre, sim, FORM);
-    sweep_exit(c, err);
 }
 
 // Many states in one launch (the serving engine's packed step): the tiles
@@ -1212,14 +948,13 @@ __global__ void __launch_bounds__(kSweepThreads, kSweepCtasPerSm)
 // belongs to another state.
 template <typename T, int A>
 __global__ void __launch_bounds__(kSweepThreads, kSweepCtasPerSm)
-    k_sweep_multi(const char *__restrict__ blob, int *__restrict__ err) {
+    k_sweep_multi(const char *__restrict__ blob) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ SweepSmem<T, A> c;
     const SweepBatch *hdr = reinterpret_cast<const SweepBatch *>(blob);
     const SweepJob *jobs = reinterpret_cast<const SweepJob *>(blob + sizeof(SweepBatch));
     const uint32_t njobs = hdr->njobs;
     const uint64_t total = hdr->total_tiles;
-    if (threadIdx.x == 0) c.bad = 0;
     int cur = -1;
     // Tiles go to CTAs round-robin (concurrent tiles stay adjacent in memory
     // and big and small jobs mix evenly); the job is looked up only when a
@@ -1245,7 +980,6 @@ __global__ void __launch_bounds__(kSweepThreads, kSweepCtasPerSm)
         process_tile(c, reinterpret_cast<T *>(J.re), reinterpret_cast<T *>(J.im), t - J.tile_start,
                      blob + J.tables_off, sre, sim, 0u);
     }
-    sweep_exit(c, err);
 }
 
 template <typename T, int A, uint32_t FORM>
@@ -1260,7 +994,7 @@ int run_sweep_form(zc_state *st, const SweepGeom &g, const char *dev_job, const 
         return fail(ZC_ERR_INVALID, "sweep shape exceeds the kernel's limits");
     const uint64_t blocks = std::min<uint64_t>(g.ntiles, (uint64_t)st->num_sms * kSweepCtasPerSm);
     k_sweep<T, A, FORM><<<(int)blocks, kSweepThreads, kSweepSmemBytes, st->stream>>>(
-        (T *)st->re, (T *)st->im, g.ntiles, dev_job, dev_tables, st->d_err);
+        (T *)st->re, (T *)st->im, g.ntiles, dev_job, dev_tables);
     ZC_CUDA(cudaGetLastError());
     return ZC_OK;
 }
@@ -1280,14 +1014,14 @@ int run_sweep(zc_state *st, const SweepGeom &g, const char *dev_job, const char 
 }
 
 template <typename T, int A>
-int run_sweep_multi(cudaStream_t stream, int num_sms, const char *dev_blob, int *d_err) {
+int run_sweep_multi(cudaStream_t stream, int num_sms, const char *dev_blob) {
     static std::atomic<bool> attr{false};  // set once per process; racing first calls repeat it
     if (!attr) {
         ZC_CUDA(cudaFuncSetAttribute(k_sweep_multi<T, A>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)kSweepSmemBytes));
         attr = true;
     }
-    k_sweep_multi<T, A><<<num_sms * kSweepCtasPerSm, kSweepThreads, kSweepSmemBytes, stream>>>(dev_blob, d_err);
+    k_sweep_multi<T, A><<<num_sms * kSweepCtasPerSm, kSweepThreads, kSweepSmemBytes, stream>>>(dev_blob);
     ZC_CUDA(cudaGetLastError());
     return ZC_OK;
 }
@@ -1323,12 +1057,12 @@ int launch_df_to_f64(zc_state *st) {
     return ZC_OK;
 }
 
-int launch_sweep_multi(cudaStream_t stream, int num_sms, int prec, bool exact, const char *dev_blob, int *d_err) {
+int launch_sweep_multi(cudaStream_t stream, int num_sms, int prec, bool exact, const char *dev_blob) {
     if (prec == 64)
-        return exact ? run_sweep_multi<double, AR_EXACT>(stream, num_sms, dev_blob, d_err)
-                     : run_sweep_multi<double, AR_DF>(stream, num_sms, dev_blob, d_err);
-    return exact ? run_sweep_multi<float, AR_EXACT>(stream, num_sms, dev_blob, d_err)
-                 : run_sweep_multi<float, AR_FMA>(stream, num_sms, dev_blob, d_err);
+        return exact ? run_sweep_multi<double, AR_EXACT>(stream, num_sms, dev_blob)
+                     : run_sweep_multi<double, AR_DF>(stream, num_sms, dev_blob);
+    return exact ? run_sweep_multi<float, AR_EXACT>(stream, num_sms, dev_blob)
+                 : run_sweep_multi<float, AR_FMA>(stream, num_sms, dev_blob);
 }
 
 int encode_job(int prec, bool exact, const SweepPlan &plan, std::vector<char> *out) {
