@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(kDfThreads) k_total_df(const T *__restrict__ r
     __shared__ bool s_last;
     using VT = typename Vec<T>::type;
     constexpr int V = Vec<T>::N, U = 4;
-    const bool inside = ONES && (1u << q) < (uint32_t)V;  // both halves in every vector
+    const bool inside = ONES && (1ull << q) < (uint64_t)V;  // both halves in every vector
     const uint64_t stride = (uint64_t)gridDim.x * kDfThreads;
     float2 acc[U] = {};
     auto element = [&](uint64_t u) {  // first element of vector u of the sum
