@@ -35,7 +35,7 @@ extern "C" {
                                  vs the f64 oracle); f64 in double-float pairs on the FP32 pipe with f64
                                  storage (max |d amp| <= 1e-12) */
 #define ZC_FLAG_NO_SWEEPS 2u  /* one launch per op: disables multi-op sweep scheduling */
-#define ZC_FLAG_FORCE_SWEEPS 4u /* schedule sweeps even for small states (testing) */
+#define ZC_FLAG_FORCE_SWEEPS 4u /* kept for callers; sweeps run from three qubits without it */
 #define ZC_FLAG_PER_SHOT 8u   /* noisy runs: replay shot by shot (zeno's order and RNG) instead of batching */
 #define ZC_FLAG_TENSOR 16u    /* f32 states: dense k>=3 blocks as 3xTF32 tensor-core GEMMs (FP32 accumulation) */
 
@@ -89,7 +89,7 @@ int zc_finish(zc_state *st);
  * not). Its scratch is a fixed ~0.9 MiB device array that every GPU loading
  * the library keeps until exit. Limits: <= 30 qubits, <= 16384 shots;
  * larger requests get ZC_ERR_INVALID. Queued ops must be flushed first
- * (zc_finish). The call synchronises the state's stream (it routes the
+ * (zc_finish; states under 14 qubits flush here). The call synchronises the state's stream (it routes the
  * draws on the host between its two kernels). The first call on a device
  * resolves the array's device address. All calls share the array: calls
  * that overlap (on the GPU or from several threads) race. */

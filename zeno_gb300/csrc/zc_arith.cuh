@@ -403,10 +403,6 @@ __device__ __forceinline__ float2 df_axpy_u(float2 x, float2 t, float2 y) {
     lo = __fmaf_rn(t.y, y.x, lo);
     return make_float2(s, __fadd_rn(x.y, lo));
 }
-__device__ __forceinline__ float2 df_axpy(float2 x, float2 t, float2 y) {
-    const float2 r = df_axpy_u(x, t, y);
-    return df_norm(r.x, r.y);
-}
 
 __device__ __forceinline__ float2 df_renorm(float2 v) { return df_norm(v.x, v.y); }
 
@@ -415,46 +411,6 @@ __device__ __forceinline__ void cscale_df_u(float2 wr, float2 wi, float2 &ar, fl
     const float2 ni = df_dot2_u(wr, ai, wi, ar);
     ar = nr;
     ai = ni;
-}
-
-// Rotation update of (a, b) with unit diagonal: [[1, -t], [t, 1]]
-// (|t| <= 1; the scale that makes it orthogonal lives in a diagonal).
-__device__ __forceinline__ void pair_update_rot_df(float2 t, float2 &ar, float2 &ai, float2 &br, float2 &bi) {
-    const float2 nt = df_neg(t);
-    const float2 nar = df_axpy(ar, nt, br);
-    const float2 nai = df_axpy(ai, nt, bi);
-    const float2 nbr = df_axpy(br, t, ar);
-    const float2 nbi = df_axpy(bi, t, ai);
-    ar = nar;
-    ai = nai;
-    br = nbr;
-    bi = nbi;
-}
-
-// The same rotation in T (FMA-contracted).
-template <typename T>
-__device__ __forceinline__ void pair_update_rot(T t, T &ar, T &ai, T &br, T &bi) {
-    const T nar = rfma(-t, br, ar);
-    const T nai = rfma(-t, bi, ai);
-    const T nbr = rfma(t, ar, br);
-    const T nbi = rfma(t, ai, bi);
-    ar = nar;
-    ai = nai;
-    br = nbr;
-    bi = nbi;
-}
-
-// The same real update in T (FMA-contracted).
-template <typename T>
-__device__ __forceinline__ void pair_update_real(const T *r, T &ar, T &ai, T &br, T &bi) {
-    const T nar = rfma(r[0], ar, rmul(r[1], br));
-    const T nai = rfma(r[0], ai, rmul(r[1], bi));
-    const T nbr = rfma(r[2], ar, rmul(r[3], br));
-    const T nbi = rfma(r[2], ai, rmul(r[3], bi));
-    ar = nar;
-    ai = nai;
-    br = nbr;
-    bi = nbi;
 }
 
 __device__ __forceinline__ void cscale_df(float2 wr, float2 wi, float2 &ar, float2 &ai) {
@@ -498,11 +454,6 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) {
     unsigned long long d;
     asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(pk_bits(a)), "l"(pk_bits(b)));
-    return pk_float2(d);
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-    unsigned long long d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(pk_bits(a)), "l"(pk_bits(b)));
     return pk_float2(d);
 }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {

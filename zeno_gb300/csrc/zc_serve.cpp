@@ -180,10 +180,14 @@ int packed_step(zc_server *s, int gi, int round, int *issued) {
         j.im = r->view.im;
         j.ntiles = plan.g.ntiles;
         j.tile_start = tiles;
-        tiles += plan.g.ntiles;
         size_t off = (body.size() + 15) & ~(size_t)15;
         int rc = encode_job(prec, ex, plan, &blk);
         if (rc) return rc;
+        // full: this request and those behind it go with the next launch (a
+        // double-float job takes ~9 KB, so that is ~1800 of them)
+        if (sizeof(SweepBatch) + (jobs.size() + 1) * sizeof(SweepJob) + 512 + off + blk.size() + plan.tables.size() >
+            kBlobBytes)
+            break;
         body.resize(off + blk.size());
         memcpy(body.data() + off, blk.data(), blk.size());
         j.job_off = off;
@@ -191,6 +195,7 @@ int packed_step(zc_server *s, int gi, int round, int *issued) {
         body.resize(off + plan.tables.size());
         if (!plan.tables.empty()) memcpy(body.data() + off, plan.tables.data(), plan.tables.size());
         j.tables_off = off;
+        tiles += plan.g.ntiles;
         jobs.push_back(j);
         planned.push_back({r, std::move(plan)});
     }
@@ -476,7 +481,7 @@ int zc_server_step(zc_server *s, zc_server_status *status) {
     s->steps++;
     int h = 0;
     ZC_CUDA(cudaMemcpy(&h, s->ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost));
-    if (h) return fail(ZC_ERR_CUDA, "packed sweep found a tile index out of range");
+    if (h) return fail(ZC_ERR_CUDA, "a kernel of this step reported an error");
     if (status) {
         status->pending = s->pending.size();
         status->active = s->active.size();

@@ -174,16 +174,8 @@ __device__ __forceinline__ PkReal rot_pairs(const OpCoef<T, A> &c) {
 }
 
 // Double-float sweeps hold each amplitude as packed pairs: slot v of the
-// re array H = (re hi, im hi), of the im array L = (re lo, im lo). The ops
-// outside register passes use the scalar routines on split pairs.
-__device__ __forceinline__ void hl_rot_df(float2 t, float2 &Ha, float2 &La, float2 &Hb, float2 &Lb) {
-    float2 ar, ai, br, bi;
-    pk_split(Ha, La, ar, ai);
-    pk_split(Hb, Lb, br, bi);
-    pair_update_rot_df(t, ar, ai, br, bi);
-    pk_join(ar, ai, Ha, La);
-    pk_join(br, bi, Hb, Lb);
-}
+// re array H = (re hi, im hi), of the im array L = (re lo, im lo). General
+// gates use the scalar routines on split pairs.
 __device__ __forceinline__ void hl_rdf(const float2 *r, float2 &Ha, float2 &La, float2 &Hb, float2 &Lb) {
     float2 ar, ai, br, bi;
     pk_split(Ha, La, ar, ai);
