@@ -28,18 +28,8 @@
 namespace zc {
 namespace {
 
-constexpr int kSweepThreads = 256;
+constexpr int kSweepThreads = 256;  // table diagonals split an index at its eighth bit
 constexpr int kSweepCtasPerSm = 3;
-constexpr uint32_t kJlutHigh = 1u << (13 - 8);  // tile index values above the low byte (tiles <= 2^13)
-constexpr uint32_t kJlutLen = 256 + kJlutHigh;
-// Sweeps without register passes (f32 and exact f64) keep the index tables
-// of their first kJobLuts table diagonals for the whole job, in the shared
-// memory the pass descriptors take in double-float sweeps; further table
-// diagonals build theirs per tile. A table diagonal's `b` field (in the
-// CTA's copy of the micro-ops) names its job table, or kNoJobLut.
-// (Exact f64 sweeps: the others' diagonals ride in register passes.)
-constexpr int kJobLuts = 5;
-constexpr uint32_t kNoJobLut = 0xffffffffu;
 // The tile's re array, then, this far behind it whatever the tile's size, im.
 constexpr uint32_t kTileArrayBytes = (uint32_t)(kSweepSmemBytes / 2);
 
@@ -210,14 +200,6 @@ struct PassOf {
     using type = typename std::conditional<A == AR_DF, GroupInfo, RegOp>::type;
     static constexpr bool any = A == AR_DF || sizeof(T) == 4;
 };
-
-template <typename R>
-__device__ __forceinline__ uint32_t jgather(const OpHead &op, uint32_t jo, uint32_t v) {
-    uint32_t j = jo;
-    for (uint32_t b = 0; b < op.k; b++)
-        if (!(op.loc[b] & kOuterFlag)) j |= ((v >> op.loc[b]) & 1) << b;
-    return j;
-}
 
 __device__ __forceinline__ uint32_t jouter(const OpHead &op, uint64_t base) {
     uint32_t jo = 0;
@@ -486,7 +468,7 @@ __device__ void run_pass_any(const GroupInfo &gi, char *tile, const OpHead *ops,
 // fuse_in / fuse_out: its first / last pass converts the tile.
 template <typename T, int A, typename R>
 __device__ void apply_ops(R *sr, R *si, const OpHead *ops, const OpCoef<T, A> *coef, int nops, uint64_t base,
-                          uint32_t size, const char *tables, uint16_t *jlut, const uint16_t *job_luts,
+                          uint32_t size, const char *tables,
                           const typename PassOf<T, A>::type *gis,
                           int fuse_in = 0, int fuse_out = 0) {
     const int tid = threadIdx.x, nt = blockDim.x;
@@ -556,52 +538,41 @@ __device__ void apply_ops(R *sr, R *si, const OpHead *ops, const OpCoef<T, A> *c
                 if constexpr (A == AR_DF) hl_cscale_df(coef[o].v[one ? 2 : 0], coef[o].v[one ? 3 : 1], xr, xi);
                 else cscale<T, A == AR_EXACT>(coef[o].v[one ? 2 : 0], coef[o].v[one ? 3 : 1], xr, xi);
             };
-            if constexpr (sizeof(R) == 4) {  // four consecutive elements per 16-byte vector
-                float4 *vr = reinterpret_cast<float4 *>(sr), *vi = reinterpret_cast<float4 *>(si);
-                for (uint32_t q = tid; q < size / 4; q += nt) {
-                    const float4 a = vr[q], b = vi[q];
-                    const uint32_t v0 = 4 * swz<16>(q);  // the elements this vector holds
-                    R xr[4] = {a.x, a.y, a.z, a.w}, xi[4] = {b.x, b.y, b.z, b.w};
+            uint32_t v = tid;
+            for (; v + 3u * nt < size; v += 4u * nt) {
+                R xr[4], xi[4];
 #pragma unroll
-                    for (int k = 0; k < 4; k++) scl(v0 + k, xr[k], xi[k]);
-                    vr[q] = make_float4(xr[0], xr[1], xr[2], xr[3]);
-                    vi[q] = make_float4(xi[0], xi[1], xi[2], xi[3]);
+                for (int k = 0; k < 4; k++) {
+                    xr[k] = sr[v + k * nt];
+                    xi[k] = si[v + k * nt];
                 }
-            } else {
-                uint32_t v = tid;
-                for (; v + 3u * nt < size; v += 4u * nt) {
-                    R xr[4], xi[4];
 #pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        xr[k] = sr[v + k * nt];
-                        xi[k] = si[v + k * nt];
-                    }
-#pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        scl(swz<(int)sizeof(R)>(v + k * nt), xr[k], xi[k]);
-                        sr[v + k * nt] = xr[k];
-                        si[v + k * nt] = xi[k];
-                    }
+                for (int k = 0; k < 4; k++) {
+                    scl(swz<(int)sizeof(R)>(v + k * nt), xr[k], xi[k]);
+                    sr[v + k * nt] = xr[k];
+                    si[v + k * nt] = xi[k];
                 }
-                for (; v < size; v += nt) scl(swz<(int)sizeof(R)>(v), sr[v], si[v]);
             }
+            for (; v < size; v += nt) scl(swz<(int)sizeof(R)>(v), sr[v], si[v]);
         } else if (op.kind == MOP_DK) {
-            const uint32_t jo = jouter(op, base);
+            // The table index of the element in slot v is linear over XOR: the
+            // bits of v select masks that the job brings along (in the op's
+            // coefficients). Gathering the op's bits through a lookup table
+            // built per tile cost the 25-qubit QFT a tenth (10.5 -> 9.5 ms).
+            const uint16_t *mask = reinterpret_cast<const uint16_t *>(&coef[o]);
+            uint32_t j0 = jouter(op, base);
+#pragma unroll
+            for (int b = 0; b < 8; b++) j0 ^= (tid >> b) & 1 ? mask[b] : 0u;
+            auto index_of = [&](uint32_t v) {
+                uint32_t j = j0;
+#pragma unroll
+                for (int b = 8; b < 13; b++) j ^= (v >> b) & 1u ? mask[b] : 0u;
+                return j;
+            };
             // (re, im) pairs of T, or double-float (re hi, re lo, im hi, im lo)
             using P2 = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
             const P2 *ptab = reinterpret_cast<const P2 *>(tables + op.table);
             const float4 *dtab = reinterpret_cast<const float4 *>(tables + op.table);
-            // table index of element v = jo | lut[v & 255] | lut[256 + (v >> 8)]:
-            // the op's local bits gathered once per job (or once per tile)
-            // instead of per element
-            const uint16_t *lut = jlut;
-            if (op.b != kNoJobLut) {
-                lut = job_luts + (size_t)op.b * kJlutLen;
-            } else {
-                for (uint32_t x = tid; x < kJlutLen; x += nt)
-                    jlut[x] = (uint16_t)jgather<R>(op, 0u, x < 256 ? x : (x - 256) << 8);
-                __syncthreads();
-            }
             // W: the table entry (T re, T im; or one float4 of double-float pairs)
             using W = typename std::conditional<A == AR_DF, float4, T>::type;
             auto load_w = [&](uint32_t j, W &wr, W &wi) {
@@ -617,47 +588,28 @@ __device__ void apply_ops(R *sr, R *si, const OpHead *ops, const OpCoef<T, A> *c
                 if constexpr (A == AR_DF) hl_cscale_df(make_float2(wr.x, wr.y), make_float2(wr.z, wr.w), xr, xi);
                 else cscale<T, A == AR_EXACT>(wr, wi, xr, xi);
             };
-            if constexpr (sizeof(R) == 4) {  // four consecutive elements per 16-byte vector
-                float4 *vr = reinterpret_cast<float4 *>(sr), *vi = reinterpret_cast<float4 *>(si);
-                for (uint32_t q = tid; q < size / 4; q += nt) {
-                    const uint32_t v0 = 4 * swz<16>(q), jh = jo | lut[256 + (v0 >> 8)];  // same high bits for all four
-                    W wr[4], wi[4];
+            uint32_t v = tid;
+            for (; v + 3u * nt < size; v += 4u * nt) {
+                R xr[4], xi[4];
+                W wr[4], wi[4];
+                const uint32_t j = index_of(v);
 #pragma unroll
-                    for (int k = 0; k < 4; k++) load_w(jh | lut[(v0 & 255u) + k], wr[k], wi[k]);
-                    const float4 a = vr[q], b = vi[q];
-                    R xr[4] = {a.x, a.y, a.z, a.w}, xi[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-                    for (int k = 0; k < 4; k++) scl(wr[k], wi[k], xr[k], xi[k]);
-                    vr[q] = make_float4(xr[0], xr[1], xr[2], xr[3]);
-                    vi[q] = make_float4(xi[0], xi[1], xi[2], xi[3]);
+                for (int k = 0; k < 4; k++) {
+                    load_w(j ^ (k & 1 ? mask[8] : 0u) ^ (k & 2 ? mask[9] : 0u), wr[k], wi[k]);
+                    xr[k] = sr[v + k * nt];
+                    xi[k] = si[v + k * nt];
                 }
-            } else {
-                uint32_t v = tid;
-                for (; v + 3u * nt < size; v += 4u * nt) {
-                    R xr[4], xi[4];
-                    W wr[4], wi[4];
 #pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        const uint32_t vk = swz<(int)sizeof(R)>(v + k * nt);
-                        const uint32_t j = jo | lut[vk & 255u] | lut[256 + (vk >> 8)];
-                        load_w(j, wr[k], wi[k]);
-                        xr[k] = sr[v + k * nt];
-                        xi[k] = si[v + k * nt];
-                    }
-#pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        scl(wr[k], wi[k], xr[k], xi[k]);
-                        sr[v + k * nt] = xr[k];
-                        si[v + k * nt] = xi[k];
-                    }
+                for (int k = 0; k < 4; k++) {
+                    scl(wr[k], wi[k], xr[k], xi[k]);
+                    sr[v + k * nt] = xr[k];
+                    si[v + k * nt] = xi[k];
                 }
-                for (; v < size; v += nt) {
-                    const uint32_t vk = swz<(int)sizeof(R)>(v);
-                    const uint32_t j = jo | lut[vk & 255u] | lut[256 + (vk >> 8)];
-                    W wr, wi;
-                    load_w(j, wr, wi);
-                    scl(wr, wi, sr[v], si[v]);
-                }
+            }
+            for (; v < size; v += nt) {
+                W wr, wi;
+                load_w(index_of(v), wr, wi);
+                scl(wr, wi, sr[v], si[v]);
             }
         } else {
             apply_perm(sr, si, op, base, size);
@@ -674,10 +626,7 @@ struct SweepSmem {
     OpCoef<T, A> coef[kMaxMicroOps];
     uint32_t rows[1u << kMaxSweepHigh];  // row r of a tile starts at element rows[r] << L of it
     JobHead job;
-    uint16_t jlut[kJlutLen];  // diagonal index tables of the current DK op
     alignas(16) typename PassOf<T, A>::type gi[PassOf<T, A>::any ? kMaxMicroOps : 1];  // register passes
-    static constexpr int kLuts = PassOf<T, A>::any ? 0 : kJobLuts;
-    uint16_t luts[kLuts * kJlutLen + 1];  // the job's diagonal index tables
 };
 static_assert(sizeof(OpHead[kMaxMicroOps]) % 16 == 0 && sizeof(GroupInfo[kMaxMicroOps]) % 16 == 0,
               "job sections are copied in 16-byte pieces");
@@ -696,7 +645,6 @@ int encode_job_as(const SweepPlan &plan, std::vector<char> *out) {
     for (uint32_t j = 0; j < h.H && j < 8; j++) h.hpos[j] = plan.g.hpos[j];
     std::vector<OpHead> ops((size_t)nops);
     std::vector<OpCoef<T, A>> coef((size_t)nops);
-    uint32_t nlut = 0;
     for (int o = 0; o < nops; o++) {
         const MicroOp &m = plan.mops[(size_t)o];
         memcpy(&ops[(size_t)o], &m, sizeof(OpHead));
@@ -712,6 +660,14 @@ int encode_job_as(const SweepPlan &plan, std::vector<char> *out) {
             } else {
                 c.v[i] = (T)m.m[i];
             }
+        }
+        if (m.kind == MOP_DK) {  // table index masks of the slot bits (see apply_ops)
+            uint16_t mask[13] = {};
+            static_assert(sizeof mask <= sizeof c, "index masks fit the op's coefficients");
+            for (uint32_t b = 0; b < h.L + h.H; b++)
+                for (uint32_t i = 0; i < m.k; i++)
+                    if (!(m.loc[i] & kOuterFlag)) mask[b] |= (uint16_t)(((swz<(int)sizeof(T)>(1u << b) >> m.loc[i]) & 1u) << i);
+            memcpy((void *)&c, mask, sizeof mask);
         }
         if constexpr (A == AR_DF) {
             if (m.kind == MOP_RT) {  // the rotation's packed pairs
@@ -754,8 +710,6 @@ int encode_job_as(const SweepPlan &plan, std::vector<char> *out) {
             q.jb_step = (uint16_t)jb;
         }
     }
-    for (OpHead &op : ops)
-        if (op.kind == MOP_DK) op.b = nlut < (uint32_t)SweepSmem<T, A>::kLuts ? nlut++ : kNoJobLut;
     auto up16 = [](size_t b) { return (b + 15) & ~(size_t)15; };
     const size_t ops_b = up16(ops.size() * sizeof(OpHead)), coef_b = up16(coef.size() * sizeof(OpCoef<T, A>));
     h.coef_off = (uint32_t)(sizeof(JobHead) + ops_b);
@@ -790,18 +744,6 @@ __device__ void load_job(SweepSmem<T, A> &c, const char *blk) {
         c.rows[r] = o;
     }
     __syncthreads();
-    if constexpr (SweepSmem<T, A>::kLuts > 0) {  // the job's diagonal index tables, once per job
-        bool any = false;
-        for (uint32_t o = 0; o < nops; o++) {
-            const OpHead &op = c.ops[o];
-            if (op.kind != MOP_DK || op.b == kNoJobLut) continue;
-            any = true;
-            uint16_t *lut = c.luts + (size_t)op.b * kJlutLen;
-            for (uint32_t x = tid; x < kJlutLen; x += blockDim.x)
-                lut[x] = (uint16_t)jgather<T>(op, 0u, x < 256 ? x : (x - 256) << 8);
-        }
-        if (any) __syncthreads();
-    }
 }
 
 // All threads: one array of a tile between global and shared memory, 16
@@ -889,7 +831,7 @@ __device__ void process_tile(SweepSmem<T, A> &c, T *re, T *im, uint64_t t, const
             for (uint32_t v = tid; v < size; v += blockDim.x) to_pairs(v);
             __syncthreads();
         }
-        apply_ops<T, A, float2>(fr, fi, c.ops, c.coef, (int)c.job.nops, base, size, tables, c.jlut, nullptr, c.gi,
+        apply_ops<T, A, float2>(fr, fi, c.ops, c.coef, (int)c.job.nops, base, size, tables, c.gi,
                                 fuse_in,
                                 fuse_out);
         if (c.job.has_arith && !fuse_out) {  // register passes leave pairs unnormalised
@@ -910,7 +852,7 @@ __device__ void process_tile(SweepSmem<T, A> &c, T *re, T *im, uint64_t t, const
             }
         }
     } else {
-        apply_ops<T, A, T>(sre, sim, c.ops, c.coef, (int)c.job.nops, base, size, tables, c.jlut, c.luts, c.gi);
+        apply_ops<T, A, T>(sre, sim, c.ops, c.coef, (int)c.job.nops, base, size, tables, c.gi);
     }
     __syncthreads();
     tile_store(c, re + base, sre, vecs);
