@@ -39,26 +39,25 @@ METRIC = "30q circuit throughput (u3 + matching-CX, depth 40, f64)"
 # DRAM read+write per launch over algorithmic bytes, from an ncu capture of
 # the f64 double-float sweep kernel at 26 qubits (state 8x the L2; the sweeps
 # between the first and the last of a flush, which hand the state over as
-# packed double-float pairs): 1.074 GB read + 1.029 GB write against
+# packed double-float pairs): 1.074 GB read + 1.022 GB write against
 # 2S = 2.147 GB.
-MEASURED_TRAFFIC_RATIO = {"sweep": (1.074e9 + 1.029e9) / 2.147e9}
-# The same capture: issue slots 50-51% busy, FMA pipe 30-31% of its
-# instruction peak and 46% of its cycles (packed f32x2 rotations), ALU pipe
-# 24-25%, FP64 0%.
-SWEEP_DF_PIPES = {"issue_active_pct": 49.6, "fma_pipe_pct": 30.0, "fma_pipe_cycles_pct": 46.2, "alu_pipe_pct": 24.3,
+MEASURED_TRAFFIC_RATIO = {"sweep": (1.074e9 + 1.022e9) / 2.147e9}
+# The same capture: issue slots 55-56% busy, FMA pipe 31-32% of its
+# instruction peak and 47-51% of its cycles (packed f32x2 rotations), ALU pipe
+# 28-31%, FP64 0%.
+SWEEP_DF_PIPES = {"issue_active_pct": 55.5, "fma_pipe_pct": 32.4, "fma_pipe_cycles_pct": 50.8, "alu_pipe_pct": 28.4,
                   "fp64_pipe_pct": 0.0}
 # FP32 operations per amplitude of each double-float sweep micro-op
 # (zeno_gb300/csrc/zc_arith.cuh; rotations issue them as packed f32x2
-# instructions, two operations each): a product is 4 (MUL + 3 FMA), TwoSum 6,
-# renormalisation 3. Complex 2x2: four 4-term dot products per pair
-# (4*4 + 3*6 + 6 + 3 = 43 each) = 86; real 2x2 and one-qubit diagonals:
-# 2-term dot products (2*4 + 6 + 2 + 3 = 19), two per amplitude = 38. Register
-# passes chain unnormalised pairs: table diagonal 2 x (2*4 + 6 + 2) = 32,
-# rotation [[1, -t], [t, 1]] 2 x (4 + 6 + 2) = 24 (one renormalisation per
-# sweep, where the tile goes back to f64, is not counted). CX and SWAP move
-# data only.
-DF_FP32_OPS_PER_AMP = {"complex": 86, "diag1": 38, "diag_table": 32, "cx": 0, "swap": 0, "real": 38,
-                         "rotation": 24}
+# instructions, two operations each): a split product is 4 (MUL + 3 FMA), TwoSum
+# 6, renormalisation 3. Complex 2x2: four 4-term dot products per pair
+# (4*4 + 3*6 + 6 + 3 = 43 each) = 86; a 2-term dot product is 12 (the residual of
+# a sum with a product is one FMA), so a real 2x2 takes 2 x (12 + 3) = 30 and a
+# diagonal 24; rotation [[1, -t], [t, 1]]: x + t*y is 10, so 20 (one
+# renormalisation per sweep, where the tile goes back to f64, is not counted).
+# CX and SWAP move data only.
+DF_FP32_OPS_PER_AMP = {"complex": 86, "diag1": 24, "diag_table": 24, "cx": 0, "swap": 0, "real": 30,
+                         "rotation": 20}
 CONFIG_NAMES = ("matching_20q", "qft", "fusion_sweep", "big_state", "trajectories", "gate_mix_tc", "serving")
 
 
@@ -493,7 +492,7 @@ def main():
                                  if dom in MEASURED_TRAFFIC_RATIO else None),
                      "ops_per_launch": len(ops) * a.steps / dd["launches"] if dom == "sweep" else 1.0,
                      "limiter": ("double-float arithmetic on the FP32 pipe, not HBM: each sweep applies many "
-                                 "gates per HBM pass; the rest is barrier and L1 latency; ncu at 26q: %s"
+                                 "gates per HBM pass; the rest is shared-memory and dependency latency; ncu at 26q: %s"
                                  % SWEEP_DF_PIPES) if df_sweep else None,
                      "compute": ({"bound": "fp32_pipe", "unit": "FP32 op/s",
                                   "achieved": fp32_ops / (dd["ms"] / 1e3),
