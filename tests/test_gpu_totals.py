@@ -32,6 +32,20 @@ def test_fast_totals(zc, prec, n):
     g.close()
 
 
+@pytest.mark.parametrize("prec,n", [(p, n) for p in (64, 32) for n in (1, 11, 12, 13, 16, 18)] + [(32, 25)])
+def test_fast_sampler_tiles(zc, prec, n):
+    """Chunks below, at and above one tile of the rescan, few chunks (wide CTAs)
+    and many: at least 99.9% of 4096 draws are exact mode's."""
+    amps = rand_state(n, 70 + n, normalize=True)
+    draws = []
+    for flags in (zc.FLAG_FAST, zc.FLAG_EXACT):
+        g = zc.CudaBackend(n, prec, flags)
+        g.load_state(amps)
+        draws.append(g.sample(4096, 5))
+        g.close()
+    assert np.mean(draws[0] == draws[1]) >= 0.999
+
+
 @pytest.mark.parametrize("prec", (64, 32))
 @pytest.mark.parametrize("n", (3, 9, 13))
 def test_noalloc_sampler_sees_queued_gates(zc, prec, n):

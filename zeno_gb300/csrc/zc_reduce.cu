@@ -302,19 +302,20 @@ __device__ __forceinline__ float2 block_sum_df(float2 v, float2 *red) {
 }
 
 // One CTA per chunk; f64 partials (the sampler's chunk masses).
-template <typename T>
-__global__ void __launch_bounds__(kDfThreads) k_chunk_sums_df(const T *__restrict__ re, const T *__restrict__ im,
-                                                              uint64_t total, uint64_t chunk,
-                                                              double *__restrict__ part) {
-    __shared__ float2 red[kDfThreads / 32];
+// NT threads: 1024 while the chunks leave SMs idle, where a chunk's latency is
+// what counts (wide_chunks), else 256.
+template <typename T, int NT>
+__global__ void __launch_bounds__(NT) k_chunk_sums_df(const T *__restrict__ re, const T *__restrict__ im,
+                                                      uint64_t total, uint64_t chunk, double *__restrict__ part) {
+    __shared__ float2 red[NT / 32];
     const uint64_t lo = (uint64_t)blockIdx.x * chunk;
     const uint64_t hi = lo + chunk < total ? lo + chunk : total;
     float2 acc[4] = {};
-    for (uint64_t h0 = lo + threadIdx.x; h0 < hi; h0 += 4 * kDfThreads) {
+    for (uint64_t h0 = lo + threadIdx.x; h0 < hi; h0 += 4 * NT) {
         T vr[4], vi[4];
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-            const uint64_t h = h0 + (uint64_t)u * kDfThreads;
+            const uint64_t h = h0 + (uint64_t)u * NT;
             vr[u] = vi[u] = (T)0;
             if (h < hi) {
                 vr[u] = re[h];
@@ -395,22 +396,21 @@ __global__ void k_total_small(const T *re, const T *im, uint64_t total, int ones
     *out = df_to_f64(a);
 }
 
-// Sampler pass 2, one CTA per touched chunk: tiles of 2048 elements get a
+// Sampler pass 2, one CTA per touched chunk: tiles of NT x 8 or 4
+// elements get a
 // CTA-wide inclusive prefix of |a|^2 (double-float) on top of the running
 // cumulative; each draw of the tile resolves by binary search to the first
 // index whose cumulative exceeds it (the reference's `us[ptr] < acc`).
 // Draws left over past the chunk go to its last nonzero index.
-constexpr int kScanPer = 8;
-constexpr int kScanTile = kDfThreads * kScanPer;
-
-template <typename T>
-__global__ void __launch_bounds__(kDfThreads) k_sample_scan_df(const T *__restrict__ re, const T *__restrict__ im,
+template <typename T, int NT>
+__global__ void __launch_bounds__(NT) k_sample_scan_df(const T *__restrict__ re, const T *__restrict__ im,
                                                                const SampleChunk *__restrict__ cs,
                                                                const double *__restrict__ us,
                                                                uint64_t *__restrict__ out, uint64_t chunk_len,
                                                                uint64_t total) {
+    constexpr int kScanPer = NT == 1024 ? 4 : 8, kScanTile = NT * kScanPer;
     __shared__ float2 s_cum[kScanTile];
-    __shared__ float2 s_wsum[kDfThreads / 32];
+    __shared__ float2 s_wsum[NT / 32];
     __shared__ unsigned long long s_last;
     const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
     const SampleChunk sc = cs[blockIdx.x];
@@ -445,7 +445,19 @@ __global__ void __launch_bounds__(kDfThreads) k_sample_scan_df(const T *__restri
         if (lane == 31) s_wsum[warp] = incl;
         __syncthreads();
         float2 wpre = make_float2(0.f, 0.f);
-        for (int w = 0; w < warp; w++) wpre = df_add(wpre, s_wsum[w]);
+        if constexpr (NT == 1024) {  // 32 warps: a scan, not 31 sums in a row
+            float2 ws = s_wsum[lane];
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const float2 v = shfl_up_df(ws, d);
+                if (lane >= d) ws = df_add(v, ws);
+            }
+            const int from = warp ? warp - 1 : 0;
+            const float2 before = make_float2(__shfl_sync(0xffffffffu, ws.x, from), __shfl_sync(0xffffffffu, ws.y, from));
+            if (warp) wpre = before;
+        } else {
+            for (int w = 0; w < warp; w++) wpre = df_add(wpre, s_wsum[w]);
+        }
         const float2 tb = df_add(base, df_add(wpre, excl));
 #pragma unroll
         for (int j = 0; j < kScanPer; j++) s_cum[tid * kScanPer + j] = df_add(tb, pre[j]);
@@ -453,7 +465,7 @@ __global__ void __launch_bounds__(kDfThreads) k_sample_scan_df(const T *__restri
         const int nvalid = hi - t0 < (uint64_t)kScanTile ? (int)(hi - t0) : kScanTile;
         const unsigned long long end_key = df_key(s_cum[nvalid - 1]);
         uint64_t resolved = 0;
-        for (uint64_t d0 = ptr; d0 < sc.s1; d0 += kDfThreads) {
+        for (uint64_t d0 = ptr; d0 < sc.s1; d0 += NT) {
             const uint64_t d = d0 + tid;
             int in = 0;
             if (d < sc.s1) {
@@ -471,7 +483,7 @@ __global__ void __launch_bounds__(kDfThreads) k_sample_scan_df(const T *__restri
             }
             const int cnt = __syncthreads_count(in);
             resolved += (uint64_t)cnt;
-            if (cnt < kDfThreads) break;
+            if (cnt < NT) break;
         }
         ptr += resolved;
         base = s_cum[nvalid - 1];
@@ -483,7 +495,7 @@ __global__ void __launch_bounds__(kDfThreads) k_sample_scan_df(const T *__restri
         if (my_last) atomicMax(&s_last, my_last);
         __syncthreads();
         const uint64_t ln = s_last ? s_last - 1 : hi - 1;
-        for (uint64_t d = ptr + tid; d < sc.s1; d += kDfThreads) out[d] = ln;
+        for (uint64_t d = ptr + tid; d < sc.s1; d += NT) out[d] = ln;
     }
 }
 
@@ -507,6 +519,7 @@ int run_chain(zc_state *st, uint64_t total, uint64_t chunk, uint64_t nrows, int 
 // Split re / im arrays -> interleaved f64 (re, im) pairs, four amplitudes per
 // thread (16-byte loads, 64 bytes of stores).
 template <typename T>
+
 __global__ void __launch_bounds__(256) k_interleave(const T *__restrict__ re, const T *__restrict__ im,
                                                     double2 *__restrict__ out, uint64_t len) {
     const uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) * 4;
@@ -541,6 +554,29 @@ int launch_interleave(zc_state *st, uint64_t first, uint64_t count, void *dst) {
     return ZC_OK;
 }
 
+// Chunks enough for two CTAs of 256 threads per SM keep HBM busy (30q: 93-97%
+// of its peak); fewer are as fast as one chunk, which 1024 threads take through
+// sooner: 1024 draws at 19 qubits (8 chunks) within a run of 1.63 -> 1.48 ms,
+// 24 served requests 7.4 -> 6.9 ms; 25 qubits (512 chunks) unchanged.
+static bool wide_chunks(const zc_state *st, size_t nch) { return nch <= (size_t)st->num_sms * 2; }
+
+template <typename T>
+void run_chunk_sums_df(zc_state *st, uint64_t total, uint64_t chunk, size_t nch, double *part) {
+    const T *re = (const T *)st->re, *im = (const T *)st->im;
+    if (wide_chunks(st, nch)) k_chunk_sums_df<T, 1024><<<(unsigned)nch, 1024, 0, st->stream>>>(re, im, total, chunk, part);
+    else k_chunk_sums_df<T, kDfThreads><<<(unsigned)nch, kDfThreads, 0, st->stream>>>(re, im, total, chunk, part);
+}
+
+template <typename T>
+void run_sample_scan_df(zc_state *st, size_t nch, const SampleChunk *cs, const double *us, uint64_t *out,
+                        uint64_t chunk_len) {
+    const T *re = (const T *)st->re, *im = (const T *)st->im;
+    if (wide_chunks(st, nch))
+        k_sample_scan_df<T, 1024><<<(unsigned)nch, 1024, 0, st->stream>>>(re, im, cs, us, out, chunk_len, st->len);
+    else
+        k_sample_scan_df<T, kDfThreads><<<(unsigned)nch, kDfThreads, 0, st->stream>>>(re, im, cs, us, out, chunk_len, st->len);
+}
+
 int launch_chunk_sums(zc_state *st, int mode, uint32_t q, size_t *nchunks_out, bool exact, double *out) {
     const uint64_t total = mode == 0 ? st->len : st->len / 2;
     const uint64_t chunk = total < (1ull << kSampleChunkLog2) ? total : (1ull << kSampleChunkLog2);
@@ -557,12 +593,8 @@ int launch_chunk_sums(zc_state *st, int mode, uint32_t q, size_t *nchunks_out, b
     *nchunks_out = nch;
     if (!exact) {  // only whole-state masses: prob_one is launch_total's
         if (mode != 0) return fail(ZC_ERR_INVALID, "fast chunk sums cover whole states");
-        if (st->prec == 64)
-            k_chunk_sums_df<double><<<(unsigned)nch, kDfThreads, 0, st->stream>>>(
-                (const double *)st->re, (const double *)st->im, total, chunk, part);
-        else
-            k_chunk_sums_df<float><<<(unsigned)nch, kDfThreads, 0, st->stream>>>(
-                (const float *)st->re, (const float *)st->im, total, chunk, part);
+        if (st->prec == 64) run_chunk_sums_df<double>(st, total, chunk, nch, part);
+        else run_chunk_sums_df<float>(st, total, chunk, nch, part);
         ZC_CUDA(cudaGetLastError());
         return ZC_OK;
     }
@@ -620,12 +652,8 @@ int launch_sample_scan(zc_state *st, const SampleChunk *d_chunks, size_t nchunks
     ProfScope ps(st, K_SAMPLE_SCAN, (double)nchunks * chunk_len * (st->prec / 8) * 2);
     st->ctr.launches++;
     if (!exact) {
-        if (st->prec == 64)
-            k_sample_scan_df<double><<<(unsigned)nchunks, kDfThreads, 0, st->stream>>>(
-                (const double *)st->re, (const double *)st->im, d_chunks, d_us, d_out, chunk_len, st->len);
-        else
-            k_sample_scan_df<float><<<(unsigned)nchunks, kDfThreads, 0, st->stream>>>(
-                (const float *)st->re, (const float *)st->im, d_chunks, d_us, d_out, chunk_len, st->len);
+        if (st->prec == 64) run_sample_scan_df<double>(st, nchunks, d_chunks, d_us, d_out, chunk_len);
+        else run_sample_scan_df<float>(st, nchunks, d_chunks, d_us, d_out, chunk_len);
         ZC_CUDA(cudaGetLastError());
         return ZC_OK;
     }

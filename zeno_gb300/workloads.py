@@ -201,7 +201,7 @@ def trajectories(peak_gbs) -> Dict[str, object]:
             "launches": r.launches, "batched": r.batched, "ops": passes, "keys": len(r.counts),
             "state_pass_GBps": 4096 * passes * 2 * S / t / 1e9,
             "note": "state passes of every trajectory (2S per op, S = 512 KiB) over wall time; each "
-                    "trajectory's state stays in its CTA's L2-resident buffer, so this is not HBM traffic"}
+                    "trajectory's state stays in shared memory and the L2, so this is not HBM traffic"}
 
 
 def gate_mix_tc(peak_gbs, tf32_tflops=None, qubits=28) -> Dict[str, object]:
