@@ -41,7 +41,7 @@ struct MicroOp {
 
 // A job as the kernel takes it (encode_job, zc_sweep.cu): this head, then at
 // 16-byte boundaries the op heads, the coefficients in the arithmetic's form
-// (coef_off), and for double-float sweeps the register passes (gi_off),
+// (coef_off), and for double-float and f32 sweeps the register passes (gi_off),
 // copied as they are into the CTA's shared tables.
 struct JobHead {
     uint32_t nops, L, H, has_arith;
