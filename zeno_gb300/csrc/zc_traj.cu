@@ -16,7 +16,8 @@
 // pending for the next pass and prepares the next op; two CTA barriers per op.
 // All draws of an op are independent of the state and come in the
 // reference's order from a per-trajectory Philox4x32-10 stream
-// (zc_philox.h). Probabilities are summed in double-float.
+// (zc_philox.h). Probabilities are summed in two floats per lane (zc_mass.h)
+// and over lanes and warps in FP64.
 //
 // Where the state lives. The pass is bound by moving the state (2S per op),
 // so it stays as close as it fits: up to 14 qubits (128 KiB) in shared
@@ -31,15 +32,18 @@
 // stands between two passes. Measured for 2048 trajectories of the 16-qubit
 // depth-20 circuit under damping: 402 ms with one scalar pass per op over
 // global memory (114 instructions per amplitude, four CTAs per SM, half the
-// traffic from DRAM), 106 ms now (15 us per op and SM; bound by the latency of
-// the L2 half of the state and the decisions between passes); 1500 shots of a
-// 13-qubit dynamic circuit: 10.2 -> 2.3 ms. Measured and dropped: two units
+// traffic from DRAM), 118 ms now (17 us per op and SM; bound by the latency of
+// the L2 half of the state, the sums of squares and the decisions between
+// passes; 106 with sums on top of a constant, which lost digits of small ones,
+// see zc_mass.h); 1500 shots of a 13-qubit dynamic circuit: 10.2 -> 2.2 ms.
+// Measured and dropped: two units
 // per thread for one-qubit ops (+17%, registers), 256-bit accesses to an
 // interleaved global part (2x, spills), passes out of line (+20%).
 #include <algorithm>
 
 #include "zc_arith.cuh"
 #include "zc_internal.h"
+#include "zc_mass.h"
 #include "zc_philox.h"
 #include "zc_traj.h"
 
@@ -102,7 +106,7 @@ struct Shared {
     uint32_t dq[3];               // all qubits of the diagonal factors, and the factors by their bits
     float dr[8], di[8];
     int nd;
-    float2 red[NT / 32][8];       // per-warp tables (double-float)
+    double red[NT / 32][8];       // per-warp tables
     double J[8];                  // joint probability table of a three-qubit op
     double seg[32], blk[32];      // final sampling: region and block masses
     double el[1024];              //   and the element masses of one block
@@ -273,57 +277,93 @@ __device__ void split_pending(Shared<NT> &s) {
     if (threadIdx.x == 0) s.npend = np;
 }
 
-// a + b in double-float (TwoSum on the high parts, low parts summed).
-__device__ __forceinline__ float2 tdf_add(float2 a, float2 b) {
-    float e;
-    const float s = two_sum(a.x, b.x, e);
-    return df_norm(s, __fadd_rn(e, __fadd_rn(a.y, b.y)));
-}
-__device__ __forceinline__ float2 shfl_xor_f2(float2 v, int m) {
-    return make_float2(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m));
+// The operations of zc_mass.h on two lanes.
+struct MassF2 {
+    typedef P2 V;
+    static __device__ __forceinline__ P2 zero() { return 0ull; }
+    static __device__ __forceinline__ P2 fma(P2 a, P2 b, P2 c) { return p2_fma(a, b, c); }
+    static __device__ __forceinline__ P2 add(P2 a, P2 b) { return p2_add(a, b); }
+    static __device__ __forceinline__ P2 sub(P2 a, P2 b) { return p2_sub(a, b); }
+    static __device__ __forceinline__ P2 neg(P2 a) { return a ^ 0x8000000080000000ull; }
+};
+
+// A folded sum as f64 (by integer operations; below 2^-75 those drop l).
+__device__ __forceinline__ double mass_f64(float2 v) {
+    if (v.x > 0.f && v.x < 0x1p-75f) return (double)v.x + (double)v.y;
+    return df_to_f64(v);
 }
 
-// Sum D per-thread double-float values over the warp into red[0..D): lanes
+__device__ __forceinline__ float2 sum_of(float2 a, float2 b) {
+    mass_join<MassF1>(a.x, a.y, b.x, b.y);
+    return a;
+}
+__device__ __forceinline__ double sum_of(double a, double b) { return a + b; }
+
+// Table values of a CTA of NT threads on their way through a warp. From eight
+// warps on they are float pairs down to the lowest four lanes: many values,
+// whose roundings average out, while FP64 takes an SM 19 cycles per warp
+// instruction (16 qubits, as above: 130 -> 126 ms when measured). Smaller CTAs
+// have fewer values, and theirs are FP64 from the start.
+template <int NT>
+using TableValue = typename std::conditional<(NT >= 256), float2, double>::type;
+
+__device__ __forceinline__ void table_value(float2 v, float2 &out) { out = v; }
+__device__ __forceinline__ void table_value(float2 v, double &out) { out = mass_f64(v); }
+// Both lanes of a sum.
+template <typename V>
+__device__ __forceinline__ V mass_end(P2 h, P2 l) {
+    mass_fold<MassF2>(h, l);
+    const float2 a = pk_float2(h), b = pk_float2(l);
+    V x, y;
+    table_value(make_float2(a.x, b.x), x);
+    table_value(make_float2(a.y, b.y), y);
+    return sum_of(x, y);
+}
+__device__ __forceinline__ float2 shfl_xor_of(float2 v, int m) {
+    return make_float2(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m));
+}
+__device__ __forceinline__ double shfl_xor_of(double v, int m) { return __shfl_xor_sync(0xffffffffu, v, m); }
+
+// Sum D per-thread values over the lanes at offsets 16 down to `last`: lanes
 // halve the values they carry as they exchange them (D - 1 + 5 - log2 D
-// additions instead of 5 D).
-template <int D>
-__device__ __forceinline__ void warp_table(float2 *v, float2 *red) {
+// additions instead of 5 D). Left in v[0]; returns which of the D it is.
+template <int D, typename V>
+__device__ __forceinline__ int lane_table(V *v, int last, int &off) {
     const int lane = threadIdx.x % 32;
-    int off = 16, base = 0;
+    int base = 0;
+    off = 16;
 #pragma unroll
     for (int w = D; w > 1; w >>= 1, off >>= 1) {
         const bool upper = lane & off;
 #pragma unroll
         for (int j = 0; j < w / 2; j++) {
-            const float2 give = upper ? v[j] : v[j + w / 2], keep = upper ? v[j + w / 2] : v[j];
-            v[j] = tdf_add(keep, shfl_xor_f2(give, off));
+            const V give = upper ? v[j] : v[j + w / 2], keep = upper ? v[j + w / 2] : v[j];
+            v[j] = sum_of(keep, shfl_xor_of(give, off));
         }
         if (upper) base += w / 2;
     }
+    const int first = off;
 #pragma unroll
-    for (int o = off; o > 0; o >>= 1) v[0] = tdf_add(v[0], shfl_xor_f2(v[0], o));
-    if ((lane & (2 * off - 1)) == 0) red[base] = v[0];
+    for (int o = first; o >= last; o >>= 1) v[0] = sum_of(v[0], shfl_xor_of(v[0], o));
+    off = first;
+    return base;
 }
 
-// |y|^2 of both halves into (h, l), h >= |y|^2: the sum's high part in one
-// FMA, t - h exact (h <= t <= 2h), and the square minus that difference is
-// what the rounding dropped. The accumulators start at kBias, above any
-// |amplitude|^2 of a normalised state, and give it back at the end; the sum
-// keeps 2^-46 of the state's norm.
-constexpr float kBias = 1.0f;
-__device__ __forceinline__ void acc_sq2(float2 y, float2 &h, float2 &l) {
-    const float2 t = fma2(y, y, h);
-    l = add2(l, fma2(y, y, sub2(h, t)));
-    h = t;
+// The warp's table into red[0..D).
+template <int D>
+__device__ __forceinline__ void warp_table(float2 *v, double *red) {
+    int off;
+    const int base = lane_table<D>(v, 4, off);
+    double t = mass_f64(v[0]);
+    t += __shfl_xor_sync(0xffffffffu, t, 2);
+    t += __shfl_xor_sync(0xffffffffu, t, 1);
+    if ((threadIdx.x % 32 & (2 * off - 1)) == 0) red[base] = t;
 }
-__device__ __forceinline__ float2 acc_end(float2 h, float2 l) {
-    return tdf_add(df_norm(__fsub_rn(h.x, kBias), l.x), df_norm(__fsub_rn(h.y, kBias), l.y));
-}
-
-__device__ __forceinline__ void acc_pair(P2 y, P2 &h, P2 &l) {
-    const P2 t = p2_fma(y, y, h);
-    l = p2_add(l, p2_fma(y, y, p2_sub(h, t)));
-    h = t;
+template <int D>
+__device__ __forceinline__ void warp_table(double *v, double *red) {
+    int off;
+    const int base = lane_table<D>(v, 1, off);
+    if ((threadIdx.x % 32 & (2 * off - 1)) == 0) red[base] = v[0];
 }
 
 // Matrix entries read where they are used: hoisted out of the pass loop, the
@@ -429,12 +469,14 @@ __device__ __forceinline__ void traj_pass_body(float *work, uint32_t n, int o, i
     // factor index bits; qubits that are not there read bit 31 of the vector
     // number, which is zero
     const uint32_t fq0 = nfv > 0 ? s.fqv[0] : 31, fq1 = nfv > 1 ? s.fqv[1] : 31, fq2 = nfv > 2 ? s.fqv[2] : 31;
-    P2 h[D], l[D];
+    // Sums per row and lane. With 64 threads the two pairs of groups have one
+    // each: as many partial sums, so as small an error, as 256 threads have.
+    constexpr int S = NT == 64 ? 2 : 1;
+    P2 h[S][D], l[S][D];
 #pragma unroll
-    for (int r = 0; r < D; r++) {
-        h[r] = p2_make(kBias, kBias);
-        l[r] = p2_make(0.f, 0.f);
-    }
+    for (int i = 0; i < S; i++)
+#pragma unroll
+        for (int r = 0; r < D; r++) h[i][r] = l[i][r] = 0ull;
     // the thread's vectors: unit u spread around the spanned bits, then those
     auto vector = [&](uint32_t u, int v) {
         uint32_t vb = ((u >> plo) << (plo + 1)) | (u & ((1u << plo) - 1));
@@ -503,16 +545,19 @@ __device__ __forceinline__ void traj_pass_body(float *work, uint32_t n, int o, i
                                 bi[r] = p2_fma(wr, ai, c ? p2_fma(wi, ar, bi[r]) : p2_mul(wi, ar));
                             }
                         }
-                        if (acc) {
-                            acc_pair(br[r], h[r], l[r]);
-                            acc_pair(bi[r], h[r], l[r]);
-                        }
                     }
 #pragma unroll
                     for (int r = 0; r < D; r++) {
                         xr[i][r][p] = br[r];
                         xi[i][r][p] = bi[r];
                     }
+                }
+                if (acc) {  // one branch for all rows: one per row kept their arithmetic apart (126 -> 118 ms)
+#pragma unroll
+                    for (int p = 0; p < 2; p++)
+#pragma unroll
+                        for (int r = 0; r < D; r++)
+                            mass_add2<MassF2>(xr[i][r][p], xi[i][r][p], h[p % S][r], l[p % S][r]);
                 }
                 if (!MONO) {
                     lanes<K, false>(xr[i], low);
@@ -525,11 +570,22 @@ __device__ __forceinline__ void traj_pass_body(float *work, uint32_t n, int o, i
                     *sm.im4(vi) = make_ulonglong2(xi[i][v][0], xi[i][v][1]);
                 }
             }
-    }
-    float2 tab[D];
+        if ((u0 / NT) % (kMassFold / 4) == kMassFold / 4 - 1) {  // four squares per row, lane and unit
 #pragma unroll
-    for (int r = 0; r < D; r++) tab[r] = acc_end(pk_float2(h[r]), pk_float2(l[r]));
-    if (acc) warp_table<D>(tab, s.red[threadIdx.x / 32]);
+            for (int i = 0; i < S; i++)
+#pragma unroll
+                for (int r = 0; r < D; r++) mass_fold<MassF2>(h[i][r], l[i][r]);
+        }
+    }
+    if (!acc) return;
+    using V = TableValue<NT>;
+    V tab[D];
+#pragma unroll
+    for (int r = 0; r < D; r++) {
+        tab[r] = mass_end<V>(h[0][r], l[0][r]);
+        if (S == 2) tab[r] = sum_of(tab[r], mass_end<V>(h[S - 1][r], l[S - 1][r]));
+    }
+    warp_table<D>(tab, s.red[threadIdx.x / 32]);
 }
 
 // A dense two-qubit op's pass, out of line: its registers would crowd the
@@ -547,11 +603,15 @@ __device__ __noinline__ void traj_pass_general(float *work, uint32_t n, int o, i
     const StateMem<SMEM> sm(work, n);
     const uint64_t len = 1ull << n;
     const uint32_t k = s.op(o).k, dim = 1u << k;
-    float2 acc[8];
+    // Sums per row, for CTAs of up to 128 threads two: a thread's groups in turn.
+    constexpr int S = NT <= 128 ? 2 : 1;
+    float h[S][8], l[S][8];
 #pragma unroll
-    for (int r = 0; r < 8; r++) acc[r] = make_float2(kBias, 0.f);
+    for (int i = 0; i < S; i++)
+#pragma unroll
+        for (int r = 0; r < 8; r++) h[i][r] = l[i][r] = 0.f;
     const uint64_t groups = len >> k;
-    for (uint64_t g = threadIdx.x; g < groups; g += NT) {
+    auto group = [&](uint64_t g, float (&hs)[8], float (&ls)[8]) {
         const uint64_t base = insert_zeros(g, s.op(o).qs, (int)k);
         float xr[8], xi[8];
 #pragma unroll
@@ -580,18 +640,31 @@ __device__ __noinline__ void traj_pass_general(float *work, uint32_t n, int o, i
             for (uint32_t b = 0; b < k; b++) idx |= (uint64_t)((r >> b) & 1) << s.op(o).qs[b];
             sm.re(idx) = yr;
             sm.im(idx) = yi;
-            float2 h = make_float2(acc[r].x, kBias), l = make_float2(acc[r].y, 0.f);
-            acc_sq2(make_float2(yr, 0.f), h, l);
-            acc_sq2(make_float2(yi, 0.f), h, l);
-            acc[r] = make_float2(h.x, l.x);
+            mass_add2<MassF1>(yr, yi, hs[r], ls[r]);
+        }
+        if ((g / NT) % (kMassFold / 2) >= kMassFold / 2 - S) {
+#pragma unroll
+            for (int r = 0; r < 8; r++) mass_fold<MassF1>(hs[r], ls[r]);
+        }
+    };
+    for (uint64_t g = threadIdx.x; g < groups; g += S * NT) {
+        group(g, h[0], l[0]);
+        if (S == 2 && g + NT < groups) group(g + NT, h[S - 1], l[S - 1]);
+    }
+    if (!table) return;
+    TableValue<NT> tab[8], x;
+#pragma unroll
+    for (int r = 0; r < 8; r++) {
+#pragma unroll
+        for (int i = 0; i < S; i++) {
+            mass_fold<MassF1>(h[i][r], l[i][r]);
+            table_value(make_float2(h[i][r], l[i][r]), x);
+            tab[r] = i ? sum_of(tab[r], x) : x;
         }
     }
-#pragma unroll
-    for (int r = 0; r < 8; r++) acc[r] = df_norm(__fsub_rn(acc[r].x, kBias), acc[r].y);
-    if (!table) return;
-    if (k == 1) warp_table<2>(acc, s.red[threadIdx.x / 32]);
-    else if (k == 2) warp_table<4>(acc, s.red[threadIdx.x / 32]);
-    else warp_table<8>(acc, s.red[threadIdx.x / 32]);
+    if (k == 1) warp_table<2>(tab, s.red[threadIdx.x / 32]);
+    else if (k == 2) warp_table<4>(tab, s.red[threadIdx.x / 32]);
+    else warp_table<8>(tab, s.red[threadIdx.x / 32]);
 }
 
 // One warp: the next 32 Philox blocks of trajectory t, one per lane, when
@@ -920,19 +993,15 @@ __device__ __noinline__ void finish_op(int o, int cur, bool acc, const TrajRec *
 #pragma unroll
     for (int j = 0; j < D; j++) J[j] = 0.0;
     if (acc) {
-        float2 v[D];
+        double v[D];
 #pragma unroll
         for (int j = 0; j < D; j += G) v[j] = s.red[lane % NW][(j + lane / NW) & (D - 1)];
 #pragma unroll
         for (int o = NW / 2; o > 0; o >>= 1)
 #pragma unroll
-            for (int j = 0; j < D; j += G) v[j] = tdf_add(v[j], shfl_xor_f2(v[j], o));
+            for (int j = 0; j < D; j += G) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
 #pragma unroll
-        for (int j = 0; j < D; j++) {
-            const int src = (j % G) * NW;
-            const float hi = __shfl_sync(0xffffffffu, v[j - j % G].x, src), lo = __shfl_sync(0xffffffffu, v[j - j % G].y, src);
-            J[j] = (double)hi + (double)lo;
-        }
+        for (int j = 0; j < D; j++) J[j] = __shfl_sync(0xffffffffu, v[j - j % G], (j % G) * NW);
     }
     const bool gate = s.op(o).kind == TOP_GATE;
     if constexpr (K == 3) {
@@ -967,20 +1036,32 @@ __device__ __forceinline__ double mass_at(const StateMem<SMEM> &sm, const Shared
     return (double)xr * xr + (double)xi * xi;
 }
 
-// Warp: the mass of elements [i0, i1) in double-float.
+// Warp: the mass of elements [i0, i1).
 template <int NT, bool SMEM>
 __device__ double range_mass(const StateMem<SMEM> &sm, const Shared<NT> &s, uint64_t i0, uint64_t i1) {
-    float2 h = make_float2(kBias, kBias), l = make_float2(0.f, 0.f);
-    for (uint64_t i = i0 + threadIdx.x % 32; i < i1; i += 32) {
+    P2 h[2] = {0, 0}, l[2] = {0, 0};  // a lane's elements in turn
+    const uint64_t first = i0 + threadIdx.x % 32;
+    auto value = [&](uint64_t i) {
+        if (i >= i1) return MassF2::zero();
         float fr, fi;
         diag_factor(s, i, fr, fi);
         const float a = sm.re(i), c = sm.im(i);
-        acc_sq2(make_float2(fr * a - fi * c, fr * c + fi * a), h, l);
-    }
-    float2 v = acc_end(h, l);
+        return p2_make(fr * a - fi * c, fr * c + fi * a);
+    };
+    uint32_t folded = 0;
+    for (uint64_t i = first; i < i1; i += 128) {
+        mass_add2<MassF2>(value(i), value(i + 64), h[0], l[0]);
+        mass_add2<MassF2>(value(i + 32), value(i + 96), h[1], l[1]);
+        if (++folded == kMassFold / 2) {
+            folded = 0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = tdf_add(v, shfl_xor_f2(v, o));
-    return (double)v.x + (double)v.y;
+            for (int j = 0; j < 2; j++) mass_fold<MassF2>(h[j], l[j]);
+        }
+    }
+    double v = mass_end<double>(h[0], l[0]) + mass_end<double>(h[1], l[1]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
 }
 
 // One basis index from |psi|^2 by the draw u in [0, 1): region (one per
