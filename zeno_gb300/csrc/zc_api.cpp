@@ -196,13 +196,6 @@ int launch_single(zc_state *st, const QOp &op) {
     }
 }
 
-static uint64_t touch_mask(const QOp &op) {
-    if (op.kind == Q_CX || op.kind == Q_SWAP) return (1ull << op.a) | (1ull << op.b);
-    uint64_t m = 0;
-    for (uint32_t i = 0; i < op.k; i++) m |= 1ull << op.qs[i];
-    return m;
-}
-
 // Qubits that must be local for `op` to run inside a sweep.
 static uint64_t need_mask(const QOp &op) {
     switch (op.kind) {
@@ -266,20 +259,24 @@ static uint32_t loc_of(uint32_t q, uint32_t L, const std::vector<uint32_t> &high
 // rules above). Fills `plan` and returns how many ops it took; 0 or 1 means
 // the front op should simply run on its own.
 size_t plan_sweep(uint32_t n, int prec, bool ex, uint32_t L, uint32_t Hcap, const std::vector<QOp> &q,
-                  SweepPlan *plan) {
+                  SweepPlan *plan, size_t head, uint64_t touch_all) {
     const uint64_t low_mask = L >= 64 ? ~0ull : ((1ull << L) - 1);
     uint64_t blocked = 0, highs_mask = 0;
     uint32_t nhigh = 0;
     bool arith_deferred = false;
     std::vector<size_t> &taken = plan->taken;
     taken.clear();
-    const size_t window = std::min(q.size(), kQueueWindow);
+    const size_t window = head + std::min(q.size() - head, kQueueWindow);
+    const uint64_t qubits = touch_all & (n >= 64 ? ~0ull : (1ull << n) - 1);
     // Under double-float lowering a diagonal joins the pending tables and
     // becomes a micro-op only when flushed, so it does not count against the
     // micro-op budget here (the lowered count is checked below).
     const bool df_lowering = !ex && prec == 64;
     size_t counted = 0;
-    for (size_t i = 0; i < window && counted < (size_t)kMaxMicroOps && taken.size() < 4 * (size_t)kMaxMicroOps;
+    // once every qubit is blocked no later op can join (walking the rest of the
+    // window regardless cost 5 us per lone op)
+    for (size_t i = head; i < window && counted < (size_t)kMaxMicroOps &&
+                          taken.size() < 4 * (size_t)kMaxMicroOps && (blocked & qubits) != qubits;
          i++) {
         const QOp &op = q[i];
         const uint64_t touch = touch_mask(op);
@@ -419,7 +416,7 @@ size_t plan_sweep(uint32_t n, int prec, bool ex, uint32_t L, uint32_t Hcap, cons
     const size_t fit = taken.size() * (size_t)kMaxMicroOps / low.size();
     taken.resize(std::min(fit, taken.size() - 1));
     if (taken.size() <= 1) {
-        taken.resize(1);
+        taken.assign(1, head);
         plan->carry.clear();
         return taken.size();
     }
@@ -474,30 +471,34 @@ size_t plan_sweep(uint32_t n, int prec, bool ex, uint32_t L, uint32_t Hcap, cons
     return taken.size();
 }
 
-// Remove the ops at the (ascending) indices `taken`, keeping the rest in order.
-void erase_taken(std::vector<QOp> &q, const std::vector<size_t> &taken) {
-    std::vector<QOp> rest;
-    rest.reserve(q.size() - taken.size());
-    size_t ti = 0;
-    for (size_t i = 0; i < q.size(); i++) {
-        if (ti < taken.size() && taken[ti] == i) {
-            ti++;
-            continue;
+// The ops that stay move up against those behind the plan's reach, so the cost
+// is that of the plan's own span. The carried diagonals act after every op the
+// sweep took and touch only qubits those ops touched; no op deferred ahead of
+// them touches those qubits, so the queue front is their place in program order.
+void consume_plan(std::vector<QOp> &q, SweepPlan &plan, size_t *head) {
+    size_t from = head ? *head : 0;
+    if (!plan.taken.empty()) {
+        size_t w = plan.taken.back() + 1, ti = plan.taken.size();
+        for (size_t i = w; i-- > from;) {
+            if (ti && plan.taken[ti - 1] == i) {
+                ti--;
+                std::vector<double>().swap(q[i].data);
+                continue;
+            }
+            if (--w != i) q[w] = std::move(q[i]);
         }
-        rest.push_back(std::move(q[i]));
+        from = w;
     }
-    q.swap(rest);
-}
-
-// The carried diagonals act after every op the sweep took and touch only
-// qubits those ops touched; no op deferred ahead of them touches those qubits,
-// so the queue front is their place in program order.
-void consume_plan(std::vector<QOp> &q, SweepPlan &plan) {
-    erase_taken(q, plan.taken);
-    if (!plan.carry.empty()) {
-        q.insert(q.begin(), std::make_move_iterator(plan.carry.begin()), std::make_move_iterator(plan.carry.end()));
-        plan.carry.clear();
+    if (plan.carry.size() > from) {  // (a plan carries fewer diagonals than it took ops)
+        q.insert(q.begin() + (long)from, plan.carry.size() - from, QOp{});
+        from = plan.carry.size();
     }
+    while (!plan.carry.empty()) {
+        q[--from] = std::move(plan.carry.back());
+        plan.carry.pop_back();
+    }
+    if (head) *head = from;
+    else q.erase(q.begin(), q.begin() + (long)from);
 }
 
 // Ops of a fast f64 state that read and leave packed double-float pairs.
@@ -512,19 +513,19 @@ static int settle_form(zc_state *st) {
     return launch_df_to_f64(st);
 }
 
-// Plan and launch one sweep starting at the queue front; erases what ran.
+// Plan and launch one sweep starting at the queue front; takes out what ran.
 static int run_one_sweep(zc_state *st) {
-    std::vector<QOp> &q = st->queue;
+    OpQueue &q = st->queue;
     const SweepShape sh = shape_for(st);
     SweepPlan plan;
-    if (plan_sweep(st->n, st->prec, program_order(st), sh.L, sh.Hcap, q, &plan) <= 1) {
+    if (plan_sweep(st->n, st->prec, program_order(st), sh.L, sh.Hcap, q.ops, &plan, q.head, q.touch) <= 1) {
         // nothing to batch: the per-op kernel is the same work (a permutation
         // moves slots whatever they hold)
         const bool perm = q.front().kind == Q_CX || q.front().kind == Q_SWAP;
         int rc = perm ? ZC_OK : settle_form(st);
         if (rc) return rc;
         rc = launch_single(st, q.front());
-        q.erase(q.begin());
+        q.pop();
         return rc;
     }
     std::vector<char> blob;
@@ -536,7 +537,7 @@ static int run_one_sweep(zc_state *st) {
     const void *dev = nullptr;
     rc = arena_put(st, blob.data(), blob.size(), &dev);
     if (rc) return rc;
-    consume_plan(q, plan);
+    consume_plan(q.ops, plan, &q.head);
     // Fast f64: consecutive sweeps of one flush hand the state over as
     // (hi, lo) float pairs, also to and from small dense blocks; the last one
     // (nothing that takes pairs queued behind it) rounds it back to f64.
@@ -567,7 +568,7 @@ int flush(zc_state *st) {
                 rc = settle_form(st);
                 if (rc == ZC_OK) rc = launch_single(st, op);
             }
-            st->queue.erase(st->queue.begin());
+            st->queue.pop();
             continue;
         }
         rc = run_one_sweep(st);
@@ -580,7 +581,7 @@ int flush(zc_state *st) {
 static int enqueue(zc_state *st, QOp &&op) {
     st->ctr.ops++;
     if (!sweeps_enabled(st)) return launch_single(st, op);
-    st->queue.push_back(std::move(op));
+    st->queue.push(std::move(op));
     if (st->queue.size() >= kQueueFlushAt) return flush(st);
     return ZC_OK;
 }

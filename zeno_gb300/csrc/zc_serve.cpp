@@ -44,7 +44,7 @@ struct Request {
     uint32_t n = 0;
     int prec = 32;
     uint64_t shots = 0, seed = 0;
-    std::vector<QOp> queue;
+    OpQueue queue;
     std::vector<std::pair<uint32_t, uint32_t>> finals;
     size_t off = 0, bytes = 0;
     zc_state view;  // re/im in the pool; stream and scratch borrowed from the server
@@ -163,14 +163,14 @@ int packed_step(zc_server *s, int gi, int round, int *issued) {
         uint32_t L, Hcap;
         tile_shape(r, &L, &Hcap);
         SweepPlan plan;
-        if (plan_sweep(r->n, r->prec, ex, L, Hcap, r->queue, &plan) <= 1) {
+        if (plan_sweep(r->n, r->prec, ex, L, Hcap, r->queue.ops, &plan, r->queue.head, r->queue.touch) <= 1) {
             // the front op runs on its own (a dense k >= 2 block, or nothing to batch);
             // the view shares the server's parameter ring
             r->view.arena = s->ctx->arena;
             int rc = launch_single(&r->view, r->queue.front());
             s->ctx->arena = r->view.arena;
             if (rc) return rc;
-            r->queue.erase(r->queue.begin());
+            r->queue.pop();
             s->launches++;
             (*issued)++;
             continue;
@@ -230,7 +230,7 @@ int packed_step(zc_server *s, int gi, int round, int *issued) {
     s->packed_launches++;
     g.launches++;
     (*issued)++;
-    for (auto &pr : planned) consume_plan(pr.first->queue, pr.second);
+    for (auto &pr : planned) consume_plan(pr.first->queue.ops, pr.second, &pr.first->queue.head);
     return ZC_OK;
 }
 
@@ -410,7 +410,7 @@ int zc_server_submit(zc_server *s, const zc_program *p, int prec, uint64_t shots
             delete r;
             return rc;
         }
-        r->queue.push_back(to_qop(v));
+        r->queue.push(to_qop(v));
     }
     for (uint64_t i = 0; i < info.nfinal; i++) {
         uint32_t q, c;
