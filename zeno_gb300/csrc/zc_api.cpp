@@ -150,9 +150,6 @@ static int grow(void **p, size_t *cap, size_t need) {
 static constexpr size_t kQueueWindow = 2048;  // ops examined per sweep plan
 static constexpr size_t kQueueFlushAt = 8192; // queue length that forces a flush
 static constexpr uint32_t kMinSweepQubits = 3;
-// f32 states below this size keep program order in fast mode too (see
-// program_order).
-static constexpr uint32_t kF32OrderQubits = 14;
 
 int launch_single(zc_state *st, const QOp &op) {
     const bool ex = exact(st);
@@ -233,7 +230,7 @@ static SweepShape shape_for(const zc_state *st) {
         T = n <= 15 ? 8 : n <= 17 ? 9 : n <= 21 ? 10 : Tmax;
     } else if (st->prec == 64) {
         T = std::max<uint32_t>(8, n / 2 + 2);
-    } else if (n >= kF32OrderQubits) {
+    } else if (n >= kSmallStateQubits) {
         uint32_t tiles_log2 = 0;
         while ((1u << tiles_log2) < (uint32_t)(2 * st->num_sms)) tiles_log2++;
         T = n - std::min(tiles_log2, n - L);
@@ -242,10 +239,22 @@ static SweepShape shape_for(const zc_state *st) {
 }
 
 // Whether ops keep program order. Exact mode does (reordering two gates
-// changes the rounding); so do f32 states under kF32OrderQubits, whose
-// results stay those of one launch per op.
+// changes the rounding); so do small f32 states, whose results stay those of
+// one launch per op.
 static bool program_order(const zc_state *st) {
-    return exact(st) || (st->prec == 32 && st->n < kF32OrderQubits);
+    return exact(st) || (st->prec == 32 && st->n < kSmallStateQubits);
+}
+
+// Fewer queued ops than this on a small state go one by one: a sweep costs ~20
+// us (double-float ~40) of planning, copy and latency before its first op, a
+// single launch ~5. Measured from a caller's first op to the end, 8 qubits, us,
+// in sweeps / one by one: fast f64 2 ops 41/32, 4 62/44, 6 74/58, 10 92/89, 20
+// 137/167 (13 qubits: 10 102/92, 20 156/172); f32 2 34/26, 3 39/38, 4 42/44,
+// 6 51/57; exact f64 2 33/34, 4 42/46.
+static size_t min_batch(const zc_state *st) {
+    if (st->n >= kSmallStateQubits || (st->flags & ZC_FLAG_FORCE_SWEEPS)) return 0;
+    if (st->prec == 32) return 4;
+    return exact(st) ? 0 : 11;
 }
 
 static uint32_t loc_of(uint32_t q, uint32_t L, const std::vector<uint32_t> &highs) {
@@ -557,6 +566,11 @@ static bool sweeps_enabled(const zc_state *st) {
 // Launch everything queued (program order preserved where results depend on it).
 int flush(zc_state *st) {
     int rc = ZC_OK;
+    if (st->queue.size() < min_batch(st))
+        while (!st->queue.empty() && rc == ZC_OK) {
+            rc = launch_single(st, st->queue.front());
+            st->queue.pop();
+        }
     while (!st->queue.empty() && rc == ZC_OK) {
         if (!sweeps_enabled(st) || !sweepable(st->queue.front())) {
             const QOp &op = st->queue.front();

@@ -24,6 +24,9 @@ int cuda_fail(cudaError_t e, const char *where);
 constexpr int kMaxUnitaryQubits = 7;
 constexpr int kMaxDiagQubits = 12;
 constexpr int kSampleChunkLog2 = 16;  // sample.rs CHUNK = 1 << 16
+// States below this size are small: a few ops on one take as long as their
+// launches, and f32 ones keep program order in fast mode too (program_order).
+constexpr uint32_t kSmallStateQubits = 14;
 constexpr int kErrWords = 16;         // device error record (d_err) in ints
 // A state's status block (d_scalar): the scalar result, the device error
 // record and a ticket for one-launch sums; one copy reads result and record.
