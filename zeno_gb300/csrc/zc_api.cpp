@@ -118,6 +118,8 @@ static int check_support(const zc_state *st, const uint32_t *qs, uint32_t k, uin
 }
 
 static inline bool exact(const zc_state *st) { return (st->flags & ZC_FLAG_FAST) == 0; }
+// The arithmetic of the ops being launched (see few_in_exact).
+static inline bool exact_ops(const zc_state *st) { return exact(st) || st->exact_flush; }
 
 
 int sync_status(zc_state *st) {
@@ -152,7 +154,7 @@ static constexpr size_t kQueueFlushAt = 8192; // queue length that forces a flus
 static constexpr uint32_t kMinSweepQubits = 3;
 
 int launch_single(zc_state *st, const QOp &op) {
-    const bool ex = exact(st);
+    const bool ex = exact_ops(st);
     switch (op.kind) {
         case Q_UNITARY: {
             if (op.k == 1) return launch_1q(st, op.qs[0], op.data.data(), ex);
@@ -226,7 +228,7 @@ static SweepShape shape_for(const zc_state *st) {
     uint32_t Hcap = std::min<uint32_t>(Tmax - L, n - L);
     if (st->sweep_high) return SweepShape{L, std::min<uint32_t>(Hcap, st->sweep_high)};  // tuned
     uint32_t T = Tmax;
-    if (st->prec == 64 && exact(st)) {
+    if (st->prec == 64 && exact_ops(st)) {
         T = n <= 15 ? 8 : n <= 17 ? 9 : n <= 21 ? 10 : Tmax;
     } else if (st->prec == 64) {
         T = std::max<uint32_t>(8, n / 2 + 2);
@@ -242,19 +244,31 @@ static SweepShape shape_for(const zc_state *st) {
 // changes the rounding); so do small f32 states, whose results stay those of
 // one launch per op.
 static bool program_order(const zc_state *st) {
-    return exact(st) || (st->prec == 32 && st->n < kSmallStateQubits);
+    return exact_ops(st) || (st->prec == 32 && st->n < kSmallStateQubits);
 }
 
-// Fewer queued ops than this on a small state go one by one: a sweep costs ~20
-// us (double-float ~40) of planning, copy and latency before its first op, a
-// single launch ~5. Measured from a caller's first op to the end, 8 qubits, us,
-// in sweeps / one by one: fast f64 2 ops 41/32, 4 62/44, 6 74/58, 10 92/89, 20
-// 137/167 (13 qubits: 10 102/92, 20 156/172); f32 2 34/26, 3 39/38, 4 42/44,
-// 6 51/57; exact f64 2 33/34, 4 42/46.
-static size_t min_batch(const zc_state *st) {
-    if (st->n >= kSmallStateQubits || (st->flags & ZC_FLAG_FORCE_SWEEPS)) return 0;
-    if (st->prec == 32) return 4;
-    return exact(st) ? 0 : 11;
+// A few queued ops on a small state. A sweep costs ~20 us of planning, copy and
+// latency before its first op, a double-float one ~40. Measured from a caller's
+// first op to the end, us:
+//   f32, 8 qubits, in a sweep / one by one: 2 ops 34/24, 3 39/32, 4 42/44, 6
+//   51/57: fewer than four go one by one, the same bits
+//   fast f64, 8 qubits, in double-float / in exact arithmetic: 2 ops 41/33, 3
+//   59/38, 6 74/50, 10 92/66; through zc_run (whole calls) 4 167/153, 7 168/169,
+//   8 174/195, at 13 qubits 4 176/170, 6 181/183, 8 182/209: two to seven run
+//   in exact arithmetic, which is also the closer one (6 ops at 8 qubits: 5e-17
+//   off, 1e-15 in double-float). One by one in double-float 2 ops take 32 but
+//   are twenty times further off: each launch truncates to pairs. Dense blocks,
+//   whose exact sums take twice as long, keep their own way.
+static constexpr size_t kFewF32 = 4, kFewF64 = 8;
+static bool few_ops(const zc_state *st, size_t few) {
+    return st->n < kSmallStateQubits && !(st->flags & ZC_FLAG_FORCE_SWEEPS) && st->queue.size() < few;
+}
+static bool few_one_by_one(const zc_state *st) { return st->prec == 32 && few_ops(st, kFewF32); }
+static bool few_in_exact(const zc_state *st) {
+    if (st->prec == 32 || exact(st) || !few_ops(st, kFewF64) || st->queue.size() < 2) return false;
+    for (size_t i = 0; i < st->queue.size(); i++)
+        if (!sweepable(st->queue[i])) return false;
+    return true;
 }
 
 static uint32_t loc_of(uint32_t q, uint32_t L, const std::vector<uint32_t> &highs) {
@@ -538,7 +552,7 @@ static int run_one_sweep(zc_state *st) {
         return rc;
     }
     std::vector<char> blob;
-    int rc = encode_job(st->prec, exact(st), plan, &blob);
+    int rc = encode_job(st->prec, exact_ops(st), plan, &blob);
     if (rc) return rc;
     const size_t tab_off = (blob.size() + 255) & ~(size_t)255;
     blob.resize(tab_off + plan.tables.size());
@@ -550,10 +564,10 @@ static int run_one_sweep(zc_state *st) {
     // Fast f64: consecutive sweeps of one flush hand the state over as
     // (hi, lo) float pairs, also to and from small dense blocks; the last one
     // (nothing that takes pairs queued behind it) rounds it back to f64.
-    const bool df = st->prec == 64 && !exact(st);
+    const bool df = st->prec == 64 && !exact_ops(st);
     const bool out_df = df && !q.empty() && takes_pairs(q.front());
     plan.g.form = (st->df_resident ? kFormInDf : 0u) | (out_df ? kFormOutDf : 0u);
-    rc = launch_sweep(st, plan.g, (const char *)dev, (const char *)dev + tab_off, exact(st));
+    rc = launch_sweep(st, plan.g, (const char *)dev, (const char *)dev + tab_off, exact_ops(st));
     st->df_resident = out_df;
     for (const MicroOp &m : plan.mops) st->ctr.micro_ops[m.kind & 7]++;
     return rc;
@@ -566,7 +580,8 @@ static bool sweeps_enabled(const zc_state *st) {
 // Launch everything queued (program order preserved where results depend on it).
 int flush(zc_state *st) {
     int rc = ZC_OK;
-    if (st->queue.size() < min_batch(st))
+    st->exact_flush = few_in_exact(st);
+    if (few_one_by_one(st))
         while (!st->queue.empty() && rc == ZC_OK) {
             rc = launch_single(st, st->queue.front());
             st->queue.pop();
@@ -574,7 +589,7 @@ int flush(zc_state *st) {
     while (!st->queue.empty() && rc == ZC_OK) {
         if (!sweeps_enabled(st) || !sweepable(st->queue.front())) {
             const QOp &op = st->queue.front();
-            if (st->prec == 64 && !exact(st) && sweeps_enabled(st) && takes_pairs(op)) {  // a small dense block
+            if (st->prec == 64 && !exact_ops(st) && sweeps_enabled(st) && takes_pairs(op)) {  // a small dense block
                 const bool out_df = st->queue.size() > 1 && takes_pairs(st->queue[1]);
                 rc = launch_kq_small(st, op.qs, op.k, op.data.data(), false, st->df_resident, out_df);
                 st->df_resident = out_df;
@@ -588,6 +603,7 @@ int flush(zc_state *st) {
         rc = run_one_sweep(st);
     }
     st->queue.clear();
+    st->exact_flush = false;
     const int rc2 = settle_form(st);  // every other entry point sees f64
     return rc ? rc : rc2;
 }

@@ -124,6 +124,7 @@ struct zc_state {
     void *d_samp = nullptr;      // sampler work area
     size_t samp_cap = 0;
     int *d_err = nullptr;        // device error record, inside the status block
+    bool exact_flush = false;    // inside a flush: a few fast f64 ops run in exact arithmetic
     bool df_resident = false;    // inside a flush: fast f64 sweeps left packed float pairs in re / im
     zc::OpQueue queue;           // ops waiting to be scheduled into sweeps
     bool prof = false;            // record CUDA events around every launch
