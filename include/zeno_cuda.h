@@ -127,7 +127,10 @@ uint32_t zc_max_qubits(uint64_t budget, int precision_bits);
 
 /* Overwrite the state with 2^n interleaved (re, im) doubles. */
 int zc_load_state(zc_state *st, const double *amps_c64);
-/* The CUDA stream (cudaStream_t) all of this state's work runs on. */
+/* The CUDA stream (cudaStream_t) all of this state's work runs on. Ops wait on
+ * the host for a sweep, so it holds them only after a call that needs the
+ * state (zc_finish, zc_prob_one, ...). On states under 14 qubits this call
+ * launches what waits, and from then on ops go to the stream as they are applied. */
 int zc_get_stream(zc_state *st, void **stream);
 
 typedef struct {
@@ -138,6 +141,7 @@ typedef struct {
     uint64_t micro_ops[8];   /* ops inside multi-op sweeps, by kind: 1 complex 2x2, 2 one-qubit
                                 diagonal, 3 table diagonal, 4 CX, 5 SWAP, 6 real 2x2, 7 rotation */
 } zc_counters;
+/* Of the work launched so far; states under 14 qubits launch what waits first. */
 int zc_get_counters(zc_state *st, zc_counters *out);
 
 /* Sweep tile shape: at most `max_high` (1..7) qubits above the 256-byte row

@@ -261,7 +261,7 @@ static bool program_order(const zc_state *st) {
 //   whose exact sums take twice as long, keep their own way.
 static constexpr size_t kFewF32 = 4, kFewF64 = 8;
 static bool few_ops(const zc_state *st, size_t few) {
-    return st->n < kSmallStateQubits && !(st->flags & ZC_FLAG_FORCE_SWEEPS) && st->queue.size() < few;
+    return hides_queue(st) && st->queue.size() < few;
 }
 static bool few_one_by_one(const zc_state *st) { return st->prec == 32 && few_ops(st, kFewF32); }
 static bool few_in_exact(const zc_state *st) {
@@ -610,7 +610,7 @@ int flush(zc_state *st) {
 
 static int enqueue(zc_state *st, QOp &&op) {
     st->ctr.ops++;
-    if (!sweeps_enabled(st)) return launch_single(st, op);
+    if (!sweeps_enabled(st) || st->stream_out) return launch_single(st, op);
     st->queue.push(std::move(op));
     if (st->queue.size() >= kQueueFlushAt) return flush(st);
     return ZC_OK;
@@ -1106,6 +1106,11 @@ int zc_finish(zc_state *st) {
 
 int zc_get_stream(zc_state *st, void **stream) {
     if (!st || !stream) return fail(ZC_ERR_INVALID, "null argument");
+    if (hides_queue(st)) {  // what the caller puts on the stream comes behind the ops applied so far
+        const int rc = flush(st);
+        if (rc) return rc;
+        st->stream_out = true;
+    }
     *stream = (void *)st->stream;
     return ZC_OK;
 }
@@ -1159,6 +1164,10 @@ int zc_set_sweep_shape(zc_state *st, uint32_t max_high) {
 
 int zc_get_counters(zc_state *st, zc_counters *out) {
     if (!st || !out) return fail(ZC_ERR_INVALID, "null argument");
+    if (hides_queue(st)) {
+        const int rc = flush(st);
+        if (rc) return rc;
+    }
     *out = st->ctr;
     return ZC_OK;
 }

@@ -124,6 +124,7 @@ struct zc_state {
     void *d_samp = nullptr;      // sampler work area
     size_t samp_cap = 0;
     int *d_err = nullptr;        // device error record, inside the status block
+    bool stream_out = false;     // a small state's caller has its stream: ops are launched as they come
     bool exact_flush = false;    // inside a flush: a few fast f64 ops run in exact arithmetic
     bool df_resident = false;    // inside a flush: fast f64 sweeps left packed float pairs in re / im
     zc::OpQueue queue;           // ops waiting to be scheduled into sweeps
@@ -135,6 +136,13 @@ struct zc_state {
 };
 
 namespace zc {
+
+// A small state's ops look launched once their call has returned, unless its
+// creator asked for sweeps: whatever shows a caller the difference (the stream,
+// the counters, sampling without allocation) launches what is queued first.
+inline bool hides_queue(const zc_state *st) {
+    return st->n < kSmallStateQubits && !(st->flags & ZC_FLAG_FORCE_SWEEPS);
+}
 
 // Kernel launchers (zc_gates.cu / zc_reduce.cu). All are asynchronous on
 // st->stream and return ZC_OK or an error code.
