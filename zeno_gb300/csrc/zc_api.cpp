@@ -8,6 +8,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -608,9 +609,34 @@ int flush(zc_state *st) {
     return rc ? rc : rc2;
 }
 
+// The kernels a queued op of a small state may launch, loaded as it is applied:
+// its launch may come inside a call that allocates nothing. Once per device,
+// arithmetic and kind of op (2 MB of device memory for the double-float sweeps,
+// the other kinds none that shows).
+static int load_for(const zc_state *st, const QOp &op) {
+    static std::atomic<uint64_t> loaded[64];
+    const bool ex = exact(st), tc = op.kind == Q_UNITARY && op.k >= 3 && st->prec == 32 && (st->flags & ZC_FLAG_TENSOR);
+    const uint32_t k = sweepable(op) ? 1 : op.k;
+    const uint64_t bit = 1ull << ((st->prec == 64) * 32 + ex * 16 + tc * 8 + k);
+    std::atomic<uint64_t> &mask = loaded[st->device & 63];
+    if (mask.load(std::memory_order_relaxed) & bit) return ZC_OK;
+    int rc = tc ? load_tc_kernels(k) : load_op_kernels(st->prec, ex, k);
+    if (rc == ZC_OK && k == 1) rc = load_sweep_kernels(st->prec, ex);
+    if (rc == ZC_OK && k == 1 && st->prec == 64 && !ex) {  // few_in_exact
+        rc = load_op_kernels(64, true, 1);
+        if (rc == ZC_OK) rc = load_sweep_kernels(64, true);
+    }
+    if (rc == ZC_OK) mask.fetch_or(bit, std::memory_order_relaxed);
+    return rc;
+}
+
 static int enqueue(zc_state *st, QOp &&op) {
     st->ctr.ops++;
     if (!sweeps_enabled(st) || st->stream_out) return launch_single(st, op);
+    if (hides_queue(st)) {
+        const int rc = load_for(st, op);
+        if (rc) return rc;
+    }
     st->queue.push(std::move(op));
     if (st->queue.size() >= kQueueFlushAt) return flush(st);
     return ZC_OK;

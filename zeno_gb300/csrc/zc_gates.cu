@@ -658,6 +658,50 @@ __global__ void k_set_one(T *re) {
 
 }  // namespace
 
+// (States too short for vectors queue nothing: their scalar kernels are left out.)
+template <typename T, int A, bool EXACT>
+static int load_ops(uint32_t k) {
+    constexpr int V = Vec<T>::N;
+    if (k == 1) {
+        ZC_LOAD(k_1q_rows<T, A>);
+        ZC_LOAD(k_1q_inreg<T, A>);
+        ZC_LOAD(k_diag1<T, A>);
+        ZC_LOAD(k_diagk<T, A>);
+        ZC_LOAD(k_pair_swap<T, V>);
+        ZC_LOAD(k_pair_swap<T, 1>);
+    } else if constexpr (A == AR_DF) {
+        if (k == 2) {
+            ZC_LOAD(k_kq_reg_df<2, false, false>);
+            ZC_LOAD(k_kq_reg_df<2, false, true>);
+            ZC_LOAD(k_kq_reg_df<2, true, false>);
+            ZC_LOAD(k_kq_reg_df<2, true, true>);
+        } else if (k == 3) {
+            ZC_LOAD(k_kq_reg_df<3, false, false>);
+            ZC_LOAD(k_kq_reg_df<3, false, true>);
+            ZC_LOAD(k_kq_reg_df<3, true, false>);
+            ZC_LOAD(k_kq_reg_df<3, true, true>);
+        } else if (k == 4) {
+            ZC_LOAD(k_kq_reg_df<4, false, false>);
+            ZC_LOAD(k_kq_reg_df<4, false, true>);
+            ZC_LOAD(k_kq_reg_df<4, true, false>);
+            ZC_LOAD(k_kq_reg_df<4, true, true>);
+        } else {
+            ZC_LOAD(k_kq_df);
+        }
+    } else {
+        if (k == 2) ZC_LOAD(k_kq_reg<T, EXACT, 2>);
+        else if (k == 3) ZC_LOAD(k_kq_reg<T, EXACT, 3>);
+        else if (k == 4) ZC_LOAD(k_kq_reg<T, EXACT, 4>);
+        else ZC_LOAD(k_kq<T, EXACT>);
+    }
+    return ZC_OK;
+}
+
+int load_op_kernels(int prec, bool exact, uint32_t k) {
+    if (prec == 64) return exact ? load_ops<double, AR_EXACT, true>(k) : load_ops<double, AR_DF, false>(k);
+    return exact ? load_ops<float, AR_EXACT, true>(k) : load_ops<float, AR_FMA, false>(k);
+}
+
 int launch_1q(zc_state *st, uint32_t q, const double *m8, bool exact) {
     ProfScope ps(st, K_1Q, 2.0 * st->len * (st->prec / 8) * 2);
     st->ctr.launches++;

@@ -15,6 +15,13 @@ namespace zc {
 int fail(int code, const std::string &msg);
 int cuda_fail(cudaError_t e, const char *where);
 
+// Load a kernel now.
+#define ZC_LOAD(...)                                       \
+    do {                                                   \
+        cudaFuncAttributes fa_;                            \
+        ZC_CUDA(cudaFuncGetAttributes(&fa_, __VA_ARGS__)); \
+    } while (0)
+
 #define ZC_CUDA(call)                                   \
     do {                                                \
         cudaError_t e_ = (call);                        \
@@ -166,6 +173,12 @@ int sync_status(zc_state *st);
 int plan_state(uint32_t n, int prec, uint64_t budget);
 int create_state(uint32_t n, int prec, uint32_t flags, uint64_t budget, zc_state **out);
 
+// Load the kernels that ops of one kind may launch (k: qubits of a dense block;
+// 1: every op that sweeps take), without launching any. CUDA loads a kernel on
+// its first launch otherwise, which can allocate device memory.
+int load_op_kernels(int prec, bool exact, uint32_t k);
+int load_sweep_kernels(int prec, bool exact);
+int load_tc_kernels(uint32_t k);
 int launch_1q(zc_state *st, uint32_t q, const double *m8, bool exact);
 // Dense blocks of 2 to kMaxRegUnitary qubits, a group per thread; mat: row-major
 // interleaved complex. in_df / out_df (fast f64): packed pairs in the slots.

@@ -213,9 +213,10 @@ extern "C" int zc_sample_noalloc(zc_state *st, uint64_t shots, uint64_t seed, ui
     if (!st) return fail(ZC_ERR_INVALID, "null state");
     if (shots == 0) return ZC_OK;
     if (!out) return fail(ZC_ERR_INVALID, "sample_noalloc: null output");
-    // states below 14 qubits never needed a zc_finish before this call; their
-    // few queued ops are launched here (from the parameter ring: no allocation)
-    if (!st->queue.empty() && st->n < 14) {
+    // small states need no zc_finish before this call: what waits is launched
+    // here, from the parameter ring and with kernels loaded when the ops were
+    // applied, so nothing is allocated
+    if (hides_queue(st)) {
         const int rc = flush(st);
         if (rc) return rc;
     }

@@ -979,6 +979,22 @@ __global__ void __launch_bounds__(256) k_df_to_f64(double *__restrict__ re, doub
 
 }  // namespace
 
+int load_sweep_kernels(int prec, bool exact) {
+    if (prec == 32) {
+        if (exact) ZC_LOAD(k_sweep<float, AR_EXACT, 0>);
+        else ZC_LOAD(k_sweep<float, AR_FMA, 0>);
+    } else if (exact) {
+        ZC_LOAD(k_sweep<double, AR_EXACT, 0>);
+    } else {
+        ZC_LOAD(k_sweep<double, AR_DF, 0>);
+        ZC_LOAD(k_sweep<double, AR_DF, kFormInDf>);
+        ZC_LOAD(k_sweep<double, AR_DF, kFormOutDf>);
+        ZC_LOAD(k_sweep<double, AR_DF, kFormInDf | kFormOutDf>);
+        ZC_LOAD(k_df_to_f64);
+    }
+    return ZC_OK;
+}
+
 int launch_df_to_f64(zc_state *st) {
     ProfScope ps(st, K_SWEEP, 2.0 * st->len * 8 * 2);
     st->ctr.launches++;

@@ -485,6 +485,15 @@ static double real_form(const double *mat, size_t D, size_t r, size_t kk) {
     return (r < D) == (kk < D) ? mr : (r < D ? -mi : mi);
 }
 
+int load_tc_kernels(uint32_t k) {
+    if (k == 3) ZC_LOAD(k_block_tc<16>);
+    else if (k == 4) ZC_LOAD(k_block_umma<32>);
+    else if (k == 5) ZC_LOAD(k_block_umma<64>);
+    else if (k == 6) ZC_LOAD(k_block_umma<128>);
+    else ZC_LOAD(k_block_umma<256>);
+    return ZC_OK;
+}
+
 int launch_block_tc(zc_state *st, const uint32_t *qs, uint32_t k, const double *mat) {
     st->ctr.launches++;
     st->ctr.sweeps++;
