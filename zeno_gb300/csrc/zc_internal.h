@@ -34,9 +34,8 @@ constexpr int kSampleChunkLog2 = 16;  // sample.rs CHUNK = 1 << 16
 // States below this size are small: a few ops on one take as long as their
 // launches, and f32 ones keep program order in fast mode too (program_order).
 constexpr uint32_t kSmallStateQubits = 14;
-constexpr int kErrWords = 16;         // device error record (d_err) in ints
-// A state's status block (d_scalar): the scalar result, the device error
-// record and a ticket for one-launch sums; one copy reads result and record.
+// A state's status block (d_scalar): the scalar result, the device error code
+// (d_err) and a ticket for one-launch sums; one copy reads result and code.
 constexpr size_t kStatusErr = 64, kStatusTicket = 128, kStatusBytes = 256;
 
 // Device parameter arena: tables (matrices, diagonals) for queued ops are
@@ -130,7 +129,7 @@ struct zc_state {
     double *h_scalar = nullptr;  // pinned copy of it
     void *d_samp = nullptr;      // sampler work area
     size_t samp_cap = 0;
-    int *d_err = nullptr;        // device error record, inside the status block
+    int *d_err = nullptr;        // device error code, inside the status block
     bool stream_out = false;     // a small state's caller has its stream: ops are launched as they come
     bool exact_flush = false;    // inside a flush: a few fast f64 ops run in exact arithmetic
     bool df_resident = false;    // inside a flush: fast f64 sweeps left packed float pairs in re / im
@@ -161,9 +160,8 @@ struct ProfScope {
     ~ProfScope();
 };
 
-// Reads the state's device error record after a sync (a kernel that gave
-// up on a bounded wait or found an index out of range): ZC_ERR_CUDA with
-// the record's text, and the record cleared; else ZC_OK.
+// Reads the state's device error code after a sync (nonzero: a kernel gave up
+// on a bounded wait): ZC_ERR_CUDA, and the code cleared; else ZC_OK.
 int check_device_error(zc_state *st);
 // The same where the stream is not yet synchronised: reads the status block
 // with one copy and one synchronisation (h_scalar[0] is the scalar result).

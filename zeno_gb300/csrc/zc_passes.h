@@ -29,6 +29,28 @@ static_assert(sizeof(OpHead) == 72 && offsetof(MicroOp, table) == offsetof(OpHea
                   offsetof(MicroOp, m) == sizeof(OpHead),
               "OpHead is the head of MicroOp");
 
+// Whether the kernel can run an op on a tile of 2^tile_log2 slots of an n-qubit
+// state: every operand a tile bit or, where that is allowed, an outer qubit.
+// The kernel indexes shared memory with them unchecked.
+inline bool operands_ok(const OpHead &op, uint32_t tile_log2, uint32_t n) {
+    auto local = [&](uint32_t x) { return x < tile_log2; };
+    auto any = [&](uint32_t x) { return (x & kOuterFlag) ? (x & ~kOuterFlag) < n : local(x); };
+    switch (op.kind) {
+        case MOP_U1:
+        case MOP_R1:
+        case MOP_RT: return local(op.a);
+        case MOP_D1: return any(op.a);
+        case MOP_DK:
+            if (op.k < 1 || op.k > 12) return false;
+            for (uint32_t b = 0; b < op.k; b++)
+                if (!any(op.loc[b])) return false;
+            return true;
+        case MOP_CX: return any(op.a) && local(op.b) && op.a != op.b;
+        case MOP_SWAP: return local(op.a) && local(op.b) && op.a != op.b;
+    }
+    return false;
+}
+
 inline int popcount32(uint32_t v) {
     int n = 0;
     for (; v; v &= v - 1) n++;
@@ -147,7 +169,7 @@ inline void plan_passes(const OpHead *ops, int nops, uint32_t tile_log2, bool fo
             bits[g] = ops[first + g].a;
             in_tile &= bits[g] < tile_log2;
         }
-        if (!in_tile) {  // cannot happen for a planned sweep: recorded, ops run one by one
+        if (!in_tile) {  // not a planned sweep: encode_job refuses the job
             *bad = 0x80000000u | (uint32_t)o;
             o++;
             continue;
@@ -267,7 +289,7 @@ inline void plan_reg_passes(const OpHead *ops, int nops, uint32_t tile_log2, Reg
             uint32_t add = 0;
             if (op.kind == MOP_U1 || op.kind == MOP_CX) {
                 const uint32_t bit = op.kind == MOP_U1 ? op.a : op.b;
-                if (bit >= tile_log2) break;  // not a planned op: the plain loop reports it
+                if (bit >= tile_log2) break;  // (encode_job refuses such an op)
                 add = 1u << bit;
             } else if (op.kind != MOP_D1 && op.kind != MOP_DK) {
                 break;

@@ -638,6 +638,8 @@ static_assert(sizeof(OpHead[kMaxMicroOps]) % 16 == 0 && sizeof(GroupInfo[kMaxMic
 template <typename T, int A>
 int encode_job_as(const SweepPlan &plan, std::vector<char> *out) {
     const int nops = (int)plan.mops.size();
+    if (((size_t)2 << (plan.g.L + plan.g.H)) * sizeof(T) > kSweepSmemBytes)
+        return fail(ZC_ERR_INVALID, "sweep shape exceeds the kernel's limits");
     JobHead h{};
     h.nops = (uint32_t)nops;
     h.L = plan.g.L;
@@ -650,8 +652,11 @@ int encode_job_as(const SweepPlan &plan, std::vector<char> *out) {
         memcpy(&ops[(size_t)o], &m, sizeof(OpHead));
         h.has_arith |= m.kind != MOP_CX && m.kind != MOP_SWAP;
         const int cnt = m.kind == MOP_U1 ? 8 : m.kind == MOP_RT ? 1 : m.kind == MOP_D1 || m.kind == MOP_R1 ? 4 : 0;
-        if ((is_1q(m.kind) && m.a >= h.L + h.H) || (m.kind == MOP_CX && m.b >= h.L + h.H))
-            return fail(ZC_ERR_INVALID, "sweep plan: a gate bit lies outside the tile");
+        if (!operands_ok(ops[(size_t)o], h.L + h.H, plan.g.n))
+            return fail(ZC_ERR_INVALID, "sweep plan: an operand lies outside the tile and the state");
+        constexpr size_t entry = A == AR_DF ? 16 : 2 * sizeof(T);
+        if (m.kind == MOP_DK && (m.table % 16 || m.table + (entry << m.k) > plan.tables.size()))
+            return fail(ZC_ERR_INVALID, "sweep plan: a diagonal lies outside the tables");
         OpCoef<T, A> &c = coef[(size_t)o];
         for (int i = 0; i < cnt; i++) {
             if constexpr (A == AR_DF) {
@@ -924,8 +929,6 @@ int run_sweep_form(zc_state *st, const SweepGeom &g, const char *dev_job, const 
                                      (int)kSweepSmemBytes));
         attr = true;
     }
-    if (((size_t)2 << (g.L + g.H)) * sizeof(T) > kSweepSmemBytes || g.H > kMaxSweepHigh)
-        return fail(ZC_ERR_INVALID, "sweep shape exceeds the kernel's limits");
     const uint64_t blocks = std::min<uint64_t>(g.ntiles, (uint64_t)st->num_sms * kSweepCtasPerSm);
     k_sweep<T, A, FORM><<<(int)blocks, kSweepThreads, kSweepSmemBytes, st->stream>>>(
         (T *)st->re, (T *)st->im, g.ntiles, dev_job, dev_tables);
