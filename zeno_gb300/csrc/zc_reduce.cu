@@ -519,19 +519,19 @@ int run_chain(zc_state *st, uint64_t total, uint64_t chunk, uint64_t nrows, int 
 // Split re / im arrays -> interleaved f64 (re, im) pairs, four amplitudes per
 // thread (16-byte loads, 64 bytes of stores).
 template <typename T>
-
 __global__ void __launch_bounds__(256) k_interleave(const T *__restrict__ re, const T *__restrict__ im,
                                                     double2 *__restrict__ out, uint64_t len) {
     const uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) * 4;
     if (i + 4 <= len) {
-        T r[4], m[4];
         using VT = typename Vec<T>::type;
         constexpr int V = Vec<T>::N;
+        VT vr[4 / V], vm[4 / V];
 #pragma unroll
-        for (int k = 0; k < 4; k += V) {
-            *reinterpret_cast<VT *>(r + k) = *reinterpret_cast<const VT *>(re + i + k);
-            *reinterpret_cast<VT *>(m + k) = *reinterpret_cast<const VT *>(im + i + k);
+        for (int k = 0; k < 4 / V; k++) {
+            vr[k] = reinterpret_cast<const VT *>(re + i)[k];
+            vm[k] = reinterpret_cast<const VT *>(im + i)[k];
         }
+        const T *r = reinterpret_cast<const T *>(vr), *m = reinterpret_cast<const T *>(vm);
 #pragma unroll
         for (int k = 0; k < 4; k++) out[i + k] = make_double2(widen(r[k]), widen(m[k]));
     } else {
