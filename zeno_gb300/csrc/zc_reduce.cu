@@ -577,15 +577,26 @@ void run_sample_scan_df(zc_state *st, size_t nch, const SampleChunk *cs, const d
         k_sample_scan_df<T, kDfThreads><<<(unsigned)nch, kDfThreads, 0, st->stream>>>(re, im, cs, us, out, chunk_len, st->len);
 }
 
+// The partial sums' buffer, at least `count` long. Its capacity is zero while
+// there is none: one left over from before a failed allocation would send the
+// next, smaller sum to a null pointer.
+static int grow_part(zc_state *st, size_t count) {
+    if (count <= st->part_cap) return ZC_OK;
+    if (st->d_part) cudaFree(st->d_part);
+    st->d_part = nullptr;
+    st->part_cap = 0;
+    ZC_CUDA(cudaMalloc(&st->d_part, count * sizeof(double)));
+    st->part_cap = count;
+    return ZC_OK;
+}
+
 int launch_chunk_sums(zc_state *st, int mode, uint32_t q, size_t *nchunks_out, bool exact, double *out) {
     const uint64_t total = mode == 0 ? st->len : st->len / 2;
     const uint64_t chunk = total < (1ull << kSampleChunkLog2) ? total : (1ull << kSampleChunkLog2);
     const uint64_t nch = (total + chunk - 1) / chunk;
-    if (!out && nch > st->part_cap) {
-        if (st->d_part) cudaFree(st->d_part);
-        st->d_part = nullptr;
-        ZC_CUDA(cudaMalloc(&st->d_part, nch * sizeof(double)));
-        st->part_cap = nch;
+    if (!out) {
+        const int rc = grow_part(st, nch);
+        if (rc) return rc;
     }
     double *part = out ? out : st->d_part;
     ProfScope ps(st, K_CHUNK_SUMS, (mode == 0 ? 1.0 : 0.5) * st->len * (st->prec / 8) * 2);
@@ -614,13 +625,8 @@ int run_total(zc_state *st, bool ones, uint32_t q) {
         const uint64_t units = (ones && (1ull << q) >= V ? st->len / 2 : st->len) / V;
         const uint64_t want = (units + kDfThreads - 1) / kDfThreads, cap = (uint64_t)st->num_sms * 8;
         const unsigned blocks = (unsigned)std::min(want, cap);
-        if (blocks > st->part_cap) {
-            if (st->d_part) cudaFree(st->d_part);
-            st->d_part = nullptr;
-            st->part_cap = 0;
-            ZC_CUDA(cudaMalloc(&st->d_part, cap * sizeof(double)));
-            st->part_cap = cap;
-        }
+        const int rc = blocks > st->part_cap ? grow_part(st, cap) : ZC_OK;
+        if (rc) return rc;
         if (ones) k_total_df<T, true><<<blocks, kDfThreads, 0, st->stream>>>(re, im, units, q, st->d_part, ticket, st->d_scalar);
         else k_total_df<T, false><<<blocks, kDfThreads, 0, st->stream>>>(re, im, units, q, st->d_part, ticket, st->d_scalar);
     }
