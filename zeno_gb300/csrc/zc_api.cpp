@@ -161,7 +161,8 @@ int launch_single(zc_state *st, const QOp &op) {
             if (op.k == 1) return launch_1q(st, op.qs[0], op.data.data(), ex);
             if (op.k >= 3 && st->prec == 32 && (st->flags & ZC_FLAG_TENSOR))
                 return launch_block_tc(st, op.qs, op.k, op.data.data());
-            if (op.k <= kMaxRegUnitary) return launch_kq_small(st, op.qs, op.k, op.data.data(), ex);
+            if (op.k <= kMaxRegUnitary && !(op.k == 4 && ex && st->prec == 64 && st->n < kStagedK4Qubits))
+                return launch_kq_small(st, op.qs, op.k, op.data.data(), ex);
             const void *dev = nullptr;
             if (st->prec == 64 && !ex) {  // fast f64: double-float on the FP32 pipe
                 const size_t cnt = (size_t)1 << (2 * op.k);

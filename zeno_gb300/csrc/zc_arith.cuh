@@ -184,9 +184,12 @@ __device__ __forceinline__ void cscale(T wr, T wi, T &ar, T &ai) {
 
 // One term of the fused k-qubit matvec (kern_kq_scalar, src/state.rs:382-383):
 // ar = (ar + wr*xr) - wi*xi ; ai = (ai + wr*xi) + wi*xr.
-template <typename T, bool EXACT>
+// SOFT: exact f64 products on the integer pipe, for callers with enough of them
+// in flight. (k_kq's rows, one product after another from shared memory, took
+// longer with it: 7 qubits on 12 623 -> 681 us, on 24 33.3 -> 33.6 ms.)
+template <typename T, bool EXACT, bool SOFT = false>
 __device__ __forceinline__ void cmac(T wr, T wi, T xr, T xi, T &ar, T &ai) {
-    if constexpr (EXACT && sizeof(T) == 8) {
+    if constexpr (EXACT && SOFT && sizeof(T) == 8) {
         double p0, p1, p2, p3;
         if (soft_pair_ok(xr, xi, wr, wi)) {  // products on the integer pipe
             const SoftOp sr = soft_left(f64_bits(xr)), si = soft_left(f64_bits(xi));

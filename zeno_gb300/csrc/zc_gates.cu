@@ -121,8 +121,8 @@ struct KqParams {
 
 constexpr int kKqTile = 2048;  // amplitudes staged per CTA iteration
 
-// Fused k-qubit unitary of five to seven qubits (kern_kq_scalar,
-// src/state.rs:355-392): a CTA stages G = 2048 / 2^k groups in shared memory (gather), each thread
+// Fused k-qubit unitary of five to seven qubits, and of four on exact f64 states
+// under kStagedK4Qubits (kern_kq_scalar, src/state.rs:355-392): a CTA stages G = 2048 / 2^k groups in shared memory (gather), each thread
 // forms output rows with the column sum in ascending order, then scatters.
 template <typename T, bool EXACT>
 __global__ void __launch_bounds__(kThreads) k_kq(T *__restrict__ re, T *__restrict__ im, KqParams p,
@@ -208,7 +208,9 @@ int run_kq(zc_state *st, const uint32_t *qs, uint32_t k, const void *dev_mat) {
 // registers, each output row is summed and stored at once, and the matrix
 // comes as a kernel parameter (constant bank: uniform loads, no shared memory,
 // no barriers). Staging groups in shared memory (k_kq below five qubits
-// before) spent more on the staging than on the sums.
+// before) spent more on the staging than on the sums: 24 qubits, exact f64, k =
+// 2, 3, 4: 1.16, 2.20, 4.26 ms staged, 0.90, 1.90, 4.08 here; fast f32 0.23,
+// 0.27, 0.32 and 0.05, 0.05, 0.08.
 // The sums are k_kq's, column by column, so results are the same bits.
 template <typename T, int K>
 struct KqMat {
@@ -245,7 +247,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_kq_reg(T *__restrict__ re, T *_
         for (int r = 0; r < D; r++) {  // (unrolled, the compiler takes minutes over it)
             T ar = T(0), ai = T(0);
 #pragma unroll
-            for (int c = 0; c < D; c++) cmac<T, EXACT>(m.re[r * D + c], m.im[r * D + c], xr[c], xi[c], ar, ai);
+            for (int c = 0; c < D; c++) cmac<T, EXACT, true>(m.re[r * D + c], m.im[r * D + c], xr[c], xi[c], ar, ai);
             const uint64_t i = base | kq_offset<K>(qs, r);
             re[i] = ar;
             im[i] = ai;
@@ -283,8 +285,10 @@ int run_kq_small(zc_state *st, const uint32_t *qs, uint32_t k, const double *mat
 // every eight terms; the row is (A.re - B.im, A.im + B.re).
 // in_df / out_df: the slots hold packed pairs on entry / exit, as sweeps hand
 // them over, instead of f64 (a conversion costs as much as two entries).
-// Measured at 22 qubits, K = 3: 132 us per block staged through shared memory,
-// 54 here.
+// Measured at 30 qubits, K = 2, 3, 4: 22.2, 31.9, 49.4 ms per block staged
+// through shared memory, 7.2, 12.9, 50.3 here. K = 4 gains nothing by itself (each
+// thread reads its 8 KB of matrix through the constant cache); it stays for the
+// pairs it hands on: staged, the state is truncated to pairs for each block.
 template <int K>
 struct KqMatDf {
     float2 rh[1 << (2 * K)], rl[1 << (2 * K)], ih[1 << (2 * K)], il[1 << (2 * K)];  // each value twice
@@ -692,7 +696,7 @@ static int load_ops(uint32_t k) {
         if (k == 2) ZC_LOAD(k_kq_reg<T, EXACT, 2>);
         else if (k == 3) ZC_LOAD(k_kq_reg<T, EXACT, 3>);
         else if (k == 4) ZC_LOAD(k_kq_reg<T, EXACT, 4>);
-        else ZC_LOAD(k_kq<T, EXACT>);
+        if (k >= 4) ZC_LOAD(k_kq<T, EXACT>);
     }
     return ZC_OK;
 }

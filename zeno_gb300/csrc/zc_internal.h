@@ -181,6 +181,11 @@ int launch_1q(zc_state *st, uint32_t q, const double *m8, bool exact);
 // Dense blocks of 2 to kMaxRegUnitary qubits, a group per thread; mat: row-major
 // interleaved complex. in_df / out_df (fast f64): packed pairs in the slots.
 constexpr uint32_t kMaxRegUnitary = 4;
+// Exact f64 blocks of four qubits on states below this size run staged: a
+// thread's 256 complex products in a row leave the chip idle (12, 18, 20, 21
+// qubits 161, 164, 306, 599 us in registers, 97, 98, 320, 549 staged; 22 and 24
+// qubits 1.06 and 4.08 ms in registers, 1.11 and 4.26 staged).
+constexpr uint32_t kStagedK4Qubits = 22;
 int launch_kq_small(zc_state *st, const uint32_t *qs, uint32_t k, const double *mat, bool exact, bool in_df = false,
                     bool out_df = false);
 int launch_kq(zc_state *st, const uint32_t *qs, uint32_t k, const void *dev_mat, bool exact);
