@@ -18,7 +18,10 @@ typedef __float128 Q;
 
 struct Sum {
     float h = 0.f, l = 0.f;
-    void add(float x, float y) { zc::mass_add2<Ops>(x, y, h, l); }
+    void add(float x, float y, bool pair = false) {
+        if (pair) zc::mass_add_pair<Ops>(x, y, h, l);
+        else zc::mass_add2<Ops>(x, y, h, l);
+    }
     void fold() { zc::mass_fold<Ops>(h, l); }
     void join(const Sum &o) { zc::mass_join<Ops>(h, l, o.h, o.l); }
     double value() const { return (double)h + (double)l; }
@@ -39,7 +42,7 @@ static double row_by_lanes(const std::vector<float> &re, const std::vector<float
         for (size_t p = 0; p < 2; p++)
             for (size_t lane = 0; lane < 2; lane++) {
                 Sum &s = sums[(u % NT) * 4 + (p % S) * 2 + lane];
-                s.add(re[4 * u + 2 * p + lane], im[4 * u + 2 * p + lane]);
+                s.add(re[4 * u + 2 * p + lane], im[4 * u + 2 * p + lane], NT >= 256);
                 if (p + 1 >= 2 / S && (u / NT) % (zc::kMassFold / 4) == zc::kMassFold / 4 - 1) s.fold();
             }
     // a thread's sums, then the lanes of a warp: from eight warps on joined as
@@ -81,34 +84,37 @@ int main() {
     std::normal_distribution<float> gauss;
     // one lane: relative error within the roundings of its additions. A
     // square and a residual are exact; of a pair of squares the two sums of
-    // residuals and their sum are rounded (at most 2^-48 of the total each),
-    // l is (at most kMassFold + 1/2 ulps, 2^-24 of the total each, before),
-    // a fold is exact.
+    // residuals and their sum are rounded (at most 2^-48 of the total each; of
+    // a joined pair the FMA's error, its sum with the other and theirs), l is
+    // (at most kMassFold + 1/2 ulps, 2^-24 of the total each, before), a fold is
+    // exact.
     double worst = 0.0;
     for (int kind = 0; kind < 5; kind++)
         for (int lg = 1; lg <= 18; lg++)
-            for (int t = 0; t < (lg <= 12 ? 64 : 4); t++) {
-                const size_t n = (size_t)1 << lg;
-                Sum s;
-                Q exact = 0;
-                float pair[2] = {0.f, 0.f};
-                for (size_t i = 0; i < n; i++) {
-                    float x = gauss(g) / std::sqrt((float)n);
-                    if (kind == 1 && i) x *= 1e-4f;                               // one large amplitude, first
-                    if (kind == 2) x = std::ldexp(x, -(int)(g() % 20));           // a wide range
-                    if (kind == 3) x *= 1e-9f;                                    // a branch of small mass
-                    if (kind == 4 && i + 1 < n) x = g() % 8 ? 0.f : x * 1e-3f;    // sparse, the largest last
-                    pair[i % 2] = x;
-                    exact += (Q)x * x;
-                    if (i % 2) s.add(pair[0], pair[1]);
-                    if (i % zc::kMassFold == zc::kMassFold - 1) s.fold();
+            for (int pair = 0; pair < 2; pair++)
+                for (int t = 0; t < (lg <= 12 ? 64 : 4); t++) {
+                    const size_t n = (size_t)1 << lg;
+                    Sum s;
+                    Q exact = 0;
+                    float two[2] = {0.f, 0.f};
+                    for (size_t i = 0; i < n; i++) {
+                        float x = gauss(g) / std::sqrt((float)n);
+                        if (kind == 1 && i) x *= 1e-4f;                               // one large amplitude, first
+                        if (kind == 2) x = std::ldexp(x, -(int)(g() % 20));           // a wide range
+                        if (kind == 3) x *= 1e-9f;                                    // a branch of small mass
+                        if (kind == 4 && i + 1 < n) x = g() % 8 ? 0.f : x * 1e-3f;    // sparse, the largest last
+                        two[i % 2] = x;
+                        exact += (Q)x * x;
+                        if (i % 2) s.add(two[0], two[1], pair);
+                        if (i % zc::kMassFold == zc::kMassFold - 1) s.fold();
+                    }
+                    s.fold();
+                    const double e = std::fabs((double)(((Q)s.h + (Q)s.l - exact) / exact));
+                    const double bound = (double)(n / 2) * std::ldexp(3.0 + zc::kMassFold + 0.5, -48);
+                    if (!(e <= bound))
+                        return std::printf("FAIL kind %d 2^%d: error %.3e, bound %.3e\n", kind, lg, e, bound), 1;
+                    worst = std::max(worst, e / bound);
                 }
-                s.fold();
-                const double e = std::fabs((double)(((Q)s.h + (Q)s.l - exact) / exact));
-                const double bound = (double)(n / 2) * std::ldexp(3.0 + zc::kMassFold + 0.5, -48);
-                if (!(e <= bound)) return std::printf("FAIL kind %d 2^%d: error %.3e, bound %.3e\n", kind, lg, e, bound), 1;
-                worst = std::max(worst, e / bound);
-            }
     // table entries: rms errors over T states, each known to 1 / sqrt(2 T)
     // of itself: three times that of their difference, and the result's own
     // last bit, are let pass

@@ -32,7 +32,7 @@
 // stands between two passes. Measured for 2048 trajectories of the 16-qubit
 // depth-20 circuit under damping: 402 ms with one scalar pass per op over
 // global memory (114 instructions per amplitude, four CTAs per SM, half the
-// traffic from DRAM), 118 ms now (17 us per op and SM; bound by the latency of
+// traffic from DRAM), 113 ms now (16 us per op and SM; bound by the latency of
 // the L2 half of the state, the sums of squares and the decisions between
 // passes; 106 with sums on top of a constant, which lost digits of small ones,
 // see zc_mass.h); 1500 shots of a 13-qubit dynamic circuit: 10.2 -> 2.2 ms.
@@ -285,6 +285,22 @@ struct MassF2 {
     static __device__ __forceinline__ P2 add(P2 a, P2 b) { return p2_add(a, b); }
     static __device__ __forceinline__ P2 sub(P2 a, P2 b) { return p2_sub(a, b); }
     static __device__ __forceinline__ P2 neg(P2 a) { return a ^ 0x8000000080000000ull; }
+    static __device__ __forceinline__ void by_size(P2 x, P2 y, P2 &a, P2 &b) {
+        const float2 u = pk_float2(x), v = pk_float2(y);
+        a = p2_make(larger(u.x, v.x), larger(u.y, v.y));
+        b = p2_make(smaller(u.x, v.x), smaller(u.y, v.y));
+    }
+    // of two magnitudes, NaN if either is
+    static __device__ __forceinline__ float larger(float x, float y) {
+        float r;
+        asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(fabsf(x)), "f"(fabsf(y)));
+        return r;
+    }
+    static __device__ __forceinline__ float smaller(float x, float y) {
+        float r;
+        asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(fabsf(x)), "f"(fabsf(y)));
+        return r;
+    }
 };
 
 // A folded sum as f64 (by integer operations; below 2^-75 those drop l).
@@ -557,7 +573,8 @@ __device__ __forceinline__ void traj_pass_body(float *work, uint32_t n, int o, i
                     for (int p = 0; p < 2; p++)
 #pragma unroll
                         for (int r = 0; r < D; r++)
-                            mass_add2<MassF2>(xr[i][r][p], xi[i][r][p], h[p % S][r], l[p % S][r]);
+                            if (NT >= 256) mass_add_pair<MassF2>(xr[i][r][p], xi[i][r][p], h[p % S][r], l[p % S][r]);
+                            else mass_add2<MassF2>(xr[i][r][p], xi[i][r][p], h[p % S][r], l[p % S][r]);
                 }
                 if (!MONO) {
                     lanes<K, false>(xr[i], low);
