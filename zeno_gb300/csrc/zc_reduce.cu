@@ -29,6 +29,7 @@ constexpr int kChainThreads = 256;
 constexpr int kStageElems = 32;  // elements per row: one warp-wide load, one recorded chain value
 constexpr int kRowsPerWarp = 8;
 constexpr int kTileRows = kRowsPerWarp * kChainThreads / 32;  // 64 rows, two per lane in the scan
+constexpr uint64_t kShortChain = 128;  // elements up to which one warp adds a chain up one by one
 
 __device__ __forceinline__ ChainFn shfl_down_fn(const ChainFn &f, int o) {
     return ChainFn{__shfl_down_sync(0xffffffffu, f.a, o), __shfl_down_sync(0xffffffffu, f.b, o)};
@@ -65,7 +66,9 @@ __device__ __forceinline__ ChainFn row_fn(uint64_t vbits, uint32_t e) {
 // rounded as f64), 60 us per 2^16-element chunk on one SM, with about
 // twelve serial rows of 1 us per chunk beside them. One lane per chain, fed
 // by producer warps, took 2.9 ms per chunk at any state size (2^16 dependent
-// adds of 64 cycles).
+// adds of 64 cycles). A chain of up to kShortChain elements crosses a binade in
+// nearly every row: one warp adds it up one by one (a draw from an exact 5-qubit
+// state 78 -> 57 us; at 256 elements the rows are as fast).
 //
 // SCAN = false: chunk blockIdx.x of the index space (mode 0: index h; mode 1,
 //   prob_one of qubit q: insert_zero(h, q) + 2^q; mode 2: re holds the
@@ -98,6 +101,38 @@ __global__ void __launch_bounds__(kChainThreads, 2)
     const uint64_t first = c * chunk, len = total - first < chunk ? total - first : chunk;
     const uint64_t sbit = 1ull << q;
     const uint32_t nst = (uint32_t)((len + kStageElems - 1) / kStageElems);
+    if (len <= kShortChain) {
+        if (warp) return;
+        double a = __longlong_as_double((long long)acc);
+        auto value = [&](uint32_t r) {
+            const uint64_t e = (uint64_t)r * kStageElems + lane, h = first + e;
+            if (e >= len) return 0ull;
+            const uint64_t idx = mode == 1 ? insert_zero(h, q) + sbit : h;
+            return dkey(mode == 2 ? widen(re[idx]) : p2(widen(re[idx]), widen(im[idx])));
+        };
+        unsigned long long v = value(0);
+        for (uint32_t r = 0; r < nst; r++) {
+            const unsigned long long next = r + 1 < nst ? value(r + 1) : 0ull;
+            if (SCAN) {
+                if (lane == 0) rec[row * rec_stride + r] = a;
+                const uint32_t mass = __ballot_sync(0xffffffffu, v != 0ull);
+                if (mass) my_last = (unsigned long long)r * kStageElems + 32 - __clz(mass);
+            }
+#pragma unroll 8
+            for (int i = 0; i < 32; i++)
+                a = radd(a, __longlong_as_double((long long)__shfl_sync(0xffffffffu, v, i)));
+            v = next;
+        }
+        if (lane == 0) {
+            if (SCAN) {
+                rec_nst[row] = nst;
+                rec_last[row] = my_last;
+            } else {
+                part[row] = a;
+            }
+        }
+        return;
+    }
     uint32_t ran = nst;
     T nr[kRowsPerWarp], ni[kRowsPerWarp];  // the next tile's amplitudes, in flight while this one is summed
     auto fetch = [&](uint64_t t0) {
@@ -236,11 +271,15 @@ __global__ void __launch_bounds__(kResolveThreads) k_resolve(const T *__restrict
         const uint64_t e0 = (uint64_t)lo * kStageElems;
         const uint64_t e1 = e0 + kStageElems < len ? e0 + kStageElems : len;
         uint64_t res = ~0ull;
-        for (uint64_t e = e0; e < e1; e++) {
-            acc = radd(acc, p2(widen(re[first + e]), widen(im[first + e])));
-            if (uk < dkey(acc)) {
-                res = first + e;
-                break;
+        for (uint64_t e = e0; e < e1 && res == ~0ull; e += 4) {  // four loads in flight
+            double v[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                v[j] = e + j < e1 ? p2(widen(re[first + e + j]), widen(im[first + e + j])) : 0.0;
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                acc = radd(acc, v[j]);
+                if (res == ~0ull && uk < dkey(acc)) res = first + e + j;
             }
         }
         if (res == ~0ull) res = rec_last[b] ? first + rec_last[b] - 1 : first + len - 1;
