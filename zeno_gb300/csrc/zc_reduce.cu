@@ -597,7 +597,11 @@ int launch_interleave(zc_state *st, uint64_t first, uint64_t count, void *dst) {
 // of its peak); fewer are as fast as one chunk, which 1024 threads take through
 // sooner: 1024 draws at 19 qubits (8 chunks) within a run of 1.63 -> 1.48 ms,
 // 24 served requests 7.4 -> 6.9 ms; 25 qubits (512 chunks) unchanged.
-static bool wide_chunks(const zc_state *st, size_t nch) { return nch <= (size_t)st->num_sms * 2; }
+// (States of up to 4096 amplitudes are a few vectors per thread: 256 threads, 8
+// qubits 64 -> 57 us.)
+static bool wide_chunks(const zc_state *st, size_t nch) {
+    return nch <= (size_t)st->num_sms * 2 && st->len > 4096;
+}
 
 template <typename T>
 void run_chunk_sums_df(zc_state *st, uint64_t total, uint64_t chunk, size_t nch, double *part) {
