@@ -413,7 +413,17 @@ size_t plan_sweep(uint32_t n, int prec, bool ex, uint32_t L, uint32_t Hcap, cons
     if (df) {
         std::vector<const QOp *> seq;
         for (size_t t : order) seq.push_back(&q[taken[t]]);
-        lower_df(seq, 2, &low, &plan->carry);
+        // a sweep with no sweep to follow at once (the queue ends or a dense block
+        // is next) applies its pending diagonals itself, if they fit: carried,
+        // they would be a launch of their own
+        size_t next = head;
+        while (next - head < taken.size() && taken[next - head] == next) next++;
+        const bool last = next == q.size() || !sweepable(q[next]);
+        lower_df(seq, 2, &low, last ? nullptr : &plan->carry);
+        if (last && low.size() > (size_t)kMaxMicroOps) {
+            low.clear();
+            lower_df(seq, 2, &low, &plan->carry);
+        }
     } else {
         for (size_t t : order) {
             const QOp &op = q[taken[t]];
