@@ -953,8 +953,7 @@ int zc_run(const zc_program *p, const zc_run_options *opt, zc_run_result *res, u
         for (const Op &op : p->ops)
             if ((rc = apply_gate_op(st, op))) return done(rc);
         if ((rc = flush(st))) return done(rc);
-        if (sv)  // take the array's page faults while the device works
-            for (size_t b = 0; b < st->len * 2 * sizeof(double); b += 4096) reinterpret_cast<volatile char *>(sv)[b] = 0;
+        if (sv) touch_pages(sv, st->len * 2 * sizeof(double));  // while the device works
         if ((rc = zc_finish(st))) return done(rc);
         if (sv && (rc = zc_statevector(st, sv))) return done(rc);
         if (!p->finals.empty() && opt->shots > 0) {

@@ -166,6 +166,9 @@ int check_device_error(zc_state *st);
 // The same where the stream is not yet synchronised: reads the status block
 // with one copy and one synchronisation (h_scalar[0] is the scalar result).
 int sync_status(zc_state *st);
+// Fault in the pages of [p, p + bytes): one byte of each, inside the range, is
+// written.
+void touch_pages(void *p, size_t bytes);
 // mem::plan against `budget` bytes (ZC_ERR_MEMORY with zeno's text), and
 // zc_create_ex with that budget in place of 0.75 of the device memory.
 int plan_state(uint32_t n, int prec, uint64_t budget);
