@@ -60,9 +60,8 @@ inline int popcount32(uint32_t v) {
 ZC_HD bool is_1q(uint32_t kind) { return kind == MOP_U1 || kind == MOP_R1 || kind == MOP_RT; }
 
 // The register group starting at one-qubit op o: three rotations on distinct
-// bits when max_group is two (f64 states outside FMA mode), else up to
-// max_group one-qubit ops on distinct bits. Returns its size; *rot3 tells the
-// first kind.
+// bits (max_group two, the kernel's), else up to max_group one-qubit ops on
+// distinct bits. Returns its size; *rot3 tells the first kind.
 ZC_HD int group_at(const OpHead *ops, int o, int nops, int max_group, bool *rot3) {
     *rot3 = false;
     if (max_group == 2 && o + 2 < nops && ops[o].kind == MOP_RT && ops[o + 1].kind == MOP_RT &&
@@ -114,10 +113,11 @@ struct GroupInfo {
     uint32_t tab_off;
 };
 
-// Walk the ops the way apply_ops will and describe each pass
-// (max_group: the kernel's register group size). *fuse_in / *fuse_out: the
-// job starts / ends with a pass, which then also converts the tile between
-// f64 and double-float in registers.
+// Walk the ops the way apply_ops will and describe each pass. The kernel's jobs
+// have CX blocks folded (fold) and groups of two (max_group); the host check of
+// the pass logic also tries single gates and unfolded blocks. *fuse_in /
+// *fuse_out: the job starts / ends with a pass, which then also converts the
+// tile between f64 and double-float in registers.
 inline void plan_passes(const OpHead *ops, int nops, uint32_t tile_log2, bool fold, int max_group, GroupInfo *gi,
                         uint32_t *bad, int *fuse_in, int *fuse_out) {
     for (int i = 0; i < nops; i++) gi[i].G = 0;

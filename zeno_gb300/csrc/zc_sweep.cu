@@ -139,7 +139,7 @@ __device__ void apply_perm(T *sr, T *si, const OpHead &op, uint64_t base, uint32
     }
 }
 
-// Per-op coefficients converted once per CTA into the compute representation.
+// Per-op coefficients in the compute representation, as encode_job leaves them.
 // U1: the 2x2 matrix; D1: entries 0..3 = d0r d0i d1r d1i. Double-float
 // pairs for A == AR_DF, else values of T. Double-float RT: v[0] = t, and
 // v[2..6) its packed pairs (PkReal: t hi, t lo, -t hi, -t lo, each twice).
@@ -1003,7 +1003,7 @@ int launch_df_to_f64(zc_state *st) {
     st->ctr.launches++;
     st->ctr.sweeps++;
     st->ctr.bytes_moved += 2 * st->len * 8 * 2;
-    const uint64_t n2 = st->len / 2;  // two elements per thread step; len >= 2^14 for sweeps
+    const uint64_t n2 = st->len / 2;  // two elements per thread step (sweeps have at least 2^3)
     const uint64_t blocks = std::min<uint64_t>((n2 + 255) / 256, (uint64_t)st->num_sms * 8);
     k_df_to_f64<<<(int)blocks, 256, 0, st->stream>>>((double *)st->re, (double *)st->im, n2);
     ZC_CUDA(cudaGetLastError());

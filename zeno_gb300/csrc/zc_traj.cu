@@ -104,7 +104,7 @@ struct Shared {
     uint32_t fqv[3];              // high qubits of the factor table, in vector units
     int nfv;                      // -1: no factor differs from one
     uint32_t dq[3];               // all qubits of the diagonal factors, and the factors by their bits
-    float dr[8], di[8];
+    float dr[8];
     int nd;
     double red[NT / 32][8];       // per-warp tables
     double J[8];                  // joint probability table of a three-qubit op
@@ -213,11 +213,10 @@ __device__ __noinline__ void apply_nondiag_pending(float *work, uint32_t n) {
 
 // Per-element factor of the diagonal pending operators.
 template <int NT>
-__device__ __forceinline__ void diag_factor(const Shared<NT> &s, uint64_t idx, float &fr, float &fi) {
+__device__ __forceinline__ float diag_factor(const Shared<NT> &s, uint64_t idx) {
     uint32_t j = 0;
     for (int b = 0; b < s.nd; b++) j |= (uint32_t)((idx >> s.dq[b]) & 1) << b;
-    fr = s.dr[j];
-    fi = s.di[j];
+    return s.dr[j];
 }
 
 // Warp 0, every lane with the same arguments: the tables of the real diagonal
@@ -242,10 +241,7 @@ __device__ __forceinline__ void factor_tables(Shared<NT> &s, int nd, const uint3
             }
             if (lane == 0) s.dq[b] = q[b];
         }
-    if (lane < 8) {
-        s.dr[lane] = f;
-        s.di[lane] = 0.f;
-    }
+    if (lane < 8) s.dr[lane] = f;
     reinterpret_cast<float *>(s.ft)[lane] = fv;
     if (lane == 0) {
         s.nd = nd;
@@ -503,91 +499,81 @@ __device__ __forceinline__ void traj_pass_body(float *work, uint32_t n, int o, i
     };
     auto source = [&](int v) { return MONO ? col[v] : v; };
     const uint32_t units = 1u << (n - 2 - K);
-    constexpr int U = 1;
 #pragma unroll 1
-    for (uint32_t u0 = threadIdx.x; u0 < units; u0 += U * NT) {
-        P2 xr[U][D][2], xi[U][D][2];
+    for (uint32_t u = threadIdx.x; u < units; u += NT) {
+        P2 xr[D][2], xi[D][2];
 #pragma unroll
-        for (int i = 0; i < U; i++)
-            if (i == 0 || u0 + i * NT < units) {
+        for (int v = 0; v < D; v++) {
+            const uint32_t vi = vector(u, source(v));
+            const ulonglong2 a = *sm.re4(vi), c = *sm.im4(vi);
+            xr[v][0] = a.x;
+            xr[v][1] = a.y;
+            xi[v][0] = c.x;
+            xi[v][1] = c.y;
+        }
+        if (nfv >= 0) {  // factors are real: flips and damping have real operators
 #pragma unroll
-                for (int v = 0; v < D; v++) {
-                    const uint32_t vi = vector(u0 + i * NT, source(v));
-                    const ulonglong2 a = *sm.re4(vi), c = *sm.im4(vi);
-                    xr[i][v][0] = a.x;
-                    xr[i][v][1] = a.y;
-                    xi[i][v][0] = c.x;
-                    xi[i][v][1] = c.y;
+            for (int v = 0; v < D; v++) {
+                const uint32_t vi = vector(u, source(v));
+                uint32_t j = ((vi >> fq0) & 1u) | (((vi >> fq1) & 1u) << 1);
+                if (nfv > 2) j |= ((vi >> fq2) & 1u) << 2;
+                const ulonglong2 f = *reinterpret_cast<const ulonglong2 *>(&s.ft[j]);
+                xr[v][0] = p2_mul(f.x, xr[v][0]);
+                xr[v][1] = p2_mul(f.y, xr[v][1]);
+                xi[v][0] = p2_mul(f.x, xi[v][0]);
+                xi[v][1] = p2_mul(f.y, xi[v][1]);
+            }
+        }
+        if (!MONO) {
+            lanes<K, true>(xr, low);
+            lanes<K, true>(xi, low);
+        }
+        // one pair of groups at a time, results over the inputs they came from
+#pragma unroll
+        for (int p = 0; p < 2; p++) {
+            P2 br[D], bi[D];
+#pragma unroll
+            for (int r = 0; r < D; r++) {
+                P2 wr, wi, nwi;
+                if (MONO) {
+                    entry<(K > 1)>(&W[r * D + col[r]], &NW[r * D + col[r]], wr, wi, nwi);
+                    br[r] = p2_fma(wr, xr[r][p], p2_mul(nwi, xi[r][p]));
+                    bi[r] = p2_fma(wr, xi[r][p], p2_mul(wi, xr[r][p]));
+                } else {
+#pragma unroll
+                    for (int c = 0; c < D; c++) {
+                        entry<(K > 1)>(&W[r * D + c], &NW[r * D + c], wr, wi, nwi);
+                        const P2 ar = xr[c][p], ai = xi[c][p];
+                        br[r] = p2_fma(wr, ar, c ? p2_fma(nwi, ai, br[r]) : p2_mul(nwi, ai));
+                        bi[r] = p2_fma(wr, ai, c ? p2_fma(wi, ar, bi[r]) : p2_mul(wi, ar));
+                    }
                 }
             }
 #pragma unroll
-        for (int i = 0; i < U; i++)
-            if (i == 0 || u0 + i * NT < units) {
-                const uint32_t u = u0 + i * NT;
-                if (nfv >= 0) {  // factors are real: flips and damping have real operators
-#pragma unroll
-                    for (int v = 0; v < D; v++) {
-                        const uint32_t vi = vector(u, source(v));
-                        uint32_t j = ((vi >> fq0) & 1u) | (((vi >> fq1) & 1u) << 1);
-                        if (nfv > 2) j |= ((vi >> fq2) & 1u) << 2;
-                        const ulonglong2 f = *reinterpret_cast<const ulonglong2 *>(&s.ft[j]);
-                        xr[i][v][0] = p2_mul(f.x, xr[i][v][0]);
-                        xr[i][v][1] = p2_mul(f.y, xr[i][v][1]);
-                        xi[i][v][0] = p2_mul(f.x, xi[i][v][0]);
-                        xi[i][v][1] = p2_mul(f.y, xi[i][v][1]);
-                    }
-                }
-                if (!MONO) {
-                    lanes<K, true>(xr[i], low);
-                    lanes<K, true>(xi[i], low);
-                }
-                // one pair of groups at a time, results over the inputs they came from
-#pragma unroll
-                for (int p = 0; p < 2; p++) {
-                    P2 br[D], bi[D];
-#pragma unroll
-                    for (int r = 0; r < D; r++) {
-                        P2 wr, wi, nwi;
-                        if (MONO) {
-                            entry<(K > 1)>(&W[r * D + col[r]], &NW[r * D + col[r]], wr, wi, nwi);
-                            br[r] = p2_fma(wr, xr[i][r][p], p2_mul(nwi, xi[i][r][p]));
-                            bi[r] = p2_fma(wr, xi[i][r][p], p2_mul(wi, xr[i][r][p]));
-                        } else {
-#pragma unroll
-                            for (int c = 0; c < D; c++) {
-                                entry<(K > 1)>(&W[r * D + c], &NW[r * D + c], wr, wi, nwi);
-                                const P2 ar = xr[i][c][p], ai = xi[i][c][p];
-                                br[r] = p2_fma(wr, ar, c ? p2_fma(nwi, ai, br[r]) : p2_mul(nwi, ai));
-                                bi[r] = p2_fma(wr, ai, c ? p2_fma(wi, ar, bi[r]) : p2_mul(wi, ar));
-                            }
-                        }
-                    }
-#pragma unroll
-                    for (int r = 0; r < D; r++) {
-                        xr[i][r][p] = br[r];
-                        xi[i][r][p] = bi[r];
-                    }
-                }
-                if (acc) {  // one branch for all rows: one per row kept their arithmetic apart (126 -> 118 ms)
-#pragma unroll
-                    for (int p = 0; p < 2; p++)
-#pragma unroll
-                        for (int r = 0; r < D; r++)
-                            if (NT >= 256) mass_add_pair<MassF2>(xr[i][r][p], xi[i][r][p], h[p % S][r], l[p % S][r]);
-                            else mass_add2<MassF2>(xr[i][r][p], xi[i][r][p], h[p % S][r], l[p % S][r]);
-                }
-                if (!MONO) {
-                    lanes<K, false>(xr[i], low);
-                    lanes<K, false>(xi[i], low);
-                }
-#pragma unroll
-                for (int v = 0; v < D; v++) {
-                    const uint32_t vi = vector(u, v);
-                    *sm.re4(vi) = make_ulonglong2(xr[i][v][0], xr[i][v][1]);
-                    *sm.im4(vi) = make_ulonglong2(xi[i][v][0], xi[i][v][1]);
-                }
+            for (int r = 0; r < D; r++) {
+                xr[r][p] = br[r];
+                xi[r][p] = bi[r];
             }
-        if ((u0 / NT) % (kMassFold / 4) == kMassFold / 4 - 1) {  // four squares per row, lane and unit
+        }
+        if (acc) {  // one branch for all rows: one per row kept their arithmetic apart (126 -> 118 ms)
+#pragma unroll
+            for (int p = 0; p < 2; p++)
+#pragma unroll
+                for (int r = 0; r < D; r++)
+                    if (NT >= 256) mass_add_pair<MassF2>(xr[r][p], xi[r][p], h[p % S][r], l[p % S][r]);
+                    else mass_add2<MassF2>(xr[r][p], xi[r][p], h[p % S][r], l[p % S][r]);
+        }
+        if (!MONO) {
+            lanes<K, false>(xr, low);
+            lanes<K, false>(xi, low);
+        }
+#pragma unroll
+        for (int v = 0; v < D; v++) {
+            const uint32_t vi = vector(u, v);
+            *sm.re4(vi) = make_ulonglong2(xr[v][0], xr[v][1]);
+            *sm.im4(vi) = make_ulonglong2(xi[v][0], xi[v][1]);
+        }
+        if ((u / NT) % (kMassFold / 4) == kMassFold / 4 - 1) {  // four squares per row, lane and unit
 #pragma unroll
             for (int i = 0; i < S; i++)
 #pragma unroll
@@ -636,11 +622,9 @@ __device__ __noinline__ void traj_pass_general(float *work, uint32_t n, int o, i
             if (j >= dim) break;
             uint64_t idx = base;
             for (uint32_t b = 0; b < k; b++) idx |= (uint64_t)((j >> b) & 1) << s.op(o).qs[b];
-            float fr, fi;
-            diag_factor(s, idx, fr, fi);
-            const float a = sm.re(idx), c = sm.im(idx);
-            xr[j] = fr * a - fi * c;
-            xi[j] = fr * c + fi * a;
+            const float f = diag_factor(s, idx);
+            xr[j] = f * sm.re(idx);
+            xi[j] = f * sm.im(idx);
         }
 #pragma unroll
         for (uint32_t r = 0; r < 8; r++) {
@@ -1046,10 +1030,7 @@ __device__ __noinline__ void finish_op(int o, int cur, bool acc, const TrajRec *
 // |a|^2 of element i with the pending factors, as f64.
 template <int NT, bool SMEM>
 __device__ __forceinline__ double mass_at(const StateMem<SMEM> &sm, const Shared<NT> &s, uint64_t i) {
-    float fr, fi;
-    diag_factor(s, i, fr, fi);
-    const float a = sm.re(i), c = sm.im(i);
-    const float xr = fr * a - fi * c, xi = fr * c + fi * a;
+    const float f = diag_factor(s, i), xr = f * sm.re(i), xi = f * sm.im(i);
     return (double)xr * xr + (double)xi * xi;
 }
 
@@ -1060,10 +1041,8 @@ __device__ double range_mass(const StateMem<SMEM> &sm, const Shared<NT> &s, uint
     const uint64_t first = i0 + threadIdx.x % 32;
     auto value = [&](uint64_t i) {
         if (i >= i1) return MassF2::zero();
-        float fr, fi;
-        diag_factor(s, i, fr, fi);
-        const float a = sm.re(i), c = sm.im(i);
-        return p2_make(fr * a - fi * c, fr * c + fi * a);
+        const float f = diag_factor(s, i);
+        return p2_make(f * sm.re(i), f * sm.im(i));
     };
     uint32_t folded = 0;
     for (uint64_t i = first; i < i1; i += 128) {
