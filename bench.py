@@ -15,8 +15,8 @@ drop-in's default exact arithmetic (bit-identical to zeno's CPU kernels).
 `roofline` = the dominant kernel's algorithmic HBM bytes per launch over its
 CUDA-event duration; `cpu_baseline` = the oracle (the C restatement of
 zeno's CPU backend) on all host cores for a bounded sample of the same
-workload. `configs` = every other seeded workload at its own shape
-(zeno_gb300/workloads.py).
+workload. Every other seeded workload runs at its own shape
+(zeno_gb300/workloads.py); their records are one JSON line on stderr.
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 """
@@ -392,6 +392,15 @@ def run_configs(a, peak, pk, line):
     line["configs"] = out
 
 
+def emit(line):
+    """The result as one short line on stdout; the other workloads' records,
+    18 KB that a reader of the line would have to hold, as one line on stderr."""
+    configs = line.pop("configs", None)
+    if configs is not None:
+        print(json.dumps({"configs": configs}), file=sys.stderr, flush=True)
+    print(json.dumps(line), flush=True)
+
+
 def main():
     a = parse()
     if a.impl == "reference":
@@ -544,7 +553,7 @@ def main():
     if rank == 0 and not a.no_cpu:
         line["cpu_baseline"] = cpu_baseline(a)
     if rank == 0:
-        print(json.dumps(line), flush=True)
+        emit(line)
     if ws > 1:
         torch.distributed.destroy_process_group()
 
