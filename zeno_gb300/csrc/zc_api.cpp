@@ -265,9 +265,10 @@ static bool program_order(const zc_state *st) {
 //   59/38, 6 74/50, 10 92/66; through zc_run (whole calls) 4 167/153, 7 168/169,
 //   8 174/195, at 13 qubits 4 176/170, 6 181/183, 8 182/209: two to seven run
 //   in exact arithmetic, which is also the closer one (6 ops at 8 qubits: 5e-17
-//   off, 1e-15 in double-float). One by one in double-float 2 ops take 32 but
-//   are twenty times further off: each launch truncates to pairs. Dense blocks,
-//   whose exact sums take twice as long, keep their own way.
+//   off, 1e-15 in a double-float sweep). One by one in double-float 2 ops take
+//   32 but are five times further off than in a sweep: each launch converts to
+//   pairs and back. Dense blocks, whose exact sums take twice as long, keep
+//   their own way.
 static constexpr size_t kFewF32 = 4, kFewF64 = 8;
 static bool few_ops(const zc_state *st, size_t few) {
     return hides_queue(st) && st->queue.size() < few;

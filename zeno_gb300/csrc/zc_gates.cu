@@ -288,7 +288,7 @@ int run_kq_small(zc_state *st, const uint32_t *qs, uint32_t k, const double *mat
 // Measured at 30 qubits, K = 2, 3, 4: 22.2, 31.9, 49.4 ms per block staged
 // through shared memory, 7.2, 12.9, 50.3 here. K = 4 gains nothing by itself (each
 // thread reads its 8 KB of matrix through the constant cache); it stays for the
-// pairs it hands on: staged, the state is truncated to pairs for each block.
+// pairs it hands on: staged, the state goes to pairs and back for each block.
 template <int K>
 struct KqMatDf {
     float2 rh[1 << (2 * K)], rl[1 << (2 * K)], ih[1 << (2 * K)], il[1 << (2 * K)];  // each value twice

@@ -458,7 +458,7 @@ __global__ void __launch_bounds__(NT) k_sample_scan_df(const T *__restrict__ re,
     const uint64_t lo = sc.chunk * chunk_len;
     const uint64_t hi = lo + chunk_len < total ? lo + chunk_len : total;
     uint64_t ptr = sc.s0;
-    float2 base = df_from_f64(sc.cum);  // truncated: never above the host's cum
+    float2 base = df_from_f64<true>(sc.cum);  // never above the host's cum
     unsigned long long my_last = 0;     // 1 + last index with nonzero mass seen
     for (uint64_t t0 = lo; t0 < hi && ptr < sc.s1; t0 += kScanTile) {
         const uint64_t e0 = t0 + (uint64_t)tid * kScanPer;

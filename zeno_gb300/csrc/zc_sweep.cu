@@ -182,10 +182,14 @@ __device__ __forceinline__ void hl_udf(const MatDF &m, float2 &Ha, float2 &La, f
     pk_join(ar, ai, Ha, La);
     pk_join(br, bi, Hb, Lb);
 }
-// Diagonal factors leave the pairs unnormalised, as in register passes: the
-// ops after them accept that, and the sweep's exit renormalises.
+// Diagonals outside register passes take normalised pairs (the product drops lo x
+// lo, which after a chain of unnormalised rotations is no longer below the last
+// bit: 20-qubit QFT off by 8.4e-15 so, 1.1e-14 without, in the same time) and
+// leave them unnormalised, as register passes do: the ops after them accept
+// that, and the sweep's exit renormalises.
 __device__ __forceinline__ void hl_cscale_df(float2 wr, float2 wi, float2 &H, float2 &L) {
     float2 ar, ai;
+    pk_renorm(H, L);
     pk_split(H, L, ar, ai);
     cscale_df_u(wr, wi, ar, ai);
     pk_join(ar, ai, H, L);
