@@ -23,7 +23,7 @@ struct Sum {
         else zc::mass_add2<Ops>(x, y, h, l);
     }
     void fold() { zc::mass_fold<Ops>(h, l); }
-    void join(const Sum &o) { zc::mass_join<Ops>(h, l, o.h, o.l); }
+    zc::MassSum<Ops> sum3() const { return zc::MassSum<Ops>{h, l, 0.f}; }
     double value() const { return (double)h + (double)l; }
 };
 
@@ -45,28 +45,29 @@ static double row_by_lanes(const std::vector<float> &re, const std::vector<float
                 s.add(re[4 * u + 2 * p + lane], im[4 * u + 2 * p + lane], NT >= 256);
                 if (p + 1 >= 2 / S && (u / NT) % (zc::kMassFold / 4) == zc::kMassFold / 4 - 1) s.fold();
             }
-    // a thread's sums, then the lanes of a warp: from eight warps on joined as
-    // float pairs down to offset 4 and then added in f64, else in f64 throughout
+    // a thread's sums and the lanes of a warp, joined (from eight warps on without
+    // the third float down to offset 4); warps added in f64
     std::vector<double> warps;
     for (size_t w = 0; w < NT; w += 32) {
-        std::vector<double> v;
-        Sum t[32];
+        zc::MassSum<Ops> t[32];
         for (size_t j = 0; j < 32; j++) {
             Sum *s = &sums[4 * (w + j)];
             for (size_t i = 0; i < 4; i++) s[i].fold();
-            if (NT < 256) {
-                v.push_back((s[0].value() + s[1].value()) + (s[2].value() + s[3].value()));
+            zc::MassSum<Ops> a = s[0].sum3(), b = s[2].sum3();
+            if (NT >= 256) {
+                zc::mass_join<false>(a, s[1].sum3());
             } else {
-                t[j] = s[0];
-                t[j].join(s[1]);
+                zc::mass_join<true>(a, s[1].sum3());
+                zc::mass_join<true>(b, s[3].sum3());
+                zc::mass_join<true>(a, b);
             }
+            t[j] = a;
         }
-        if (NT >= 256) {
-            for (size_t o = 16; o >= 4; o /= 2)
-                for (size_t j = 0; j < o; j++) t[j].join(t[j + o]);
-            for (size_t j = 0; j < 4; j++) v.push_back(t[j].value());
-        }
-        warps.push_back(tree(v));
+        for (size_t o = 16; o; o /= 2)
+            for (size_t j = 0; j < o; j++)
+                if (NT >= 256 && o >= 4) zc::mass_join<false>(t[j], t[j + o]);
+                else zc::mass_join<true>(t[j], t[j + o]);
+        warps.push_back((double)((long double)t[0].h + t[0].l + t[0].c));
     }
     return tree(warps);
 }

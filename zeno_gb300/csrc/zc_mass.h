@@ -93,13 +93,27 @@ ZC_MASS_HD void mass_fold(typename Ops::V &h, typename Ops::V &l) {
     h = s;
 }
 
-// (h, l) += (g, k), folded sums both.
+// A folded sum on its way through the additions over lanes.
 template <typename Ops>
-ZC_MASS_HD void mass_join(typename Ops::V &h, typename Ops::V &l, typename Ops::V g, typename Ops::V k) {
-    typename Ops::V s = h;
-    const typename Ops::V e = mass_two_sum<Ops>(s, g), r = Ops::add(e, Ops::add(l, k));
-    h = Ops::add(s, r);
-    l = Ops::sub(r, Ops::sub(h, s));
+struct MassSum {
+    typename Ops::V h, l, c;
+};
+
+// a += b. THIRD: c takes what h and l lose, so that the sum keeps ~2^-70 and a
+// table of few values is as good as they are. Without it 2^-48, for the
+// additions of many values, whose roundings average out.
+template <bool THIRD, typename Ops>
+ZC_MASS_HD void mass_join(MassSum<Ops> &a, const MassSum<Ops> &b) {
+    typename Ops::V s = a.h, t = a.l;
+    const typename Ops::V e = mass_two_sum<Ops>(s, b.h);
+    if (THIRD) {
+        const typename Ops::V f = mass_two_sum<Ops>(t, b.l), g = mass_two_sum<Ops>(t, e);
+        a.c = Ops::add(Ops::add(a.c, b.c), Ops::add(f, g));
+    } else {
+        t = Ops::add(e, Ops::add(t, b.l));
+    }
+    a.h = Ops::add(s, t);
+    a.l = Ops::sub(t, Ops::sub(a.h, s));
 }
 
 }  // namespace zc

@@ -16,8 +16,8 @@
 // pending for the next pass and prepares the next op; two CTA barriers per op.
 // All draws of an op are independent of the state and come in the
 // reference's order from a per-trajectory Philox4x32-10 stream
-// (zc_philox.h). Probabilities are summed in two floats per lane (zc_mass.h)
-// and over lanes and warps in FP64.
+// (zc_philox.h). Probabilities are summed in two floats per lane and three over
+// lanes (zc_mass.h), and over warps in FP64.
 //
 // Where the state lives. The pass is bound by moving the state (2S per op),
 // so it stays as close as it fits: up to 14 qubits (128 KiB) in shared
@@ -299,83 +299,68 @@ struct MassF2 {
     }
 };
 
-// A folded sum as f64 (by integer operations; below 2^-75 those drop l).
-__device__ __forceinline__ double mass_f64(float2 v) {
-    if (v.x > 0.f && v.x < 0x1p-75f) return (double)v.x + (double)v.y;
-    return df_to_f64(v);
+// Table values on their way through a warp: float sums (zc_mass.h), not FP64, of
+// which an SM takes one warp instruction per 19 cycles (9 qubits, 2048
+// trajectories: 1.70 ms with FP64 additions, 1.20 so). CTAs of eight warps and
+// more have many values and join them without the third float down to the
+// lowest four lanes (2048 trajectories at 16 qubits: 114 -> 112 ms).
+typedef MassSum<MassF1> Sum3;
+
+// The f64 nearest h + l + c, by integer operations: as df_to_f64, with c and what
+// rounding l to f64 units left added in those units. Masses are scaled by 2^48
+// on the way, below 2^-123 they are h alone.
+__device__ __forceinline__ double mass_f64(const Sum3 &v) {
+    const float h = v.h * 0x1p48f, t = v.l + v.c, l = t * 0x1p48f, c = (v.c - (t - v.l)) * 0x1p48f;
+    const unsigned hb = __float_as_uint(h), eh = hb >> 23, mant = hb & 0x7fffffu;  // h >= 0
+    if (eh == 0u) return 0.0;
+    if (eh == 255u) return (double)v.h;  // inf, NaN
+    const long long hbits = (long long)((unsigned long long)((eh + 896u - 48u) << 20 | mant >> 3) << 32 |
+                                        (unsigned long long)(mant << 29));
+    const unsigned se = 306u - eh + (mant == 0u && l < 0.f ? 1u : 0u);  // f32 exponent field of 1 / (f64 unit)
+    if (se >= 255u) return __longlong_as_double(hbits);
+    const float units = __uint_as_float(se << 23), f = __fmul_rn(l, units);
+    const int L = __float2int_rn(f);
+    return __longlong_as_double(hbits + L + __float2int_rn(__fmaf_rn(c, units, __fsub_rn(f, (float)L))));
 }
 
-__device__ __forceinline__ float2 sum_of(float2 a, float2 b) {
-    mass_join<MassF1>(a.x, a.y, b.x, b.y);
+template <bool THIRD>
+__device__ __forceinline__ Sum3 sum_of(Sum3 a, const Sum3 &b) {
+    mass_join<THIRD>(a, b);
     return a;
 }
-__device__ __forceinline__ double sum_of(double a, double b) { return a + b; }
-
-// Table values of a CTA of NT threads on their way through a warp. From eight
-// warps on they are float pairs down to the lowest four lanes: many values,
-// whose roundings average out, while FP64 takes an SM 19 cycles per warp
-// instruction (16 qubits, as above: 130 -> 126 ms when measured). Smaller CTAs
-// have fewer values, and theirs are FP64 from the start.
-template <int NT>
-using TableValue = typename std::conditional<(NT >= 256), float2, double>::type;
-
-__device__ __forceinline__ void table_value(float2 v, float2 &out) { out = v; }
-__device__ __forceinline__ void table_value(float2 v, double &out) { out = mass_f64(v); }
 // Both lanes of a sum.
-template <typename V>
-__device__ __forceinline__ V mass_end(P2 h, P2 l) {
+template <bool THIRD>
+__device__ __forceinline__ Sum3 mass_end(P2 h, P2 l) {
     mass_fold<MassF2>(h, l);
     const float2 a = pk_float2(h), b = pk_float2(l);
-    V x, y;
-    table_value(make_float2(a.x, b.x), x);
-    table_value(make_float2(a.y, b.y), y);
-    return sum_of(x, y);
+    return sum_of<THIRD>(Sum3{a.x, b.x, 0.f}, Sum3{a.y, b.y, 0.f});
 }
-__device__ __forceinline__ float2 shfl_xor_of(float2 v, int m) {
-    return make_float2(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m));
+__device__ __forceinline__ Sum3 shfl_xor_of(const Sum3 &v, int m) {
+    return Sum3{__shfl_xor_sync(0xffffffffu, v.h, m), __shfl_xor_sync(0xffffffffu, v.l, m),
+                __shfl_xor_sync(0xffffffffu, v.c, m)};
 }
-__device__ __forceinline__ double shfl_xor_of(double v, int m) { return __shfl_xor_sync(0xffffffffu, v, m); }
 
-// Sum D per-thread values over the lanes at offsets 16 down to `last`: lanes
-// halve the values they carry as they exchange them (D - 1 + 5 - log2 D
-// additions instead of 5 D). Left in v[0]; returns which of the D it is.
-template <int D, typename V>
-__device__ __forceinline__ int lane_table(V *v, int last, int &off) {
+// The warp's table into red[0..D) from D sums per thread: lanes halve the values
+// they carry as they exchange them (D - 1 + 5 - log2 D additions instead of 5 D).
+template <int D, int NT>
+__device__ __forceinline__ void warp_table(Sum3 *v, double *red) {
+    constexpr bool THIRD = NT < 256;
     const int lane = threadIdx.x % 32;
-    int base = 0;
-    off = 16;
+    int off = 16, base = 0;
 #pragma unroll
     for (int w = D; w > 1; w >>= 1, off >>= 1) {
         const bool upper = lane & off;
 #pragma unroll
         for (int j = 0; j < w / 2; j++) {
-            const V give = upper ? v[j] : v[j + w / 2], keep = upper ? v[j + w / 2] : v[j];
-            v[j] = sum_of(keep, shfl_xor_of(give, off));
+            const Sum3 give = upper ? v[j] : v[j + w / 2], keep = upper ? v[j + w / 2] : v[j];
+            v[j] = sum_of<THIRD>(keep, shfl_xor_of(give, off));
         }
         if (upper) base += w / 2;
     }
-    const int first = off;
 #pragma unroll
-    for (int o = first; o >= last; o >>= 1) v[0] = sum_of(v[0], shfl_xor_of(v[0], o));
-    off = first;
-    return base;
-}
-
-// The warp's table into red[0..D).
-template <int D>
-__device__ __forceinline__ void warp_table(float2 *v, double *red) {
-    int off;
-    const int base = lane_table<D>(v, 4, off);
-    double t = mass_f64(v[0]);
-    t += __shfl_xor_sync(0xffffffffu, t, 2);
-    t += __shfl_xor_sync(0xffffffffu, t, 1);
-    if ((threadIdx.x % 32 & (2 * off - 1)) == 0) red[base] = t;
-}
-template <int D>
-__device__ __forceinline__ void warp_table(double *v, double *red) {
-    int off;
-    const int base = lane_table<D>(v, 1, off);
-    if ((threadIdx.x % 32 & (2 * off - 1)) == 0) red[base] = v[0];
+    for (int o = off; o > 0; o >>= 1)
+        v[0] = o >= 4 ? sum_of<THIRD>(v[0], shfl_xor_of(v[0], o)) : sum_of<true>(v[0], shfl_xor_of(v[0], o));
+    if ((lane & (2 * off - 1)) == 0) red[base] = mass_f64(v[0]);
 }
 
 // Matrix entries read where they are used: hoisted out of the pass loop, the
@@ -581,14 +566,13 @@ __device__ __forceinline__ void traj_pass_body(float *work, uint32_t n, int o, i
         }
     }
     if (!acc) return;
-    using V = TableValue<NT>;
-    V tab[D];
+    Sum3 tab[D];
 #pragma unroll
     for (int r = 0; r < D; r++) {
-        tab[r] = mass_end<V>(h[0][r], l[0][r]);
-        if (S == 2) tab[r] = sum_of(tab[r], mass_end<V>(h[S - 1][r], l[S - 1][r]));
+        tab[r] = mass_end<(NT < 256)>(h[0][r], l[0][r]);
+        if (S == 2) tab[r] = sum_of<true>(tab[r], mass_end<true>(h[S - 1][r], l[S - 1][r]));
     }
-    warp_table<D>(tab, s.red[threadIdx.x / 32]);
+    warp_table<D, NT>(tab, s.red[threadIdx.x / 32]);
 }
 
 // A dense two-qubit op's pass, out of line: its registers would crowd the
@@ -653,19 +637,19 @@ __device__ __noinline__ void traj_pass_general(float *work, uint32_t n, int o, i
         if (S == 2 && g + NT < groups) group(g + NT, h[S - 1], l[S - 1]);
     }
     if (!table) return;
-    TableValue<NT> tab[8], x;
+    Sum3 tab[8];
 #pragma unroll
     for (int r = 0; r < 8; r++) {
 #pragma unroll
         for (int i = 0; i < S; i++) {
             mass_fold<MassF1>(h[i][r], l[i][r]);
-            table_value(make_float2(h[i][r], l[i][r]), x);
-            tab[r] = i ? sum_of(tab[r], x) : x;
+            const Sum3 x{h[i][r], l[i][r], 0.f};
+            tab[r] = i ? sum_of<true>(tab[r], x) : x;
         }
     }
-    if (k == 1) warp_table<2>(tab, s.red[threadIdx.x / 32]);
-    else if (k == 2) warp_table<4>(tab, s.red[threadIdx.x / 32]);
-    else warp_table<8>(tab, s.red[threadIdx.x / 32]);
+    if (k == 1) warp_table<2, NT>(tab, s.red[threadIdx.x / 32]);
+    else if (k == 2) warp_table<4, NT>(tab, s.red[threadIdx.x / 32]);
+    else warp_table<8, NT>(tab, s.red[threadIdx.x / 32]);
 }
 
 // One warp: the next 32 Philox blocks of trajectory t, one per lane, when
@@ -1054,10 +1038,10 @@ __device__ double range_mass(const StateMem<SMEM> &sm, const Shared<NT> &s, uint
             for (int j = 0; j < 2; j++) mass_fold<MassF2>(h[j], l[j]);
         }
     }
-    double v = mass_end<double>(h[0], l[0]) + mass_end<double>(h[1], l[1]);
+    Sum3 v = sum_of<true>(mass_end<true>(h[0], l[0]), mass_end<true>(h[1], l[1]));
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+    for (int o = 16; o > 0; o >>= 1) v = sum_of<true>(v, shfl_xor_of(v, o));
+    return mass_f64(v);
 }
 
 // One basis index from |psi|^2 by the draw u in [0, 1): region (one per
@@ -1148,11 +1132,10 @@ __global__ void __launch_bounds__(NT, CTAS)
                    const float *__restrict__ mats, const uint32_t *__restrict__ fq, const uint32_t *__restrict__ fc,
                    int nfinal, TrajNoise nz, uint64_t ntraj, uint64_t seed, uint64_t *__restrict__ out) {
     Shared<NT> &s = shared_of<NT>();
-    constexpr int NW = NT / 32;
     const uint64_t len = 1ull << n;
     if (!SMEM) work += (size_t)blockIdx.x * 2 * len;
     const StateMem<SMEM> sm(work, n);
-    const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+    const int tid = threadIdx.x, warp = tid / 32;
     const bool vec = n >= 5 && n <= 31;
     if (tid == 0) {
         s.keep = sqrt(1.0 - nz.p[4]);
